@@ -215,20 +215,24 @@ class _Memory:
 
 def _seen(t, shape, dtype):
     """A result [.., columns] as a torch tensor over the same memory; its rows may lie further apart than they are long."""
-    ptr, L = [], _lib.load()
-    flat = (int(np.prod(shape[:-1])), shape[-1])
-    for row in range(min(2, flat[0])):
+    L, flat, size, keep = _lib.load(), (int(np.prod(shape[:-1])), shape[-1]), {"float32": 4}.get(dtype, 2), [t]
+
+    def at(x):
+        return int(L.applegpu_ffi_device_ptr(x.id) or 0)
+
+    def row(i):
         r = t
-        at = np.unravel_index(row, shape[:-1])
-        for dim, i in enumerate(at):
-            r = gpu.slice(r, dim, int(i), int(i) + 1)
-        ptr.append((int(L.applegpu_ffi_device_ptr(r.id) or 0), r))
-        if not ptr[-1][0]:
-            raise RuntimeError(L.applegpu_ffi_last_error())
-    size = {"float32": 4}.get(dtype, 2)
-    pitch = (ptr[1][0] - ptr[0][0]) // size if flat[0] > 1 else flat[1]
-    m = _Memory([t, ptr], ptr[0][0], flat, (pitch, 1), size)
-    return torch.as_tensor(m, device="cuda").view(_TORCH[dtype])
+        for dim, j in enumerate(np.unravel_index(i, shape[:-1])):
+            r = gpu.slice(r, dim, int(j), int(j) + 1)
+        keep.append(r)
+        return at(r)
+    ptr, pitch = at(t), flat[1]
+    if not ptr:                                           # rows with a pitch
+        ptr = row(0)
+        pitch = (row(1) - ptr) // size
+    if not ptr:
+        raise RuntimeError(L.applegpu_ffi_last_error())
+    return torch.as_tensor(_Memory(keep, ptr, flat, (pitch, 1), size), device="cuda").view(_TORCH[dtype])
 
 
 def run(state):
