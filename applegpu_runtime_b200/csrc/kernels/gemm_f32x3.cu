@@ -1,0 +1,442 @@
+// float32 products on the tensor cores.
+//
+// Both operands are split into three bf16 planes, x = x0 + x1 + x2 (each the bf16 rounding of what the planes before it left), and
+// the six largest cross terms a0 b0, a0 b1, a1 b0, a0 b2, a1 b1, a2 b0 are multiplied by tcgen05 (error about 2^-22 of the product).
+// A pipeline stage holds the three planes of one 64-deep k-block of A and B, and its six products run from that one copy: 72 KB per
+// 24 MMAs and CTA, where a GEMM over a six-fold K extent (what this replaces) fetches 12 tiles for the same work, and the planes are
+// written once instead of each term as often as a product names it (10 bytes per element moved instead of 16).
+// The tensor core truncates where it adds, so a long accumulation drifts (K = 768 in one go: 7.3e-7 of the result's norm off, all of it
+// towards zero, against 5.0e-7 for the CUDA-core kernel's rounded sums). a0 b0 therefore has an accumulator of its own, and no
+// accumulation runs over more than kF3Chunk k-blocks: the epilogue warps add the chunks up in registers, rounded to nearest, under the
+// next chunk's products.
+//
+// Tiles of 256 x 128 on CTA pairs (cta_group::2); two accumulator pairs of 2 x 128 TMEM columns, so the epilogue of a tile runs under the
+// next one's products. A product with few tiles also splits K: each share is one unit of the persistent grid, leaves its sum in
+// a workspace, and a second kernel adds the shares in K order and applies the epilogue.
+//
+// Bound: shared-memory bandwidth beside the tensor pipe (a 256 x 128 tile reads 96 to 128 bytes a clock and SM for its operands): about 2 250
+// cycles a k-block against 1 536 at the tensor rate; sm__pipe_tensor_cycles_active 68 % on 1024 x 50257 x 768. Before -> after in a GPT-2-small
+// forward of 1024 rows, us: the 48 linears 2 910 -> 1 370 with 93 for the shares, LM head 519 -> 339, planes 555 -> 397, whole 4 430 -> 2 690.
+#include "common.cuh"
+#include "sm100.cuh"
+#include <algorithm>
+#include <cmath>
+
+namespace ag { namespace k {
+using namespace sm100;
+
+Status make_map(CUtensorMap* out, DType dt, const void* ptr, uint64_t inner, uint64_t rows, uint64_t nbi, uint64_t nbo, uint64_t row_stride, uint64_t bi_stride,
+                uint64_t bo_stride, uint32_t b0, uint32_t b1);
+int* matmul_status_word();
+
+// ── planes ──────────────────────────────────────────────────────────────────
+struct PlaneJob { const float* in; __nv_bfloat16* out; long long rows, cols, row_stride, batch_stride; int batches, blocks; };
+
+__global__ void __launch_bounds__(256) f32_planes_kernel(const __grid_constant__ PlaneJob ja, const __grid_constant__ PlaneJob jb) {
+  pdl_trigger();
+  pdl_wait();
+  const bool second = (int)blockIdx.x >= ja.blocks;
+  const PlaneJob& j = second ? jb : ja;
+  const long long packs = j.cols / 8, plane = j.rows * j.cols, per = j.rows * packs, total = per * j.batches;
+  const long long step = (long long)j.blocks * 256;
+  for (long long i = (long long)(blockIdx.x - (second ? ja.blocks : 0)) * 256 + threadIdx.x; i < total; i += step) {
+    const long long b = j.batches > 1 ? i / per : 0, q = i - b * per, r = q / packs, c = (q - r * packs) * 8;
+    const float* src = j.in + b * j.batch_stride + r * j.row_stride + c;
+    const float4 x0 = __ldcs(reinterpret_cast<const float4*>(src)), x1 = __ldcs(reinterpret_cast<const float4*>(src + 4));
+    const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+    Pack<__nv_bfloat16> t[3];
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      const __nv_bfloat16 h0 = __float2bfloat16_rn(x[e]);
+      const float r1 = x[e] - __bfloat162float(h0);
+      const __nv_bfloat16 h1 = __float2bfloat16_rn(r1);
+      const float r2 = r1 - __bfloat162float(h1);
+      t[0].v[e] = h0; t[1].v[e] = h1; t[2].v[e] = __float2bfloat16_rn(r2);
+    }
+    __nv_bfloat16* dst = j.out + b * 3 * plane + r * j.cols + c;
+#pragma unroll
+    for (int k = 0; k < 3; k++) st16(dst + k * plane, t[k]);
+  }
+}
+
+// ── the product ─────────────────────────────────────────────────────────────
+constexpr int kF3Bm = 128, kF3Bn = 128, kF3Bk = 64, kF3Stages = 3, kF3EpiWarps = 8, kF3Threads = 64 + 32 * kF3EpiWarps;
+constexpr int kF3ATile = kF3Bm * kF3Bk * 2, kF3BTile = (kF3Bn / 2) * kF3Bk * 2;      // one plane: this CTA's rows of A, its half of B's columns
+constexpr int kF3Stage = 3 * (kF3ATile + kF3BTile);
+constexpr int kF3Chunk = 4;                                                          // k-blocks per accumulation
+constexpr int kF3StgPitch = 9;                                                       // floats: 32 rows x 8 columns per warp, no bank conflicts
+constexpr int kF3Stg = 32 * kF3StgPitch * 4;
+constexpr int kF3Smem = kF3Stages * kF3Stage + kF3EpiWarps * kF3Stg + 1024;
+static_assert(kF3Smem + 512 <= 232448, "shared memory of a CTA");
+
+struct F3Params {
+  float* c; const float* bias; const float* residual; float* partial;
+  float alpha; int act, m, n, batch, a_one, b_one, num_kb, tiles_m, tiles_n, splits, kb_per_split, vec;
+  long long c_row, c_batch, p_row;
+  const float* a; const float* b;        // the operands as they were given, for results that are not finite
+  int k; long long a_row, a_batch, b_row, b_col, b_batch;
+  int* status;
+};
+
+// Out of line: 64 copies of the two GELUs would be most of the kernel's code, fetched anew by every launch.
+__device__ __noinline__ float4 f3_act(float4 v, int act) {
+  switch ((Act)act) {
+    case Act::GeluTanh: return make_float4(gelu_tanh_f(v.x), gelu_tanh_f(v.y), gelu_tanh_f(v.z), gelu_tanh_f(v.w));
+    case Act::GeluErf: return make_float4(gelu_erf_f(v.x), gelu_erf_f(v.y), gelu_erf_f(v.z), gelu_erf_f(v.w));
+    case Act::Relu: return make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+    default: return v;
+  }
+}
+
+// A sum that is not finite may owe it to the planes: an infinity, or a number that bf16 rounds to one, leaves a NaN for its remainder,
+// and infinity times a plane that is zero is another. Such an element (and one that truly overflows) is taken again in float32.
+__device__ __noinline__ void f3_plain(const F3Params& p, int b, long long row, int col0, int n, float* v) {
+  const float* a = p.a + b * p.a_batch + row * p.a_row;
+  for (int e = 0; e < n && col0 + e < p.n; e++) {
+    if (isfinite(v[e])) continue;
+    const float* w = p.b + b * p.b_batch + (col0 + e) * p.b_col;
+    float t = 0.f;
+    for (int i = 0; i < p.k; i++) t = fmaf(__ldg(a + i), __ldg(w + i * p.b_row), t);
+    v[e] = t;
+  }
+}
+
+// One MMA of a CTA pair whose descriptors differ from one another in their low words only. 24 of them take 1 536 cycles of a
+// k-block, so the issuing thread has 64 cycles for each: the words are sums with constants, nothing is packed in 64 bits.
+__device__ __forceinline__ void f3_mma(uint32_t d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n .reg .b64 da, db;\n mov.b64 da, {%1, %2};\n mov.b64 db, {%3, %4};\n setp.ne.b32 p, %6, 0;\n"
+      " tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n}"
+      ::"r"(d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+template <bool B_MN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kF3Threads, 1)
+gemm_f32x3_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ F3Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t full_bar[kF3Stages], empty_bar[kF3Stages], tmem_full_bar[2], tmem_empty_bar[2];
+  __shared__ uint32_t tmem_base_slot;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int tiles = p.tiles_m * p.tiles_n;
+  const long long units = (long long)tiles * p.batch * p.splits, first = blockIdx.x >> 1, step = gridDim.x >> 1;
+  // unit -> share of K (outermost), batch entry, column block, row block (innermost: neighbours share B)
+  auto unit = [&](long long u, int& m0, int& n0, int& b, int& kb0, int& kb1, int& split) {
+    const long long t = u % ((long long)tiles * p.batch);
+    split = (int)(u / ((long long)tiles * p.batch));
+    b = (int)(t / tiles);
+    const int rem = (int)(t % tiles);
+    m0 = (rem % p.tiles_m) * 2 * kF3Bm + (int)rank * kF3Bm;
+    n0 = rem / p.tiles_m * kF3Bn;
+    kb0 = split * p.kb_per_split;
+    kb1 = min(p.num_kb, kb0 + p.kb_per_split);
+  };
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kF3Stages; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int a = 0; a < 2; a++) { mbar_init(&tmem_full_bar[a], 1); mbar_init(&tmem_empty_bar[a], 2 * kF3EpiWarps); }
+    mbar_fence_init();
+    prefetch_tmap(&tmap_a);
+    prefetch_tmap(&tmap_b);
+  }
+  if (warp == 1) { tmem_alloc_pair(&tmem_base_slot, 512); tmem_relinquish_pair(); }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = tmem_base_slot;
+  pdl_wait();
+  pdl_trigger();
+  int m0, n0, b, kb0, kb1, split;
+
+  if (warp == 0) {
+    if (lane == 0) {                                   // loads (both CTAs; the even CTA's barriers count the bytes of both)
+      int stage = 0; uint32_t phase = 0;
+      bool ok = true;
+      for (long long u = first; u < units && ok; u += step) {
+        unit(u, m0, n0, b, kb0, kb1, split);
+        const int nh = n0 + (int)rank * (kF3Bn / 2), ba = p.a_one ? 0 : b, bb = p.b_one ? 0 : b;
+        for (int kb = kb0; kb < kb1; kb++) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.status, 1)) { ok = false; break; }
+          if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * kF3Stage);
+          const uint32_t bar = mapa_u32(smem_u32(&full_bar[stage]), 0);
+          uint8_t* sa = smem + stage * kF3Stage;
+          uint8_t* sb = sa + 3 * kF3ATile;
+#pragma unroll
+          for (int q = 0; q < 3; q++) {
+            tma_load_4d_pair(sa + q * kF3ATile, &tmap_a, bar, kb * kF3Bk, m0, q, ba);
+            if (B_MN) tma_load_4d_pair(sb + q * kF3BTile, &tmap_b, bar, nh, kb * kF3Bk, q, bb);
+            else tma_load_4d_pair(sb + q * kF3BTile, &tmap_b, bar, kb * kF3Bk, nh, q, bb);
+          }
+          if (++stage == kF3Stages) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {                      // products
+      constexpr uint32_t idesc = make_idesc_f16(1, 0, B_MN ? 1 : 0, 2 * kF3Bm, kF3Bn);
+      int stage = 0, acc = 0; uint32_t phase = 0, acc_phase = 0;
+      bool ok = true;
+      for (long long u = first; u < units && ok; u += step) {
+        unit(u, m0, n0, b, kb0, kb1, split);
+        for (int kc = kb0; kc < kb1 && ok; kc += kF3Chunk) {
+          if (!mbar_wait(&tmem_empty_bar[acc], acc_phase ^ 1, p.status, 2)) { ok = false; break; }
+          tc_fence_after_sync();
+          const uint32_t d_hi = tmem_base + (uint32_t)(acc * 256), d_lo = d_hi + 128;
+          for (int kb = kc; kb < min(kb1, kc + kF3Chunk); kb++) {
+            if (!mbar_wait(&full_bar[stage], phase, p.status, 3)) { ok = false; break; }
+            tc_fence_after_sync();
+            const uint32_t sa = smem_u32(smem + stage * kF3Stage);
+            const uint64_t a0 = make_smem_desc_sw128(sa, 16, 1024), b0 = make_smem_desc_sw128(sa + 3 * kF3ATile, B_MN ? 64 * 128 : 16, 1024);
+            const uint32_t ah = (uint32_t)(a0 >> 32), bh = (uint32_t)(b0 >> 32), al = (uint32_t)a0, bl = (uint32_t)b0;
+            uint32_t on = kb > kc ? 1u : 0u;
+#pragma unroll
+            for (int kk = 0; kk < kF3Bk / 16; kk++) {
+              auto mma = [&](uint32_t d, int qa, int qb, uint32_t acc_on) {
+                f3_mma(d, al + (uint32_t)((qa * kF3ATile + kk * 32) >> 4), ah, bl + (uint32_t)((qb * kF3BTile + kk * (B_MN ? 16 * 128 : 32)) >> 4), bh, idesc, acc_on);
+              };
+              mma(d_lo, 2, 0, on);
+              mma(d_lo, 1, 1, 1u);
+              mma(d_lo, 0, 2, 1u);
+              mma(d_lo, 1, 0, 1u);
+              mma(d_lo, 0, 1, 1u);
+              mma(d_hi, 0, 0, on);
+              on = 1u;
+            }
+            const uint32_t eb = smem_u32(&empty_bar[stage]);
+            mma_commit_pair(mapa_u32(eb, 0));
+            mma_commit_pair(mapa_u32(eb, 1));
+            if (++stage == kF3Stages) { stage = 0; phase ^= 1; }
+          }
+          if (!ok) break;
+          const uint32_t fb = smem_u32(&tmem_full_bar[acc]);
+          mma_commit_pair(mapa_u32(fb, 0));
+          mma_commit_pair(mapa_u32(fb, 1));
+          if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        }
+      }
+    }
+  } else {                                             // epilogue: a warp has 32 rows of its CTA and 64 of the tile's columns
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    float* stg = reinterpret_cast<float*>(smem + kF3Stages * kF3Stage) + (warp - 2) * (32 * kF3StgPitch);
+    int acc = 0; uint32_t acc_phase = 0;
+    bool ok = true;
+    for (long long u = first; u < units; u += step) {
+      unit(u, m0, n0, b, kb0, kb1, split);
+      const long long row0 = m0 + quarter * 32, gm = row0 + lane;
+      float bias_l[2];
+#pragma unroll
+      for (int g = 0; g < 2; g++) {
+        const int col = n0 + half * 64 + g * 32 + lane;
+        bias_l[g] = p.bias && !p.partial && col < p.n ? __ldg(p.bias + col) : 0.f;
+      }
+      float sum[2][32];
+#pragma unroll
+      for (int g = 0; g < 2; g++)
+#pragma unroll
+        for (int e = 0; e < 32; e++) sum[g][e] = 0.f;
+      for (int kc = kb0; kc < kb1; kc += kF3Chunk) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full_bar[acc], acc_phase, p.status, 4))) { ok = false; break; }
+        tc_fence_after_sync();
+        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * 256 + half * 64);
+#pragma unroll
+        for (int g = 0; g < 2; g++) {
+          uint32_t hi[32], lo[32];
+          tmem_ld_32x32(taddr + g * 32, hi);
+          tmem_ld_32x32(taddr + 128 + g * 32, lo);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; e++) sum[g][e] += __uint_as_float(hi[e]) + __uint_as_float(lo[e]);
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty_bar[acc]), 0));
+        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+      }
+      if (!ok) break;
+#pragma unroll
+      for (int g = 0; g < 2; g++) {
+        const int col0 = n0 + half * 64 + g * 32;
+        if (row0 >= p.m || col0 >= p.n) continue;      // uniform across the warp
+        float (&v)[32] = sum[g];
+        if (p.partial) {
+          float* dst = p.partial + ((long long)(split * p.batch + b) * p.m + gm) * p.p_row + col0;
+          if (gm < p.m) {
+#pragma unroll
+            for (int e = 0; e < 32; e += 4) if (col0 + e < p.n) *reinterpret_cast<float4*>(dst + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+          }
+          continue;
+        }
+        bool odd = false;
+#pragma unroll
+        for (int e = 0; e < 32; e++) odd |= !isfinite(v[e]);
+        if (odd && gm < p.m) {
+          float t[32];
+#pragma unroll
+          for (int e = 0; e < 32; e++) t[e] = v[e];
+          f3_plain(p, b, gm, col0, 32, t);
+#pragma unroll
+          for (int e = 0; e < 32; e++) v[e] = t[e];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < 32; e++) v[e] = fmaf(v[e], p.alpha, __shfl_sync(0xffffffffu, bias_l[g], e));
+        if (p.act) {
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            const float4 o = f3_act(make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]), p.act);
+            v[e] = o.x; v[e + 1] = o.y; v[e + 2] = o.z; v[e + 3] = o.w;
+          }
+        }
+        const long long at = (long long)b * p.c_batch + row0 * p.c_row + col0;
+        if (p.vec && col0 + 32 <= p.n) {
+          if (gm < p.m) {
+            float* crow = p.c + at + lane * p.c_row;
+            const float* rrow = p.residual ? p.residual + at + lane * p.c_row : nullptr;
+#pragma unroll
+            for (int e = 0; e < 32; e += 4) {
+              float4 o = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+              if (rrow) { const float4 r = *reinterpret_cast<const float4*>(rrow + e); o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w; }
+              *reinterpret_cast<float4*>(crow + e) = o;
+            }
+          }
+          continue;
+        }
+        // rows on any 4-byte boundary, or a ragged column block: four rows of eight columns per store instead of 32 rows of one
+#pragma unroll
+        for (int e0 = 0; e0 < 32; e0 += 8) {
+          __syncwarp();
+#pragma unroll
+          for (int e = 0; e < 8; e++) stg[lane * kF3StgPitch + e] = v[e0 + e];
+          __syncwarp();
+          const int c = lane & 7, col = col0 + e0 + c;
+#pragma unroll
+          for (int r = lane >> 3; r < 32; r += 4) {
+            if (row0 + r < p.m && col < p.n) {
+              const long long o = at + r * p.c_row + e0 + c;
+              const float x = stg[r * kF3StgPitch + c];
+              p.c[o] = p.residual ? x + p.residual[o] : x;
+            }
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();      // neither CTA leaves while its peer can still signal its barriers or run MMAs on its shared memory
+  tc_fence_after_sync();
+  if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
+}
+
+// The shares of K added in order, then what the single-launch epilogue does.
+__global__ void __launch_bounds__(256) f32x3_finish_kernel(const __grid_constant__ F3Params p) {
+  pdl_trigger();
+  pdl_wait();
+  const long long q = p.p_row / 4, total = (long long)p.batch * p.m * q, share = (long long)p.batch * p.m * p.p_row;
+  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
+    const long long row = i / q, col = (i - row * q) * 4, b = row / p.m;
+    const float* src = p.partial + row * p.p_row + col;
+    float4 x[8];
+#pragma unroll
+    for (int s = 0; s < 8; s++) if (s < p.splits) x[s] = __ldcg(reinterpret_cast<const float4*>(src + s * share));
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int s = 0; s < 8; s++) if (s < p.splits) { v[0] += x[s].x; v[1] += x[s].y; v[2] += x[s].z; v[3] += x[s].w; }
+    const long long at = b * p.c_batch + (row - b * p.m) * p.c_row + col;
+    if (!(isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]) && isfinite(v[3]))) {
+      float t[4] = {v[0], v[1], v[2], v[3]};
+      f3_plain(p, (int)b, row - b * p.m, (int)col, 4, t);
+#pragma unroll
+      for (int e = 0; e < 4; e++) v[e] = t[e];
+    }
+#pragma unroll
+    for (int e = 0; e < 4; e++) v[e] = fmaf(v[e], p.alpha, p.bias && col + e < p.n ? __ldg(p.bias + col + e) : 0.f);
+    if (p.act) { const float4 o = f3_act(make_float4(v[0], v[1], v[2], v[3]), p.act); v[0] = o.x; v[1] = o.y; v[2] = o.z; v[3] = o.w; }
+    if (p.vec && col + 4 <= p.n) {
+      float4 o = make_float4(v[0], v[1], v[2], v[3]);
+      if (p.residual) { const float4 r = *reinterpret_cast<const float4*>(p.residual + at); o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w; }
+      *reinterpret_cast<float4*>(p.c + at) = o;
+    } else {
+      for (int e = 0; e < 4 && col + e < p.n; e++) p.c[at + e] = p.residual ? v[e] + p.residual[at + e] : v[e];
+    }
+  }
+}
+
+// Shares of K. A unit of kb k-blocks takes about 1 600 cycles per k-block (24 MMAs of 256 x 128 x 16) and 3 000 around it (first
+// loads, last epilogue); splitting costs one more launch and the shares' way through the L2 (about 2 600 bytes per cycle).
+int f32x3_splits(int64_t m, int64_t n, int64_t k, int64_t batch) {
+  const double pairs = sm_count() / 2, num_kb = (double)((k + kF3Bk - 1) / kF3Bk);
+  const double tiles = (double)((m + 2 * kF3Bm - 1) / (2 * kF3Bm)) * (double)((n + kF3Bn - 1) / kF3Bn) * (double)batch;
+  int best = 1; double best_cost = 0;
+  for (int s = 1; s <= 8; s++) {
+    const double kb = std::ceil(num_kb / s);
+    if (s > 1 && (kb < 3 || kb * (s - 1) >= num_kb || tiles * s > 4 * pairs)) continue;
+    double cost = std::ceil(tiles * s / pairs) * kb * 1600 + 3000;
+    if (s > 1) cost += 5000 + (double)m * n * batch * 4 * (2 * s + 1) / 2600;
+    if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
+  }
+  return best;
+}
+
+// float32 A [m, k] with rows along k; B [k, n] with either dimension along its rows; bytes of the workspace for the planes and shares
+bool f32x3_eligible(const GemmDesc& g) {
+  if (g.dtype != DType::F32 || g.b_dtype != DType::F32 || g.batch_inner != 1 || g.k % 8 || g.a_col != 1 || g.a_row % 4 || g.a_batch % 4 || g.b_batch % 4) return false;
+  if (g.ep.b_scales || g.ep.argmax_keys || g.ep.ln_stats || g.ep.stats_out || g.ep.stats_zero || g.ep.glu_n || g.ln_gamma) return false;
+  if (g.m > 0x3fffffff || g.n > 0x3fffffff || g.k > 0x3fffffff || g.batch > 65535) return false;
+  if (g.b_col == 1) { if (g.n % 8 || g.b_row % 4) return false; }
+  else if (g.b_row != 1 || g.b_col % 4) return false;
+  return aligned16(g.a) && aligned16(g.b);
+}
+static int64_t f3_pad(int64_t bytes) { return (bytes + 255) / 256 * 256; }
+int64_t f32x3_workspace(const GemmDesc& g) {
+  const int64_t ca = g.batch > 1 && g.a_batch ? g.batch : 1, cb = g.batch > 1 && g.b_batch ? g.batch : 1;
+  const int s = f32x3_splits(g.m, g.n, g.k, g.batch);
+  return f3_pad(6 * ca * g.m * g.k) + f3_pad(6 * cb * g.n * g.k) + (s > 1 ? (int64_t)s * g.batch * g.m * ((g.n + 3) / 4 * 4) * 4 : 0);
+}
+
+Status matmul_f32x3(cudaStream_t s, const GemmDesc& g, void* workspace) {
+  if (!f32x3_eligible(g) || !workspace || !aligned16(workspace)) return Status::invalid("matmul_f32x3: operands");
+  int* st = matmul_status_word();
+  if (!st) return Status::compute("matmul: the kernel workspace is not initialised");
+  const int64_t ca = g.batch > 1 && g.a_batch ? g.batch : 1, cb = g.batch > 1 && g.b_batch ? g.batch : 1;
+  const bool b_mn = g.b_col == 1;
+  uint8_t* ws = static_cast<uint8_t*>(workspace);
+  __nv_bfloat16* pa = reinterpret_cast<__nv_bfloat16*>(ws);
+  __nv_bfloat16* pb = reinterpret_cast<__nv_bfloat16*>(ws + f3_pad(6 * ca * g.m * g.k));
+  const int64_t b_rows = b_mn ? g.k : g.n, b_cols = b_mn ? g.n : g.k;
+  PlaneJob ja{static_cast<const float*>(g.a), pa, g.m, g.k, g.a_row, g.a_batch, (int)ca, grid_for(ca * g.m * (g.k / 8), 256, 4)};
+  PlaneJob jb{static_cast<const float*>(g.b), pb, b_rows, b_cols, b_mn ? g.b_row : g.b_col, g.b_batch, (int)cb, grid_for(cb * b_rows * (b_cols / 8), 256, 8)};
+  cudaError_t e = launch_pdl(f32_planes_kernel, dim3((unsigned)(ja.blocks + jb.blocks)), dim3(256), 0, s, ja, jb);
+  if (e != cudaSuccess) return cuda_status(e, "matmul_f32x3 planes");
+  CUtensorMap ma, mb;
+  AG_RETURN_IF_ERROR(make_map(&ma, DType::BF16, pa, (uint64_t)g.k, (uint64_t)g.m, 3, (uint64_t)ca, (uint64_t)g.k, (uint64_t)(g.m * g.k), (uint64_t)(3 * g.m * g.k), kF3Bk, kF3Bm));
+  AG_RETURN_IF_ERROR(make_map(&mb, DType::BF16, pb, (uint64_t)b_cols, (uint64_t)b_rows, 3, (uint64_t)cb, (uint64_t)b_cols, (uint64_t)(b_rows * b_cols), (uint64_t)(3 * b_rows * b_cols), 64, 64));
+  F3Params p;
+  p.c = static_cast<float*>(g.c); p.bias = static_cast<const float*>(g.ep.bias); p.residual = static_cast<const float*>(g.ep.residual);
+  p.alpha = g.ep.alpha; p.act = (int)g.ep.act; p.m = (int)g.m; p.n = (int)g.n; p.batch = (int)g.batch; p.a_one = ca == 1; p.b_one = cb == 1;
+  p.num_kb = (int)((g.k + kF3Bk - 1) / kF3Bk); p.tiles_m = (int)((g.m + 2 * kF3Bm - 1) / (2 * kF3Bm)); p.tiles_n = (int)((g.n + kF3Bn - 1) / kF3Bn);
+  p.splits = f32x3_splits(g.m, g.n, g.k, g.batch); p.kb_per_split = (p.num_kb + p.splits - 1) / p.splits;
+  p.c_row = g.c_row; p.c_batch = g.c_batch; p.p_row = (g.n + 3) / 4 * 4; p.status = st;
+  p.a = static_cast<const float*>(g.a); p.b = static_cast<const float*>(g.b); p.k = (int)g.k; p.a_row = g.a_row; p.a_batch = g.a_batch; p.b_row = g.b_row; p.b_col = g.b_col; p.b_batch = g.b_batch;
+  p.partial = p.splits > 1 ? reinterpret_cast<float*>(ws + f3_pad(6 * ca * g.m * g.k) + f3_pad(6 * cb * g.n * g.k)) : nullptr;
+  p.vec = aligned16(g.c) && g.c_row % 4 == 0 && g.c_batch % 4 == 0 && (!g.ep.residual || aligned16(g.ep.residual)) ? 1 : 0;
+  static bool attr = false;
+  if (!attr) {
+    e = cudaFuncSetAttribute(gemm_f32x3_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kF3Smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_f32x3_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kF3Smem);
+    if (e != cudaSuccess) return cuda_status(e, "matmul_f32x3 smem attribute");
+    attr = true;
+  }
+  const long long units = (long long)p.tiles_m * p.tiles_n * p.batch * p.splits;
+  const dim3 grid((unsigned)(2 * std::min<long long>(units, sm_count() / 2)));
+  e = b_mn ? launch_pdl(gemm_f32x3_kernel<true>, grid, dim3(kF3Threads), (size_t)kF3Smem, s, ma, mb, p) : launch_pdl(gemm_f32x3_kernel<false>, grid, dim3(kF3Threads), (size_t)kF3Smem, s, ma, mb, p);
+  if (e != cudaSuccess) return cuda_status(e, "matmul_f32x3");
+  if (p.splits > 1) {
+    e = launch_pdl(f32x3_finish_kernel, dim3((unsigned)grid_for((int64_t)p.batch * p.m * (p.p_row / 4), 256, 8)), dim3(256), 0, s, p);
+    if (e != cudaSuccess) return cuda_status(e, "matmul_f32x3 shares");
+  }
+  return Status::OK();
+}
+
+}}  // namespace ag::k

@@ -335,7 +335,7 @@ __device__ __forceinline__ void epilogue_group(const TcParams& p, uint32_t taddr
   for (int e = 0; e < 32; e++) v[e] = __uint_as_float(acc[e]);
 
   if (p.c_f32) {
-    // float32 output (split-precision fp32 product): bias (staged as floats where the int8 scales
+    // float32 output: bias (staged as floats where the int8 scales
     // would be) and residual are float32; each lane stores its own row's 32 columns, 128 contiguous bytes.
     float* Cf = reinterpret_cast<float*>(p.c) + c_off;
     const float* Rf = p.residual ? reinterpret_cast<const float*>(p.residual) + c_off : nullptr;
@@ -2266,6 +2266,7 @@ static int initial_tile_override() {
 static const int g_tile_override_init = (g_tile_override = initial_tile_override());
 void set_gemm_tile(int code) { g_tile_override = code; }
 
+bool matmul_simt_forced() { return g_force_path == 1; }
 bool matmul_tc_ready(const GemmDesc& d) { return g_force_path != 1 && tc_eligible(d); }
 const char* matmul_path(const GemmDesc& d) {
   if (g_force_path == 1) return "simt";

@@ -496,3 +496,39 @@ def test_attention_on_strided_head_views(gpu_dev):
     hq, hk, hv = (np.ascontiguousarray(qkv[:, i * d:(i + 1) * d].reshape(B, T, h, dh).transpose(0, 2, 1, 3)) for i in range(3))
     ref = R.attention(hq, hk, hv, True).transpose(0, 2, 1, 3).reshape(B * T, d)
     assert rel_err(out, ref.astype(np.float64)) <= 2e-2
+
+
+@pytest.mark.parametrize("m,n,k,kmajor", [(17, 96, 768, False), (33, 3072, 768, False), (255, 136, 2056, False), (257, 768, 1000, False), (256, 128, 704, False), (1024, 768, 3072, False),
+                                          (100, 1003, 776, True), (513, 2049, 64, True), (300, 64, 1032, True)])
+def test_float32_products_through_bf16_planes(gpu_dev, m, n, k, kmajor):
+    """Edges of the 256 x 128 tiles, a last k-block that is short, split and whole K, rows of the result on any 4-byte boundary, with
+    and without epilogue. Bar: an accumulation covers at most 256 of K, 16 additions that each drop less than 2^-23 of the sum so far;
+    sums of standard normal products stay below 4 of their final deviation, so 16 * 4 * 2^-23 / 2 of it on average, 4e-6."""
+    rng = np.random.default_rng(m + 3 * n + k)
+    a = rng.standard_normal((m, k)).astype(np.float32); b = rng.standard_normal((n, k) if kmajor else (k, n)).astype(np.float32)
+    bias = rng.standard_normal(n).astype(np.float32); res = rng.standard_normal((m, n)).astype(np.float32)
+    ga, gb = gpu_dev.from_numpy(a), gpu_dev.from_numpy(b)
+    w = gpu_dev.transpose(gb) if kmajor else gb
+    ref = a.astype(np.float64) @ (b.T if kmajor else b).astype(np.float64)
+    got = (ga @ w).to_numpy()
+    assert np.max(np.abs(got - ref)) <= 4e-6 * np.sqrt(k)
+    assert np.array_equal(got, (ga @ w).to_numpy())
+    y = (gpu_dev.from_numpy(res) + gpu_dev.gelu(gpu_dev.add_bias(ga @ w, gpu_dev.from_numpy(bias)))).to_numpy()
+    want = R.gelu((ref + bias).astype(np.float32)).astype(np.float64) + res
+    np.testing.assert_allclose(y, want, rtol=1e-4, atol=1e-4)
+    assert gpu_dev.pipeline_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(64, 256, 256), (40, 768, 3072)])
+def test_float32_products_keep_infinities_and_nans(gpu_dev, m, n, k):
+    """What three bf16 planes cannot hold (infinities, the largest floats, NaN) comes out as the plain sums have it, split K or not."""
+    rng = np.random.default_rng(m + n)
+    a = rng.standard_normal((m, k)).astype(np.float32); b = rng.standard_normal((k, n)).astype(np.float32)
+    b[[6, 8]] /= 8      # products with the largest floats stay finite: a float32 sum that overflows on the way has no value apart from its order
+    a[3, 5] = np.inf; a[4, 6] = 3.4e38; a[5, 7] = np.nan; a[6] = 0; b[9, 10] = -np.inf; a[7, 8] = -3.4028235e38; b[8, 20] = 1e-38; b[11, 12] = 0
+    got = (gpu_dev.from_numpy(a) @ gpu_dev.from_numpy(b)).to_numpy()
+    with np.errstate(all="ignore"):
+        ref = (a.astype(np.float64) @ b.astype(np.float64)).astype(np.float32)
+    assert np.array_equal(np.isnan(got), np.isnan(ref)) and np.array_equal(np.isinf(got), np.isinf(ref)) and np.array_equal(np.sign(got[np.isinf(got)]), np.sign(ref[np.isinf(ref)]))
+    ok = np.isfinite(ref)
+    assert np.all(np.abs(got[ok] - ref[ok]) <= 4e-6 * np.sqrt(k) + 1e-5 * np.abs(ref[ok]))
