@@ -7,11 +7,12 @@
 // row in place and attends over rows 0 .. len: the step has the same launch list at every length, so it can be
 // captured once as a CUDA graph and replayed.
 #include "common.cuh"
+#include "mma_sync.cuh"
+#include "sm100.cuh"
 
 namespace ag { namespace k {
 
-float* skinny_partials();            // workspace.cu: created with the device context (shared with the skinny matmul; launches of one
-unsigned int* skinny_counters();     // stream never overlap past their dependency wait)
+float* skinny_partials();            // workspace.cu: created with the device context (shared with the skinny matmul)
 
 __device__ __forceinline__ unsigned long long globaltimer_ns_dec() {
   unsigned long long t;
@@ -25,127 +26,168 @@ constexpr int kDlRows = 128;      // K rows per CTA
 constexpr int kDlThreads = 256;
 constexpr int kDlMaxM = 16;
 
-// One (sequence, head) of a decode step's attention, by the first 128 threads of the block (any others only join
-// the barriers and contribute neutral elements to the block reductions, which leaves every sum bit-identical).
+// One (sequence, head) of a decode step's attention, by a block of kDlThreads threads.
 // s_qkv: this head's q | k | v of the new token as floats that hold storage-type values; kc / vc: the head's cache
 // [t_max, 64]; out_row: 64 outputs; len = tokens already in the cache (the new token becomes row len).
+// A thread has one key of each 256 for the scores, and for the weighted sum 16 bytes of the rows of one key in 256 / (threads
+// that share a row); the first 256 keys' pieces of both are asked for before anything else (AttnDecodeRegs). What bounds it is the
+// chain of L2 round trips of one block, so nothing is read twice and no load waits for a sum: 7.4 -> 3.8 us a launch at 8 x 12
+// heads and 64 to 114 keys.
 struct AttnDecodeSmem {
   float s_q[64];
-  float s_o[2][64];
+  float s_o[kDlThreads / 32][64];
   float s_red[33];
 };
+template <typename T> struct AttnDecodeRegs {
+  static constexpr int kPacks = 64 / Pack<T>::N;              // 16-byte pieces of a row
+  static constexpr int kGroups = kDlThreads / kPacks;         // keys whose values are read at once
+  static constexpr int kPre = 8;                              // rounds of them asked for ahead
+  Pack<T> k[kPacks], v[kPre];
+};
+__device__ __forceinline__ int attn_decode_len(int len, int t_max) { return len < 0 ? 0 : len > t_max - 1 ? t_max - 1 : len; }   // a full cache overwrites its last row
 template <typename T>
-__device__ __forceinline__ void attn_decode_item(const float* s_qkv, T* kc, T* vc, T* out_row, int len, int t_max, float scale, float* s_scores, AttnDecodeSmem& sm) {
+__device__ __forceinline__ void attn_decode_fetch(const T* kc, const T* vc, int len, AttnDecodeRegs<T>& r) {
+  using R = AttnDecodeRegs<T>;
+  const int tid = threadIdx.x, grp = tid / R::kPacks, c = tid % R::kPacks;
+  if (tid < len) {
+#pragma unroll
+    for (int i = 0; i < R::kPacks; i++) r.k[i] = ld16(kc + (long long)tid * 64 + i * Pack<T>::N);
+  }
+#pragma unroll
+  for (int i = 0; i < R::kPre; i++) if (grp + i * R::kGroups < len) r.v[i] = ld16(vc + (long long)(grp + i * R::kGroups) * 64 + c * Pack<T>::N);
+}
+template <typename T>
+__device__ __forceinline__ void attn_decode_item(const float* s_qkv, T* kc, T* vc, T* out_row, int len, float scale, float* s_scores, AttnDecodeSmem& sm, AttnDecodeRegs<T>& pre) {
+  using R = AttnDecodeRegs<T>;
+  constexpr int N = Pack<T>::N;
   const int tid = threadIdx.x;
-  if (len < 0) len = 0;
-  if (len > t_max - 1) len = t_max - 1;      // a full cache overwrites its last row instead of writing past the end
-  const int n_keys = len + 1;
-  // append the new key / value row in place; stage q (pre-scaled) as floats
+  // append the new key / value row in place; q pre-scaled. Nothing below reads the new row from global memory.
   if (tid < 64) { kc[(long long)len * 64 + tid] = Cvt<T>::from(s_qkv[64 + tid]); sm.s_q[tid] = s_qkv[tid] * scale; }
   else if (tid < 128) vc[(long long)len * 64 + (tid - 64)] = Cvt<T>::from(s_qkv[128 + (tid - 64)]);
-  __syncthreads();                             // the block's own global writes are visible to it from here
-  // scores: one key per thread and pass, the key row read as 16-byte packs
-  constexpr int N = Pack<T>::N;                // elements per 16 bytes
+  __syncthreads();
   float m_local = -INFINITY;
-  if (tid < 128) {
-    for (int j = tid; j < n_keys; j += 128) {
-      const T* kr = kc + (long long)j * 64;
-      float acc = 0.f;
+  for (int j = tid; j <= len; j += kDlThreads) {
+    float acc = 0.f;
+    if (j == len) {
+      for (int c = 0; c < 64; c++) acc = fmaf(sm.s_q[c], s_qkv[64 + c], acc);
+    } else {
+      if (j != tid) {
 #pragma unroll
-      for (int c = 0; c < 64 / N; c++) {
-        Pack<T> pk = ld16(kr + c * N);
-#pragma unroll
-        for (int e = 0; e < N; e++) acc = fmaf(sm.s_q[c * N + e], Cvt<T>::to(pk.v[e]), acc);
+        for (int i = 0; i < R::kPacks; i++) pre.k[i] = ld16(kc + (long long)j * 64 + i * N);
       }
-      s_scores[j] = acc;
-      m_local = fmaxf(m_local, acc);
+#pragma unroll
+      for (int i = 0; i < R::kPacks; i++)
+#pragma unroll
+        for (int e = 0; e < N; e++) acc = fmaf(sm.s_q[i * N + e], Cvt<T>::to(pre.k[i].v[e]), acc);
     }
+    s_scores[j] = acc;
+    m_local = fmaxf(m_local, acc);
   }
   const float m = block_max(m_local, sm.s_red);
   float l_local = 0.f;
-  if (tid < 128) {
-    for (int j = tid; j < n_keys; j += 128) { float p = __expf(s_scores[j] - m); s_scores[j] = p; l_local += p; }
+  for (int j = tid; j <= len; j += kDlThreads) { const float p = __expf(s_scores[j] - m); s_scores[j] = p; l_local += p; }
+  const float l = block_sum(l_local, sm.s_red);          // its barriers make the weights visible as well
+  const int grp = tid / R::kPacks, c = tid % R::kPacks;
+  float o[N];
+#pragma unroll
+  for (int e = 0; e < N; e++) o[e] = 0.f;
+#pragma unroll
+  for (int i = 0; i < R::kPre; i++) {
+    const int j = grp + i * R::kGroups;
+    if (j < len) {
+      const float p = s_scores[j];
+#pragma unroll
+      for (int e = 0; e < N; e++) o[e] = fmaf(p, Cvt<T>::to(pre.v[i].v[e]), o[e]);
+    }
   }
-  const float l = block_sum(l_local, sm.s_red);
-  __syncthreads();
-  // output: thread (e, half) sums p_j * V[j][e] over its half of the keys; consecutive threads read consecutive elements
-  if (tid < 128) {
-    const int e = tid & 63, half = tid >> 6;
-    float o = 0.f;
-    for (int j = half; j < n_keys; j += 2) o = fmaf(s_scores[j], Cvt<T>::to(vc[(long long)j * 64 + e]), o);
-    sm.s_o[half][e] = o;
+#pragma unroll 4
+  for (int j = grp + R::kPre * R::kGroups; j < len; j += R::kGroups) {
+    const Pack<T> v = ld16(vc + (long long)j * 64 + c * N);
+    const float p = s_scores[j];
+#pragma unroll
+    for (int e = 0; e < N; e++) o[e] = fmaf(p, Cvt<T>::to(v.v[e]), o[e]);
+  }
+  if (grp == len % R::kGroups) {
+    const float p = s_scores[len];
+#pragma unroll
+    for (int e = 0; e < N; e++) o[e] = fmaf(p, s_qkv[128 + c * N + e], o[e]);
+  }
+#pragma unroll
+  for (int e = 0; e < N; e++) {
+#pragma unroll
+    for (int d = R::kPacks; d < 32; d *= 2) o[e] += __shfl_xor_sync(0xffffffffu, o[e], d);
+  }
+  if ((tid & 31) < R::kPacks) {
+#pragma unroll
+    for (int e = 0; e < N; e++) sm.s_o[tid >> 5][c * N + e] = o[e];
   }
   __syncthreads();
-  if (tid < 64) out_row[tid] = Cvt<T>::from((sm.s_o[0][tid] + sm.s_o[1][tid]) / l);
+  if (tid < 64) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < kDlThreads / 32; w++) t += sm.s_o[w][tid];
+    out_row[tid] = Cvt<T>::from(t / l);
+  }
 }
 
-// grid = B * heads, 128 threads. qkv: [B, 3 * d] rows (q | k | v of the new token); caches: [B, heads, t_max, 64];
-// out: [B, d] (heads merged). *len_ptr = tokens already in the cache; the new token becomes row *len_ptr.
-// `part` non-null: qkv is not materialised; the projection left `slabs` (at most 8) float partials [slab][16][3 * d] and
-// this kernel adds them in K order, adds `bias` and rounds to the storage type, exactly as the projection's own last CTA
-// would have (all loads of a value in flight before the first addition).
+// grid = B * heads. qkv: [B, 3 * d] rows (q | k | v of the new token); caches: [B, heads, t_max, 64]; out: [B, d] (heads
+// merged). *len_ptr = tokens already in the cache; the new token becomes row *len_ptr.
+// The length and the cached rows are read before the dependency wait: the length is older than the launch before this one (the
+// step's embedding and projection lie between, and every kernel of a step waits for the one before it ahead of letting the next one
+// start), and so are the rows below it.
 template <typename T>
-__global__ void __launch_bounds__(128) attention_decode_kernel(const T* __restrict__ qkv, T* __restrict__ kcache, T* __restrict__ vcache, T* __restrict__ out,
-                                                               const int* __restrict__ len_ptr, int heads, int t_max, float scale,
-                                                               const float* __restrict__ part, int slabs, const T* __restrict__ bias) {
+__global__ void __launch_bounds__(kDlThreads) attention_decode_kernel(const T* __restrict__ qkv, T* kcache, T* vcache, T* __restrict__ out, const int* len_ptr, int heads, int t_max,
+                                                                      float scale) {
   extern __shared__ float s_scores[];          // [t_max]
   __shared__ AttnDecodeSmem sm;
   __shared__ float s_qkv[192];
-  pdl_wait();
-  pdl_trigger();
   const int b = blockIdx.x / heads, h = blockIdx.x % heads;
   const int d = heads * 64;
-  if (part) {
-    for (int i = threadIdx.x; i < 192; i += blockDim.x) {
-      const int col = (i >> 6) * d + h * 64 + (i & 63);
-      float v[8];
-#pragma unroll
-      for (int ks = 0; ks < 8; ks++) v[ks] = ks < slabs ? __ldcg(part + ((long long)ks * kDlMaxM + b) * 3 * d + col) : 0.f;
-      float t = 0.f;
-#pragma unroll
-      for (int ks = 0; ks < 8; ks++) if (ks < slabs) t += v[ks];
-      if (bias) t += Cvt<T>::to(bias[col]);
-      s_qkv[i] = Cvt<T>::to(Cvt<T>::from(t));
-    }
-  } else {
-    const T* row = qkv + (long long)b * 3 * d;
-    for (int i = threadIdx.x; i < 192; i += blockDim.x) s_qkv[i] = Cvt<T>::to(row[(i >> 6) * d + h * 64 + (i & 63)]);
-  }
-  __syncthreads();
   T* kc = kcache + ((long long)b * heads + h) * (long long)t_max * 64;
   T* vc = vcache + ((long long)b * heads + h) * (long long)t_max * 64;
-  attn_decode_item<T>(s_qkv, kc, vc, out + (long long)b * d + h * 64, *len_ptr, t_max, scale, s_scores, sm);
+  const int len = attn_decode_len(*len_ptr, t_max);
+  AttnDecodeRegs<T> pre;
+  attn_decode_fetch<T>(kc, vc, len, pre);
+  pdl_wait();
+  pdl_trigger();
+  const T* row = qkv + (long long)b * 3 * d;
+  if (threadIdx.x < 192) s_qkv[threadIdx.x] = Cvt<T>::to(row[(threadIdx.x >> 6) * d + h * 64 + (threadIdx.x & 63)]);
+  __syncthreads();
+  attn_decode_item<T>(s_qkv, kc, vc, out + (long long)b * d + h * 64, len, scale, s_scores, sm, pre);
 }
 
-Status attention_decode(cudaStream_t s, DType dt, const void* qkv, void* kcache, void* vcache, void* out, const int* len_ptr, int batch, int heads,
-                        int t_max, float scale, const float* part, int slabs, const void* bias) {
+Status attention_decode(cudaStream_t s, DType dt, const void* qkv, void* kcache, void* vcache, void* out, const int* len_ptr, int batch, int heads, int t_max, float scale) {
   if (batch <= 0 || heads <= 0) return Status::OK();
-  if (part && (slabs < 1 || slabs > 8 || batch > kDlMaxM)) return Status::invalid("attention_decode: 1..8 partial slabs of at most 16 rows");
-  if (!part && !qkv) return Status::invalid("attention_decode: no q / k / v");
+  if (!qkv) return Status::invalid("attention_decode: no q / k / v");
   if (t_max <= 0 || t_max > 8192) return Status::invalid("attention_decode: cache length must be in 1..8192");
   if (!aligned16(kcache) || !aligned16(vcache)) return Status::compute("attention_decode needs 16-byte aligned caches");
   const size_t smem = (size_t)t_max * sizeof(float);
   cudaError_t le = cudaSuccess;
-  AG_DISPATCH_FLOAT(dt, T, (le = launch_pdl(attention_decode_kernel<T>, dim3((unsigned)(batch * heads)), dim3(128), smem, s, (const T*)qkv, (T*)kcache,
-                                             (T*)vcache, (T*)out, len_ptr, heads, t_max, scale, part, slabs, (const T*)bias)));
+  AG_DISPATCH_FLOAT(dt, T, (le = launch_pdl(attention_decode_kernel<T>, dim3((unsigned)(batch * heads)), dim3(kDlThreads), smem, s, (const T*)qkv, (T*)kcache,
+                                             (T*)vcache, (T*)out, len_ptr, heads, t_max, scale)));
   if (le != cudaSuccess) return cuda_status(le, "attention_decode");
   return Status::OK();
 }
 
 // ── linear layer of a decode step ───────────────────────────────────────────
 // y[M, N] = act(layer_norm?(x)[M, K] @ W[K, N] + bias) + residual with M <= 16 and W as the reference stores its
-// Conv1D weights ([in, out], rows along N). The product is bound by streaming W once, so the grid is
-// (N / 64 column slabs) x (K / 128 row slabs) and every CTA has all its weight loads (8-byte loads, two 128-byte rows
-// per warp instruction) in flight before it waits for anything. Three things set it apart from the general skinny
-// matmul kernel:
+// Conv1D weights ([in, out], rows along N). The product reads W once, and what a launch takes is the chain of round trips behind
+// its inputs, so:
+//   * a CTA has 64 columns and a share of K in slabs of 128 rows; the (at most eight) shares of a column slab are a cluster, whose
+//     sums meet over distributed shared memory in K order: no partials in global memory, no fence, counter and reload;
 //   * W is a model weight, never written by a kernel of the step, so its loads are issued BEFORE the programmatic
 //     dependency wait: they overlap the previous kernel's tail, and x (which that kernel produces) is read after it;
 //   * layer_norm of x runs in the prologue: every CTA takes the row statistics over the whole rows itself
-//     (kernel_templates.rs:1097-1109: mean, population variance, 1/sqrt(var + eps)) and normalises its K slab on the
+//     (kernel_templates.rs:1097-1109: mean, population variance, 1/sqrt(var + eps)) and normalises its K share on the
 //     way into shared memory, which removes the separate layer_norm launches of the step;
-//   * same deterministic reduction: fp32 partials per K slab in a workspace, the last CTA of a column slab (a
-//     counter) adds them in K order and applies bias / activation / residual.
-
+//   * 16-bit weights are multiplied by mma.m16n8k16 from registers (dl_products16). Stored inputs have the weight's type and enter as they
+//     are; a normalised input is float32 and enters as the sum of three 16-bit numbers, which holds it to 2^-24. float32 weights keep
+//     CUDA-core multiply-adds.
+// Every thread runs this code once per launch, so a launch takes about as long as its instructions: options are template parameters and
+// nothing is unrolled beyond what the shape needs. GPT-2 small, 8 rows, bf16, a launch's share of a replayed step: 7.8 us with
+// multiply-adds, partials in the L2 and a last CTA that adds them; 7.9 us with cluster sums and MMAs but x through shared memory and one
+// kernel for all options (38 to 68 KB of code); now 3.5 (no layer_norm), 3.6 (K = 3072) and 4.8 us (layer_norm), 12 to 20 KB. Four shares
+// in place of eight: 25 against 23 ms a generation, measured with the second form.
 
 struct DecodeLinearParams {
   const void* x; const void* w; void* y;
@@ -153,238 +195,474 @@ struct DecodeLinearParams {
   float ln_eps; int act;
   int m, n, k;
   long long x_row, w_row, y_row;
-  float* partial;            // [k_slabs][16][n]
-  unsigned int* counters;    // one per column slab, zero between launches
-  // x not materialised: it is act(sum over xp_slabs of xp[slab][m][.] + xp_bias) rounded to the storage type, i.e. the
+  // the persistent engine only:
+  float* partial;            // [shares][16][n]
+  // x not materialised: it is act(sum over xp_shares of xp[share][m][.] + xp_bias) rounded to the storage type, i.e. the
   // unfinished result of the previous linear of the step (its row length is this linear's k)
-  const float* xp = nullptr; int xp_slabs = 0; const void* xp_bias = nullptr; int xp_act = 0;
-  // leave the result unfinished: only the partials are written, and the kernel that consumes them adds them up (no
-  // fence, counter and reload by a last CTA on this launch's tail); y, bias, act and residual are then unused
-  int partial_only = 0;
+  const float* xp = nullptr; int xp_shares = 0; const void* xp_bias = nullptr; int xp_act = 0;
 };
 
-template <typename T> struct DlVec { using type = uint2; };      // four consecutive 16-bit weights
-template <> struct DlVec<float> { using type = uint4; };
+constexpr int kDlShares = 8;      // shares of K at most: a cluster of portable size
+__host__ __device__ __forceinline__ int dl_per(int slabs) { return (slabs + kDlShares - 1) / kDlShares; }       // slabs of one share
+__host__ __device__ __forceinline__ int dl_shares(int k) { const int slabs = (k + kDlRows - 1) / kDlRows, per = dl_per(slabs); return (slabs + per - 1) / per; }
 
-// Shared memory of one linear work item (a 64-column x 128-row slab of W against all rows of x).
+constexpr int kDlXPad = 16, kDlSumPitch = kDlCols + 4;       // floats; keep the 16-byte accesses of eight lanes on different banks
+// Shared memory of one linear work item of the persistent engine (a 64-column x 128-row slab of W against all rows of x).
+struct DlStats { float mean[kDlMaxM], rstd[kDlMaxM]; };
 struct DlSmem {
-  float sX[kDlMaxM][kDlRows];                 // this item's slab of x (normalised if asked), as float
-  float sSum[kDlThreads / 32][kDlMaxM][kDlCols];
-  float s_mean[kDlMaxM], s_rstd[kDlMaxM];
+  alignas(16) float sX[kDlMaxM][kDlRows + kDlXPad];       // float32 weights: this item's slab of x (normalised if asked)
+  alignas(16) float sSum[kDlThreads / 32][kDlMaxM][kDlSumPitch];
+  DlStats st;
 };
 
-// The item's weights: a warp owns 16 consecutive K rows, a lane four consecutive columns of two of them.
+// A slab's weights: a warp owns 16 consecutive K rows. 16-bit: a lane has eight consecutive columns of four of them; float32: four
+// columns of eight.
+template <typename T> constexpr int kDlWv = sizeof(T) == 4 ? 8 : 4;
 template <typename T>
-__device__ __forceinline__ void dl_load_weights(const DecodeLinearParams& p, int n0, int k0, typename DlVec<T>::type (&wv)[8]) {
-  using V = typename DlVec<T>::type;
+__device__ __forceinline__ void dl_load_weights(const DecodeLinearParams& p, int n0, int k0, uint4 (&wv)[kDlWv<T>]) {
   const T* W = reinterpret_cast<const T*>(p.w);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int half = lane >> 4, cl = lane & 15;
-  const int col = n0 + cl * 4;
+  if constexpr (sizeof(T) == 4) {
+    const int col = n0 + (lane & 15) * 4;
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const int kk = k0 + warp * 16 + i * 2 + half;
-    wv[i] = V{};
-    if (kk < p.k && col < p.n) wv[i] = __ldcs(reinterpret_cast<const V*>(W + (long long)kk * p.w_row + col));
+    for (int i = 0; i < 8; i++) {
+      const int kk = k0 + warp * 16 + i * 2 + (lane >> 4);
+      wv[i] = kk < p.k && col < p.n ? __ldcs(reinterpret_cast<const uint4*>(W + (long long)kk * p.w_row + col)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  } else {
+    const bool wide = ((reinterpret_cast<uintptr_t>(W) | (uintptr_t)(p.w_row * 2)) & 15u) == 0;
+    const int col = n0 + (lane >> 2) * 8;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int kk = k0 + warp * 16 + (lane & 3) * 4 + i;
+      const T* at = W + (long long)kk * p.w_row + col;
+      wv[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (kk >= p.k) continue;
+      if (wide && col + 8 <= p.n) wv[i] = __ldcs(reinterpret_cast<const uint4*>(at));
+      else {                                             // rows on 8 bytes, or half a piece at the end of one
+        if (col < p.n) { const uint2 u = __ldcs(reinterpret_cast<const uint2*>(at)); wv[i].x = u.x; wv[i].y = u.y; }
+        if (col + 4 < p.n) { const uint2 u = __ldcs(reinterpret_cast<const uint2*>(at + 4)); wv[i].z = u.x; wv[i].w = u.y; }
+      }
+    }
   }
 }
 
 // Row statistics of layer_norm over the whole rows of x: a warp per row, the row in registers after one round of
 // 16-byte loads (kernel_templates.rs:1097-1109: mean, population variance, 1/sqrt(var + eps)). Ends with a block barrier.
-template <typename T>
-__device__ __forceinline__ void dl_ln_stats(const DecodeLinearParams& p, DlSmem& sm) {
+// IT: 32 x 16-byte rounds of a row at most (the persistent engine: 2048 columns of any type).
+template <typename T, int IT = 8>
+__device__ __forceinline__ void dl_ln_stats(const DecodeLinearParams& p, DlStats& sm) {
   constexpr int N16 = Pack<T>::N;
   const T* X = reinterpret_cast<const T*>(p.x);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int m = warp; m < p.m; m += kDlThreads / 32) {
     const T* xr = X + (long long)m * p.x_row;
     const int packs = p.k / N16;
-    float v[8][N16];                                   // up to 8 x 32 packs per row: k <= 256 * N16
+    Pack<T> q[IT];
     float sum = 0.f;
 #pragma unroll
-    for (int it = 0; it < 8; it++) {
-      const int pk = lane + it * 32;
-      if (pk < packs) {
-        Pack<T> q = ld16(xr + pk * N16);
+    for (int it = 0; it < IT; it++) if (lane + it * 32 < packs) q[it] = ld16(xr + (lane + it * 32) * N16);
 #pragma unroll
-        for (int e = 0; e < N16; e++) { v[it][e] = Cvt<T>::to(q.v[e]); sum += v[it][e]; }
-      } else {
+    for (int it = 0; it < IT; it++) {
+      if (lane + it * 32 < packs) {
 #pragma unroll
-        for (int e = 0; e < N16; e++) v[it][e] = 0.f;
+        for (int e = 0; e < N16; e++) sum += Cvt<T>::to(q[it].v[e]);
       }
     }
     const float mean = warp_sum(sum) / (float)p.k;
     float sq = 0.f;
 #pragma unroll
-    for (int it = 0; it < 8; it++) {
+    for (int it = 0; it < IT; it++) {
       if (lane + it * 32 < packs) {
 #pragma unroll
-        for (int e = 0; e < N16; e++) { const float dlt = v[it][e] - mean; sq += dlt * dlt; }
+        for (int e = 0; e < N16; e++) { const float dlt = Cvt<T>::to(q[it].v[e]) - mean; sq += dlt * dlt; }
       }
     }
     const float var = warp_sum(sq) / (float)p.k;
-    if (lane == 0) { sm.s_mean[m] = mean; sm.s_rstd[m] = 1.0f / sqrtf(var + p.ln_eps); }
+    if (lane == 0) { sm.mean[m] = mean; sm.rstd[m] = 1.0f / sqrtf(var + p.ln_eps); }
   }
   __syncthreads();
 }
 
-// The item's partial product into p.partial[k_slab][m][n0 ..]: x slab to shared memory (layer_norm applied on the way
-// if asked; the statistics must be in sm), the products, the reduction over the CTA's warps in K order.
+// 128 columns of x from k0 on go into shared memory as floats, layer_norm applied on the way if asked. A thread has eight columns of
+// one row: dl_ask_norm and dl_ask_x ask for them (the former before the dependency wait: gamma and beta are model weights), dl_put_x
+// writes them once the statistics are there. K is a multiple of eight.
+constexpr int kDlPer = kDlRows / 16;
+template <typename T> struct DlX { Pack<T> x[kDlPer / Pack<T>::N], g[kDlPer / Pack<T>::N], b[kDlPer / Pack<T>::N]; };
+__device__ __forceinline__ int dl_x_col(int k0) { return k0 + (threadIdx.x & 15) * kDlPer; }
 template <typename T>
-__device__ __forceinline__ void dl_partial(const DecodeLinearParams& p, DlSmem& sm, int n0, int k0, int k_slab, const typename DlVec<T>::type (&wv)[8]) {
-  const T* X = reinterpret_cast<const T*>(p.x);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int half = lane >> 4, cl = lane & 15;
-  // x slab -> shared as float (M x 128, zero beyond M and K): one 16-byte load per thread
-  {
-    const int m = threadIdx.x >> 4, ch = threadIdx.x & 15;
-    constexpr int PER = kDlRows / 16;                    // 8 elements per thread
-    float v[PER];
+__device__ __forceinline__ void dl_ask_norm(const DecodeLinearParams& p, int k0, DlX<T>& r) {
+  const int kk = dl_x_col(k0);
+  if (!p.ln_gamma || kk >= p.k) return;
+  const T* G = reinterpret_cast<const T*>(p.ln_gamma) + kk;
+  const T* B = reinterpret_cast<const T*>(p.ln_beta) + kk;
+  constexpr int N = Pack<T>::N;
+  if (((reinterpret_cast<uintptr_t>(G) | reinterpret_cast<uintptr_t>(B)) & 15u) == 0) {
 #pragma unroll
-    for (int e = 0; e < PER; e++) v[e] = 0.f;
-    const int kk = k0 + ch * PER;
-    if (p.xp && m < p.m && kk + PER <= p.k && p.xp_slabs <= 8) {
-      // the previous linear's partials, added in K order, + bias, activation, rounded as it would have been stored; all
-      // loads of the (at most eight) slabs are in flight before the first addition
-      float4 q[8][2];
+    for (int i = 0; i < kDlPer / N; i++) { r.g[i] = ld16(G + i * N); r.b[i] = ld16(B + i * N); }
+  } else {
 #pragma unroll
-      for (int ks = 0; ks < 8; ks++) {
-        if (ks < p.xp_slabs) {
-          const float4* src = reinterpret_cast<const float4*>(p.xp + ((long long)ks * kDlMaxM + m) * p.k + kk);
-          q[ks][0] = __ldcg(src); q[ks][1] = __ldcg(src + 1);
-        } else {
-          q[ks][0] = make_float4(0.f, 0.f, 0.f, 0.f); q[ks][1] = q[ks][0];
-        }
-      }
-      float t[PER];
+    for (int i = 0; i < kDlPer / N; i++)
 #pragma unroll
-      for (int e = 0; e < PER; e++) t[e] = 0.f;
+      for (int e = 0; e < N; e++) { r.g[i].v[e] = G[i * N + e]; r.b[i].v[e] = B[i * N + e]; }
+  }
+}
+template <typename T>
+__device__ __forceinline__ void dl_ask_x(const DecodeLinearParams& p, int k0, DlX<T>& r) {
+  const int m = threadIdx.x >> 4, kk = dl_x_col(k0);
+  if (m >= p.m || kk >= p.k) return;
+  const T* src = reinterpret_cast<const T*>(p.x) + (long long)m * p.x_row + kk;
 #pragma unroll
-      for (int ks = 0; ks < 8; ks++) {
-        if (ks < p.xp_slabs) {
-          t[0] += q[ks][0].x; t[1] += q[ks][0].y; t[2] += q[ks][0].z; t[3] += q[ks][0].w;
-          t[4] += q[ks][1].x; t[5] += q[ks][1].y; t[6] += q[ks][1].z; t[7] += q[ks][1].w;
-        }
-      }
+  for (int i = 0; i < kDlPer / Pack<T>::N; i++) r.x[i] = ld16(src + i * Pack<T>::N);
+}
+template <typename T>
+__device__ __forceinline__ void dl_put_x(const DecodeLinearParams& p, const DlStats& st, float* sX, int pitch, int k0, const DlX<T>& r) {
+  const int m = threadIdx.x >> 4, kk = dl_x_col(k0);
+  constexpr int N = Pack<T>::N;
+  float v[kDlPer];
 #pragma unroll
-      for (int e = 0; e < PER; e++) {
-        if (p.xp_bias) t[e] += Cvt<T>::to(reinterpret_cast<const T*>(p.xp_bias)[kk + e]);
-        v[e] = Cvt<T>::to(Cvt<T>::from(apply_act(t[e], (Act)p.xp_act)));
-      }
-    } else if (p.xp && m < p.m && kk < p.k) {
-      for (int e = 0; e < PER; e++) {
-        if (kk + e < p.k) {
-          float t = 0.f;
-          for (int ks = 0; ks < p.xp_slabs; ks++) t += __ldcg(p.xp + ((long long)ks * kDlMaxM + m) * p.k + kk + e);
-          if (p.xp_bias) t += Cvt<T>::to(reinterpret_cast<const T*>(p.xp_bias)[kk + e]);
-          v[e] = Cvt<T>::to(Cvt<T>::from(apply_act(t, (Act)p.xp_act)));
-        }
-      }
-    } else if (m < p.m && kk < p.k) {
-      const T* src = X + (long long)m * p.x_row + kk;
-      if (kk + PER <= p.k) {
-        if constexpr (sizeof(T) == 4) {
-          const float4 q0 = *reinterpret_cast<const float4*>(src), q1 = *reinterpret_cast<const float4*>(src + 4);
-          v[0] = q0.x; v[1] = q0.y; v[2] = q0.z; v[3] = q0.w; v[4] = q1.x; v[5] = q1.y; v[6] = q1.z; v[7] = q1.w;
-        } else {
-          Pack<T> q = ld16(src);
+  for (int e = 0; e < kDlPer; e++) v[e] = 0.f;
+  if (m < p.m && kk < p.k) {
 #pragma unroll
-          for (int e = 0; e < PER; e++) v[e] = Cvt<T>::to(q.v[e]);
-        }
-      } else {
-        for (int e = 0; e < PER; e++) if (kk + e < p.k) v[e] = Cvt<T>::to(src[e]);
-      }
-      if (p.ln_gamma) {
-        const T* G = reinterpret_cast<const T*>(p.ln_gamma);
-        const T* Bt = reinterpret_cast<const T*>(p.ln_beta);
-        const float mean = sm.s_mean[m], rstd = sm.s_rstd[m];
-        for (int e = 0; e < PER; e++) if (kk + e < p.k) v[e] = Cvt<T>::to(G[kk + e]) * (v[e] - mean) * rstd + Cvt<T>::to(Bt[kk + e]);
+    for (int e = 0; e < kDlPer; e++) v[e] = Cvt<T>::to(r.x[e / N].v[e % N]);
+    if (p.ln_gamma) {
+      const float mean = st.mean[m], rstd = st.rstd[m];
+#pragma unroll
+      for (int e = 0; e < kDlPer; e++) v[e] = Cvt<T>::to(r.g[e / N].v[e % N]) * (v[e] - mean) * rstd + Cvt<T>::to(r.b[e / N].v[e % N]);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < kDlPer; e += 4) *reinterpret_cast<float4*>(sX + m * pitch + (threadIdx.x & 15) * kDlPer + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+}
+// The persistent engine's x that is not materialised: the previous linear's partials, added in K order, + bias, activation, rounded as
+// they would have been stored.
+template <typename T>
+__device__ __forceinline__ void dl_put_partials(const DecodeLinearParams& p, float* sX, int pitch, int k0) {
+  const int m = threadIdx.x >> 4, kk = dl_x_col(k0);
+  float v[kDlPer];
+#pragma unroll
+  for (int e = 0; e < kDlPer; e++) v[e] = 0.f;
+  if (m < p.m && kk < p.k) {
+    float4 q[kDlShares][2];                              // all loads are in flight before the first addition
+#pragma unroll
+    for (int ks = 0; ks < kDlShares; ks++) {
+      if (ks < p.xp_shares) {
+        const float4* src = reinterpret_cast<const float4*>(p.xp + ((long long)ks * kDlMaxM + m) * p.k + kk);
+        q[ks][0] = __ldcg(src); q[ks][1] = __ldcg(src + 1);
       }
     }
 #pragma unroll
-    for (int e = 0; e < PER; e++) sm.sX[m][ch * PER + e] = v[e];
-  }
-  __syncthreads();
-  float acc[kDlMaxM][4];
+    for (int ks = 0; ks < kDlShares; ks++) {
+      if (ks < p.xp_shares) {
+        v[0] += q[ks][0].x; v[1] += q[ks][0].y; v[2] += q[ks][0].z; v[3] += q[ks][0].w;
+        v[4] += q[ks][1].x; v[5] += q[ks][1].y; v[6] += q[ks][1].z; v[7] += q[ks][1].w;
+      }
+    }
 #pragma unroll
-  for (int m = 0; m < kDlMaxM; m++) { acc[m][0] = 0.f; acc[m][1] = 0.f; acc[m][2] = 0.f; acc[m][3] = 0.f; }
+    for (int e = 0; e < kDlPer; e++) {
+      if (p.xp_bias) v[e] += Cvt<T>::to(reinterpret_cast<const T*>(p.xp_bias)[kk + e]);
+      v[e] = Cvt<T>::to(Cvt<T>::from(apply_act(v[e], (Act)p.xp_act)));
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < kDlPer; e += 4) *reinterpret_cast<float4*>(sX + m * pitch + (threadIdx.x & 15) * kDlPer + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+}
+
+// float32 weights: this warp's 16 rows of a slab against the staged x, added to acc (two columns' halves: see dl_store_f32).
+__device__ __forceinline__ void dl_products_f32(const float* sX, int pitch, const uint4 (&wv)[8], float (&acc)[kDlMaxM][4]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
-    const int kk = warp * 16 + i * 2 + half;
-    const T* pr = reinterpret_cast<const T*>(&wv[i]);
-    const float b0 = Cvt<T>::to(pr[0]), b1 = Cvt<T>::to(pr[1]), b2 = Cvt<T>::to(pr[2]), b3 = Cvt<T>::to(pr[3]);
+    const float* at = sX + warp * 16 + i * 2 + (lane >> 4);
+    const float* pr = reinterpret_cast<const float*>(&wv[i]);
 #pragma unroll
     for (int m = 0; m < kDlMaxM; m++) {
-      const float a = sm.sX[m][kk];                      // two addresses per warp (one per half): broadcasts
-      acc[m][0] = fmaf(a, b0, acc[m][0]); acc[m][1] = fmaf(a, b1, acc[m][1]);
-      acc[m][2] = fmaf(a, b2, acc[m][2]); acc[m][3] = fmaf(a, b3, acc[m][3]);
+      const float a = at[m * pitch];                         // two addresses per warp (one per half): broadcasts
+#pragma unroll
+      for (int e = 0; e < 4; e++) acc[m][e] = fmaf(a, pr[e], acc[m][e]);
     }
   }
-  // the two half-warps hold different rows of the same columns
+}
+// the two half-warps hold different rows of the same columns
+__device__ __forceinline__ void dl_store_f32(float (&acc)[kDlMaxM][4], float (*sSum)[kDlMaxM][kDlSumPitch]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int m = 0; m < kDlMaxM; m++) {
 #pragma unroll
     for (int e = 0; e < 4; e++) acc[m][e] += __shfl_xor_sync(0xffffffffu, acc[m][e], 16);
-  }
-  if (half == 0) {
-#pragma unroll
-    for (int m = 0; m < kDlMaxM; m++) *reinterpret_cast<float4*>(&sm.sSum[warp][m][cl * 4]) = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
-  }
-  __syncthreads();
-  float* my_partial = p.partial + ((long long)k_slab * kDlMaxM) * p.n;
-  for (int i = threadIdx.x; i < kDlMaxM * kDlCols; i += kDlThreads) {
-    int m = i / kDlCols, c = i % kDlCols;
-    if (m < p.m && n0 + c < p.n) {
-      float v = 0.f;
-#pragma unroll
-      for (int w8 = 0; w8 < kDlThreads / 32; w8++) v += sm.sSum[w8][m][c];    // warp order = K order
-      my_partial[(long long)m * p.n + n0 + c] = v;
-    }
+    if (lane < 16) *reinterpret_cast<float4*>(&sSum[warp][m][lane * 4]) = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
   }
 }
 
-// One finished element: the K slabs' partials added in K order (deterministic), bias, activation, residual.
+template <typename T> __device__ __forceinline__ T dl_piece(float v) { return Cvt<T>::from(v); }
+template <> __device__ __forceinline__ __half dl_piece<__half>(float v) {         // a value beyond the type leaves the rest to the next piece
+  return __float2half_rn(fabsf(v) > 65504.f ? copysignf(65504.f, v) : v);
+}
+template <typename T> __device__ __forceinline__ uint32_t dl_pair(T lo, T hi) {
+  return (uint32_t)*reinterpret_cast<const uint16_t*>(&lo) | ((uint32_t)*reinterpret_cast<const uint16_t*>(&hi) << 16);
+}
+template <typename T> __device__ __forceinline__ float dl_elem(uint2 v, int e) {
+  const uint32_t w = e < 2 ? v.x : v.y;
+  const uint16_t h = (uint16_t)(e & 1 ? w >> 16 : w & 0xffffu);
+  return Cvt<T>::to(*reinterpret_cast<const T*>(&h));
+}
+
+// 16-bit weights: a lane (g, q) has rows 4q .. 4q + 3 of the warp's 16 and columns 8g .. 8g + 7. The order of K in a product and of the
+// columns is free as long as both operands agree, so mma.m16n8k16 takes the weights as they lie: product j has columns 8g + j and
+// 8g + j + 4 in its rows, eight rows of x in its columns and the lane's four rows as its K, and the x operand is four neighbouring
+// elements of row g, straight from memory.
+__device__ __forceinline__ int dl_k_of(int k0) { return k0 + (threadIdx.x >> 5) * 16 + (threadIdx.x & 3) * 4; }
 template <typename T>
-__device__ __forceinline__ float dl_finish_element(const DecodeLinearParams& p, int k_slabs, int m, int col) {
+__device__ __forceinline__ uint2 dl_ask4(const void* base, long long at) { return *reinterpret_cast<const uint2*>(reinterpret_cast<const T*>(base) + at); }
+template <typename T, int NT>
+__device__ __forceinline__ void dl_ask_x16(const DecodeLinearParams& p, int k0, uint2 (&x)[NT]) {
+  const int kk = dl_k_of(k0), g = (threadIdx.x & 31) >> 2;
+#pragma unroll
+  for (int t = 0; t < NT; t++) x[t] = kk < p.k && g + 8 * t < p.m ? dl_ask4<T>(p.x, (long long)(g + 8 * t) * p.x_row + kk) : make_uint2(0u, 0u);
+}
+template <typename T>
+__device__ __forceinline__ void dl_ask_norm16(const DecodeLinearParams& p, int k0, uint2& gam, uint2& bet) {
+  const int kk = dl_k_of(k0);
+  gam = make_uint2(0u, 0u); bet = gam;
+  if (kk >= p.k) return;
+  if (((reinterpret_cast<uintptr_t>(p.ln_gamma) | reinterpret_cast<uintptr_t>(p.ln_beta)) & 7u) == 0) { gam = dl_ask4<T>(p.ln_gamma, kk); bet = dl_ask4<T>(p.ln_beta, kk); return; }
+  const T* G = reinterpret_cast<const T*>(p.ln_gamma) + kk;
+  const T* B = reinterpret_cast<const T*>(p.ln_beta) + kk;
+  gam.x = dl_pair(G[0], G[1]); gam.y = dl_pair(G[2], G[3]); bet.x = dl_pair(B[0], B[1]); bet.y = dl_pair(B[2], B[3]);
+}
+template <typename T, int NT, bool LN>
+__device__ __forceinline__ void dl_products16(const uint4 (&wv)[4], const uint2 (&x)[NT], uint2 gam, uint2 bet, const DlStats& st, float (&acc)[NT][4][4]) {
+  const int g = (threadIdx.x & 31) >> 2;
+  uint32_t a[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    auto word = [&](int i, int c) { return c < 2 ? wv[i].x : c < 4 ? wv[i].y : c < 6 ? wv[i].z : wv[i].w; };
+    const uint32_t sel = j & 1 ? 0x7632u : 0x5410u;
+    a[j][0] = __byte_perm(word(0, j), word(1, j), sel); a[j][1] = __byte_perm(word(0, j + 4), word(1, j + 4), sel);
+    a[j][2] = __byte_perm(word(2, j), word(3, j), sel); a[j][3] = __byte_perm(word(2, j + 4), word(3, j + 4), sel);
+  }
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    if constexpr (!LN) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) mma_16816<T>(acc[t][j], a[j][0], a[j][1], a[j][2], a[j][3], x[t].x, x[t].y);
+    } else {
+      const float mean = st.mean[g + 8 * t], rstd = st.rstd[g + 8 * t];
+      float r[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) r[e] = dl_elem<T>(gam, e) * (dl_elem<T>(x[t], e) - mean) * rstd + dl_elem<T>(bet, e);
+#pragma unroll
+      for (int piece = 0; piece < 3; piece++) {            // float32 as the sum of three 16-bit numbers
+        T h[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) { h[e] = dl_piece<T>(r[e]); r[e] -= Cvt<T>::to(h[e]); }
+        const uint32_t b0 = dl_pair(h[0], h[1]), b1 = dl_pair(h[2], h[3]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) mma_16816<T>(acc[t][j], a[j][0], a[j][1], a[j][2], a[j][3], b0, b1);
+      }
+    }
+  }
+}
+template <int NT>
+__device__ __forceinline__ void dl_store16(const float (&acc)[NT][4][4], float (*sSum)[kDlSumPitch]) {     // this warp's [NT * 8][64]
+  const int g = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
+#pragma unroll
+  for (int t = 0; t < NT; t++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {                          // rows 2q and 2q + 1 of x; columns 8g + 0 .. 3, then 4 .. 7
+      float* at = &sSum[t * 8 + q * 2 + h][g * 8];
+      *reinterpret_cast<float4*>(at) = make_float4(acc[t][0][h], acc[t][1][h], acc[t][2][h], acc[t][3][h]);
+      *reinterpret_cast<float4*>(at + 4) = make_float4(acc[t][0][h + 2], acc[t][1][h + 2], acc[t][2][h + 2], acc[t][3][h + 2]);
+    }
+}
+template <int NT>
+__device__ __forceinline__ void dl_zero(float (&acc)[NT][4][4]) {
+#pragma unroll
+  for (int t = 0; t < NT; t++)
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) acc[t][j][e] = 0.f;
+}
+
+// The persistent engine's item: one share's partial product into p.partial[share][m][n0 ..]. Its sums are those of decode_linear_kernel,
+// in the same order.
+template <typename T>
+__device__ __forceinline__ void dl_partial(const DecodeLinearParams& p, DlSmem& sm, int n0, int share, int per, uint4 (&wv)[kDlWv<T>]) {
+  if constexpr (sizeof(T) == 4) {
+    float acc[kDlMaxM][4];
+#pragma unroll
+    for (int m = 0; m < kDlMaxM; m++) { acc[m][0] = 0.f; acc[m][1] = 0.f; acc[m][2] = 0.f; acc[m][3] = 0.f; }
+    for (int i = 0; i < per; i++) {
+      const int k0 = (share * per + i) * kDlRows;
+      if (i) { __syncthreads(); dl_load_weights<T>(p, n0, k0, wv); }
+      if (p.xp) dl_put_partials<T>(p, &sm.sX[0][0], kDlRows + kDlXPad, k0);
+      else {
+        DlX<T> x;
+        dl_ask_norm<T>(p, k0, x);
+        dl_ask_x<T>(p, k0, x);
+        dl_put_x<T>(p, sm.st, &sm.sX[0][0], kDlRows + kDlXPad, k0, x);
+      }
+      __syncthreads();
+      dl_products_f32(&sm.sX[0][0], kDlRows + kDlXPad, wv, acc);
+    }
+    dl_store_f32(acc, sm.sSum);
+  } else {
+    float acc[2][4][4];
+    dl_zero<2>(acc);
+    for (int i = 0; i < per; i++) {
+      const int k0 = (share * per + i) * kDlRows;
+      if (i) dl_load_weights<T>(p, n0, k0, wv);
+      uint2 x[2], gam = make_uint2(0u, 0u), bet = gam;
+      if (p.xp) {                                          // values of type T again: dl_put_partials has rounded them
+        __syncthreads();
+        dl_put_partials<T>(p, &sm.sX[0][0], kDlRows + kDlXPad, k0);
+        __syncthreads();
+        const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+          const float4 f = *reinterpret_cast<const float4*>(&sm.sX[(lane >> 2) + 8 * t][(threadIdx.x >> 5) * 16 + (lane & 3) * 4]);
+          x[t] = make_uint2(dl_pair(Cvt<T>::from(f.x), Cvt<T>::from(f.y)), dl_pair(Cvt<T>::from(f.z), Cvt<T>::from(f.w)));
+        }
+      } else dl_ask_x16<T, 2>(p, k0, x);
+      if (p.ln_gamma) { dl_ask_norm16<T>(p, k0, gam, bet); dl_products16<T, 2, true>(wv, x, gam, bet, sm.st, acc); }
+      else dl_products16<T, 2, false>(wv, x, gam, bet, sm.st, acc);
+    }
+    dl_store16<2>(acc, sm.sSum[threadIdx.x >> 5]);
+  }
+  __syncthreads();
+  float* my_partial = p.partial + ((long long)share * kDlMaxM) * p.n;
+  for (int i = threadIdx.x; i < kDlMaxM * kDlCols; i += kDlThreads) {
+    const int m = i / kDlCols, c = i % kDlCols;
+    float v = 0.f;
+#pragma unroll
+    for (int w8 = 0; w8 < kDlThreads / 32; w8++) v += sm.sSum[w8][m][c];      // warp order = K order
+    if (m < p.m && n0 + c < p.n) my_partial[(long long)m * p.n + n0 + c] = v;
+  }
+}
+
+// One finished element: the shares' partials added in K order (deterministic), bias, activation, residual.
+template <typename T>
+__device__ __forceinline__ float dl_finish_element(const DecodeLinearParams& p, int shares, int m, int col) {
   float v = 0.f;
-  for (int ks = 0; ks < k_slabs; ks++) v += __ldcg(p.partial + ((long long)ks * kDlMaxM + m) * p.n + col);
+  for (int ks = 0; ks < shares; ks++) v += __ldcg(p.partial + ((long long)ks * kDlMaxM + m) * p.n + col);
   if (p.bias) v += Cvt<T>::to(reinterpret_cast<const T*>(p.bias)[col]);
   v = apply_act(v, (Act)p.act);
   if (p.residual) v += Cvt<T>::to(reinterpret_cast<const T*>(p.residual)[(long long)m * p.y_row + col]);
   return v;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kDlThreads) decode_linear_kernel(const DecodeLinearParams p) {
-  using V = typename DlVec<T>::type;
-  __shared__ DlSmem sm;
-  __shared__ unsigned int s_last;
-  const int n0 = blockIdx.x * kDlCols, k0 = blockIdx.y * kDlRows;
-  // weights first, before the dependency wait (they are not produced by the step)
-  V wv[8];
-  dl_load_weights<T>(p, n0, k0, wv);
-  pdl_wait();      // x, the residual and the workspace belong to the step: nothing of them is touched above this line
-  pdl_trigger();
-  if (p.ln_gamma) dl_ln_stats<T>(p, sm);
-  dl_partial<T>(p, sm, n0, k0, (int)blockIdx.y, wv);
-  if (p.partial_only) return;     // the consumer adds the partials up; the end of this grid orders them before its reads
-  const int k_slabs = gridDim.y;
-  // the last CTA of this column slab finishes it
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned int prev = atomicAdd(p.counters + blockIdx.x, 1u);
-    s_last = (prev == (unsigned int)(k_slabs - 1)) ? 1u : 0u;
+// The CTA's sums for its share (sSum, eight warps of them) to the results. Row m is finished by share m % shares: every CTA adds its warps'
+// sums in K order and stores them in that CTA's sFin, and after one cluster barrier the finisher adds the shares in K order. The barrier
+// that says the peers' shared memory exists was arrived at when the kernel started.
+constexpr int kDlFinRows = kDlMaxM + kDlShares;            // shares x rows a share finishes, at most
+template <typename T, int ROWS>
+__device__ __forceinline__ void dl_finish(const DecodeLinearParams& p, int n0, int rank, int ranks, const float* sSum, float* sFin) {
+  const int c = threadIdx.x & (kDlCols - 1), m0 = threadIdx.x / kDlCols;
+  constexpr int STEP = kDlThreads / kDlCols;
+  const int mine = (p.m - rank + ranks - 1) / ranks;       // rows this CTA finishes: rank, rank + ranks, ..
+  const bool live = n0 + c < p.n;
+  float bias = 0.f, res = 0.f;
+  if (live && p.bias) bias = Cvt<T>::to(reinterpret_cast<const T*>(p.bias)[n0 + c]);
+  if (live && p.residual && m0 < mine) res = Cvt<T>::to(reinterpret_cast<const T*>(p.residual)[(long long)(rank + m0 * ranks) * p.y_row + n0 + c]);
+  if (ranks > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const int per = (p.m + ranks - 1) / ranks;
+#pragma unroll
+  for (int j = 0; j < ROWS / STEP; j++) {
+    const int m = m0 + j * STEP;
+    if (m >= p.m) break;
+    float v = 0.f;
+#pragma unroll
+    for (int w8 = 0; w8 < kDlThreads / 32; w8++) v += sSum[(w8 * ROWS + m) * kDlSumPitch + c];      // warp order = K order
+    float* at = sFin + (rank * per + m / ranks) * kDlCols + c;
+    if (ranks > 1) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(sm100::mapa_u32(sm100::smem_u32(at), (uint32_t)(m % ranks))), "f"(v) : "memory");
+    else *at = v;
   }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
+  if (ranks > 1) sm100::cluster_sync_all(); else __syncthreads();
   T* Y = reinterpret_cast<T*>(p.y);
-  for (int i = threadIdx.x; i < kDlMaxM * kDlCols; i += kDlThreads) {
-    int m = i / kDlCols, c = i % kDlCols;
-    if (m < p.m && n0 + c < p.n) Y[(long long)m * p.y_row + n0 + c] = Cvt<T>::from(dl_finish_element<T>(p, k_slabs, m, n0 + c));
+  for (int i = m0; i < mine && live; i += STEP) {
+    const int m = rank + i * ranks;
+    float v = 0.f;
+    for (int r = 0; r < ranks; r++) v += sFin[(r * per + i) * kDlCols + c];
+    if (i != m0 && p.residual) res = Cvt<T>::to(reinterpret_cast<const T*>(p.residual)[(long long)m * p.y_row + n0 + c]);
+    v = apply_act(v + bias, (Act)p.act);
+    Y[(long long)m * p.y_row + n0 + c] = Cvt<T>::from(p.residual ? v + res : v);
   }
-  if (threadIdx.x == 0) p.counters[blockIdx.x] = 0;   // ready for the next launch on this stream
+}
+
+// grid = (column slabs, shares of K), a cluster per column slab; `per` slabs of 128 K rows in a share, PRE of them asked for ahead of the
+// dependency wait (they are not produced by the step). NT groups of eight rows of x.
+// LN: 0 or the rounds of layer_norm's statistics (IT above).
+template <typename T, int NT, int PRE, int LN>
+__global__ void __launch_bounds__(kDlThreads) decode_linear_kernel(const __grid_constant__ DecodeLinearParams p, int per) {
+  __shared__ __align__(16) float sSum[kDlThreads / 32][NT * 8][kDlSumPitch];
+  __shared__ float sFin[kDlFinRows * kDlCols];
+  __shared__ DlStats st;
+  const int ranks = gridDim.y, rank = ranks > 1 ? (int)sm100::cluster_ctarank() : 0;
+  if (ranks > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  const int n0 = blockIdx.x * kDlCols, k0 = rank * per * kDlRows;
+  uint4 wv[PRE][4];
+  uint2 x[PRE][NT], gam[PRE], bet[PRE];
+#pragma unroll
+  for (int s = 0; s < PRE; s++) dl_load_weights<T>(p, n0, s < per ? k0 + s * kDlRows : p.k, wv[s]);
+  if constexpr (LN) {
+#pragma unroll
+    for (int s = 0; s < PRE; s++) dl_ask_norm16<T>(p, s < per ? k0 + s * kDlRows : p.k, gam[s], bet[s]);
+  }
+  pdl_wait();      // x and the residual belong to the step: nothing of them is touched above this line
+  pdl_trigger();
+#pragma unroll
+  for (int s = 0; s < PRE; s++) dl_ask_x16<T, NT>(p, s < per ? k0 + s * kDlRows : p.k, x[s]);
+  if constexpr (LN) dl_ln_stats<T, LN>(p, st);
+  float acc[NT][4][4];
+  dl_zero<NT>(acc);
+#pragma unroll
+  for (int s = 0; s < PRE; s++) dl_products16<T, NT, LN != 0>(wv[s], x[s], gam[s], bet[s], st, acc);
+  for (int s = PRE; s < per; s++) {
+    dl_load_weights<T>(p, n0, k0 + s * kDlRows, wv[0]);
+    dl_ask_x16<T, NT>(p, k0 + s * kDlRows, x[0]);
+    if constexpr (LN) dl_ask_norm16<T>(p, k0 + s * kDlRows, gam[0], bet[0]);
+    dl_products16<T, NT, LN != 0>(wv[0], x[0], gam[0], bet[0], st, acc);
+  }
+  dl_store16<NT>(acc, sSum[threadIdx.x >> 5]);
+  __syncthreads();
+  dl_finish<T, NT * 8>(p, n0, rank, ranks, &sSum[0][0][0], sFin);
+}
+
+// float32 weights: the same on CUDA cores, x staged in shared memory.
+__global__ void __launch_bounds__(kDlThreads) decode_linear_f32_kernel(const __grid_constant__ DecodeLinearParams p, int per) {
+  __shared__ __align__(16) float sSum[kDlThreads / 32][kDlMaxM][kDlSumPitch];
+  __shared__ __align__(16) float sBuf[kDlMaxM * (kDlRows + kDlXPad)];       // x, then the shares' sums
+  static_assert(kDlFinRows * kDlCols <= kDlMaxM * (kDlRows + kDlXPad), "the shares' sums take the place of x");
+  __shared__ DlStats st;
+  const int ranks = gridDim.y, rank = ranks > 1 ? (int)sm100::cluster_ctarank() : 0;
+  const int n0 = blockIdx.x * kDlCols, k0 = rank * per * kDlRows;
+  uint4 wv[8];
+  DlX<float> x;
+  dl_load_weights<float>(p, n0, k0, wv);
+  dl_ask_norm<float>(p, k0, x);
+  pdl_wait();
+  pdl_trigger();
+  dl_ask_x<float>(p, k0, x);
+  if (p.ln_gamma) dl_ln_stats<float>(p, st);
+  float acc[kDlMaxM][4];
+#pragma unroll
+  for (int m = 0; m < kDlMaxM; m++) { acc[m][0] = 0.f; acc[m][1] = 0.f; acc[m][2] = 0.f; acc[m][3] = 0.f; }
+  for (int s = 0; s < per; s++) {
+    if (s) {
+      __syncthreads();
+      dl_load_weights<float>(p, n0, k0 + s * kDlRows, wv);
+      dl_ask_norm<float>(p, k0 + s * kDlRows, x);
+      dl_ask_x<float>(p, k0 + s * kDlRows, x);
+    }
+    dl_put_x<float>(p, st, sBuf, kDlRows + kDlXPad, k0 + s * kDlRows, x);
+    __syncthreads();
+    dl_products_f32(sBuf, kDlRows + kDlXPad, wv, acc);
+  }
+  dl_store_f32(acc, sSum);
+  __syncthreads();
+  if (ranks > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");     // every CTA is done with its x
+  dl_finish<float, kDlMaxM>(p, n0, rank, ranks, &sSum[0][0][0], sBuf);
 }
 
 
@@ -399,36 +677,37 @@ bool decode_linear_eligible(const GemmDesc& d) {
   if (d.a_row % n16 != 0 || (reinterpret_cast<uintptr_t>(d.a) & 15u) != 0 || d.k % 8 != 0) return false;   // 16-byte loads of x
   if (d.ln_gamma && (d.k % n16 != 0 || d.k > 256 * n16)) return false;                                     // a row fits the registers of one warp
   const int64_t ks = (d.k + kDlRows - 1) / kDlRows;
-  if (ks > 64 || ks * kDlMaxM * d.n > (int64_t)kDecodeRegionFloats) return false;                         // one workspace region: [k_slabs][16][n] floats
-  return true;
+  return ks <= 64;
 }
 
-float* decode_partial_region(int region) {
-  float* base = skinny_partials();
-  return base ? base + (size_t)region * kDecodeRegionFloats : nullptr;
+template <typename K>
+static cudaError_t launch_dl(cudaStream_t s, K kernel, const DecodeLinearParams& p, int per, int ranks) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((p.n + kDlCols - 1) / kDlCols), (unsigned)ranks); cfg.blockDim = dim3(kDlThreads); cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  at[1].id = cudaLaunchAttributeClusterDimension; at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = (unsigned)ranks; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = ranks > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, p, per);
+}
+template <typename T, int NT>
+static cudaError_t launch_dl16(cudaStream_t s, const DecodeLinearParams& p, int per, int ranks) {
+  if (!p.ln_gamma) return per == 1 ? launch_dl(s, decode_linear_kernel<T, NT, 1, 0>, p, per, ranks) : launch_dl(s, decode_linear_kernel<T, NT, 3, 0>, p, per, ranks);
+  return p.k <= 1024 ? launch_dl(s, decode_linear_kernel<T, NT, 1, 4>, p, per, ranks) : launch_dl(s, decode_linear_kernel<T, NT, 1, 8>, p, per, ranks);
 }
 
-Status decode_linear(cudaStream_t s, const GemmDesc& d, const DecodeLinearOpts& o) {
+Status decode_linear(cudaStream_t s, const GemmDesc& d) {
   if (!decode_linear_eligible(d)) return Status::invalid("decode_linear: shape or layout not supported");
-  if (o.region < 0 || o.region >= kDecodeRegions) return Status::invalid("decode_linear: partial region");
-  if (o.xp && (o.xp_slabs < 1 || o.xp_slabs > 64)) return Status::invalid("decode_linear: partial slabs of the input");
-  if (((d.k + kDlRows - 1) / kDlRows) * kDlMaxM * d.n > (int64_t)kDecodeRegionFloats) return Status::invalid("decode_linear: partials exceed a workspace region");
-  float* partial = decode_partial_region(o.region);
-  unsigned int* counters = skinny_counters();
-  if (!partial || !counters) return Status::compute("decode_linear: the kernel workspace is not initialised");
   DecodeLinearParams p;
   p.x = d.a; p.w = d.b; p.y = d.c; p.bias = d.ep.bias; p.residual = d.ep.residual; p.ln_gamma = d.ln_gamma; p.ln_beta = d.ln_beta; p.ln_eps = d.ln_eps;
   p.act = (int)d.ep.act; p.m = (int)d.m; p.n = (int)d.n; p.k = (int)d.k;
-  p.x_row = d.a_row; p.w_row = d.b_row; p.y_row = d.c_row; p.partial = partial; p.counters = counters;
-  p.partial_only = o.partial_only ? 1 : 0;
-  p.xp = o.xp; p.xp_slabs = o.xp_slabs; p.xp_bias = o.xp_bias; p.xp_act = (int)o.xp_act;
+  p.x_row = d.a_row; p.w_row = d.b_row; p.y_row = d.c_row; p.partial = nullptr;
+  const int per = dl_per((int)((d.k + kDlRows - 1) / kDlRows)), ranks = dl_shares((int)d.k);
   cudaError_t e;
-  dim3 grid((unsigned)((d.n + kDlCols - 1) / kDlCols), (unsigned)((d.k + kDlRows - 1) / kDlRows), 1);
-  if (d.dtype == DType::BF16) e = launch_pdl(decode_linear_kernel<__nv_bfloat16>, grid, dim3(kDlThreads), 0, s, p);
-  else if (d.dtype == DType::F16) e = launch_pdl(decode_linear_kernel<__half>, grid, dim3(kDlThreads), 0, s, p);
-  else e = launch_pdl(decode_linear_kernel<float>, grid, dim3(kDlThreads), 0, s, p);
-  if (e != cudaSuccess) return cuda_status(e, "decode_linear");
-  return Status::OK();
+  if (d.dtype == DType::F32) e = launch_dl(s, decode_linear_f32_kernel, p, per, ranks);
+  else if (d.dtype == DType::BF16) e = d.m <= 8 ? launch_dl16<__nv_bfloat16, 1>(s, p, per, ranks) : launch_dl16<__nv_bfloat16, 2>(s, p, per, ranks);
+  else e = d.m <= 8 ? launch_dl16<__half, 1>(s, p, per, ranks) : launch_dl16<__half, 2>(s, p, per, ranks);
+  return cuda_status(e, "decode_linear");
 }
 
 // ── the layers of a decode step as one persistent kernel ────────────────────
@@ -442,7 +721,7 @@ Status decode_linear(cudaStream_t s, const GemmDesc& d, const DecodeLinearOpts& 
 //   P3   partial products of att @ W_proj                         (12 x 6 items)
 //   P3b  x2 = x + sum of P3's partials + bias                     (element-wise)
 //   P4   partial products of ln_2(x2) @ W_fc                      (48 x 6 items)
-//   P5   partial products of gelu(P4 + bias) @ W_fc2, the operand summed from P4's partials on the way in   (12 x 24 items)
+//   P5   partial products of gelu(P4 + bias) @ W_fc2, the operand summed from P4's partials on the way in   (12 x 8 items)
 //   P5b  x = x2 + sum of P5's partials + bias                     (element-wise)
 // Every item runs the same device functions, in the same order of additions, as the per-op kernels above, so the
 // stream of tokens is the one the per-op engine produces. The barrier: one counter in global memory, cleared by a
@@ -501,7 +780,6 @@ __device__ __forceinline__ bool mega_barrier(const MegaParams& p, unsigned int& 
 
 template <typename T>
 __global__ void __launch_bounds__(kDlThreads, 2) decode_layers_kernel(const MegaParams p) {
-  using V = typename DlVec<T>::type;
 #ifdef AG_DECODE_PROBE
   if (blockIdx.x == 0 && threadIdx.x == 0) { g_mega_probe_n = 0; g_mega_probe[g_mega_probe_n++] = globaltimer_ns_dec(); }
 #endif
@@ -513,45 +791,45 @@ __global__ void __launch_bounds__(kDlThreads, 2) decode_layers_kernel(const Mega
   const int G = (int)gridDim.x, cta = (int)blockIdx.x;
   unsigned int target = 0;
   float* part_qkv = p.partial;
-  float* part_proj = part_qkv + (long long)((D + kDlRows - 1) / kDlRows) * kDlMaxM * 3 * D;
-  float* part_fc = part_proj + (long long)((D + kDlRows - 1) / kDlRows) * kDlMaxM * D;
-  float* part_fc2 = part_fc + (long long)((D + kDlRows - 1) / kDlRows) * kDlMaxM * 4 * D;
-  const int ks_d = (D + kDlRows - 1) / kDlRows, ks_4d = (4 * D + kDlRows - 1) / kDlRows;
+  const int ks_d = dl_shares(D), ks_4d = dl_shares(4 * D);
+  float* part_proj = part_qkv + (long long)ks_d * kDlMaxM * 3 * D;
+  float* part_fc = part_proj + (long long)ks_d * kDlMaxM * D;
+  float* part_fc2 = part_fc + (long long)ks_d * kDlMaxM * 4 * D;
 
   // The weights of this CTA's first item of the next linear phase are fetched as soon as the current linear phase is
   // done (they are constants of the model): the loads fly during the barriers and the phases in between, as the per-op
   // kernels fetch theirs ahead of the dependency wait.
-  V wv_next[8];
+  uint4 wv_next[kDlWv<T>];
   auto prefetch = [&](const void* wgt, int n, int k) {
     DecodeLinearParams lp{};
     lp.w = wgt; lp.n = n; lp.k = k; lp.w_row = n;
-    const int n_slabs = (n + kDlCols - 1) / kDlCols, k_slabs = (k + kDlRows - 1) / kDlRows;
-    if (cta < n_slabs * k_slabs) dl_load_weights<T>(lp, (cta % n_slabs) * kDlCols, (cta / n_slabs) * kDlRows, wv_next);
+    const int n_slabs = (n + kDlCols - 1) / kDlCols, shares = dl_shares(k), per = dl_per((k + kDlRows - 1) / kDlRows);
+    if (cta < n_slabs * shares) dl_load_weights<T>(lp, (cta % n_slabs) * kDlCols, (cta / n_slabs) * per * kDlRows, wv_next);
   };
   // one linear's partial products over the grid
   auto linear_partials = [&](DecodeLinearParams lp) {
-    const int n_slabs = (lp.n + kDlCols - 1) / kDlCols, k_slabs = (lp.k + kDlRows - 1) / kDlRows;
+    const int n_slabs = (lp.n + kDlCols - 1) / kDlCols, shares = dl_shares(lp.k), per = dl_per((lp.k + kDlRows - 1) / kDlRows);
     bool stats = false;
-    for (int it = cta; it < n_slabs * k_slabs; it += G) {
+    for (int it = cta; it < n_slabs * shares; it += G) {
       const int ns = it % n_slabs, ks = it / n_slabs;
-      V wv[8];
+      uint4 wv[kDlWv<T>];
       if (it == cta) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) wv[i] = wv_next[i];
+        for (int i = 0; i < kDlWv<T>; i++) wv[i] = wv_next[i];
       } else {
-        dl_load_weights<T>(lp, ns * kDlCols, ks * kDlRows, wv);
+        dl_load_weights<T>(lp, ns * kDlCols, ks * per * kDlRows, wv);
       }
       __syncthreads();                       // the previous item's shared-memory reads are done
-      if (lp.ln_gamma && !stats) { dl_ln_stats<T>(lp, sm); stats = true; }
-      dl_partial<T>(lp, sm, ns * kDlCols, ks * kDlRows, ks, wv);
+      if (lp.ln_gamma && !stats) { dl_ln_stats<T, 64 / Pack<T>::N>(lp, sm.st); stats = true; }
+      dl_partial<T>(lp, sm, ns * kDlCols, ks, per, wv);
     }
   };
   // y = round(sum of partials + bias + residual) over the grid
-  auto finish_rows = [&](const DecodeLinearParams& lp, int k_slabs) {
+  auto finish_rows = [&](const DecodeLinearParams& lp, int shares) {
     T* Y = reinterpret_cast<T*>(lp.y);
     for (int i = cta * kDlThreads + threadIdx.x; i < lp.m * lp.n; i += G * kDlThreads) {
       const int m = i / lp.n, c = i % lp.n;
-      Y[(long long)m * lp.y_row + c] = Cvt<T>::from(dl_finish_element<T>(lp, k_slabs, m, c));
+      Y[(long long)m * lp.y_row + c] = Cvt<T>::from(dl_finish_element<T>(lp, shares, m, c));
     }
   };
 
@@ -589,7 +867,10 @@ __global__ void __launch_bounds__(kDlThreads, 2) decode_layers_kernel(const Mega
       __syncthreads();
       T* kc = reinterpret_cast<T*>(w.kcache) + ((long long)b * p.heads + h) * (long long)p.t_max * 64;
       T* vc = reinterpret_cast<T*>(w.vcache) + ((long long)b * p.heads + h) * (long long)p.t_max * 64;
-      attn_decode_item<T>(s_qkv, kc, vc, reinterpret_cast<T*>(p.att) + (long long)b * D + h * 64, *p.len_ptr, p.t_max, p.scale, s_scores, asm_);
+      const int len = attn_decode_len(*p.len_ptr, p.t_max);
+      AttnDecodeRegs<T> pre;
+      attn_decode_fetch<T>(kc, vc, len, pre);
+      attn_decode_item<T>(s_qkv, kc, vc, reinterpret_cast<T*>(p.att) + (long long)b * D + h * 64, len, p.scale, s_scores, asm_, pre);
     }
     if (!mega_barrier(p, target)) return;
     // P3: att @ W_proj, then x2 = x + that + bias
@@ -610,7 +891,7 @@ __global__ void __launch_bounds__(kDlThreads, 2) decode_layers_kernel(const Mega
     if (!mega_barrier(p, target)) return;
     // P5: gelu(P4 + bias) @ W_fc2, then x = x2 + that + bias
     lp = DecodeLinearParams{};
-    lp.x = nullptr; lp.xp = part_fc; lp.xp_slabs = ks_d; lp.xp_bias = w.b_fc; lp.xp_act = (int)Act::GeluTanh;
+    lp.x = nullptr; lp.xp = part_fc; lp.xp_shares = ks_d; lp.xp_bias = w.b_fc; lp.xp_act = (int)Act::GeluTanh;
     lp.w = w.w_fc2; lp.m = B; lp.n = D; lp.k = 4 * D; lp.x_row = 4 * D; lp.w_row = D; lp.y_row = D; lp.partial = part_fc2;
     linear_partials(lp);
     if (l + 1 < p.n_layer) prefetch(p.layers[l + 1].w_qkv, 3 * D, D);
@@ -627,14 +908,14 @@ Status decode_layers(cudaStream_t s, DType dt, const void* layers, int n_layer, 
   if (batch < 1 || batch > kDlMaxM || d != heads * 64 || d % 8 != 0 || t_max < 1 || t_max > 8192) return Status::invalid("decode_layers: shape not supported");
   float* partial = skinny_partials();
   if (!partial) return Status::compute("decode_layers: the kernel workspace is not initialised");
-  const long long ks_d = (d + kDlRows - 1) / kDlRows, ks_4d = (4 * d + kDlRows - 1) / kDlRows;
+  const long long ks_d = dl_shares(d), ks_4d = dl_shares(4 * d);
   const long long need = (ks_d * kDlMaxM * 3 * d) + (ks_d * kDlMaxM * d) + (ks_d * kDlMaxM * 4 * d) + (ks_4d * kDlMaxM * d);
   if (need > ((long long)1 << 18) * 16) return Status::invalid("decode_layers: the partial sums do not fit the workspace");
   MegaParams p;
   p.layers = static_cast<const MegaLayerW*>(layers); p.n_layer = n_layer; p.heads = heads; p.d = d; p.t_max = t_max; p.batch = batch;
   p.wte = wte; p.wpe = wpe; p.tok = tok; p.pos = pos; p.len_ptr = len_ptr; p.x = x; p.x2 = x2; p.att = att;
   p.partial = partial; p.bar = bar; p.err = err; p.scale = 1.0f / sqrtf(64.0f);
-  // 42 KB of static shared memory leave ~5 KB of the default 48 KB for the scores: longer caches need the opt-in (set
+  // 47 KB of static shared memory leave next to nothing of the default 48 KB for the scores: longer caches need the opt-in (set
   // on the first, uncaptured call)
   static bool attr_set = false;
   if (!attr_set) {

@@ -242,3 +242,19 @@ def test_layer_norm_folded_into_the_linears_matches_the_layer_norm_kernels(gpu_d
         for other in (again, taped, replayed):
             assert np.array_equal(other, got), (dtype, float(np.max(np.abs(other - got))) / scale)
     assert gpu_dev.pipeline_status() == 0
+
+
+@pytest.mark.parametrize("heads,batch,dtype", [(5, 3, "float16"), (5, 16, "bfloat16"), (21, 9, "bfloat16"), (21, 2, "float16"), (5, 9, "float32"), (21, 16, "float32")])
+def test_decode_linears_at_the_edges_of_their_shares(gpu_dev, heads, batch, dtype):
+    """Widths of 5 x 64 (a last slab of 64 rows, three shares) and 21 x 64 (two and six slabs in a share, rows beyond 1024 for the
+    statistics), one and two groups of eight rows: the step replayed, issued launch by launch and as one persistent kernel adds in the
+    same order, so tokens are equal; the engine that keeps its cache by concatenation sums in another (and float32 rows beyond 1024
+    take their layer_norm in a launch of its own there)."""
+    cfg = {"n_layer": 2, "n_head": heads, "n_embd": 64 * heads, "vocab_size": 300, "n_positions": 320}
+    m = gpu_dev.init_gpt2_weights(cfg, seed=heads + batch, dtype=dtype)
+    ids = np.random.default_rng(batch).integers(0, 300, (batch, 250))
+    out = {e: gpu_dev.greedy_generate(m, ids, max_tokens=16, use_cache=True, engine=e) for e in ("graph", "direct", "persistent", "tape")}
+    assert out["graph"].tolist() == out["direct"].tolist() == out["persistent"].tolist()
+    new = out["graph"][:, 250:]
+    assert np.array_equal(new, out["tape"][:, 250:]) if dtype == "float32" else np.mean(new == out["tape"][:, 250:]) >= 0.85
+    assert gpu_dev.pipeline_status() == 0
