@@ -32,6 +32,21 @@ def padded(parts):
 
 
 # ── norms and the feed-forward activation ───────────────────────────────────
+@pytest.mark.parametrize("width", [4, 508, 1020, 1024, 1028, 2044, 2048, 2052, 4100])
+def test_rms_add_where_a_row_fits_the_registers(gpu_dev, width):
+    """Both sides of the widths (1024, 2048, 4096) at which the kernel changes, and rows that end inside a block's last access. float32 sums
+    of `width` squares: 1e-6 of the largest entry, as for the other widths."""
+    rng = np.random.default_rng(width)
+    x, y = rng.standard_normal((3, width)).astype(np.float32), rng.standard_normal((3, width)).astype(np.float32)
+    post, w = rng.standard_normal(width).astype(np.float32), rng.standard_normal(width).astype(np.float32)
+    g = gpu_dev
+    gx = g.from_numpy(x)
+    got = g.rms_add(gx, g.from_numpy(y), g.from_numpy(post), g.from_numpy(w), eps=2e-3, dtype="float32").to_numpy()
+    s = x + R.rms_norm(y.astype(np.float64), post, 2e-3)
+    assert rel(gx.to_numpy(), s) < 1e-6
+    assert rel(got, R.rms_norm(s, w, 2e-3)) < 1e-6
+
+
 @pytest.mark.parametrize("rows,width", [(1, 24), (5, 33), (40, 200), (3, 1024), (2, 9000)])
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_rms_add(gpu_dev, rows, width, dtype):
