@@ -91,36 +91,51 @@ __global__ void __launch_bounds__(256) grouped_decode_kernel(const GaParams p, i
   const int split = (int)sm100::cluster_ctarank(), splits = (int)gridDim.x;
   const int kh = (int)blockIdx.y / p.h_parts, part = (int)blockIdx.y % p.h_parts, h0 = kh * p.group + part * p.hg, nh = min(p.hg, p.group - part * p.hg);
   const int r = blockIdx.z, s = r / p.T, t = r % p.T, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  pdl_wait();
-  pdl_trigger();
-  const int last = min(p.pos[s] + t + 1, p.max_len), from = p.window ? max(0, last - p.window) : 0;
+  // Positions and the rows below them are older than the launch before this one, which has appended this portion's rows and waited for
+  // its own predecessor ahead of letting this one start: they are read before the dependency wait.
+  const int old_rows = p.pos[s], last = min(old_rows + t + 1, p.max_len), from = p.window ? max(0, last - p.window) : 0;
   const int per = ((last - from + splits - 1) / splits + 7) / 8 * 8;
   const int k_lo = min(last, from + split * per), k_hi = min(last, k_lo + per);
   const T* Q = reinterpret_cast<const T*>(p.proj) + (long long)r * p.ld + p.q_off + (long long)h0 * p.dim;
   const T* K = reinterpret_cast<const T*>(p.cache) + (long long)s * p.seq_stride + (long long)kh * p.dim;
   const T* V = reinterpret_cast<const T*>(p.cache) + (long long)s * p.seq_stride + p.v_col + (long long)kh * p.vdim;
+  const bool kvec = p.dim % N == 0, vvec = p.vdim % N == 0;        // rows of a head then start on 16 bytes
+  // rows k0 + [0, kGdKeys) that lie in [lo, hi) into shared memory: neighbouring lanes take a row's pieces
+  auto stage = [&](T* dst, int pitch, const T* src, int n, bool vec, int k0, int lo, int hi) {
+    if (vec) {
+      const int q = n / N, rows = 256 / q;                         // q <= 256 pieces where a head fits
+      const int j0 = q <= 256 ? (int)threadIdx.x / q : 0, c0 = q <= 256 ? (int)threadIdx.x % q : (int)threadIdx.x;
+      if (q <= 256 && j0 >= rows) return;
+      for (int j = j0; j < kGdKeys; j += q <= 256 ? rows : 1) {
+        if (k0 + j < lo || k0 + j >= hi) continue;
+        for (int c = c0; c < q; c += q <= 256 ? q : 256)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sm100::smem_u32(dst + j * pitch + c * N)), "l"(src + (long long)(k0 + j) * p.cld + c * N));
+      }
+    } else {
+      const int q = (n + N - 1) / N * N;
+      for (int i = threadIdx.x; i < kGdKeys * q; i += 256) {
+        const int j = i / q, c = i % q;
+        if (k0 + j >= lo && k0 + j < hi) dst[j * pitch + c] = c < n ? src[(long long)(k0 + j) * p.cld + c] : Cvt<T>::from(0.f);
+      }
+    }
+  };
+  auto stage_both = [&](int k0, int lo, int hi) { stage(sk, kp, K, p.dim, kvec, k0, lo, hi); stage(sv, vp, V, p.vdim, vvec, k0, lo, hi); };
+  stage_both(k_lo, k_lo, min(k_hi, old_rows));
+  pdl_wait();
+  pdl_trigger();
   for (int i = threadIdx.x; i < p.hg * kp; i += 256) { const int hh = i / kp, c = i % kp; sq[i] = hh < nh && c < p.dim ? Cvt<T>::to(Q[(long long)hh * p.dim + c]) * p.scale : 0.f; }
   if (threadIdx.x < p.hg) { s_m[threadIdx.x] = -INFINITY; s_l[threadIdx.x] = 0.f; }
   float acc[NO];
 #pragma unroll
   for (int n = 0; n < NO; n++) acc[n] = 0.f;
   const int outs = nh * p.vdim;
-  const bool kvec = p.dim % N == 0, vvec = p.vdim % N == 0;        // rows of a head then start on 16 bytes
   const int kpacks = (p.dim + N - 1) / N;
   for (int k0 = k_lo; k0 < k_hi; k0 += kGdKeys) {
     const int nk = min(kGdKeys, k_hi - k0);
-    __syncthreads();
-    auto stage = [&](T* dst, int pitch, const T* src, int n, bool vec) {
-      if (vec) {
-        const int q = n / N;
-        for (int i = threadIdx.x; i < nk * q; i += 256) st16(dst + i / q * pitch + i % q * N, ld16(src + (long long)(k0 + i / q) * p.cld + i % q * N));
-      } else {
-        const int q = (n + N - 1) / N * N;
-        for (int i = threadIdx.x; i < nk * q; i += 256) dst[i / q * pitch + i % q] = i % q < n ? src[(long long)(k0 + i / q) * p.cld + i % q] : Cvt<T>::from(0.f);
-      }
-    };
-    stage(sk, kp, K, p.dim, kvec);
-    stage(sv, vp, V, p.vdim, vvec);
+    if (k0 != k_lo) __syncthreads();
+    stage_both(k0, k0 == k_lo ? max(k0, old_rows) : k0, k_hi);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     const int key = threadIdx.x & (kGdKeys - 1);
     for (int hh = threadIdx.x / kGdKeys; hh < nh; hh += 256 / kGdKeys) {
