@@ -254,6 +254,9 @@ static Status key_decay_step(cudaStream_t s, DType dt, const KdParams& p) {
     const int most = 32 * vec;
     *ranks = 1;
     while (*ranks < 8 && (p.vdim + *ranks - 1) / *ranks > most) *ranks *= 2;
+    // As long as SMs are idle a CTA's time is the number of its columns and what every CTA of the head repeats. Rurunex of width 1024, eight
+    // sequences (64 CTAs before, 128 now): 19.06 -> 18.48 ms for 1024 + 48 tokens.
+    while (*ranks < 8 && p.vdim / *ranks >= 64 && 2 * *ranks * p.heads * p.n_seq <= sm_count()) *ranks *= 2;
     *slice = ((p.vdim + *ranks - 1) / *ranks + vec - 1) / vec * vec;
     *tx_n = 4;
     while (*tx_n < 32 && *tx_n * vec < *slice) *tx_n *= 2;
