@@ -317,8 +317,10 @@ __device__ __forceinline__ ArgPair arg_better(ArgPair a, ArgPair b) {
   if (b.v > a.v || (b.v == a.v && b.i < a.i)) return b;
   return a;
 }
+// One block per row, whose time is its rounds of loads: long rows that leave SMs idle take blocks of 1024 threads (eight rows of 32768
+// floats in a step: 18.50 -> 18.34 ms for 49 steps, about 3 us a launch).
 template <typename T>
-__global__ void __launch_bounds__(256) argmax_kernel(const T* __restrict__ in, int32_t* __restrict__ out, int64_t rows, int64_t cols, int64_t row_stride) {
+__global__ void __launch_bounds__(1024) argmax_kernel(const T* __restrict__ in, int32_t* __restrict__ out, int64_t rows, int64_t cols, int64_t row_stride) {
   __shared__ float sv[32];
   __shared__ int si[32];
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -411,10 +413,11 @@ Status argmax(cudaStream_t s, const TView& in, const TView& out) {
   }
   if (rows == 0) return Status::OK();
   int grid = (int)(rows < (int64_t)sm_count() * 8 ? rows : (int64_t)sm_count() * 8);
+  const int threads = rows <= sm_count() && cols >= 8192 ? 1024 : 256;
   switch (in.dtype) {
-    case DType::F32: argmax_kernel<float><<<grid, 256, 0, s>>>((const float*)in.ptr, (int32_t*)out.ptr, rows, cols, row_stride); break;
-    case DType::F16: argmax_kernel<__half><<<grid, 256, 0, s>>>((const __half*)in.ptr, (int32_t*)out.ptr, rows, cols, row_stride); break;
-    case DType::BF16: argmax_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)in.ptr, (int32_t*)out.ptr, rows, cols, row_stride); break;
+    case DType::F32: argmax_kernel<float><<<grid, threads, 0, s>>>((const float*)in.ptr, (int32_t*)out.ptr, rows, cols, row_stride); break;
+    case DType::F16: argmax_kernel<__half><<<grid, threads, 0, s>>>((const __half*)in.ptr, (int32_t*)out.ptr, rows, cols, row_stride); break;
+    case DType::BF16: argmax_kernel<__nv_bfloat16><<<grid, threads, 0, s>>>((const __nv_bfloat16*)in.ptr, (int32_t*)out.ptr, rows, cols, row_stride); break;
     case DType::I32: argmax_int_kernel<int32_t><<<(int)((rows + 127) / 128), 128, 0, s>>>((const int32_t*)in.ptr, (int32_t*)out.ptr, rows, cols); break;
     case DType::I64: argmax_int_kernel<int64_t><<<(int)((rows + 127) / 128), 128, 0, s>>>((const int64_t*)in.ptr, (int32_t*)out.ptr, rows, cols); break;
     case DType::U8: argmax_int_kernel<uint8_t><<<(int)((rows + 127) / 128), 128, 0, s>>>((const uint8_t*)in.ptr, (int32_t*)out.ptr, rows, cols); break;

@@ -404,3 +404,18 @@ def test_bf16_and_f16_bandwidth_ops(gpu_dev):
     assert np.mean(goth == refh) > 0.97 and np.max(np.abs(goth - refh) / np.maximum(np.abs(refh), 1e-3)) <= 2 ** -9
     got = gpu_dev.add_bias(up_bf16(gpu_dev, x), up_bf16(gpu_dev, g)).to_numpy()
     assert np.array_equal(got, R.from_bf16(R.add_bias(xb, gb, st=2)))
+
+
+@pytest.mark.parametrize("rows,cols", [(3, 8191), (3, 8192), (1, 50257), (8, 32768), (148, 8200), (149, 8200)])
+def test_argmax_of_long_rows(gpu_dev, rows, cols):
+    """Both sides of the sizes at which a row takes a larger block: the lowest index among equals, NaNs never, a NaN in front always."""
+    rng = np.random.default_rng(rows + cols)
+    x = rng.integers(-50, 50, (rows, cols)).astype(np.float32)
+    x[0, cols - 1] = 60
+    want = x.argmax(-1)
+    if rows > 2:
+        x[1, 7] = x[1, want[1] + 1 if want[1] + 1 < cols else 3] = np.nan
+        want[1] = np.nanargmax(x[1])
+        x[2, 0] = np.nan
+        want[2] = 0
+    assert np.array_equal(gpu_dev.argmax(gpu_dev.from_numpy(x)).to_numpy().reshape(-1), want)
