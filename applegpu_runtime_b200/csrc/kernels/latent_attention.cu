@@ -113,23 +113,25 @@ Status latent_append(cudaStream_t s, const LatentDesc& d) {
 // ── decode ──────────────────────────────────────────────────────────────────
 // A generated token has one row, so the work on a head's slices of W_uk and W_uv (dim or vdim times the rank) is cut into `cuts`
 // CTAs, which start their share towards the L2 before the dependency wait. Gedenex at width 2048, one sequence, prepare / attend / merge:
-// 7.5 / 12.0 / 8.7 us a launch in a step with one CTA per head, index divisions and no load ahead of the wait, 4.7 / 8.9 / 6.8 us now.
+// 7.5 / 12.0 / 8.7 us a launch in a step with one CTA per head, index divisions and no load ahead of the wait, 4.7 / 8.9 / 6.8 us with them (the
+// prepare kernel with other sums than today's, whose step is 0.4 % longer).
 __device__ __forceinline__ void la_prefetch(const void* at, int bytes) {
   for (int i = threadIdx.x * 128; i < bytes; i += 256 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t*>(at) + i));
 }
-// prepare: CTA h * cuts + c: the c-th part of the query of head h in cache-row coordinates, scaled: (q W_uk | 0 | rotated part | 0); the
-// last CTA appends the row to the cache.
-template <typename T>
-__global__ void __launch_bounds__(256) latent_decode_prepare_kernel(const LaParams p, int cuts) {
+// prepare: CTA h * CUTS + c: the c-th part of the query of head h in cache-row coordinates, scaled: (q W_uk | 0 | rotated part | 0); the
+// last CTA appends the row to the cache. A thread of a finer cut has fewer columns of the same rows of W_uk, so a sequence's query
+// has the same bits however many rows, and hence CTAs per head, a call has.
+template <typename T, int V> struct alignas(V * sizeof(T)) LaPart { T v[V]; };
+template <typename T, int CUTS>
+__global__ void __launch_bounds__(256) latent_decode_prepare_kernel(const LaParams p) {
   extern __shared__ __align__(16) float sq[];            // [dim]
   __shared__ float red[33];
-  constexpr int N = Pack<T>::N;
-  const int h = blockIdx.x / cuts, cut = blockIdx.x % cuts, r = blockIdx.y, s = r / p.T, t = r % p.T;
-  // this CTA's 16-byte pieces of a row of W_uk
-  const int all = p.coff / N, each = (all + cuts - 1) / cuts, v0 = cut * each, nv = min(each, all - v0);
-  const T* uk = reinterpret_cast<const T*>(p.uk) + (long long)min(h, p.heads - 1) * p.dim * p.w_ld + v0 * N;
-  if (h < p.heads && nv > 0) {
-    const int lines = (nv * 16 + 127) / 128;
+  constexpr int V = Pack<T>::N / CUTS;                   // columns of a thread
+  const int h = blockIdx.x / CUTS, cut = blockIdx.x % CUTS, r = blockIdx.y, s = r / p.T, t = r % p.T;
+  const int nv = p.coff / Pack<T>::N, v0 = cut * nv * V; // this CTA's columns of W_uk: nv * V from v0 on
+  const T* uk = reinterpret_cast<const T*>(p.uk) + (long long)min(h, p.heads - 1) * p.dim * p.w_ld + v0;
+  if (h < p.heads) {
+    const int lines = (nv * V * (int)sizeof(T) + 127) / 128;
     for (int d = threadIdx.x / lines; d < p.dim; d += 256 / lines)
       if (threadIdx.x < 256 / lines * lines) asm volatile("prefetch.global.L2 [%0];" ::"l"(uk + (long long)d * p.w_ld + threadIdx.x % lines * (128 / (int)sizeof(T))));
   }
@@ -157,30 +159,30 @@ __global__ void __launch_bounds__(256) latent_decode_prepare_kernel(const LaPara
     }
   }
   __syncthreads();
-  if (nv <= 0) return;
-  // a thread owns one piece's columns and every G-th row, the G partial sums meet in shared memory
+  // a thread owns V columns and every G-th row, the G partial sums meet in shared memory
   float* part = sq + p.dim;
-  const int G = nv >= 256 ? 1 : 256 / nv, g = threadIdx.x / nv, col = threadIdx.x % nv;
+  const int G = nv >= 256 ? 1 : 256 / nv, g = threadIdx.x / nv, col = threadIdx.x % nv * V;
   if (g < G) {
-    float a[N];
+    float a[V];
 #pragma unroll
-    for (int e = 0; e < N; e++) a[e] = 0.f;
-#pragma unroll 8
+    for (int e = 0; e < V; e++) a[e] = 0.f;
+    constexpr int U = 8 * CUTS;                          // the same bytes in flight
+#pragma unroll U
     for (int d = g; d < p.dim; d += G) {
-      const Pack<T> w = ld16(uk + (long long)d * p.w_ld + col * N);
+      const LaPart<T, V> w = *reinterpret_cast<const LaPart<T, V>*>(uk + (long long)d * p.w_ld + col);
       const float x = sq[d];
 #pragma unroll
-      for (int e = 0; e < N; e++) a[e] = fmaf(x, Cvt<T>::to(w.v[e]), a[e]);
+      for (int e = 0; e < V; e++) a[e] = fmaf(x, Cvt<T>::to(w.v[e]), a[e]);
     }
 #pragma unroll
-    for (int e = 0; e < N; e++) part[(g * nv + col) * N + e] = a[e];
+    for (int e = 0; e < V; e++) part[g * nv * V + col + e] = a[e];
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < nv * N; i += 256) {
+  for (int i = threadIdx.x; i < nv * V; i += 256) {
     float a = 0.f;
 #pragma unroll 4
-    for (int k = 0; k < G; k++) a += part[k * nv * N + i];
-    out[v0 * N + i] = v0 * N + i < p.rank ? a * p.scale : 0.f;
+    for (int k = 0; k < G; k++) a += part[k * nv * V + i];
+    out[v0 + i] = v0 + i < p.rank ? a * p.scale : 0.f;
   }
 }
 
@@ -520,7 +522,9 @@ static cudaError_t latent_decode_t(cudaStream_t s, const LaParams& p) {
   const size_t psmem = ((size_t)p.dim + 256 * Pack<T>::N) * sizeof(float);
   int cuts = 1;                                            // CTAs per head and row: as many as an SM each, at most four
   while (cuts < 4 && 2 * cuts * p.heads * rows <= sm_count()) cuts *= 2;
-  cudaError_t e = launch_pdl(latent_decode_prepare_kernel<T>, dim3((unsigned)(p.heads * cuts + 1), (unsigned)rows), dim3(256), psmem, s, p, cuts);
+  const dim3 pgrid((unsigned)(p.heads * cuts + 1), (unsigned)rows);
+  cudaError_t e = cuts == 4 ? launch_pdl(latent_decode_prepare_kernel<T, 4>, pgrid, dim3(256), psmem, s, p)
+                  : cuts == 2 ? launch_pdl(latent_decode_prepare_kernel<T, 2>, pgrid, dim3(256), psmem, s, p) : launch_pdl(latent_decode_prepare_kernel<T, 1>, pgrid, dim3(256), psmem, s, p);
   if (e != cudaSuccess) return e;
   bool done = false;
   if constexpr (sizeof(T) == 2) {

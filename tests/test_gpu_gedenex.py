@@ -207,6 +207,21 @@ def test_latent_attention_forms_and_portions(gpu_dev, size, dtype):
     assert g.pipeline_status() == 0
 
 
+@pytest.mark.parametrize("size", range(len(LATENT_SIZES)))
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+def test_latent_step_has_the_same_bits_alone_and_in_a_batch(gpu_dev, size, dtype):
+    """Few rows leave SMs idle and a head's slice of W_uk then takes up to four CTAs; 32 cached rows are one share of the keys in any batch."""
+    g, z = gpu_dev, LATENT_SIZES[size]
+    c = latent_case(g, 4, 160, z, dtype, 30 + size, 32)
+    out = []
+    for n in (160, 1, 20, 50):
+        few, cache = dict(c, B=n, proj=c["proj"][:n]), new_cache(g, dict(c, B=n))
+        out.append(np.concatenate([latent_run(g, few, t, t + 1, cache, "latent") for t in range(4)], axis=1))
+    for y in out[1:]:
+        assert np.array_equal(y, out[0][:len(y)])
+    assert rel(out[0][0], latent_want(c, 0, 4)) < {"float32": 3e-5, "float16": 4e-3, "bfloat16": 2e-2}[dtype]
+
+
 @pytest.mark.parametrize("form", ["expanded", "latent", "tensor"])
 @pytest.mark.parametrize("key,query", [(0, 299), (63, 299), (64, 128), (127, 128), (128, 128), (191, 255), (255, 256), (200, 201), (299, 299)])
 def test_latent_attention_far_key(gpu_dev, form, key, query):
