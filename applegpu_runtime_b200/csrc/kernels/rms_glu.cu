@@ -136,7 +136,8 @@ __global__ void __launch_bounds__(kRmsThreads) rms_rows_kernel(const RmsParams p
 // The same for rows that fit the registers, in 16-byte pieces (the kernel above takes what is wider or lies otherwise): every operand of
 // the row is asked for at once and read once. A generated token has one block per sequence, whose time is its chain of round trips (two of
 // them and two sums, where the kernel above has four); a prompt is bound by memory, 14 bytes per element with `post`.
-// 1024 columns, 8 rows: 5.1 -> 3.0 us a launch in a step; 8192 rows of 2048 with `post`: 56 -> 54 us.
+// 1024 columns, 8 rows: 5.1 -> 3.0 us a launch in a step; 8192 rows of 2048 with `post`: 56 -> 54 us. It adds in the order of the kernel
+// above: which of the two a row takes (an unaligned weight, say) does not show in its bits.
 template <typename T, int NREG>
 __global__ void __launch_bounds__(kRmsThreads) rms_row_kernel(const __grid_constant__ RmsParams p) {
   constexpr int W = kRmsThreads / 32;
@@ -149,10 +150,8 @@ __global__ void __launch_bounds__(kRmsThreads) rms_row_kernel(const __grid_const
     v = warp_sum(v);
     if ((threadIdx.x & 31) == 0) at[threadIdx.x >> 5] = v;
     __syncthreads();
-    float t = 0.f;
-#pragma unroll
-    for (int w = 0; w < W; w++) t += at[w];
-    return t;
+    static_assert(W == 4, "the order in which block_sum adds four warps");
+    return (at[0] + at[2]) + (at[1] + at[3]);
   };
   auto piece = [&](const float* base, int it) {
     const int i = threadIdx.x + it * kRmsThreads;

@@ -47,6 +47,20 @@ def test_rms_add_where_a_row_fits_the_registers(gpu_dev, width):
     assert rel(got, R.rms_norm(s, w, 2e-3)) < 1e-6
 
 
+@pytest.mark.parametrize("width", [4, 512, 1020, 1024, 1028, 2048])
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+def test_rms_add_has_the_same_bits_in_either_kernel(gpu_dev, width, dtype):
+    """A weight that does not lie on 16 bytes takes the kernel for rows of any kind: same stream, same outputs."""
+    g, rng = gpu_dev, np.random.default_rng(width)
+    x, y = rng.standard_normal((2, 40, width)).astype(np.float32)
+    post, w = rng.standard_normal((2, width)).astype(np.float32)
+    out = []
+    for off in (0, 1):
+        gx, gw = g.from_numpy(x), g.slice(g.from_numpy(np.concatenate([np.zeros(off, np.float32), w])), 0, off, off + width)
+        out.append((g.rms_add(gx, g.from_numpy(y), g.from_numpy(post), gw, eps=2e-3, dtype=dtype).to_numpy(), gx.to_numpy()))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
 @pytest.mark.parametrize("rows,width", [(1, 24), (5, 33), (40, 200), (3, 1024), (2, 9000)])
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_rms_add(gpu_dev, rows, width, dtype):
