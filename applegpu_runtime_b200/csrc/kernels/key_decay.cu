@@ -4,6 +4,9 @@
 // sums of squares over distributed shared memory). With r = (diag(a) S)^T k and p = (diag(a) S)^T q taken in one pass over S, the
 // rest of a token is u = beta (v - r) (or v), o = p + (k . q) u and the update S <- diag(a) S + k u^T, which is the order of the
 // recurrence (o includes what the token itself wrote). S stays in registers from token to token where the CTA's columns fit.
+// While SMs are idle a group of 128 columns is cut again, into up to four CTAs whose threads have two columns, or one, in place of four:
+// the rows a thread adds up and the order in which its neighbours' sums and the norm's squares meet stay, so a sequence's bits do not
+// depend on how many others are in the call.
 #include "key_decay.cuh"
 #include "sm100.cuh"
 #include <algorithm>
@@ -36,14 +39,19 @@ __device__ __forceinline__ void kd_rows(const T* w, int ld, int rank, const floa
     if (i < n && lane == 0) out[i] = a;
   }
 }
+__device__ __forceinline__ float kd_peer(const float* at, int rank) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(sm100::mapa_u32(sm100::smem_u32(at), (uint32_t)rank)));
+  return v;
+}
 __device__ __forceinline__ void kd_prefetch(const void* at, int bytes) {
   for (int i = threadIdx.x * 128; i < bytes; i += kKsThreads * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t*>(at) + i));
 }
 
 template <typename T, int VEC, int NR>          // NR rows of S per thread, VEC neighbouring columns of each
-__global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_step_kernel(const KdParams p, int slice, int tx_n) {
+__global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_step_kernel(const KdParams p, int slice, int tx_n, int sub) {      // sub: CTAs of one group of columns
   extern __shared__ __align__(16) float sm[];
-  __shared__ float s_sq[2];
+  __shared__ float s_sq[2], s_group[8];
   const int D = p.dim, E = p.vdim, cw = tx_n * VEC;       // cw: columns of a pass
   const int rank = (int)sm100::cluster_ctarank(), n_rank = (int)gridDim.x;
   const int h = blockIdx.y, s = blockIdx.z, qh = h / p.group;
@@ -56,8 +64,8 @@ __global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_
   float* sa = sk + D;
   float* sv = sa + D;                    // [slice] each
   float* sg = sv + slice;
-  float* so = sg + slice;
-  float* sx = so + slice;                // a1 and g1 of the token, padded with zeros to whole packs
+  float* so_all = sg + slice;            // two of them where peers read the values: one may still be at the previous token's
+  float* sx = so_all + (sub > 1 ? 2 : 1) * slice;      // a1 and g1 of the token, padded with zeros to whole packs
   float* sy = sx + p.a_ld;
   // weights start towards the L2 before the previous kernel is waited for
   kd_prefetch(p.bias + h * D, D * 4);
@@ -83,6 +91,9 @@ __global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_
       if constexpr (VEC == 4) {
         const float4 f = in ? *reinterpret_cast<const float4*>(at) : make_float4(0.f, 0.f, 0.f, 0.f);
         st[n][0] = f.x; st[n][1] = f.y; st[n][2] = f.z; st[n][3] = f.w;
+      } else if constexpr (VEC == 2) {
+        const float2 f = in ? *reinterpret_cast<const float2*>(at) : make_float2(0.f, 0.f);
+        st[n][0] = f.x; st[n][1] = f.y;
       } else st[n][0] = in ? *at : 0.f;
     }
   };
@@ -92,6 +103,7 @@ __global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_
     for (int n = 0; n < NR; n++, at += step) {
       if (n * ty_n + ty >= D || c >= ne) continue;
       if constexpr (VEC == 4) *reinterpret_cast<float4*>(at) = make_float4(st[n][0], st[n][1], st[n][2], st[n][3]);
+      else if constexpr (VEC == 2) *reinterpret_cast<float2*>(at) = make_float2(st[n][0], st[n][1]);
       else *at = st[n][0];
     }
   };
@@ -101,6 +113,7 @@ __global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_
   T* ring = p.ring_of<T>(s);
   const float rate = p.softplus ? p.rate[h] : 0.f;
   for (int t = 0; t < p.T; t++) {
+    float* so = so_all + (sub > 1 && (t & 1) ? slice : 0);
     const T* row = base + (long long)t * p.ld;
     const long long r = (long long)s * p.T + t;
     const float beta_raw = p.delta ? p.beta[r * p.beta_ld + h] : 0.f;
@@ -166,6 +179,9 @@ __global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_
       if constexpr (VEC == 4) {
         *reinterpret_cast<float4*>(part + threadIdx.x * 4) = make_float4(rk[0], rk[1], rk[2], rk[3]);
         *reinterpret_cast<float4*>(part + (kKsThreads + threadIdx.x) * 4) = make_float4(rq[0], rq[1], rq[2], rq[3]);
+      } else if constexpr (VEC == 2) {
+        *reinterpret_cast<float2*>(part + threadIdx.x * 2) = make_float2(rk[0], rk[1]);
+        *reinterpret_cast<float2*>(part + (kKsThreads + threadIdx.x) * 2) = make_float2(rq[0], rq[1]);
       } else { part[threadIdx.x] = rk[0]; part[kKsThreads + threadIdx.x] = rq[0]; }
       __syncthreads();
       for (int i = threadIdx.x; i < 2 * cw; i += kKsThreads) {
@@ -197,18 +213,36 @@ __global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_
     }
     __syncthreads();
     float ss = 0.f;
-    for (int i = lane; i < ne; i += 32) ss = fmaf(so[i], so[i], ss);
-    ss = warp_sum(ss);
-    if (n_rank > 1) {
-      if (threadIdx.x == 0) s_sq[t & 1] = ss;
-      sm100::cluster_sync_all();
-      float tot = 0.f;
-      for (int q = 0; q < n_rank; q++) {
-        float v;
-        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(sm100::mapa_u32(sm100::smem_u32(&s_sq[t & 1]), (uint32_t)q)));
-        tot += v;
+    if (sub == 1) {
+      for (int i = lane; i < ne; i += 32) ss = fmaf(so[i], so[i], ss);
+      ss = warp_sum(ss);
+      if (n_rank > 1) {
+        if (threadIdx.x == 0) s_sq[t & 1] = ss;
+        sm100::cluster_sync_all();
+        ss = 0.f;
+        for (int q = 0; q < n_rank; q++) ss += kd_peer(&s_sq[t & 1], q);
       }
-      ss = tot;
+    } else {                                              // a warp for a group, whose values lie in `sub` CTAs
+      sm100::cluster_sync_all();
+      const int groups = n_rank / sub, g = threadIdx.x >> 5, width = slice * sub;
+      if (g < groups) {
+        const int n = min(width, E - g * width);
+        for (int i0 = lane; i0 < n; i0 += 128) {
+          float v[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const int i = i0 + j * 32, c = (i >= slice) + (i >= 2 * slice) + (i >= 3 * slice);
+            v[j] = i < n ? kd_peer(so + i - c * slice, g * sub + c) : 0.f;
+          }
+#pragma unroll
+          for (int j = 0; j < 4; j++) ss = fmaf(v[j], v[j], ss);
+        }
+        ss = warp_sum(ss);
+        if (lane == 0) s_group[g] = ss;
+      }
+      __syncthreads();
+      ss = 0.f;
+      for (int q = 0; q < groups; q++) ss += s_group[q];
     }
     const float rs = 1.0f / sqrtf(ss / (float)E + p.eps);
     T* y = reinterpret_cast<T*>(p.y) + r * p.y_ld + h * E + e0;
@@ -232,7 +266,7 @@ __global__ void __launch_bounds__(256) key_decay_tail_kernel(const KdParams p) {
 }
 
 template <typename T, int VEC, int NR>
-static cudaError_t launch_ks(cudaStream_t s, const KdParams& p, int ranks, int slice, int tx_n, size_t smem) {
+static cudaError_t launch_ks(cudaStream_t s, const KdParams& p, int ranks, int slice, int tx_n, int sub, size_t smem) {
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(key_decay_step_kernel<T, VEC, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
@@ -245,7 +279,7 @@ static cudaError_t launch_ks(cudaStream_t s, const KdParams& p, int ranks, int s
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   at[1].id = cudaLaunchAttributeClusterDimension; at[1].val.clusterDim.x = (unsigned)ranks; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
   cfg.attrs = at; cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, key_decay_step_kernel<T, VEC, NR>, p, slice, tx_n);
+  return cudaLaunchKernelEx(&cfg, key_decay_step_kernel<T, VEC, NR>, p, slice, tx_n, sub);
 }
 
 static Status key_decay_step(cudaStream_t s, DType dt, const KdParams& p) {
@@ -254,9 +288,6 @@ static Status key_decay_step(cudaStream_t s, DType dt, const KdParams& p) {
     const int most = 32 * vec;
     *ranks = 1;
     while (*ranks < 8 && (p.vdim + *ranks - 1) / *ranks > most) *ranks *= 2;
-    // As long as SMs are idle a CTA's time is the number of its columns and what every CTA of the head repeats. Rurunex of width 1024, eight
-    // sequences (64 CTAs before, 128 now): 19.06 -> 18.48 ms for 1024 + 48 tokens.
-    while (*ranks < 8 && p.vdim / *ranks >= 64 && 2 * *ranks * p.heads * p.n_seq <= sm_count()) *ranks *= 2;
     *slice = ((p.vdim + *ranks - 1) / *ranks + vec - 1) / vec * vec;
     *tx_n = 4;
     while (*tx_n < 32 && *tx_n * vec < *slice) *tx_n *= 2;
@@ -264,13 +295,18 @@ static Status key_decay_step(cudaStream_t s, DType dt, const KdParams& p) {
   };
   int ranks, slice, tx_n, vec = 4, nr = shape(4, &ranks, &slice, &tx_n);
   if (p.vdim % 4 || nr > 16) { vec = 1; nr = shape(1, &ranks, &slice, &tx_n); }
-  const size_t smem = (2 * (size_t)kKsThreads * vec + 2 * (size_t)tx_n * vec + 3 * (size_t)p.dim + 3 * (size_t)slice + p.a_ld + p.g_ld) * sizeof(float);
+  // As long as SMs are idle a CTA's time is the number of its columns and what every CTA of the head repeats. Rurunex of width 1024, eight
+  // sequences (64 CTAs before, 128 now): 19.06 -> 18.48 ms for 1024 + 48 tokens.
+  int sub = 1;
+  while (vec > 1 && ranks < 8 && p.vdim / ranks >= 64 && 2 * ranks * p.heads * p.n_seq <= sm_count()) { ranks *= 2; sub *= 2; slice /= 2; vec /= 2; }
+  const size_t smem = (2 * (size_t)kKsThreads * vec + 2 * (size_t)tx_n * vec + 3 * (size_t)p.dim + (sub > 1 ? 4 : 3) * (size_t)slice + p.a_ld + p.g_ld) * sizeof(float);
   if (nr > 32 || smem > 100 * 1024) return Status::unsupported("key decay: head too large");
   cudaError_t e = cudaSuccess;
   AG_DISPATCH_FLOAT(dt, T, {
-    if (vec == 4) e = nr <= 2 ? launch_ks<T, 4, 2>(s, p, ranks, slice, tx_n, smem) : nr <= 4 ? launch_ks<T, 4, 4>(s, p, ranks, slice, tx_n, smem)
-                    : nr <= 8 ? launch_ks<T, 4, 8>(s, p, ranks, slice, tx_n, smem) : launch_ks<T, 4, 16>(s, p, ranks, slice, tx_n, smem);
-    else e = nr <= 8 ? launch_ks<T, 1, 8>(s, p, ranks, slice, tx_n, smem) : launch_ks<T, 1, 32>(s, p, ranks, slice, tx_n, smem);
+    if (vec == 4) e = nr <= 2 ? launch_ks<T, 4, 2>(s, p, ranks, slice, tx_n, sub, smem) : nr <= 4 ? launch_ks<T, 4, 4>(s, p, ranks, slice, tx_n, sub, smem)
+                    : nr <= 8 ? launch_ks<T, 4, 8>(s, p, ranks, slice, tx_n, sub, smem) : launch_ks<T, 4, 16>(s, p, ranks, slice, tx_n, sub, smem);
+    else if (vec == 2) e = nr <= 8 ? launch_ks<T, 2, 8>(s, p, ranks, slice, tx_n, sub, smem) : launch_ks<T, 2, 16>(s, p, ranks, slice, tx_n, sub, smem);
+    else e = nr <= 8 ? launch_ks<T, 1, 8>(s, p, ranks, slice, tx_n, sub, smem) : launch_ks<T, 1, 32>(s, p, ranks, slice, tx_n, sub, smem);
   });
   return cuda_status(e, "key decay step");
 }

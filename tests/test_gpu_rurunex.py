@@ -177,6 +177,22 @@ def test_key_decay_portions(gpu_dev, name, dtype, form):
     assert gpu_dev.pipeline_status() == 0
 
 
+@pytest.mark.parametrize("name", ["delta_128", "gla_wide", "delta_values_200", "delta_96", "gla_odd"])
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+def test_key_decay_steps_have_the_same_bits_alone_and_in_a_batch(gpu_dev, name, dtype):
+    """Few sequences leave SMs idle and a head then takes more CTAs: up to eight, down to 32 value columns each. Outputs and states of a
+    sequence stay what they are in a batch that fills the chip, and right (the bars of test_key_decay_portions)."""
+    c = kd_case(KD_CASES[name], 19, 100, seed=5, decay=-1.0 if KD_CASES[name]["softplus"] else 2.0)
+    cuts = [1, 1, 16, 1]
+    got, S = kd_run(gpu_dev, c, cuts, dtype, "steps")
+    for n in (1, 3, 16, 50):
+        few = dict(c, B=n, **{x: c[x][:n] for x in ("q", "k", "v", "a1", "g", "beta")})
+        y, state = kd_run(gpu_dev, few, cuts, dtype, "steps")
+        assert np.array_equal(y, got[:n]) and np.array_equal(state, S[:n])
+    want, state = kd_want(c, 0)
+    assert rel(S[0], state) < (2e-5 if dtype == "float32" else 2e-4) and rel(got[0], want) < {"float32": 1e-4, "float16": 4e-3, "bfloat16": 2e-2}[dtype]
+
+
 @pytest.mark.parametrize("kind", ["gla", "delta"])
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("where", [0, 1, 7, 8, 15, 16, 31, 32, 63, 96, 288])
