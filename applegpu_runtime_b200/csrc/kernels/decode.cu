@@ -249,7 +249,7 @@ __device__ __forceinline__ void dl_load_weights(const DecodeLinearParams& p, int
 
 // Row statistics of layer_norm over the whole rows of x: a warp per row, the row in registers after one round of
 // 16-byte loads (kernel_templates.rs:1097-1109: mean, population variance, 1/sqrt(var + eps)). Ends with a block barrier.
-// IT: 32 x 16-byte rounds of a row at most (the persistent engine: 2048 columns of any type).
+// IT: 32 x 16-byte rounds of a row at most; what lies behind them would be left out.
 template <typename T, int IT = 8>
 __device__ __forceinline__ void dl_ln_stats(const DecodeLinearParams& p, DlStats& sm) {
   constexpr int N16 = Pack<T>::N;
@@ -727,6 +727,7 @@ Status decode_linear(cudaStream_t s, const GemmDesc& d) {
 // memset node before the launch; each CTA adds one and spins (bounded: 2 s, then an error word is set and every CTA
 // leaves at its next barrier) until the count reaches phases-so-far x CTAs. The launch is cooperative, so all CTAs
 // are resident and the spin cannot wait for a CTA that has not started.
+constexpr int kMegaCols = 2048;      // of a row at most: what the statistics of layer_norm keep in registers
 struct MegaLayerW {
   const void *ln1_g, *ln1_b, *w_qkv, *b_qkv, *w_proj, *b_proj, *ln2_g, *ln2_b, *w_fc, *b_fc, *w_fc2, *b_fc2;
   void *kcache, *vcache;
@@ -819,7 +820,7 @@ __global__ void __launch_bounds__(kDlThreads, 2) decode_layers_kernel(const Mega
         dl_load_weights<T>(lp, ns * kDlCols, ks * per * kDlRows, wv);
       }
       __syncthreads();                       // the previous item's shared-memory reads are done
-      if (lp.ln_gamma && !stats) { dl_ln_stats<T, 64 / Pack<T>::N>(lp, sm.st); stats = true; }
+      if (lp.ln_gamma && !stats) { dl_ln_stats<T, kMegaCols / (32 * Pack<T>::N)>(lp, sm.st); stats = true; }
       dl_partial<T>(lp, sm, ns * kDlCols, ks, per, wv);
     }
   };
@@ -905,6 +906,7 @@ __global__ void __launch_bounds__(kDlThreads, 2) decode_layers_kernel(const Mega
 Status decode_layers(cudaStream_t s, DType dt, const void* layers, int n_layer, int heads, int d, int t_max, int batch, const void* wte, const void* wpe,
                      const int32_t* tok, const int32_t* pos, const int* len_ptr, void* x, void* x2, void* att, unsigned int* bar, int* err) {
   if (batch < 1 || batch > kDlMaxM || d != heads * 64 || d % 8 != 0 || t_max < 1 || t_max > 8192) return Status::invalid("decode_layers: shape not supported");
+  if (d > kMegaCols) return Status::unsupported("decode_layers: rows of more than " + std::to_string(kMegaCols) + " columns");
   float* partial = skinny_partials();
   if (!partial) return Status::compute("decode_layers: the kernel workspace is not initialised");
   const long long ks_d = dl_shares(d), ks_4d = dl_shares(4 * d);

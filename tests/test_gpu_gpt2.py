@@ -258,3 +258,26 @@ def test_decode_linears_at_the_edges_of_their_shares(gpu_dev, heads, batch, dtyp
     new = out["graph"][:, 250:]
     assert np.array_equal(new, out["tape"][:, 250:]) if dtype == "float32" else np.mean(new == out["tape"][:, 250:]) >= 0.85
     assert gpu_dev.pipeline_status() == 0
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_persistent_decode_refuses_rows_beyond_its_statistics(gpu_dev, dtype):
+    """Its layer_norm keeps 2048 columns of a row: 32 heads give the step engine's tokens, 33 are refused and leave the step engine usable."""
+    from applegpu_runtime_b200.generate import Gpt2Decoder
+    for heads in (32, 33):
+        m = gpu_dev.init_gpt2_weights({"n_layer": 1, "n_head": heads, "n_embd": 64 * heads, "vocab_size": 300, "n_positions": 32}, seed=heads, dtype=dtype)
+        ids = np.random.default_rng(heads).integers(0, 300, (2, 9))
+        want = gpu_dev.greedy_generate(m, ids, max_tokens=8, engine="graph")
+        if heads == 32:
+            assert np.array_equal(gpu_dev.greedy_generate(m, ids, max_tokens=8, engine="persistent"), want)
+            continue
+        logits, kv = gpu_dev.gpt2_forward(m, ids, last_only=True)
+        dec = Gpt2Decoder(m, 2, 17)
+        dec.set_engine(persistent=True)
+        dec.prefill(kv, gpu_dev.argmax(logits), 9)
+        for graph in (True, False):
+            with pytest.raises(ValueError, match="2048 columns"):
+                dec.steps(7, use_graph=graph)
+        dec.set_engine(persistent=False)
+        assert np.array_equal(dec.steps(7), want[:, 10:].T)
+    assert gpu_dev.pipeline_status() == 0
