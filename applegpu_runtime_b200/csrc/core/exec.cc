@@ -327,7 +327,8 @@ static Status matmul_f32_split(cudaStream_t s, const k::GemmDesc& g, bool* done)
   if (g.batch > 1 ? flops < 2.0e9 || g.m < 64 : flops < 2.0e7 || g.m <= 16) return Status::OK();
   if (g.n < 64 || k::matmul_simt_forced() || !k::f32x3_eligible(g)) return Status::OK();
   TensorRec ws;
-  AG_RETURN_IF_ERROR(alloc_out({k::f32x3_workspace(g)}, DType::U8, &ws, nullptr));
+  const Status got = alloc_out({k::f32x3_workspace(g)}, DType::U8, &ws, nullptr);
+  if (!got.ok()) return flops < 2.0e9 ? Status::OK() : got;      // what CUDA cores do within 0.1 ms is not refused for want of a workspace
   AG_LAUNCH(k::matmul_f32x3(s, g, ws.data()));
   *done = true;
   return Status::OK();

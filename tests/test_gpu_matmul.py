@@ -532,3 +532,23 @@ def test_float32_products_keep_infinities_and_nans(gpu_dev, m, n, k):
     assert np.array_equal(np.isnan(got), np.isnan(ref)) and np.array_equal(np.isinf(got), np.isinf(ref)) and np.array_equal(np.sign(got[np.isinf(got)]), np.sign(ref[np.isinf(ref)]))
     ok = np.isfinite(ref)
     assert np.all(np.abs(got[ok] - ref[ok]) <= 4e-6 * np.sqrt(k) + 1e-5 * np.abs(ref[ok]))
+
+
+def test_float32_product_without_room_for_its_planes(gpu_dev):
+    """A product of less than 2 GFLOP whose workspace cannot be had is computed all the same; a larger one reports the failure."""
+    from applegpu_runtime_b200 import _lib
+    lib, rng = _lib.load(), np.random.default_rng(0)
+    for m, n, k, runs in ((64, 512, 1024, True), (1024, 1024, 1024, False)):
+        a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+        ga, gb = gpu_dev.from_numpy(a), gpu_dev.from_numpy(b)
+        gpu_dev.pool_drain()
+        room = gpu_dev.from_numpy(np.zeros((m, n), np.float32))
+        del room                                          # the result's buffer is there, the planes' is not
+        lib.applegpu_pool_fail_next(1)
+        if runs:
+            got = (ga @ gb).to_numpy()
+            assert np.max(np.abs(got - a.astype(np.float64) @ b.astype(np.float64))) <= 1e-4 * np.sqrt(k)
+        else:
+            with pytest.raises(ValueError, match="allocate"):
+                (ga @ gb).to_numpy()
+        lib.applegpu_pool_fail_next(0)
