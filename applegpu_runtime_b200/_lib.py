@@ -193,6 +193,7 @@ EXT_SYMBOLS = {
     "applegpu_gpt2_decoder_create": (u64, [u64p, u32, u32, u32, u32, u32, u32, u32, u32]),
     "applegpu_gpt2_decoder_prefill": (i32, [u64, u64p, u32, u64, u32]),
     "applegpu_gpt2_decoder_steps": (i32, [u64, u32, vp, cbool]),
+    "applegpu_gpt2_decoder_cache": (u64, [u64, u32, cbool]),
     "applegpu_gpt2_decoder_launches_per_step": (i32, [u64]),
     "applegpu_gpt2_decoder_uses_graph": (i32, [u64]),
     "applegpu_gpt2_decoder_set_engine": (i32, [u64, i32]),

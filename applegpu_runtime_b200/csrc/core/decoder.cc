@@ -296,6 +296,23 @@ Status decoder_steps(uint64_t handle, int n_steps, int32_t* host_tokens, bool us
   return download(hist, host_tokens, (size_t)n_steps * c.batch * 4, true);   // waits, and reports a timed-out tensor-core wait
 }
 
+// The filled rows of a layer's keys or values as a tensor of its own, [batch, heads, tokens so far, 64].
+Status decoder_cache(uint64_t handle, int layer, bool values, TensorRec* out) {
+  std::lock_guard<std::mutex> g(g_dec_mu);
+  Gpt2Decoder* dec = find_decoder(handle);
+  if (!dec) return Status::invalid("decoder: unknown handle");
+  const Gpt2DecoderCfg& c = dec->cfg;
+  if (!dec->primed) return Status::invalid("decoder: prefill first");
+  if (layer < 0 || layer >= c.n_layer) return Status::invalid("decoder: no such layer");
+  TView src;
+  src.ptr = values ? dec->vcache(layer) : dec->kcache(layer);
+  src.dtype = dec->dtype; src.shape = {c.batch, c.n_head, dec->prompt_len + dec->steps_done, 64};
+  src.strides = {(int64_t)c.n_head * c.max_len * 64, (int64_t)c.max_len * 64, 64, 1};
+  out->shape = src.shape; out->strides = contiguous_strides(src.shape); out->dtype = dec->dtype; out->byte_offset = 0; out->has_meta = true;
+  AG_RETURN_IF_ERROR(Shared::get().pool.acquire((size_t)numel_of(src.shape) * dec->esz(), &out->buf));
+  return k::copy_strided(DeviceCtx::get().stream, src, out->view());
+}
+
 // engine 0: one kernel per op; 1: the layers as one persistent cooperative kernel. A captured step of the other engine is dropped.
 Status decoder_set_engine(uint64_t handle, int engine) {
   std::lock_guard<std::mutex> g(g_dec_mu);

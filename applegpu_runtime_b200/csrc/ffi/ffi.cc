@@ -28,6 +28,7 @@ Status decoder_prefill(uint64_t handle, const std::vector<TensorRec>& kvs, const
 Status decoder_steps(uint64_t handle, int n_steps, int32_t* host_tokens, bool use_graph);
 int decoder_launches_per_step(uint64_t handle);
 int decoder_uses_graph(uint64_t handle);
+Status decoder_cache(uint64_t handle, int layer, bool values, TensorRec* out);
 Status decoder_set_engine(uint64_t handle, int engine);
 void decoder_destroy(uint64_t handle);
 namespace k {
@@ -1342,6 +1343,17 @@ int32_t applegpu_gpt2_decoder_steps(uint64_t decoder, uint32_t n_steps, int32_t*
   Status s = decoder_steps(decoder, (int)n_steps, host_tokens, use_graph);
   if (!s.ok()) { set_ffi_error("gpt2_decoder_steps failed: " + s.to_string()); return -1; }
   return 0;
+}
+uint64_t applegpu_gpt2_decoder_cache(uint64_t decoder, uint32_t layer, bool values) {
+  if (!ffi_ready("gpt2_decoder_cache")) return 0;
+  LazyState& st = lazy_state();
+  std::lock_guard<std::mutex> g(st.mu);
+  TensorRec out;
+  Status s = decoder_cache(decoder, (int)layer, values, &out);
+  if (!s.ok()) { set_ffi_error("gpt2_decoder_cache failed: " + s.to_string()); return 0; }
+  const uint64_t id = next_tensor_id();
+  st.rt.insert_tensor(id, out);
+  return id;
 }
 int32_t applegpu_gpt2_decoder_launches_per_step(uint64_t decoder) { return decoder_launches_per_step(decoder); }
 int32_t applegpu_gpt2_decoder_uses_graph(uint64_t decoder) { return decoder_uses_graph(decoder); }

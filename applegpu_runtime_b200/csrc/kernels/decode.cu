@@ -181,8 +181,8 @@ Status attention_decode(cudaStream_t s, DType dt, const void* qkv, void* kcache,
 //     (kernel_templates.rs:1097-1109: mean, population variance, 1/sqrt(var + eps)) and normalises its K share on the
 //     way into shared memory, which removes the separate layer_norm launches of the step;
 //   * 16-bit weights are multiplied by mma.m16n8k16 from registers (dl_products16). Stored inputs have the weight's type and enter as they
-//     are; a normalised input is float32 and enters as the sum of three 16-bit numbers, which holds it to 2^-24. float32 weights keep
-//     CUDA-core multiply-adds.
+//     are; a normalised input is float32 and enters as the sum of three 16-bit numbers (DlSplit). float32 weights keep CUDA-core
+//     multiply-adds.
 // Every thread runs this code once per launch, so a launch takes about as long as its instructions: options are template parameters and
 // nothing is unrolled beyond what the shape needs. GPT-2 small, 8 rows, bf16, a launch's share of a replayed step: 7.8 us with
 // multiply-adds, partials in the L2 and a last CTA that adds them; 7.9 us with cluster sums and MMAs but x through shared memory and one
@@ -394,10 +394,16 @@ __device__ __forceinline__ void dl_store_f32(float (&acc)[kDlMaxM][4], float (*s
   }
 }
 
-template <typename T> __device__ __forceinline__ T dl_piece(float v) { return Cvt<T>::from(v); }
-template <> __device__ __forceinline__ __half dl_piece<__half>(float v) {         // a value beyond the type leaves the rest to the next piece
-  return __float2half_rn(fabsf(v) > 65504.f ? copysignf(65504.f, v) : v);
-}
+// A normalised value r as three 16-bit numbers, r = pre (h0 + h1 / step + h2 / step^2).
+// bfloat16 has float32's exponents: two truncated pieces and their remainder hold its 24 bits as they are.
+// float16: |r| <= 2^22 (sqrt(2048) times the largest gamma, plus the largest beta), so r / 2^7 <= 2^15 and, a remainder being at most
+// 2^-11 of what it remains of, every piece stays in range. The pieces hold 2^-35 of r, or 2^-43 where that is more: float32's 2^-24 from
+// |r| = 2^-18 on.
+template <typename T> struct DlSplit { static constexpr float pre = 1.f, step = 1.f; };
+template <> struct DlSplit<__half> { static constexpr float pre = 128.f, step = 4096.f; };
+template <typename T> __device__ __forceinline__ T dl_piece(float v);
+template <> __device__ __forceinline__ __nv_bfloat16 dl_piece<__nv_bfloat16>(float v) { return __float2bfloat16_rz(v); }      // no finite value becomes an infinity
+template <> __device__ __forceinline__ __half dl_piece<__half>(float v) { return __float2half_rn(v); }
 template <typename T> __device__ __forceinline__ uint32_t dl_pair(T lo, T hi) {
   return (uint32_t)*reinterpret_cast<const uint16_t*>(&lo) | ((uint32_t)*reinterpret_cast<const uint16_t*>(&hi) << 16);
 }
@@ -430,6 +436,8 @@ __device__ __forceinline__ void dl_ask_norm16(const DecodeLinearParams& p, int k
   const T* B = reinterpret_cast<const T*>(p.ln_beta) + kk;
   gam.x = dl_pair(G[0], G[1]); gam.y = dl_pair(G[2], G[3]); bet.x = dl_pair(B[0], B[1]); bet.y = dl_pair(B[2], B[3]);
 }
+// LN: acc is in units of pre. An infinity or NaN is the first pieces' alone: what it leaves for the others, or an infinite weight times
+// them, has no meaning.
 template <typename T, int NT, bool LN>
 __device__ __forceinline__ void dl_products16(const uint4 (&wv)[4], const uint2 (&x)[NT], uint2 gam, uint2 bet, const DlStats& st, float (&acc)[NT][4][4]) {
   const int g = (threadIdx.x & 31) >> 2;
@@ -450,17 +458,47 @@ __device__ __forceinline__ void dl_products16(const uint4 (&wv)[4], const uint2 
       const float mean = st.mean[g + 8 * t], rstd = st.rstd[g + 8 * t];
       float r[4];
 #pragma unroll
-      for (int e = 0; e < 4; e++) r[e] = dl_elem<T>(gam, e) * (dl_elem<T>(x[t], e) - mean) * rstd + dl_elem<T>(bet, e);
+      for (int e = 0; e < 4; e++) r[e] = (dl_elem<T>(gam, e) * (dl_elem<T>(x[t], e) - mean) * rstd + dl_elem<T>(bet, e)) * (1.f / DlSplit<T>::pre);
+      uint32_t b[3][2];
 #pragma unroll
-      for (int piece = 0; piece < 3; piece++) {            // float32 as the sum of three 16-bit numbers
+      for (int piece = 0; piece < 3; piece++) {
         T h[4];
 #pragma unroll
-        for (int e = 0; e < 4; e++) { h[e] = dl_piece<T>(r[e]); r[e] -= Cvt<T>::to(h[e]); }
-        const uint32_t b0 = dl_pair(h[0], h[1]), b1 = dl_pair(h[2], h[3]);
-#pragma unroll
-        for (int j = 0; j < 4; j++) mma_16816<T>(acc[t][j], a[j][0], a[j][1], a[j][2], a[j][3], b0, b1);
+        for (int e = 0; e < 4; e++) { h[e] = dl_piece<T>(r[e]); r[e] = (r[e] - Cvt<T>::to(h[e])) * DlSplit<T>::step; }
+        b[piece][0] = dl_pair(h[0], h[1]); b[piece][1] = dl_pair(h[2], h[3]);
       }
+      float c[4][4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        c[j][0] = 0.f; c[j][1] = 0.f; c[j][2] = 0.f; c[j][3] = 0.f;
+        mma_16816<T>(c[j], a[j][0], a[j][1], a[j][2], a[j][3], b[2][0], b[2][1]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) mma_16816<T>(acc[t][j], a[j][0], a[j][1], a[j][2], a[j][3], b[0][0], b[0][1]);
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        if constexpr (DlSplit<T>::step != 1.f) {
+#pragma unroll
+          for (int e = 0; e < 4; e++) c[j][e] *= 1.f / DlSplit<T>::step;
+        }
+        mma_16816<T>(c[j], a[j][0], a[j][1], a[j][2], a[j][3], b[1][0], b[1][1]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) if (isfinite(acc[t][j][e])) acc[t][j][e] = fmaf(c[j][e], 1.f / DlSplit<T>::step, acc[t][j][e]);
     }
+  }
+}
+template <typename T, int NT>
+__device__ __forceinline__ void dl_unit(float (&acc)[NT][4][4]) {
+  if constexpr (DlSplit<T>::pre != 1.f) {
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[t][j][e] *= DlSplit<T>::pre;
   }
 }
 template <int NT>
@@ -528,6 +566,7 @@ __device__ __forceinline__ void dl_partial(const DecodeLinearParams& p, DlSmem& 
       if (p.ln_gamma) { dl_ask_norm16<T>(p, k0, gam, bet); dl_products16<T, 2, true>(wv, x, gam, bet, sm.st, acc); }
       else dl_products16<T, 2, false>(wv, x, gam, bet, sm.st, acc);
     }
+    if (p.ln_gamma) dl_unit<T, 2>(acc);
     dl_store16<2>(acc, sm.sSum[threadIdx.x >> 5]);
   }
   __syncthreads();
@@ -592,9 +631,11 @@ __device__ __forceinline__ void dl_finish(const DecodeLinearParams& p, int n0, i
 
 // grid = (column slabs, shares of K), a cluster per column slab; `per` slabs of 128 K rows in a share, PRE of them asked for ahead of the
 // dependency wait (they are not produced by the step). NT groups of eight rows of x.
-// LN: 0 or the rounds of layer_norm's statistics (IT above).
+// LN: 0 or the rounds of layer_norm's statistics (IT above). Rows of up to 1024 columns are held to the registers of three CTAs an SM, so that the
+// next launch's weights are under way beside this one: with 88 registers, two CTAs, 50 tokens of 8 sequences of GPT-2 small in bf16 take
+// 16.7 ms in place of 14.7, and of 16 sequences 23.0 in place of 21.0.
 template <typename T, int NT, int PRE, int LN>
-__global__ void __launch_bounds__(kDlThreads) decode_linear_kernel(const __grid_constant__ DecodeLinearParams p, int per) {
+__global__ void __launch_bounds__(kDlThreads, LN == 4 ? 3 : 0) decode_linear_kernel(const __grid_constant__ DecodeLinearParams p, int per) {
   __shared__ __align__(16) float sSum[kDlThreads / 32][NT * 8][kDlSumPitch];
   __shared__ float sFin[kDlFinRows * kDlCols];
   __shared__ DlStats st;
@@ -624,6 +665,7 @@ __global__ void __launch_bounds__(kDlThreads) decode_linear_kernel(const __grid_
     if constexpr (LN) dl_ask_norm16<T>(p, k0 + s * kDlRows, gam[0], bet[0]);
     dl_products16<T, NT, LN != 0>(wv[0], x[0], gam[0], bet[0], st, acc);
   }
+  if constexpr (LN) dl_unit<T, NT>(acc);
   dl_store16<NT>(acc, sSum[threadIdx.x >> 5]);
   __syncthreads();
   dl_finish<T, NT * 8>(p, n0, rank, ranks, &sSum[0][0][0], sFin);

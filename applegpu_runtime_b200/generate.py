@@ -82,6 +82,13 @@ class Gpt2Decoder:
             raise ValueError(gpu._err())
         return out
 
+    def cache(self, layer):
+        """(keys, values) of a layer so far, each a copy [batch, heads, tokens, 64]."""
+        ids = [int(self._lib.applegpu_gpt2_decoder_cache(self.handle, int(layer), v)) for v in (False, True)]
+        if not all(ids):
+            raise ValueError(gpu._err())
+        return tuple(gpu.GpuTensor(i) for i in ids)
+
     def set_engine(self, persistent=False):
         """persistent=False (the default): one kernel per op, chained by programmatic dependent launches; True: the
         embeddings and all layers of a step run as one cooperative kernel with grid-wide barriers between phases (same

@@ -277,6 +277,8 @@ APPLEGPU_API uint64_t applegpu_gpt2_decoder_create(const uint64_t* weight_ids, u
                                                   uint32_t vocab, uint32_t n_positions, uint32_t batch, uint32_t max_len);
 APPLEGPU_API int32_t applegpu_gpt2_decoder_prefill(uint64_t decoder, const uint64_t* kv_ids, uint32_t n_kv, uint64_t first_tokens_id, uint32_t prompt_len);
 APPLEGPU_API int32_t applegpu_gpt2_decoder_steps(uint64_t decoder, uint32_t n_steps, int32_t* host_tokens, bool use_graph);
+/* A copy of the cached keys (or values) of a layer so far, [batch, heads, tokens, 64]; 0 on failure. */
+APPLEGPU_API uint64_t applegpu_gpt2_decoder_cache(uint64_t decoder, uint32_t layer, bool values);
 APPLEGPU_API int32_t applegpu_gpt2_decoder_launches_per_step(uint64_t decoder);
 APPLEGPU_API int32_t applegpu_gpt2_decoder_uses_graph(uint64_t decoder);
 /* engine 0 (default): one kernel per op, chained by programmatic dependent launches inside the captured step. engine 1:

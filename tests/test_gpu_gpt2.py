@@ -260,6 +260,125 @@ def test_decode_linears_at_the_edges_of_their_shares(gpu_dev, heads, batch, dtyp
     assert gpu_dev.pipeline_status() == 0
 
 
+# ── a step's keys and values, number by number ──────────────────────────────
+_MANTISSA = {"float32": 24, "float16": 11, "bfloat16": 8}
+
+
+def _stored(x, dtype):
+    """float64 rounded to the storage type."""
+    import torch
+    return torch.from_numpy(np.asarray(x, np.float64)).to(getattr(torch, dtype)).double().numpy()
+
+
+def _step_state(heads, layers, seed, dtype, std=0.06):
+    rng, d = np.random.default_rng(seed), 64 * heads
+    n = lambda *shape: rng.standard_normal(shape) * std  # noqa: E731
+    w = {"wte.weight": rng.standard_normal((300, d)) * 0.5, "wpe.weight": rng.standard_normal((320, d)) * 0.2, "ln_f.weight": np.ones(d), "ln_f.bias": np.zeros(d)}
+    for i in range(layers):
+        for name, k, o in (("attn.c_attn", d, 3 * d), ("attn.c_proj", d, d), ("mlp.c_fc", d, 4 * d), ("mlp.c_proj", 4 * d, d)):
+            w[f"h.{i}.{name}.weight"], w[f"h.{i}.{name}.bias"] = n(k, o), n(o) * 5
+        for name in ("ln_1", "ln_2"):
+            w[f"h.{i}.{name}.weight"], w[f"h.{i}.{name}.bias"] = 1 + 0.3 * rng.standard_normal(d), 0.3 * rng.standard_normal(d)
+    return {k: _stored(v, dtype) for k, v in w.items()}, {"n_layer": layers, "n_head": heads, "n_embd": d, "vocab_size": 300, "n_positions": 320}
+
+
+def _decoded(g, state, cfg, dtype, ids, steps, engine):
+    """Decoder behind the prompt `ids` after `steps` steps, the tokens the steps consumed [steps, batch]."""
+    from applegpu_runtime_b200.generate import Gpt2Decoder
+    m = g.load_gpt2_state_dict({"transformer." + k: v.astype(np.float32) for k, v in state.items()}, cfg, dtype, fold_layer_norms=False)
+    logits, kv = g.gpt2_forward(m, ids, last_only=True)
+    first = g.argmax(logits)
+    dec = Gpt2Decoder(m, ids.shape[0], ids.shape[1] + steps)
+    dec.set_engine(persistent=engine == "persistent")
+    dec.prefill(kv, first, ids.shape[1])
+    out = dec.steps(steps, use_graph=engine != "direct")
+    return dec, np.concatenate([first.to_numpy().reshape(1, -1), out[:-1]])
+
+
+def _norm64(x, w, b):
+    c = x - x.mean(-1, keepdims=True)
+    with np.errstate(all="ignore"):
+        return c / np.sqrt((c * c).mean(-1, keepdims=True) + 1e-5) * w + b
+
+
+def _assert_linear(got, r, w, b, dtype):
+    """got = r @ w + b rounded once: half a unit in its last place, beside what float32 arithmetic leaves open: 2^-22 for each normalised
+    value (four operations of 2^-24), and sums that each lose up to 2^-23 of the terms before them, over at most 128 of K in one chain."""
+    want, terms = r @ w + b, np.abs(r) @ np.abs(w) + np.abs(b)
+    ulp = 2.0 ** np.maximum(np.floor(np.log2(np.maximum(np.abs(want), 1e-30))) + 1 - _MANTISSA[dtype], -24 if dtype == "float16" else -140)
+    assert np.all(np.abs(got - want) <= 0.5 * ulp + 2e-6 * terms), np.max((np.abs(got - want) - 0.5 * ulp) / terms)
+
+
+@pytest.mark.parametrize("heads,batch,dtype", [(5, 1, "float16"), (5, 8, "bfloat16"), (21, 9, "float16"), (21, 16, "bfloat16"), (5, 16, "float32"), (21, 3, "float32"), (12, 8, "bfloat16")])
+@pytest.mark.parametrize("engine", ["graph", "persistent"])
+def test_decode_step_against_float64(gpu_dev, heads, batch, dtype, engine):
+    """The keys and values a step leaves. The first layer's are one linear behind layer_norm: exact up to its rounding, at ragged shares
+    of K (320 and 1344 columns), one and two groups of eight rows. The second layer's come through every kernel of a layer, with
+    attention over 300 rows (more than are asked for ahead in any type) and roundings to the storage type where the step rounds. Half a
+    storage unit of their norm: rounding them leaves 1 / sqrt(12) of a unit at most (0.2 on average over a binade), and upstream only the
+    roundings differ that float32 sums in another order turn."""
+    state, cfg = _step_state(heads, 2, 7 * heads + batch, dtype)
+    d, T = cfg["n_embd"], 300
+    ids = np.random.default_rng(batch).integers(0, 300, (batch, T))
+    dec, toks = _decoded(gpu_dev, state, cfg, dtype, ids, 3, engine)
+    (k0, v0), (k1, v1) = [[t.to_numpy().astype(np.float64) for t in dec.cache(i)] for i in range(2)]
+    merged = lambda c, t: c[:, :, t].reshape(batch, d)  # noqa: E731
+    w = lambda n: state["h.0." + n]  # noqa: E731
+    for t in range(3):
+        x = _stored(state["wte.weight"][toks[t]] + state["wpe.weight"][T + t], dtype)
+        r = _norm64(x, w("ln_1.weight"), w("ln_1.bias"))
+        _assert_linear(np.concatenate([merged(k0, T + t), merged(v0, T + t)], axis=1), r, w("attn.c_attn.weight")[:, d:], w("attn.c_attn.bias")[d:], dtype)
+        q = _stored(r @ w("attn.c_attn.weight")[:, :d] + w("attn.c_attn.bias")[:d], dtype).reshape(batch, heads, 1, 64)
+        s = (q @ k0[:, :, :T + t + 1].transpose(0, 1, 3, 2)) / 8
+        p = np.exp(s - s.max(-1, keepdims=True))
+        att = _stored((p @ v0[:, :, :T + t + 1] / p.sum(-1, keepdims=True)).reshape(batch, d), dtype)
+        x = _stored(att @ w("attn.c_proj.weight") + w("attn.c_proj.bias") + x, dtype)
+        h = _norm64(x, w("ln_2.weight"), w("ln_2.bias")) @ w("mlp.c_fc.weight") + w("mlp.c_fc.bias")
+        h = _stored(0.5 * h * (1 + np.tanh(0.7978845608 * (h + 0.044715 * h ** 3))), dtype)
+        x = _stored(h @ w("mlp.c_proj.weight") + w("mlp.c_proj.bias") + x, dtype)
+        r = _norm64(x, state["h.1.ln_1.weight"], state["h.1.ln_1.bias"])
+        want = r @ state["h.1.attn.c_attn.weight"][:, d:] + state["h.1.attn.c_attn.bias"][d:]
+        got = np.concatenate([merged(k1, T + t), merged(v1, T + t)], axis=1)
+        assert np.linalg.norm(got - want) <= (0.5 * 2.0 ** (1 - _MANTISSA[dtype]) + 2e-6) * np.linalg.norm(want)
+    assert gpu_dev.pipeline_status() == 0
+
+
+@pytest.mark.parametrize("gamma,std", [(1e-5, 2000.0), (3e-4, 300.0), (1.0, 0.5), (3e4, 2e-5)])
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("heads,batch", [(5, 3), (17, 16)])
+def test_decode_linear_keeps_normalised_values_in_32_bits(gpu_dev, heads, batch, dtype, gamma, std):
+    """Rows whose normalised values are tiny or (one column) beyond the storage type, next to ordinary ones."""
+    state, cfg = _step_state(heads, 1, heads, dtype)
+    state["wte.weight"][:, 3] = 40.0
+    d, rng = cfg["n_embd"], np.random.default_rng(heads)
+    state["h.0.ln_1.weight"] = _stored(gamma * rng.uniform(0.5, 2.0, d) * np.where(np.arange(d) % 7 == 0, 1e-2, 1.0), dtype)
+    state["h.0.ln_1.bias"] = _stored(gamma * 0.1 * rng.standard_normal(d), dtype)
+    state["h.0.attn.c_attn.weight"] = _stored(std * rng.standard_normal((d, 3 * d)), dtype)
+    dec, toks = _decoded(gpu_dev, state, cfg, dtype, rng.integers(0, 300, (batch, 5)), 1, "direct")
+    got = np.concatenate([t.to_numpy()[:, :, 5].reshape(batch, d) for t in dec.cache(0)], axis=1).astype(np.float64)
+    x = _stored(state["wte.weight"][toks[0]] + state["wpe.weight"][5], dtype)
+    _assert_linear(got, _norm64(x, state["h.0.ln_1.weight"], state["h.0.ln_1.bias"]), state["h.0.attn.c_attn.weight"][:, d:], state["h.0.attn.c_attn.bias"][d:], dtype)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+@pytest.mark.parametrize("where", ["gamma", "beta", "weight", "nan"])
+def test_decode_linear_keeps_infinities_and_nans(gpu_dev, dtype, where):
+    state, cfg = _step_state(5, 1, 3, dtype)
+    d, rng = cfg["n_embd"], np.random.default_rng(3)
+    if where in ("gamma", "beta"):
+        state["h.0.ln_1." + {"gamma": "weight", "beta": "bias"}[where]][77] = np.inf
+    else:
+        state["h.0.attn.c_attn.weight"][[5, 200], [d + 3, d + 90]] = np.nan if where == "nan" else np.inf
+    dec, toks = _decoded(gpu_dev, state, cfg, dtype, rng.integers(0, 300, (3, 5)), 1, "direct")
+    got = np.concatenate([t.to_numpy()[:, :, 5].reshape(3, d) for t in dec.cache(0)], axis=1).astype(np.float64)
+    x = _stored(state["wte.weight"][toks[0]] + state["wpe.weight"][5], dtype)
+    with np.errstate(all="ignore"):
+        want = _norm64(x, state["h.0.ln_1.weight"], state["h.0.ln_1.bias"]) @ state["h.0.attn.c_attn.weight"][:, d:] + state["h.0.attn.c_attn.bias"][d:]
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    inf = np.isinf(want)
+    assert inf.any() == (where != "nan") and np.array_equal(np.isinf(got), inf) and np.array_equal(got[inf], want[inf])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_persistent_decode_refuses_rows_beyond_its_statistics(gpu_dev, dtype):
     """Its layer_norm keeps 2048 columns of a row: 32 heads give the step engine's tokens, 33 are refused and leave the step engine usable."""
