@@ -395,15 +395,32 @@ __device__ __forceinline__ void dl_store_f32(float (&acc)[kDlMaxM][4], float (*s
 }
 
 // A normalised value r as three 16-bit numbers, r = pre (h0 + h1 / step + h2 / step^2).
-// bfloat16 has float32's exponents: two truncated pieces and their remainder hold its 24 bits as they are.
+// bfloat16 has float32's exponents: its pieces are eight bits each, cut off and so of the value's sign, and hold the 24 as they are. The
+// NaN that arithmetic leaves has its payload in the upper half.
 // float16: |r| <= 2^22 (sqrt(2048) times the largest gamma, plus the largest beta), so r / 2^7 <= 2^15 and, a remainder being at most
 // 2^-11 of what it remains of, every piece stays in range. The pieces hold 2^-35 of r, or 2^-43 where that is more: float32's 2^-24 from
 // |r| = 2^-18 on.
 template <typename T> struct DlSplit { static constexpr float pre = 1.f, step = 1.f; };
 template <> struct DlSplit<__half> { static constexpr float pre = 128.f, step = 4096.f; };
-template <typename T> __device__ __forceinline__ T dl_piece(float v);
-template <> __device__ __forceinline__ __nv_bfloat16 dl_piece<__nv_bfloat16>(float v) { return __float2bfloat16_rz(v); }      // no finite value becomes an infinity
-template <> __device__ __forceinline__ __half dl_piece<__half>(float v) { return __float2half_rn(v); }
+__device__ __forceinline__ void dl_split(float (&r)[4], uint32_t (&b)[3][2], __half) {
+#pragma unroll
+  for (int piece = 0; piece < 3; piece++)
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const __half2 h = __floats2half2_rn(r[2 * i], r[2 * i + 1]);
+      const float2 f = __half22float2(h);
+      b[piece][i] = *reinterpret_cast<const uint32_t*>(&h);
+      r[2 * i] = (r[2 * i] - f.x) * DlSplit<__half>::step; r[2 * i + 1] = (r[2 * i + 1] - f.y) * DlSplit<__half>::step;
+    }
+}
+__device__ __forceinline__ void dl_split(float (&r)[4], uint32_t (&b)[3][2], __nv_bfloat16) {
+#pragma unroll
+  for (int piece = 0; piece < 3; piece++) {
+    b[piece][0] = __byte_perm(__float_as_uint(r[0]), __float_as_uint(r[1]), 0x7632); b[piece][1] = __byte_perm(__float_as_uint(r[2]), __float_as_uint(r[3]), 0x7632);
+#pragma unroll
+    for (int e = 0; e < 4; e++) r[e] -= __uint_as_float(__float_as_uint(r[e]) & 0xffff0000u);
+  }
+}
 template <typename T> __device__ __forceinline__ uint32_t dl_pair(T lo, T hi) {
   return (uint32_t)*reinterpret_cast<const uint16_t*>(&lo) | ((uint32_t)*reinterpret_cast<const uint16_t*>(&hi) << 16);
 }
@@ -460,13 +477,7 @@ __device__ __forceinline__ void dl_products16(const uint4 (&wv)[4], const uint2 
 #pragma unroll
       for (int e = 0; e < 4; e++) r[e] = (dl_elem<T>(gam, e) * (dl_elem<T>(x[t], e) - mean) * rstd + dl_elem<T>(bet, e)) * (1.f / DlSplit<T>::pre);
       uint32_t b[3][2];
-#pragma unroll
-      for (int piece = 0; piece < 3; piece++) {
-        T h[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) { h[e] = dl_piece<T>(r[e]); r[e] = (r[e] - Cvt<T>::to(h[e])) * DlSplit<T>::step; }
-        b[piece][0] = dl_pair(h[0], h[1]); b[piece][1] = dl_pair(h[2], h[3]);
-      }
+      dl_split(r, b, T());
       float c[4][4];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
