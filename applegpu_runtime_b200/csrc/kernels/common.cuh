@@ -178,8 +178,14 @@ inline Status cuda_status(cudaError_t e, const char* what) {
 // still draining: its CTAs run their prologue (barrier init, TMEM allocation, descriptor prefetch)
 // and then block in pdl_wait() until kernel N has completed and its writes are visible. Rules kept
 // by every kernel launched through launch_pdl: all threads call pdl_wait() before the first access
-// to global memory (so completion stays transitive along the stream), and pdl_trigger() follows
-// it (the next kernel is released for scheduling once every CTA of this one has started).
+// to memory that a kernel of the stream writes, and pdl_trigger() follows it (the next kernel is
+// released for scheduling once every CTA of this one has started and has waited). So completion is
+// transitive along the stream, and when a kernel starts, all launches but the one before it are
+// complete and their writes visible. Two kinds of load stand ahead of the wait on that ground: of
+// model weights, which no kernel of the stream writes, and, in attention_decode_kernel,
+// grouped_decode_kernel and latent_decode_attend_mma_kernel, of lengths, positions and the cached
+// rows below them: the launch right before these (a projection, an append, the prepare kernel)
+// writes none of them. A kernel that released its successor ahead of its own wait would break them.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -33,8 +33,8 @@ int* matmul_status_word();
 struct PlaneJob { const float* in; __nv_bfloat16* out; long long rows, cols, row_stride, batch_stride; int batches, blocks; };
 
 __global__ void __launch_bounds__(256) f32_planes_kernel(const __grid_constant__ PlaneJob ja, const __grid_constant__ PlaneJob jb) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const bool second = (int)blockIdx.x >= ja.blocks;
   const PlaneJob& j = second ? jb : ja;
   const long long packs = j.cols / 8, plane = j.rows * j.cols, per = j.rows * packs, total = per * j.batches;
@@ -331,8 +331,8 @@ gemm_f32x3_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
 // The shares of K added in order, then what the single-launch epilogue does.
 __global__ void __launch_bounds__(256) f32x3_finish_kernel(const __grid_constant__ F3Params p) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const long long q = p.p_row / 4, total = (long long)p.batch * p.m * q, share = (long long)p.batch * p.m * p.p_row;
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
     const long long row = i / q, col = (i - row * q) * 4, b = row / p.m;

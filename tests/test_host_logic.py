@@ -363,3 +363,19 @@ def test_interleave_advances_generators_in_lock_step():
 
     assert interleave([steps("a", 2), steps("b", 3), steps("c", 0)]) == ["A", "B", "C"]
     assert log == [("a", 0), ("b", 0), ("a", 1), ("b", 1), ("b", 2)]
+
+
+def test_kernels_wait_for_their_predecessor_before_they_release_their_successor():
+    """Loads ahead of a dependency wait are sound only while no kernel releases the next one ahead of its own wait (kernels/common.cuh)."""
+    import pathlib
+    import re
+    found = 0
+    for f in sorted((pathlib.Path(__file__).parents[1] / "applegpu_runtime_b200" / "csrc" / "kernels").glob("*.cu*")):
+        lines = [re.sub(r"//.*", "", line).strip() for line in f.read_text().splitlines()]
+        for i, line in enumerate(lines):
+            if line == "pdl_trigger();":
+                found += 1
+                assert lines[i - 1].startswith("pdl_wait();"), f"{f.name}:{i + 1}"
+            else:
+                assert "pdl_trigger();" not in line, f"{f.name}:{i + 1}"
+    assert found >= 40
