@@ -1,7 +1,12 @@
 // float32 products on the tensor cores.
 //
 // Both operands are split into three bf16 planes, x = x0 + x1 + x2 (each the bf16 rounding of what the planes before it left), and
-// the six largest cross terms a0 b0, a0 b1, a1 b0, a0 b2, a1 b1, a2 b0 are multiplied by tcgen05 (error about 2^-22 of the product).
+// the six largest cross terms a0 b0, a0 b1, a1 b0, a0 b2, a1 b1, a2 b0 are multiplied by tcgen05 (error about 2^-22 of the product, while
+// the third plane of what matters lies in bf16's range: an operand below 2^-117, 6e-36, keeps 2^-133 absolute, which a factor of 1e30 in
+// the other operand can bring to light). What is not finite in the sum of a0 b0 is the result as it stands: an infinity has no other
+// planes, and what it makes of the other operand's is not looked at. So infinities and NaN come out as float32 sums have them, at no cost
+// in time. A finite number that bf16 rounds to an infinity (0.2 % below the largest float32) is noted by the pass that writes the planes;
+// then the results that are not finite are taken again in float32, a warp to a result.
 // A pipeline stage holds the three planes of one 64-deep k-block of A and B, and its six products run from that one copy: 72 KB per
 // 24 MMAs and CTA, where a GEMM over a six-fold K extent (what this replaces) fetches 12 tiles for the same work, and the planes are
 // written once instead of each term as often as a product names it (10 bytes per element moved instead of 16).
@@ -20,6 +25,7 @@
 #include "common.cuh"
 #include "sm100.cuh"
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 
 namespace ag { namespace k {
@@ -32,13 +38,14 @@ int* matmul_status_word();
 // ── planes ──────────────────────────────────────────────────────────────────
 struct PlaneJob { const float* in; __nv_bfloat16* out; long long rows, cols, row_stride, batch_stride; int batches, blocks; };
 
-__global__ void __launch_bounds__(256) f32_planes_kernel(const __grid_constant__ PlaneJob ja, const __grid_constant__ PlaneJob jb) {
+__global__ void __launch_bounds__(256) f32_planes_kernel(const __grid_constant__ PlaneJob ja, const __grid_constant__ PlaneJob jb, unsigned long long* note, unsigned long long call) {
   pdl_wait();
   pdl_trigger();
   const bool second = (int)blockIdx.x >= ja.blocks;
   const PlaneJob& j = second ? jb : ja;
   const long long packs = j.cols / 8, plane = j.rows * j.cols, per = j.rows * packs, total = per * j.batches;
   const long long step = (long long)j.blocks * 256;
+  bool noted = false;
   for (long long i = (long long)(blockIdx.x - (second ? ja.blocks : 0)) * 256 + threadIdx.x; i < total; i += step) {
     const long long b = j.batches > 1 ? i / per : 0, q = i - b * per, r = q / packs, c = (q - r * packs) * 8;
     const float* src = j.in + b * j.batch_stride + r * j.row_stride + c;
@@ -53,10 +60,21 @@ __global__ void __launch_bounds__(256) f32_planes_kernel(const __grid_constant__
       const float r2 = r1 - __bfloat162float(h1);
       t[0].v[e] = h0; t[1].v[e] = h1; t[2].v[e] = __float2bfloat16_rn(r2);
     }
+    const uint4 w = *reinterpret_cast<const uint4*>(&t[0]);
+    auto odd = [](uint32_t u) { return (u & 0x7f807f80u) + 0x00800080u; };                     // bits 15 and 31: an exponent of ones
+    if ((odd(w.x) | odd(w.y) | odd(w.z) | odd(w.w)) & 0x80008000u) {
+#pragma unroll
+      for (int e = 0; e < 8; e++) {
+        if (isfinite(__bfloat162float(t[0].v[e]))) continue;
+        noted |= isinf(__bfloat162float(t[1].v[e]));                                           // a finite number less an infinity
+        t[1].v[e] = __float2bfloat16_rn(0.f); t[2].v[e] = t[1].v[e];
+      }
+    }
     __nv_bfloat16* dst = j.out + b * 3 * plane + r * j.cols + c;
 #pragma unroll
     for (int k = 0; k < 3; k++) st16(dst + k * plane, t[k]);
   }
+  if (noted) *note = call;
 }
 
 // ── the product ─────────────────────────────────────────────────────────────
@@ -73,8 +91,9 @@ struct F3Params {
   float* c; const float* bias; const float* residual; float* partial;
   float alpha; int act, m, n, batch, a_one, b_one, num_kb, tiles_m, tiles_n, splits, kb_per_split, vec;
   long long c_row, c_batch, p_row;
-  const float* a; const float* b;        // the operands as they were given, for results that are not finite
+  const float* a; const float* b;        // the operands as they were given; *note == call: one of them holds a finite number beyond bf16
   int k; long long a_row, a_batch, b_row, b_col, b_batch;
+  const unsigned long long* note; unsigned long long call;
   int* status;
 };
 
@@ -88,16 +107,81 @@ __device__ __noinline__ float4 f3_act(float4 v, int act) {
   }
 }
 
-// A sum that is not finite may owe it to the planes: an infinity, or a number that bf16 rounds to one, leaves a NaN for its remainder,
-// and infinity times a plane that is zero is another. Such an element (and one that truly overflows) is taken again in float32.
-__device__ __noinline__ void f3_plain(const F3Params& p, int b, long long row, int col0, int n, float* v) {
-  const float* a = p.a + b * p.a_batch + row * p.a_row;
-  for (int e = 0; e < n && col0 + e < p.n; e++) {
-    if (isfinite(v[e])) continue;
-    const float* w = p.b + b * p.b_batch + (col0 + e) * p.b_col;
-    float t = 0.f;
-    for (int i = 0; i < p.k; i++) t = fmaf(__ldg(a + i), __ldg(w + i * p.b_row), t);
-    v[e] = t;
+// n neighbouring results of each lane's row, of which those that are not finite are taken again; a warp adds one up. A unit's results take
+// the epilogue warps well below the second that the other warps wait for them (K = 2^20: 0.7 s if every result is one of them; from there
+// on they stay as they are).
+__device__ __forceinline__ bool f3_again(const F3Params& p) { return __ldcg(p.note) == p.call && p.k <= 1 << 20; }
+__device__ __noinline__ void f3_plain(const F3Params& p, bool in, int b, long long row, int col0, int n, float* v) {
+  const int lane = threadIdx.x & 31;
+  for (int e = 0; e < n; e++) {
+    for (unsigned again = __ballot_sync(0xffffffffu, in && col0 + e < p.n && !isfinite(v[e])); again; again &= again - 1) {
+      const int who = __ffs(again) - 1;
+      const float* a = p.a + __shfl_sync(0xffffffffu, b, who) * p.a_batch + __shfl_sync(0xffffffffu, row, who) * p.a_row;
+      const float* w = p.b + __shfl_sync(0xffffffffu, b, who) * p.b_batch + (__shfl_sync(0xffffffffu, col0, who) + e) * p.b_col;
+      float t = 0.f;
+#pragma unroll 4
+      for (int i = lane; i < p.k; i += 32) t = fmaf(__ldg(a + i), __ldg(w + i * p.b_row), t);
+      t = warp_sum(t);
+      if (lane == who) v[e] = t;
+    }
+  }
+}
+
+// Epilogue of 32 columns: a lane has its row's.
+__device__ __forceinline__ void f3_store(const F3Params& p, float (&v)[32], int b, long long row0, int col0, float bias_l, float* stg) {
+  const int lane = threadIdx.x & 31;
+  const long long gm = row0 + lane;
+  bool odd = false;
+#pragma unroll
+  for (int e = 0; e < 32; e++) odd |= !isfinite(v[e]);
+  if (__any_sync(0xffffffffu, odd) && f3_again(p)) {
+    float t[32];
+#pragma unroll
+    for (int e = 0; e < 32; e++) t[e] = v[e];
+    f3_plain(p, gm < p.m, b, gm, col0, 32, t);
+#pragma unroll
+    for (int e = 0; e < 32; e++) v[e] = t[e];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int e = 0; e < 32; e++) v[e] = fmaf(v[e], p.alpha, __shfl_sync(0xffffffffu, bias_l, e));
+  if (p.act) {
+#pragma unroll
+    for (int e = 0; e < 32; e += 4) {
+      const float4 o = f3_act(make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]), p.act);
+      v[e] = o.x; v[e + 1] = o.y; v[e + 2] = o.z; v[e + 3] = o.w;
+    }
+  }
+  const long long at = (long long)b * p.c_batch + row0 * p.c_row + col0;
+  if (p.vec && col0 + 32 <= p.n) {
+    if (gm < p.m) {
+      float* crow = p.c + at + lane * p.c_row;
+      const float* rrow = p.residual ? p.residual + at + lane * p.c_row : nullptr;
+#pragma unroll
+      for (int e = 0; e < 32; e += 4) {
+        float4 o = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+        if (rrow) { const float4 r = *reinterpret_cast<const float4*>(rrow + e); o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w; }
+        *reinterpret_cast<float4*>(crow + e) = o;
+      }
+    }
+    return;
+  }
+  // rows on any 4-byte boundary, or a ragged column block: four rows of eight columns per store instead of 32 rows of one
+#pragma unroll
+  for (int e0 = 0; e0 < 32; e0 += 8) {
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 8; e++) stg[lane * kF3StgPitch + e] = v[e0 + e];
+    __syncwarp();
+    const int c = lane & 7, col = col0 + e0 + c;
+#pragma unroll
+    for (int r = lane >> 3; r < 32; r += 4) {
+      if (row0 + r < p.m && col < p.n) {
+        const long long o = at + r * p.c_row + e0 + c;
+        const float x = stg[r * kF3StgPitch + c];
+        p.c[o] = p.residual ? x + p.residual[o] : x;
+      }
+    }
   }
 }
 
@@ -245,8 +329,19 @@ gemm_f32x3_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           tmem_ld_32x32(taddr + g * 32, hi);
           tmem_ld_32x32(taddr + 128 + g * 32, lo);
           tmem_ld_wait();
+          float odd = 0.f;
 #pragma unroll
-          for (int e = 0; e < 32; e++) sum[g][e] += __uint_as_float(hi[e]) + __uint_as_float(lo[e]);
+          for (int e = 0; e < 32; e++) {
+            const float x = __uint_as_float(hi[e]) + __uint_as_float(lo[e]);
+            odd = fmaf(x, 0.f, odd);
+            lo[e] = __float_as_uint(x);
+          }
+          if (odd != odd) {                            // something is not finite: the sum of a0 b0 as it stands
+#pragma unroll
+            for (int e = 0; e < 32; e++) if (!isfinite(__uint_as_float(hi[e]))) lo[e] = hi[e];
+          }
+#pragma unroll
+          for (int e = 0; e < 32; e++) sum[g][e] += __uint_as_float(lo[e]);
         }
         tc_fence_before_sync();
         __syncwarp();
@@ -267,58 +362,7 @@ gemm_f32x3_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
           continue;
         }
-        bool odd = false;
-#pragma unroll
-        for (int e = 0; e < 32; e++) odd |= !isfinite(v[e]);
-        if (odd && gm < p.m) {
-          float t[32];
-#pragma unroll
-          for (int e = 0; e < 32; e++) t[e] = v[e];
-          f3_plain(p, b, gm, col0, 32, t);
-#pragma unroll
-          for (int e = 0; e < 32; e++) v[e] = t[e];
-        }
-        __syncwarp();
-#pragma unroll
-        for (int e = 0; e < 32; e++) v[e] = fmaf(v[e], p.alpha, __shfl_sync(0xffffffffu, bias_l[g], e));
-        if (p.act) {
-#pragma unroll
-          for (int e = 0; e < 32; e += 4) {
-            const float4 o = f3_act(make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]), p.act);
-            v[e] = o.x; v[e + 1] = o.y; v[e + 2] = o.z; v[e + 3] = o.w;
-          }
-        }
-        const long long at = (long long)b * p.c_batch + row0 * p.c_row + col0;
-        if (p.vec && col0 + 32 <= p.n) {
-          if (gm < p.m) {
-            float* crow = p.c + at + lane * p.c_row;
-            const float* rrow = p.residual ? p.residual + at + lane * p.c_row : nullptr;
-#pragma unroll
-            for (int e = 0; e < 32; e += 4) {
-              float4 o = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
-              if (rrow) { const float4 r = *reinterpret_cast<const float4*>(rrow + e); o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w; }
-              *reinterpret_cast<float4*>(crow + e) = o;
-            }
-          }
-          continue;
-        }
-        // rows on any 4-byte boundary, or a ragged column block: four rows of eight columns per store instead of 32 rows of one
-#pragma unroll
-        for (int e0 = 0; e0 < 32; e0 += 8) {
-          __syncwarp();
-#pragma unroll
-          for (int e = 0; e < 8; e++) stg[lane * kF3StgPitch + e] = v[e0 + e];
-          __syncwarp();
-          const int c = lane & 7, col = col0 + e0 + c;
-#pragma unroll
-          for (int r = lane >> 3; r < 32; r += 4) {
-            if (row0 + r < p.m && col < p.n) {
-              const long long o = at + r * p.c_row + e0 + c;
-              const float x = stg[r * kF3StgPitch + c];
-              p.c[o] = p.residual ? x + p.residual[o] : x;
-            }
-          }
-        }
+        f3_store(p, v, b, row0, col0, bias_l[g], stg);
       }
     }
   }
@@ -334,8 +378,10 @@ __global__ void __launch_bounds__(256) f32x3_finish_kernel(const __grid_constant
   pdl_wait();
   pdl_trigger();
   const long long q = p.p_row / 4, total = (long long)p.batch * p.m * q, share = (long long)p.batch * p.m * p.p_row;
-  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
-    const long long row = i / q, col = (i - row * q) * 4, b = row / p.m;
+  const bool look = f3_again(p);
+  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i - (threadIdx.x & 31) < total; i += (long long)gridDim.x * 256) {      // whole warps
+    const bool in = i < total;
+    const long long row = min(i, total - 1) / q, col = (min(i, total - 1) - row * q) * 4, b = row / p.m;
     const float* src = p.partial + row * p.p_row + col;
     float4 x[8];
 #pragma unroll
@@ -344,12 +390,13 @@ __global__ void __launch_bounds__(256) f32x3_finish_kernel(const __grid_constant
 #pragma unroll
     for (int s = 0; s < 8; s++) if (s < p.splits) { v[0] += x[s].x; v[1] += x[s].y; v[2] += x[s].z; v[3] += x[s].w; }
     const long long at = b * p.c_batch + (row - b * p.m) * p.c_row + col;
-    if (!(isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]) && isfinite(v[3]))) {
+    if (look) {
       float t[4] = {v[0], v[1], v[2], v[3]};
-      f3_plain(p, (int)b, row - b * p.m, (int)col, 4, t);
+      f3_plain(p, in, (int)b, row - b * p.m, (int)col, 4, t);
 #pragma unroll
       for (int e = 0; e < 4; e++) v[e] = t[e];
     }
+    if (!in) continue;
 #pragma unroll
     for (int e = 0; e < 4; e++) v[e] = fmaf(v[e], p.alpha, p.bias && col + e < p.n ? __ldg(p.bias + col + e) : 0.f);
     if (p.act) { const float4 o = f3_act(make_float4(v[0], v[1], v[2], v[3]), p.act); v[0] = o.x; v[1] = o.y; v[2] = o.z; v[3] = o.w; }
@@ -392,7 +439,7 @@ static int64_t f3_pad(int64_t bytes) { return (bytes + 255) / 256 * 256; }
 int64_t f32x3_workspace(const GemmDesc& g) {
   const int64_t ca = g.batch > 1 && g.a_batch ? g.batch : 1, cb = g.batch > 1 && g.b_batch ? g.batch : 1;
   const int s = f32x3_splits(g.m, g.n, g.k, g.batch);
-  return f3_pad(6 * ca * g.m * g.k) + f3_pad(6 * cb * g.n * g.k) + (s > 1 ? (int64_t)s * g.batch * g.m * ((g.n + 3) / 4 * 4) * 4 : 0);
+  return 256 + f3_pad(6 * ca * g.m * g.k) + f3_pad(6 * cb * g.n * g.k) + (s > 1 ? (int64_t)s * g.batch * g.m * ((g.n + 3) / 4 * 4) * 4 : 0);
 }
 
 Status matmul_f32x3(cudaStream_t s, const GemmDesc& g, void* workspace) {
@@ -401,13 +448,16 @@ Status matmul_f32x3(cudaStream_t s, const GemmDesc& g, void* workspace) {
   if (!st) return Status::compute("matmul: the kernel workspace is not initialised");
   const int64_t ca = g.batch > 1 && g.a_batch ? g.batch : 1, cb = g.batch > 1 && g.b_batch ? g.batch : 1;
   const bool b_mn = g.b_col == 1;
-  uint8_t* ws = static_cast<uint8_t*>(workspace);
+  uint8_t* ws = static_cast<uint8_t*>(workspace) + 256;     // in front: the call whose operands hold a finite number beyond bf16
+  static std::atomic<unsigned long long> calls{0x9e3779b97f4a7c15ull};      // what a pooled buffer holds is hardly ever the next call's (it would cost time only)
+  unsigned long long* note = static_cast<unsigned long long*>(workspace);
+  const unsigned long long call = calls.fetch_add(1, std::memory_order_relaxed);
   __nv_bfloat16* pa = reinterpret_cast<__nv_bfloat16*>(ws);
   __nv_bfloat16* pb = reinterpret_cast<__nv_bfloat16*>(ws + f3_pad(6 * ca * g.m * g.k));
   const int64_t b_rows = b_mn ? g.k : g.n, b_cols = b_mn ? g.n : g.k;
   PlaneJob ja{static_cast<const float*>(g.a), pa, g.m, g.k, g.a_row, g.a_batch, (int)ca, grid_for(ca * g.m * (g.k / 8), 256, 4)};
   PlaneJob jb{static_cast<const float*>(g.b), pb, b_rows, b_cols, b_mn ? g.b_row : g.b_col, g.b_batch, (int)cb, grid_for(cb * b_rows * (b_cols / 8), 256, 8)};
-  cudaError_t e = launch_pdl(f32_planes_kernel, dim3((unsigned)(ja.blocks + jb.blocks)), dim3(256), 0, s, ja, jb);
+  cudaError_t e = launch_pdl(f32_planes_kernel, dim3((unsigned)(ja.blocks + jb.blocks)), dim3(256), 0, s, ja, jb, note, call);
   if (e != cudaSuccess) return cuda_status(e, "matmul_f32x3 planes");
   CUtensorMap ma, mb;
   AG_RETURN_IF_ERROR(make_map(&ma, DType::BF16, pa, (uint64_t)g.k, (uint64_t)g.m, 3, (uint64_t)ca, (uint64_t)g.k, (uint64_t)(g.m * g.k), (uint64_t)(3 * g.m * g.k), kF3Bk, kF3Bm));
@@ -419,6 +469,7 @@ Status matmul_f32x3(cudaStream_t s, const GemmDesc& g, void* workspace) {
   p.splits = f32x3_splits(g.m, g.n, g.k, g.batch); p.kb_per_split = (p.num_kb + p.splits - 1) / p.splits;
   p.c_row = g.c_row; p.c_batch = g.c_batch; p.p_row = (g.n + 3) / 4 * 4; p.status = st;
   p.a = static_cast<const float*>(g.a); p.b = static_cast<const float*>(g.b); p.k = (int)g.k; p.a_row = g.a_row; p.a_batch = g.a_batch; p.b_row = g.b_row; p.b_col = g.b_col; p.b_batch = g.b_batch;
+  p.note = note; p.call = call;
   p.partial = p.splits > 1 ? reinterpret_cast<float*>(ws + f3_pad(6 * ca * g.m * g.k) + f3_pad(6 * cb * g.n * g.k)) : nullptr;
   p.vec = aligned16(g.c) && g.c_row % 4 == 0 && g.c_batch % 4 == 0 && (!g.ep.residual || aligned16(g.ep.residual)) ? 1 : 0;
   static bool attr = false;

@@ -303,7 +303,7 @@ def test_matmul_argmax_epilogue_is_bit_exact_with_matmul_then_argmax(gpu_dev, dt
 @pytest.mark.parametrize("shape_a,shape_b,bt", [((1024, 1024), (1024, 1024), False), ((3, 520, 768), (3, 768, 1032), False), ((2, 1000, 512), (512, 776), False),
                                                 ((2048, 768), (1000, 768), True)])
 def test_matmul_f32_split_precision_on_tensor_cores(gpu_dev, shape_a, shape_b, bt):
-    """float32 products of at least 2 GFLOP: three bf16 terms per operand, six cross terms accumulated in
+    """float32 products large enough for the tensor cores: three bf16 planes per operand, six cross terms accumulated in
     float32 on the tensor cores. Bar: the reference's 1e-4 (python/tests/test_batched_ops.py:20-54); measured
     error is orders of magnitude below it and must match the CUDA-core kernel to 1e-5 of the largest entry."""
     rng = np.random.default_rng(sum(shape_a) + sum(shape_b))
@@ -519,7 +519,7 @@ def test_float32_products_through_bf16_planes(gpu_dev, m, n, k, kmajor):
     assert gpu_dev.pipeline_status() == 0
 
 
-@pytest.mark.parametrize("m,n,k", [(64, 256, 256), (40, 768, 3072)])
+@pytest.mark.parametrize("m,n,k", [(64, 256, 256), (96, 512, 256), (40, 768, 3072)])
 def test_float32_products_keep_infinities_and_nans(gpu_dev, m, n, k):
     """What three bf16 planes cannot hold (infinities, the largest floats, NaN) comes out as the plain sums have it, split K or not."""
     rng = np.random.default_rng(m + n)
@@ -532,6 +532,58 @@ def test_float32_products_keep_infinities_and_nans(gpu_dev, m, n, k):
     assert np.array_equal(np.isnan(got), np.isnan(ref)) and np.array_equal(np.isinf(got), np.isinf(ref)) and np.array_equal(np.sign(got[np.isinf(got)]), np.sign(ref[np.isinf(ref)]))
     ok = np.isfinite(ref)
     assert np.all(np.abs(got[ok] - ref[ok]) <= 4e-6 * np.sqrt(k) + 1e-5 * np.abs(ref[ok]))
+
+
+@pytest.mark.parametrize("m,n,k,fill", [(256, 256, 2048, "nan"), (256, 256, 2048, "inf"), (256, 384, 2048, "overflow"), (40, 768, 3072, "nan")])
+def test_float32_products_of_values_that_are_not_finite_take_no_longer(gpu_dev, m, n, k, fill):
+    """A whole operand of NaN, of infinities, or of numbers whose products overflow: right, and at the speed of any other (measured within
+    a tenth of it; what took each such element again in a loop over K took hundreds of times as long)."""
+    import time
+    rng = np.random.default_rng(k)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.uniform(0.5, 2.0, (k, n)).astype(np.float32)
+    odd = np.full((m, k), {"nan": np.nan, "inf": np.inf, "overflow": 3e38}[fill], np.float32)
+    gb, times = gpu_dev.from_numpy(b), []
+    for x in (a, odd):
+        gx = gpu_dev.from_numpy(x)
+        got = (gx @ gb).to_numpy()
+        gpu_dev.synchronize()
+        best = 1e9
+        for _ in range(5):
+            t0 = time.perf_counter()
+            (gx @ gb).eval()
+            gpu_dev.synchronize()
+            best = min(best, time.perf_counter() - t0)
+        times.append(best)
+    assert np.all(np.isnan(got)) if fill == "nan" else np.all(got == np.inf)
+    assert times[1] <= 3 * times[0] + 1e-3, times
+    assert gpu_dev.pipeline_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(96, 512, 256), (300, 264, 776)])
+def test_float32_products_of_infinities_with_any_partner(gpu_dev, m, n, k):
+    """An infinity, or the largest number, against numbers whose lower planes are zero or of the other sign, zeros and infinities."""
+    rng = np.random.default_rng(m)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    big = np.finfo(np.float32).max
+    a[:12, 3] = np.array([np.inf, -np.inf, big, -big, 3.397e38, 3.39e38, np.nan, 0, 1, -1, 1e-30, 257 / 256], np.float32)
+    b[3] /= 16                                            # a float32 sum that overflows on the way has no value apart from its order
+    b[3, :10] = np.array([1, 257 / 256, -1 + 2 ** -9, 0, np.inf, -np.inf, 1 - 2 ** -20, 1e-30, np.nan, 2 ** -10], np.float32) / 4
+    b[7, 4], a[1, 7] = np.inf, 1
+    got = (gpu_dev.from_numpy(a) @ gpu_dev.from_numpy(b)).to_numpy()
+    with np.errstate(all="ignore"):
+        ref = (a.astype(np.float64) @ b.astype(np.float64)).astype(np.float32)
+    assert np.array_equal(np.isnan(got), np.isnan(ref)) and np.array_equal(np.isinf(got), np.isinf(ref)) and np.array_equal(np.sign(got[np.isinf(got)]), np.sign(ref[np.isinf(ref)]))
+    ok = np.isfinite(ref)
+    assert np.all(np.abs(got[ok] - ref[ok]) <= 4e-6 * np.sqrt(k) + 1e-5 * np.abs(ref[ok]))
+
+
+@pytest.mark.parametrize("small,bound", [(1e-30, 2.0 ** -21), (1e-34, 2.0 ** -19), (1e-36, 2.0 ** -14), (1e-37, 2.0 ** -10)])
+def test_float32_products_of_tiny_and_huge_operands(gpu_dev, small, bound):
+    """Where bf16 ends, an operand keeps 2^-133 absolute: below 6e-36 the third plane goes, below 2e-38 the second."""
+    rng = np.random.default_rng(1)
+    a, b = (rng.uniform(1, 2, (64, 512)) * small).astype(np.float32), (rng.uniform(1, 2, (512, 512)) / small / 512).astype(np.float32)
+    ref = a.astype(np.float64) @ b.astype(np.float64)
+    assert np.max(np.abs((gpu_dev.from_numpy(a) @ gpu_dev.from_numpy(b)).to_numpy() - ref) / ref) <= bound
 
 
 def test_float32_product_without_room_for_its_planes(gpu_dev):
