@@ -15,7 +15,7 @@
 // accumulation runs over more than kF3Chunk k-blocks: the epilogue warps add the chunks up in registers, rounded to nearest, under the
 // next chunk's products.
 //
-// Tiles of 256 x 128 on CTA pairs (cta_group::2); two accumulator pairs of 2 x 128 TMEM columns, so the epilogue of a tile runs under the
+// Tiles of 256 x 128 on CTA pairs (cta_group::2), 256 x 256 for large products (f3_wide); with the former two accumulator pairs of 2 x 128 TMEM columns, so the epilogue of a tile runs under the
 // next one's products. A product with few tiles also splits K: each share is one unit of the persistent grid, leaves its sum in
 // a workspace, and a second kernel adds the shares in K order and applies the epilogue.
 //
@@ -373,6 +373,199 @@ gemm_f32x3_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
 
+// ── tiles of 256 x 256 ──────────────────────────────────────────────────────
+// A third fewer operand reads per product than in the kernel above, for products that are long in every direction. TMEM then has room for
+// one accumulator of each kind (2 x 256 columns): a0 b0, the first product of a k-block, is drained under the block's small ones, and
+// those, every kFwLowChunk blocks, under the next a0 b0. A slot of the ring is one plane of a k-block's A and B (32 KB), planes in the
+// order 1, 0, 2. Two blocks of a0 b0 in an accumulation leave less truncation than four do (4096^3: 1.6e-7 of the norm off, 2.4e-7 in the
+// kernel above); small products drained as often would cost more in rounded additions than they lose to truncation.
+// What bounds it is the power limit: 8 x 4096^3 takes 4 880 us with the planes' 400, 1.47 PFLOP/s of bf16 products (sustained rate of one
+// plain bf16 product of 8192^3: 1.44).
+constexpr int kFwBn = 256, kFwSlots = 6, kFwTile = kF3Bm * kF3Bk * 2, kFwSlot = 2 * kFwTile;
+constexpr int kFwSmem = kFwSlots * kFwSlot + kF3EpiWarps * kF3Stg + 1024;
+constexpr int kFwChunk = 2, kFwLowChunk = 16;            // k-blocks in one accumulation of a0 b0, of the small products
+static_assert(kFwLowChunk % kFwChunk == 0, "the two drains meet");
+constexpr int kFwBand = 8;                // row blocks that share a walk over the column blocks
+static_assert(kFwSmem + 512 <= 232448, "shared memory of a CTA");
+
+template <bool B_MN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kF3Threads, 1)
+gemm_f32x3_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ F3Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t full_bar[kFwSlots], empty_bar[kFwSlots], hi_full, hi_empty, lo_full, lo_empty;
+  __shared__ uint32_t tmem_base_slot;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int tiles = p.tiles_m * p.tiles_n;
+  const long long units = (long long)tiles * p.batch, first = blockIdx.x >> 1, step = gridDim.x >> 1;
+  auto unit = [&](long long u, int& m0, int& n0, int& b) {
+    b = (int)(u / tiles);
+    const int t = (int)(u % tiles), band = t / (kFwBand * p.tiles_n), r = t - band * kFwBand * p.tiles_n, high = min(kFwBand, p.tiles_m - band * kFwBand);
+    m0 = (band * kFwBand + r % high) * 2 * kF3Bm + (int)rank * kF3Bm;
+    n0 = r / high * kFwBn;
+  };
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kFwSlots; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    mbar_init(&hi_full, 1); mbar_init(&lo_full, 1);
+    mbar_init(&hi_empty, 2 * kF3EpiWarps); mbar_init(&lo_empty, 2 * kF3EpiWarps);
+    mbar_fence_init();
+    prefetch_tmap(&tmap_a);
+    prefetch_tmap(&tmap_b);
+  }
+  if (warp == 1) { tmem_alloc_pair(&tmem_base_slot, 512); tmem_relinquish_pair(); }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = tmem_base_slot;
+  pdl_wait();
+  pdl_trigger();
+  int m0, n0, b;
+
+  if (warp == 0) {
+    if (lane == 0) {                                   // loads
+      int slot = 0; uint32_t phase = 0;
+      bool ok = true;
+      for (long long u = first; u < units && ok; u += step) {
+        unit(u, m0, n0, b);
+        const int nh = n0 + (int)rank * (kFwBn / 2), ba = p.a_one ? 0 : b, bb = p.b_one ? 0 : b;
+        for (int kb = 0; kb < p.num_kb && ok; kb++) {
+          for (int i = 0; i < 3; i++) {
+            const int q = i == 2 ? 2 : 1 - i;
+            if (!mbar_wait(&empty_bar[slot], phase ^ 1, p.status, 5)) { ok = false; break; }
+            if (rank == 0) mbar_expect_tx(&full_bar[slot], 2 * kFwSlot);
+            const uint32_t bar = mapa_u32(smem_u32(&full_bar[slot]), 0);
+            uint8_t* sa = smem + slot * kFwSlot;
+            uint8_t* sb = sa + kFwTile;
+            tma_load_4d_pair(sa, &tmap_a, bar, kb * kF3Bk, m0, q, ba);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              if (B_MN) tma_load_4d_pair(sb + h * (kFwTile / 2), &tmap_b, bar, nh + h * 64, kb * kF3Bk, q, bb);
+              else tma_load_4d_pair(sb + h * (kFwTile / 2), &tmap_b, bar, kb * kF3Bk, nh + h * 64, q, bb);
+            }
+            if (++slot == kFwSlots) { slot = 0; phase ^= 1; }
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {                      // products
+      constexpr uint32_t idesc = make_idesc_f16(1, 0, B_MN ? 1 : 0, 2 * kF3Bm, kFwBn);
+      const uint64_t a0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024), b0 = make_smem_desc_sw128(smem_u32(smem) + kFwTile, B_MN ? 64 * 128 : 16, 1024);
+      const uint32_t ah = (uint32_t)(a0 >> 32), bh = (uint32_t)(b0 >> 32), al = (uint32_t)a0, bl = (uint32_t)b0;
+      const uint32_t d_hi = tmem_base, d_lo = tmem_base + 256;
+      auto products = [&](uint32_t d, int slot_a, int slot_b, uint32_t on) {
+#pragma unroll
+        for (int kk = 0; kk < kF3Bk / 16; kk++)
+          f3_mma(d, al + (uint32_t)((slot_a * kFwSlot + kk * 32) >> 4), ah, bl + (uint32_t)((slot_b * kFwSlot + kk * (B_MN ? 16 * 128 : 32)) >> 4), bh, idesc, kk ? 1u : on);
+      };
+      auto done = [&](uint64_t* bar) {                 // to both CTAs, once the products so far are done
+        const uint32_t at = smem_u32(bar);
+        mma_commit_pair(mapa_u32(at, 0));
+        mma_commit_pair(mapa_u32(at, 1));
+      };
+      int slot = 0; uint32_t phase = 0, hi_phase = 0, lo_phase = 0;
+      auto next = [&]() { const int s = slot; if (++slot == kFwSlots) { slot = 0; phase ^= 1; } return s; };
+      auto arrived = [&]() {
+        const bool here = mbar_wait(&full_bar[slot], phase, p.status, 7);
+        tc_fence_after_sync();
+        return here;
+      };
+      bool ok = true;
+      for (long long u = first; u < units && ok; u += step) {
+        for (int kb = 0; kb < p.num_kb; kb++) {
+          if (!arrived()) { ok = false; break; }
+          const int s1 = next();
+          if (!arrived()) { ok = false; break; }
+          const int s0 = next();
+          if (kb % kFwChunk == 0) {
+            if (!mbar_wait(&hi_empty, hi_phase ^ 1, p.status, 6)) { ok = false; break; }
+            hi_phase ^= 1;
+            tc_fence_after_sync();
+          }
+          products(d_hi, s0, s0, kb % kFwChunk ? 1u : 0u);
+          if (kb % kFwChunk == kFwChunk - 1 || kb + 1 == p.num_kb) done(&hi_full);
+          if (kb % kFwLowChunk == 0) {
+            if (!mbar_wait(&lo_empty, lo_phase ^ 1, p.status, 6)) { ok = false; break; }
+            lo_phase ^= 1;
+            tc_fence_after_sync();
+          }
+          products(d_lo, s1, s1, kb % kFwLowChunk ? 1u : 0u);
+          products(d_lo, s1, s0, 1u);
+          products(d_lo, s0, s1, 1u);
+          done(&empty_bar[s1]);
+          if (!arrived()) { ok = false; break; }
+          const int s2 = next();
+          products(d_lo, s2, s0, 1u);
+          products(d_lo, s0, s2, 1u);
+          done(&empty_bar[s0]);
+          done(&empty_bar[s2]);
+          if (kb % kFwLowChunk == kFwLowChunk - 1 || kb + 1 == p.num_kb) done(&lo_full);
+        }
+      }
+    }
+  } else {                                             // epilogue: a warp has 32 rows of its CTA and 128 of the tile's columns
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    float* stg = reinterpret_cast<float*>(smem + kFwSlots * kFwSlot) + (warp - 2) * (32 * kF3StgPitch);
+    const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 128);
+    uint32_t hi_phase = 0, lo_phase = 0;
+    bool ok = true;
+    for (long long u = first; u < units; u += step) {
+      unit(u, m0, n0, b);
+      const long long row0 = m0 + quarter * 32;
+      float sum[4][32];
+#pragma unroll
+      for (int g = 0; g < 4; g++)
+#pragma unroll
+        for (int e = 0; e < 32; e++) sum[g][e] = 0.f;
+      for (int kc = 0; kc < p.num_kb; kc += kFwChunk) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&hi_full, hi_phase, p.status, 8))) { ok = false; break; }
+        hi_phase ^= 1;
+        tc_fence_after_sync();
+#pragma unroll
+        for (int g = 0; g < 8; g++) {                  // 16 columns at a time: the sums take 128 of 168 registers
+          uint32_t hi[16];
+          tmem_ld_32x16(taddr + g * 16, hi);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 16; e++) sum[g / 2][g % 2 * 16 + e] += __uint_as_float(hi[e]);
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&hi_empty), 0));
+        if ((kc + kFwChunk) % kFwLowChunk && kc + kFwChunk < p.num_kb) continue;
+        if (!__all_sync(0xffffffffu, mbar_wait(&lo_full, lo_phase, p.status, 8))) { ok = false; break; }
+        lo_phase ^= 1;
+        tc_fence_after_sync();
+#pragma unroll
+        for (int g = 0; g < 8; g++) {
+          uint32_t lo[16];
+          tmem_ld_32x16(taddr + 256 + g * 16, lo);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 16; e++) if (isfinite(sum[g / 2][g % 2 * 16 + e])) sum[g / 2][g % 2 * 16 + e] += __uint_as_float(lo[e]);
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&lo_empty), 0));
+      }
+      if (!ok) break;
+#pragma unroll
+      for (int g = 0; g < 4; g++) {
+        const int col0 = n0 + half * 128 + g * 32;
+        if (row0 >= p.m || col0 >= p.n) continue;      // uniform across the warp
+        f3_store(p, sum[g], b, row0, col0, p.bias && col0 + lane < p.n ? __ldg(p.bias + col0 + lane) : 0.f, stg);
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();      // neither CTA leaves while its peer can still signal its barriers or run MMAs on its shared memory
+  tc_fence_after_sync();
+  if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
+}
+
 // The shares of K added in order, then what the single-launch epilogue does.
 __global__ void __launch_bounds__(256) f32x3_finish_kernel(const __grid_constant__ F3Params p) {
   pdl_wait();
@@ -426,6 +619,14 @@ int f32x3_splits(int64_t m, int64_t n, int64_t k, int64_t batch) {
   return best;
 }
 
+// Tiles of 256 x 256 from K = 1024 and three rounds of the grid on. Measured (narrow -> wide, us): 8 x 1536^3 318 -> 306, 16384 x 1024 x 1024
+// 224 -> 198, 4096^3 648 -> 643, 8 x 4096^3 5 809 -> 4 880, 8192^3 5 980 -> 4 600 (a six-fold K extent: 5 857, 5 776); on the other side of the
+// line 8 x 1024^3 109 -> 112 (128 tiles), 8192 x 3072 x 768 186 -> 212, 8192 x 50264 x 768 2 849 -> 2 905 (nothing runs under the end of a tile).
+static bool f3_wide(const GemmDesc& g) {
+  const int64_t tiles = (g.m + 2 * kF3Bm - 1) / (2 * kF3Bm) * ((g.n + kFwBn - 1) / kFwBn) * g.batch;
+  return g.k >= 1024 && tiles >= 3 * (sm_count() / 2);
+}
+
 // float32 A [m, k] with rows along k; B [k, n] with either dimension along its rows; bytes of the workspace for the planes and shares
 bool f32x3_eligible(const GemmDesc& g) {
   if (g.dtype != DType::F32 || g.b_dtype != DType::F32 || g.batch_inner != 1 || g.k % 8 || g.a_col != 1 || g.a_row % 4 || g.a_batch % 4 || g.b_batch % 4) return false;
@@ -438,7 +639,7 @@ bool f32x3_eligible(const GemmDesc& g) {
 static int64_t f3_pad(int64_t bytes) { return (bytes + 255) / 256 * 256; }
 int64_t f32x3_workspace(const GemmDesc& g) {
   const int64_t ca = g.batch > 1 && g.a_batch ? g.batch : 1, cb = g.batch > 1 && g.b_batch ? g.batch : 1;
-  const int s = f32x3_splits(g.m, g.n, g.k, g.batch);
+  const int s = f3_wide(g) ? 1 : f32x3_splits(g.m, g.n, g.k, g.batch);
   return 256 + f3_pad(6 * ca * g.m * g.k) + f3_pad(6 * cb * g.n * g.k) + (s > 1 ? (int64_t)s * g.batch * g.m * ((g.n + 3) / 4 * 4) * 4 : 0);
 }
 
@@ -447,7 +648,7 @@ Status matmul_f32x3(cudaStream_t s, const GemmDesc& g, void* workspace) {
   int* st = matmul_status_word();
   if (!st) return Status::compute("matmul: the kernel workspace is not initialised");
   const int64_t ca = g.batch > 1 && g.a_batch ? g.batch : 1, cb = g.batch > 1 && g.b_batch ? g.batch : 1;
-  const bool b_mn = g.b_col == 1;
+  const bool b_mn = g.b_col == 1, wide = f3_wide(g);
   uint8_t* ws = static_cast<uint8_t*>(workspace) + 256;     // in front: the call whose operands hold a finite number beyond bf16
   static std::atomic<unsigned long long> calls{0x9e3779b97f4a7c15ull};      // what a pooled buffer holds is hardly ever the next call's (it would cost time only)
   unsigned long long* note = static_cast<unsigned long long*>(workspace);
@@ -465,8 +666,8 @@ Status matmul_f32x3(cudaStream_t s, const GemmDesc& g, void* workspace) {
   F3Params p;
   p.c = static_cast<float*>(g.c); p.bias = static_cast<const float*>(g.ep.bias); p.residual = static_cast<const float*>(g.ep.residual);
   p.alpha = g.ep.alpha; p.act = (int)g.ep.act; p.m = (int)g.m; p.n = (int)g.n; p.batch = (int)g.batch; p.a_one = ca == 1; p.b_one = cb == 1;
-  p.num_kb = (int)((g.k + kF3Bk - 1) / kF3Bk); p.tiles_m = (int)((g.m + 2 * kF3Bm - 1) / (2 * kF3Bm)); p.tiles_n = (int)((g.n + kF3Bn - 1) / kF3Bn);
-  p.splits = f32x3_splits(g.m, g.n, g.k, g.batch); p.kb_per_split = (p.num_kb + p.splits - 1) / p.splits;
+  p.num_kb = (int)((g.k + kF3Bk - 1) / kF3Bk); p.tiles_m = (int)((g.m + 2 * kF3Bm - 1) / (2 * kF3Bm)); p.tiles_n = (int)((g.n + (wide ? kFwBn : kF3Bn) - 1) / (wide ? kFwBn : kF3Bn));
+  p.splits = wide ? 1 : f32x3_splits(g.m, g.n, g.k, g.batch); p.kb_per_split = (p.num_kb + p.splits - 1) / p.splits;
   p.c_row = g.c_row; p.c_batch = g.c_batch; p.p_row = (g.n + 3) / 4 * 4; p.status = st;
   p.a = static_cast<const float*>(g.a); p.b = static_cast<const float*>(g.b); p.k = (int)g.k; p.a_row = g.a_row; p.a_batch = g.a_batch; p.b_row = g.b_row; p.b_col = g.b_col; p.b_batch = g.b_batch;
   p.note = note; p.call = call;
@@ -476,12 +677,16 @@ Status matmul_f32x3(cudaStream_t s, const GemmDesc& g, void* workspace) {
   if (!attr) {
     e = cudaFuncSetAttribute(gemm_f32x3_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kF3Smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_f32x3_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kF3Smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_f32x3_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_f32x3_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwSmem);
     if (e != cudaSuccess) return cuda_status(e, "matmul_f32x3 smem attribute");
     attr = true;
   }
   const long long units = (long long)p.tiles_m * p.tiles_n * p.batch * p.splits;
   const dim3 grid((unsigned)(2 * std::min<long long>(units, sm_count() / 2)));
-  e = b_mn ? launch_pdl(gemm_f32x3_kernel<true>, grid, dim3(kF3Threads), (size_t)kF3Smem, s, ma, mb, p) : launch_pdl(gemm_f32x3_kernel<false>, grid, dim3(kF3Threads), (size_t)kF3Smem, s, ma, mb, p);
+  if (wide)
+    e = b_mn ? launch_pdl(gemm_f32x3_wide_kernel<true>, grid, dim3(kF3Threads), (size_t)kFwSmem, s, ma, mb, p) : launch_pdl(gemm_f32x3_wide_kernel<false>, grid, dim3(kF3Threads), (size_t)kFwSmem, s, ma, mb, p);
+  else e = b_mn ? launch_pdl(gemm_f32x3_kernel<true>, grid, dim3(kF3Threads), (size_t)kF3Smem, s, ma, mb, p) : launch_pdl(gemm_f32x3_kernel<false>, grid, dim3(kF3Threads), (size_t)kF3Smem, s, ma, mb, p);
   if (e != cudaSuccess) return cuda_status(e, "matmul_f32x3");
   if (p.splits > 1) {
     e = launch_pdl(f32x3_finish_kernel, dim3((unsigned)grid_for((int64_t)p.batch * p.m * (p.p_row / 4), 256, 8)), dim3(256), 0, s, p);

@@ -586,6 +586,39 @@ def test_float32_products_of_tiny_and_huge_operands(gpu_dev, small, bound):
     assert np.max(np.abs((gpu_dev.from_numpy(a) @ gpu_dev.from_numpy(b)).to_numpy() - ref) / ref) <= bound
 
 
+@pytest.mark.parametrize("batch,m,n,k,kmajor", [(1, 3700, 3904, 1024, False), (1, 3841, 3585, 1096, True), (60, 300, 264, 1160, False), (56, 300, 512, 2120, False)])
+def test_large_float32_products(gpu_dev, batch, m, n, k, kmajor):
+    """The 256 x 256 tiles: ragged rows, columns and last k-block, a last band of fewer than eight row blocks, more than one drain of the small
+    products, batches, every epilogue, and infinities, NaN and the largest numbers. The bar of the narrow tiles, and in the norm what those
+    leave (2.4e-7 at K = 2048: 16 truncated additions in each accumulation)."""
+    rng = np.random.default_rng(m + n)
+    a = rng.standard_normal((m, k) if batch == 1 else (batch, m, k)).astype(np.float32)
+    b = rng.standard_normal((n, k) if kmajor else (k, n) if batch == 1 else (batch, k, n)).astype(np.float32)
+    up = lambda x: gpu_dev.transpose(gpu_dev.from_numpy(x)) if kmajor else gpu_dev.from_numpy(x)  # noqa: E731
+    ga, gb, right = gpu_dev.from_numpy(a), up(b), b.T if kmajor else b
+    ref = np.matmul(a.astype(np.float64), right.astype(np.float64))
+    got = (ga @ gb).to_numpy()
+    assert np.max(np.abs(got - ref)) <= 4e-6 * np.sqrt(k)
+    assert np.linalg.norm(got - ref) <= 2.4e-7 * np.linalg.norm(ref)
+    if batch == 1:
+        bias, res = rng.standard_normal(n).astype(np.float32), rng.standard_normal((m, n)).astype(np.float32)
+        y = (gpu_dev.from_numpy(res) + gpu_dev.gelu(gpu_dev.add_bias(ga @ gb, gpu_dev.from_numpy(bias)))).to_numpy()
+        np.testing.assert_allclose(y, R.gelu((ref + bias).astype(np.float32)).astype(np.float64) + res, rtol=1e-4, atol=1e-4)
+        big, rows, cols = np.finfo(np.float32).max, [0, 255, 256, m - 1], [0, 127, 128, n - 1]
+        right[3] /= 16                                    # sums with the largest number stay finite
+        a[:, 7] /= 16
+        a[rows, 3], right[7, cols] = [np.inf, -np.inf, big, np.nan], [np.inf, -big, 1e-38, 0]
+        with np.errstate(all="ignore"):
+            part = np.matmul(a[rows].astype(np.float64), right.astype(np.float64)).astype(np.float32)
+            side = np.matmul(a.astype(np.float64), right[:, cols].astype(np.float64)).astype(np.float32)
+        got = (gpu_dev.from_numpy(a) @ up(b)).to_numpy()
+        for x, want in ((got[rows], part), (got[:, cols], side)):
+            assert np.array_equal(np.isnan(x), np.isnan(want)) and np.array_equal(np.isinf(x), np.isinf(want)) and np.array_equal(np.sign(x[np.isinf(x)]), np.sign(want[np.isinf(want)]))
+            ok = np.isfinite(want)
+            assert np.all(np.abs(x[ok] - want[ok]) <= 4e-6 * np.sqrt(k) + 1e-5 * np.abs(want[ok]))
+    assert gpu_dev.pipeline_status() == 0
+
+
 def test_float32_product_without_room_for_its_planes(gpu_dev):
     """A product of less than 2 GFLOP whose workspace cannot be had is computed all the same; a larger one reports the failure."""
     from applegpu_runtime_b200 import _lib
