@@ -107,14 +107,16 @@ __device__ __noinline__ float4 f3_act(float4 v, int act) {
   }
 }
 
-// n neighbouring results of each lane's row, of which those that are not finite are taken again; a warp adds one up. A unit's results take
-// the epilogue warps well below the second that the other warps wait for them (K = 2^20: 0.7 s if every result is one of them; from there
-// on they stay as they are).
-__device__ __forceinline__ bool f3_again(const F3Params& p) { return __ldcg(p.note) == p.call && p.k <= 1 << 20; }
-__device__ __noinline__ void f3_plain(const F3Params& p, bool in, int b, long long row, int col0, int n, float* v) {
+// n neighbouring results of each lane's row, of which those that are not finite are taken again; a warp adds one up. The other warps wait two
+// seconds at most for the epilogue's, so there a call takes `most` results (kF3Again; all of them up to K = 8192) and reports any beyond:
+// at 92 cycles of an SM for 32 of K, a tile's eight warps with four calls each take half a second.
+constexpr int kF3Again = 1 << 23;         // times K
+__device__ __forceinline__ bool f3_again(const F3Params& p) { return __ldcg(p.note) == p.call; }
+__device__ __noinline__ void f3_plain(const F3Params& p, bool in, int b, long long row, int col0, int n, float* v, int most) {
   const int lane = threadIdx.x & 31;
   for (int e = 0; e < n; e++) {
     for (unsigned again = __ballot_sync(0xffffffffu, in && col0 + e < p.n && !isfinite(v[e])); again; again &= again - 1) {
+      if (most-- == 0) { if (lane == 0) atomicCAS(p.status, 0, 9); return; }
       const int who = __ffs(again) - 1;
       const float* a = p.a + __shfl_sync(0xffffffffu, b, who) * p.a_batch + __shfl_sync(0xffffffffu, row, who) * p.a_row;
       const float* w = p.b + __shfl_sync(0xffffffffu, b, who) * p.b_batch + (__shfl_sync(0xffffffffu, col0, who) + e) * p.b_col;
@@ -138,7 +140,7 @@ __device__ __forceinline__ void f3_store(const F3Params& p, float (&v)[32], int 
     float t[32];
 #pragma unroll
     for (int e = 0; e < 32; e++) t[e] = v[e];
-    f3_plain(p, gm < p.m, b, gm, col0, 32, t);
+    f3_plain(p, gm < p.m, b, gm, col0, 32, t, kF3Again / p.k);
 #pragma unroll
     for (int e = 0; e < 32; e++) v[e] = t[e];
   }
@@ -585,7 +587,7 @@ __global__ void __launch_bounds__(256) f32x3_finish_kernel(const __grid_constant
     const long long at = b * p.c_batch + (row - b * p.m) * p.c_row + col;
     if (look) {
       float t[4] = {v[0], v[1], v[2], v[3]};
-      f3_plain(p, in, (int)b, row - b * p.m, (int)col, 4, t);
+      f3_plain(p, in, (int)b, row - b * p.m, (int)col, 4, t, 0x7fffffff);
 #pragma unroll
       for (int e = 0; e < 4; e++) v[e] = t[e];
     }
