@@ -313,8 +313,12 @@ static Status build_gemm(const TensorRec& a, const TensorRec& b, const TensorRec
 
 // float32 matmul on the tensor cores: three bf16 planes per operand, the six largest cross terms accumulated in float32
 // (kernels/gemm_f32x3.cu). Error is ~2^-22 relative to the exact product (inside the reference's 1e-4 tolerance by three
-// orders of magnitude), against the CUDA-core kernel's ~30 TFLOP/s. Taken for products large enough to pay for the pass
-// that writes the planes and whose layouts the TMA path accepts; *done stays false otherwise.
+// orders of magnitude) where both operands lie above 6e-36, against the CUDA-core kernel's ~30 TFLOP/s. *done stays false otherwise.
+// Taken where the layouts suit the TMA path, us a call, planes against CUDA cores:
+//   from 20 MFLOP and 17 rows: 17 x 768 x 768 12.7 / 51.3, 256 x 64 x 1024 12.7 / 66.4, 512^3 15.9 / 36.9; below, a call is its launches
+//   (128^3, 4 MFLOP: 12.0 / 13.4); at most 16 rows have a kernel that streams the weight (16 x 1024 x 1024: 13.5 / 8.4);
+//   batched from 2 GFLOP and 64 rows: 8 x 512^3 25 / 110; below it depends on the shape (8 x 256^3 15.5 / 21.0, but the scores of an
+//   attention, 96 x 128 x 128 x 64, 18.8 / 14.5) and everything stays on CUDA cores.
 namespace {
 bool g_f32_split = true;
 bool g_pitch_rows = [] { const char* v = std::getenv("APPLEGPU_PITCH_ROWS"); return !(v && v[0] == '0'); }();   // APPLEGPU_PITCH_ROWS=0: always dense outputs
