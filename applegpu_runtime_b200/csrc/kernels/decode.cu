@@ -315,7 +315,7 @@ __device__ __forceinline__ void dl_ask_x(const DecodeLinearParams& p, int k0, Dl
 #pragma unroll
   for (int i = 0; i < kDlPer / Pack<T>::N; i++) r.x[i] = ld16(src + i * Pack<T>::N);
 }
-template <typename T>
+template <typename T, int ROWS = kDlMaxM, bool LN = true>
 __device__ __forceinline__ void dl_put_x(const DecodeLinearParams& p, const DlStats& st, float* sX, int pitch, int k0, const DlX<T>& r) {
   const int m = threadIdx.x >> 4, kk = dl_x_col(k0);
   constexpr int N = Pack<T>::N;
@@ -325,12 +325,13 @@ __device__ __forceinline__ void dl_put_x(const DecodeLinearParams& p, const DlSt
   if (m < p.m && kk < p.k) {
 #pragma unroll
     for (int e = 0; e < kDlPer; e++) v[e] = Cvt<T>::to(r.x[e / N].v[e % N]);
-    if (p.ln_gamma) {
+    if (LN && p.ln_gamma) {
       const float mean = st.mean[m], rstd = st.rstd[m];
 #pragma unroll
       for (int e = 0; e < kDlPer; e++) v[e] = Cvt<T>::to(r.g[e / N].v[e % N]) * (v[e] - mean) * rstd + Cvt<T>::to(r.b[e / N].v[e % N]);
     }
   }
+  if (m >= ROWS) return;
 #pragma unroll
   for (int e = 0; e < kDlPer; e += 4) *reinterpret_cast<float4*>(sX + m * pitch + (threadIdx.x & 15) * kDlPer + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
 }
@@ -369,14 +370,15 @@ __device__ __forceinline__ void dl_put_partials(const DecodeLinearParams& p, flo
 }
 
 // float32 weights: this warp's 16 rows of a slab against the staged x, added to acc (two columns' halves: see dl_store_f32).
-__device__ __forceinline__ void dl_products_f32(const float* sX, int pitch, const uint4 (&wv)[8], float (&acc)[kDlMaxM][4]) {
+template <int ROWS>
+__device__ __forceinline__ void dl_products_f32(const float* sX, int pitch, const uint4 (&wv)[8], float (&acc)[ROWS][4]) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
     const float* at = sX + warp * 16 + i * 2 + (lane >> 4);
     const float* pr = reinterpret_cast<const float*>(&wv[i]);
 #pragma unroll
-    for (int m = 0; m < kDlMaxM; m++) {
+    for (int m = 0; m < ROWS; m++) {
       const float a = at[m * pitch];                         // two addresses per warp (one per half): broadcasts
 #pragma unroll
       for (int e = 0; e < 4; e++) acc[m][e] = fmaf(a, pr[e], acc[m][e]);
@@ -384,10 +386,11 @@ __device__ __forceinline__ void dl_products_f32(const float* sX, int pitch, cons
   }
 }
 // the two half-warps hold different rows of the same columns
-__device__ __forceinline__ void dl_store_f32(float (&acc)[kDlMaxM][4], float (*sSum)[kDlMaxM][kDlSumPitch]) {
+template <int ROWS>
+__device__ __forceinline__ void dl_store_f32(float (&acc)[ROWS][4], float (*sSum)[ROWS][kDlSumPitch]) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-  for (int m = 0; m < kDlMaxM; m++) {
+  for (int m = 0; m < ROWS; m++) {
 #pragma unroll
     for (int e = 0; e < 4; e++) acc[m][e] += __shfl_xor_sync(0xffffffffu, acc[m][e], 16);
     if (lane < 16) *reinterpret_cast<float4*>(&sSum[warp][m][lane * 4]) = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
@@ -682,40 +685,48 @@ __global__ void __launch_bounds__(kDlThreads, LN == 4 ? 3 : 0) decode_linear_ker
   dl_finish<T, NT * 8>(p, n0, rank, ranks, &sSum[0][0][0], sFin);
 }
 
-// float32 weights: the same on CUDA cores, x staged in shared memory.
+// float32 weights: the same on CUDA cores, x staged in shared memory; ROWS of it, eight or sixteen. The slabs of a share behind the first are
+// on their way to the L2 before the dependency wait. A step of GPT-2 small with 1 / 8 / 16 sequences, us: 463 / 579 / 793 with a CTA per
+// slab and partial sums in the L2, 518 / 590 / 780 with clusters and sixteen rows for any batch, now 365 / 442 / 780; four layers of
+// width 2048: 663 / 755 / 1 258, 719 / 812 / 1 303, now 594 / 676 / 1 276.
+template <int ROWS, bool LN>
 __global__ void __launch_bounds__(kDlThreads) decode_linear_f32_kernel(const __grid_constant__ DecodeLinearParams p, int per) {
-  __shared__ __align__(16) float sSum[kDlThreads / 32][kDlMaxM][kDlSumPitch];
-  __shared__ __align__(16) float sBuf[kDlMaxM * (kDlRows + kDlXPad)];       // x, then the shares' sums
-  static_assert(kDlFinRows * kDlCols <= kDlMaxM * (kDlRows + kDlXPad), "the shares' sums take the place of x");
+  __shared__ __align__(16) float sSum[kDlThreads / 32][ROWS][kDlSumPitch];
+  __shared__ __align__(16) float sBuf[ROWS * (kDlRows + kDlXPad)];       // x, then the shares' sums
+  static_assert((ROWS + kDlShares) * kDlCols <= ROWS * (kDlRows + kDlXPad), "the shares' sums take the place of x");
   __shared__ DlStats st;
   const int ranks = gridDim.y, rank = ranks > 1 ? (int)sm100::cluster_ctarank() : 0;
   const int n0 = blockIdx.x * kDlCols, k0 = rank * per * kDlRows;
   uint4 wv[8];
   DlX<float> x;
   dl_load_weights<float>(p, n0, k0, wv);
-  dl_ask_norm<float>(p, k0, x);
+  if constexpr (LN) dl_ask_norm<float>(p, k0, x);
+  for (int s = 1; s < per; s++) {                          // 256 bytes of each of 128 rows
+    const int kk = k0 + s * kDlRows + (threadIdx.x >> 1), col = n0 + (threadIdx.x & 1) * 32;
+    if (kk < p.k && col < p.n) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const float*>(p.w) + (long long)kk * p.w_row + col));
+  }
   pdl_wait();
   pdl_trigger();
   dl_ask_x<float>(p, k0, x);
-  if (p.ln_gamma) dl_ln_stats<float>(p, st);
-  float acc[kDlMaxM][4];
+  if constexpr (LN) dl_ln_stats<float>(p, st);
+  float acc[ROWS][4];
 #pragma unroll
-  for (int m = 0; m < kDlMaxM; m++) { acc[m][0] = 0.f; acc[m][1] = 0.f; acc[m][2] = 0.f; acc[m][3] = 0.f; }
+  for (int m = 0; m < ROWS; m++) { acc[m][0] = 0.f; acc[m][1] = 0.f; acc[m][2] = 0.f; acc[m][3] = 0.f; }
   for (int s = 0; s < per; s++) {
     if (s) {
       __syncthreads();
       dl_load_weights<float>(p, n0, k0 + s * kDlRows, wv);
-      dl_ask_norm<float>(p, k0 + s * kDlRows, x);
+      if constexpr (LN) dl_ask_norm<float>(p, k0 + s * kDlRows, x);
       dl_ask_x<float>(p, k0 + s * kDlRows, x);
     }
-    dl_put_x<float>(p, st, sBuf, kDlRows + kDlXPad, k0 + s * kDlRows, x);
+    dl_put_x<float, ROWS, LN>(p, st, sBuf, kDlRows + kDlXPad, k0 + s * kDlRows, x);
     __syncthreads();
     dl_products_f32(sBuf, kDlRows + kDlXPad, wv, acc);
   }
   dl_store_f32(acc, sSum);
   __syncthreads();
   if (ranks > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");     // every CTA is done with its x
-  dl_finish<float, kDlMaxM>(p, n0, rank, ranks, &sSum[0][0][0], sBuf);
+  dl_finish<float, ROWS>(p, n0, rank, ranks, &sSum[0][0][0], sBuf);
 }
 
 
@@ -749,6 +760,11 @@ static cudaError_t launch_dl16(cudaStream_t s, const DecodeLinearParams& p, int 
   return p.k <= 1024 ? launch_dl(s, decode_linear_kernel<T, NT, 1, 4>, p, per, ranks) : launch_dl(s, decode_linear_kernel<T, NT, 1, 8>, p, per, ranks);
 }
 
+template <int ROWS>
+static cudaError_t launch_dl_f32(cudaStream_t s, const DecodeLinearParams& p, int per, int ranks) {
+  return p.ln_gamma ? launch_dl(s, decode_linear_f32_kernel<ROWS, true>, p, per, ranks) : launch_dl(s, decode_linear_f32_kernel<ROWS, false>, p, per, ranks);
+}
+
 Status decode_linear(cudaStream_t s, const GemmDesc& d) {
   if (!decode_linear_eligible(d)) return Status::invalid("decode_linear: shape or layout not supported");
   DecodeLinearParams p;
@@ -757,7 +773,7 @@ Status decode_linear(cudaStream_t s, const GemmDesc& d) {
   p.x_row = d.a_row; p.w_row = d.b_row; p.y_row = d.c_row; p.partial = nullptr;
   const int per = dl_per((int)((d.k + kDlRows - 1) / kDlRows)), ranks = dl_shares((int)d.k);
   cudaError_t e;
-  if (d.dtype == DType::F32) e = launch_dl(s, decode_linear_f32_kernel, p, per, ranks);
+  if (d.dtype == DType::F32) e = d.m <= 8 ? launch_dl_f32<8>(s, p, per, ranks) : launch_dl_f32<16>(s, p, per, ranks);
   else if (d.dtype == DType::BF16) e = d.m <= 8 ? launch_dl16<__nv_bfloat16, 1>(s, p, per, ranks) : launch_dl16<__nv_bfloat16, 2>(s, p, per, ranks);
   else e = d.m <= 8 ? launch_dl16<__half, 1>(s, p, per, ranks) : launch_dl16<__half, 2>(s, p, per, ranks);
   return cuda_status(e, "decode_linear");
