@@ -687,8 +687,8 @@ __global__ void __launch_bounds__(kDlThreads, LN == 4 ? 3 : 0) decode_linear_ker
 
 // float32 weights: the same on CUDA cores, x staged in shared memory; ROWS of it, eight or sixteen. The slabs of a share behind the first are
 // on their way to the L2 before the dependency wait. A step of GPT-2 small with 1 / 8 / 16 sequences, us: 463 / 579 / 793 with a CTA per
-// slab and partial sums in the L2, 518 / 590 / 780 with clusters and sixteen rows for any batch, now 365 / 442 / 780; four layers of
-// width 2048: 663 / 755 / 1 258, 719 / 812 / 1 303, now 594 / 676 / 1 276.
+// slab and partial sums in the L2, 518 / 590 / 780 with clusters and sixteen rows for any batch, now 372 / 444 / 808 (a box
+// 2 % slower); four layers of width 2048: 663 / 755 / 1 258, 719 / 812 / 1 303, now 619 / 677 / 1 178.
 template <int ROWS, bool LN>
 __global__ void __launch_bounds__(kDlThreads) decode_linear_f32_kernel(const __grid_constant__ DecodeLinearParams p, int per) {
   __shared__ __align__(16) float sSum[kDlThreads / 32][ROWS][kDlSumPitch];
