@@ -147,6 +147,24 @@ def test_matmul_cta_pair_batched_and_epilogues(gpu_dev, pair_path):
     assert rel_err(y2, x.astype(np.float64) @ w.astype(np.float64) + bias + res) <= 1.5e-2
 
 
+@pytest.mark.parametrize("dtype,m,n,k,tile", [("bfloat16", 23900, 520, 1024, "pair256"), ("float16", 33001, 264, 768, "pair128"), ("bfloat16", 24000, 200, 1032, "pair256"),
+                                              ("bfloat16", 2049, 264, 12288, "pair256")])
+def test_cta_pair_tiles_in_bands(gpu_dev, dtype, m, n, k, tile):
+    """More rows than the L2 keeps: row tiles in bands, the last one shorter (and bands of eight tiles at the least)."""
+    import torch
+    t = {"bfloat16": torch.bfloat16, "float16": torch.float16}[dtype]
+    g = torch.Generator("cuda").manual_seed(m)
+    a, b = torch.randn((m, k), generator=g, device="cuda").to(t), torch.randn((k, n), generator=g, device="cuda").to(t)
+    gpu_dev.set_gemm_tile(tile)
+    try:
+        got = (gpu_dev.from_torch(a) @ gpu_dev.from_torch(b)).to_numpy().astype(np.float64)
+    finally:
+        gpu_dev.set_gemm_tile("auto")
+    ref = (a.double() @ b.double()).cpu().numpy()
+    # one rounding to the type (half a step: 2^-9 of the value in bfloat16) and float32 sums of k terms
+    assert rel_err(got, ref) <= 2.0 ** -8
+
+
 def test_matmul_half_batched_and_broadcast(gpu_dev):
     rng = np.random.default_rng(5)
     a = rng.standard_normal((6, 200, 64)).astype(np.float32); b = rng.standard_normal((6, 64, 136)).astype(np.float32)
