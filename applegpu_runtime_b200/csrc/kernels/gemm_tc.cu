@@ -109,13 +109,15 @@ template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) 
 
 // 256-bit global accesses (sm_100): one lane moves 32 contiguous bytes, a whole L2 sector. With one output row per
 // lane (the layout tcgen05.ld delivers) a lane's 32 columns of 16-bit results are two such stores, every sector is
-// written in full, and nothing has to be transposed through shared memory first.
+// written in full, and nothing has to be transposed through shared memory first. Neither results nor residual rows are
+// touched twice by an SM, so they are kept out of its L1: 16384 x 1280 x 1280 with residual 55.8 -> 50.7 us, 131072 x 768 x 768
+// 190 -> 159, the four linears of a block in one launch 115 -> 110. (The same stores as eight rows of 128 bytes each gained no more.)
 __device__ __forceinline__ void st_global_256(void* ptr, const uint32_t* r) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+  asm volatile("st.global.L1::no_allocate.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                ::"l"(ptr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 __device__ __forceinline__ void ld_global_256(const void* ptr, uint32_t* r) {
-  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+  asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "l"(ptr));
 }
 
@@ -724,6 +726,142 @@ __device__ __forceinline__ void epilogue_group(const TcParams& p, uint32_t taddr
   __syncwarp();
 }
 
+// The packed epilogue in units of 16 columns, for kernels with four epilogue warps per TMEM lane quarter: accumulators of one
+// unit -> registers -> epilogue math (two columns per instruction) -> one 256-bit store of this lane's row. The operations and
+// their order are those of epilogue_group's packed path; `crow` and `rrow` point at the row's first column of the unit.
+// An epilogue is a chain of latencies (tensor memory, shared memory, the store queue) beside a main loop that leaves most issue
+// slots free, so what it takes is warps: sixteen of them with 16 columns at a time fit 96 registers each, eight with 32 columns
+// take 168. Eight against sixteen warps, us, rows x N x K in bf16: 8192 x 2304 x 768 29.7 / 26.7, 8192 x 768 x 768 with residual
+// 20.5 / 17.3, 131072 x 3072 x 768 with GELU (in bands) 592 / 540, 16384 x 1280 x 1280 with residual 58.0 / 50.7, 8192 x 50257 x
+// 768 529 / 496; K >= 2048 and full tiles are equal, 16384 x 5120 x 1280 with GELU 161.6 / 164.7.
+template <typename T>
+__device__ __forceinline__ void epilogue_unit(const TcParams& p, uint32_t taddr, const float* bias_f, const float* scale_s, T* crow, const T* rrow, bool in_rows,
+                                              int col0, float ln_mean, float ln_rstd, float& row_sum, float& row_sq) {
+  const bool whole = col0 + 16 <= p.n;
+  uint32_t res[8];
+  if (rrow) {                                               // in flight beside the accumulators
+    if (in_rows && whole) ld_global_256(rrow, res);
+    else {
+      alignas(16) T tmp[16];
+#pragma unroll
+      for (int e = 0; e < 16; e++) tmp[e] = (in_rows && col0 + e < p.n) ? rrow[e] : Cvt<T>::from(0.f);
+#pragma unroll
+      for (int w = 0; w < 8; w++) res[w] = reinterpret_cast<const uint32_t*>(tmp)[w];
+    }
+  }
+  uint32_t acc[16];
+  tmem_ld_32x16(taddr, acc);
+  tmem_ld_wait();
+  uint64_t vp[8];
+#pragma unroll
+  for (int w = 0; w < 8; w++) vp[w] = pack_f32x2(__uint_as_float(acc[2 * w]), __uint_as_float(acc[2 * w + 1]));
+  if (p.alpha != 1.0f) {
+    const uint64_t a2 = pack_f32x2(p.alpha, p.alpha);
+#pragma unroll
+    for (int w = 0; w < 8; w++) vp[w] = mul_f32x2(vp[w], a2);
+  }
+  if (p.ln_stats) {
+    const uint64_t r2 = pack_f32x2(ln_rstd, ln_rstd), sh2 = pack_f32x2(ln_mean, ln_mean);
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      const ulonglong2 cs = *reinterpret_cast<const ulonglong2*>(scale_s + g * 4);   // same address in every lane: a broadcast
+      const ulonglong2 bb = *reinterpret_cast<const ulonglong2*>(bias_f + g * 4);
+      vp[2 * g] = fma_f32x2(vp[2 * g], r2, fma_f32x2(cs.x, sh2, bb.x));
+      vp[2 * g + 1] = fma_f32x2(vp[2 * g + 1], r2, fma_f32x2(cs.y, sh2, bb.y));
+    }
+  } else {
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      const ulonglong2 bb = *reinterpret_cast<const ulonglong2*>(bias_f + g * 4);
+      if (scale_s) {
+        const ulonglong2 sc = *reinterpret_cast<const ulonglong2*>(scale_s + g * 4);
+        vp[2 * g] = fma_f32x2(vp[2 * g], sc.x, bb.x);
+        vp[2 * g + 1] = fma_f32x2(vp[2 * g + 1], sc.y, bb.y);
+      } else {
+        vp[2 * g] = add_f32x2(vp[2 * g], bb.x);
+        vp[2 * g + 1] = add_f32x2(vp[2 * g + 1], bb.y);
+      }
+    }
+  }
+  if ((Act)p.act == Act::GeluTanh && std::is_same<T, __nv_bfloat16>::value) {
+    const uint64_t c0 = pack_f32x2(0.7978845608f, 0.7978845608f), c1 = pack_f32x2(0.0356774081f, 0.0356774081f), half2v = pack_f32x2(0.5f, 0.5f);
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+      const uint64_t x = vp[w];
+      const uint64_t u = mul_f32x2(x, fma_f32x2(mul_f32x2(x, x), c1, c0));
+      float u0, u1, t0, t1;
+      unpack_f32x2(u, u0, u1);
+      asm("tanh.approx.f32 %0, %1;" : "=f"(t0) : "f"(u0));
+      asm("tanh.approx.f32 %0, %1;" : "=f"(t1) : "f"(u1));
+      const uint64_t hx = mul_f32x2(x, half2v);
+      vp[w] = fma_f32x2(hx, pack_f32x2(t0, t1), hx);
+    }
+  } else if ((Act)p.act == Act::GeluErf && std::is_same<T, __nv_bfloat16>::value) {
+    const uint64_t c1 = pack_f32x2(7.97458471e-1f, 7.97458471e-1f), c3 = pack_f32x2(3.70503451e-2f, 3.70503451e-2f),
+                   c5 = pack_f32x2(-3.58732362e-4f, -3.58732362e-4f), half2v = pack_f32x2(0.5f, 0.5f);
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+      const uint64_t x = vp[w];
+      float a, b;
+      unpack_f32x2(x, a, b);
+      const uint64_t xc = pack_f32x2(fminf(fmaxf(a, -8.0f), 8.0f), fminf(fmaxf(b, -8.0f), 8.0f));
+      const uint64_t x2 = mul_f32x2(xc, xc);
+      const uint64_t u = mul_f32x2(xc, fma_f32x2(fma_f32x2(c5, x2, c3), x2, c1));
+      float u0, u1, t0, t1;
+      unpack_f32x2(u, u0, u1);
+      asm("tanh.approx.f32 %0, %1;" : "=f"(t0) : "f"(u0));
+      asm("tanh.approx.f32 %0, %1;" : "=f"(t1) : "f"(u1));
+      const uint64_t hx = mul_f32x2(x, half2v);
+      vp[w] = fma_f32x2(hx, pack_f32x2(t0, t1), hx);
+    }
+  } else if ((Act)p.act != Act::None) {
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+      float a, b;
+      unpack_f32x2(vp[w], a, b);
+      if ((Act)p.act == Act::GeluTanh) { a = gelu_tanh_f(a); b = gelu_tanh_f(b); }
+      else if ((Act)p.act == Act::GeluErf) { a = gelu_erf_fast_f(a); b = gelu_erf_fast_f(b); }
+      else if ((Act)p.act == Act::Relu) { a = fmaxf(a, 0.f); b = fmaxf(b, 0.f); }
+      vp[w] = pack_f32x2(a, b);
+    }
+  }
+  if (rrow) {
+#pragma unroll
+    for (int w = 0; w < 8; w++) vp[w] = add_f32x2(vp[w], widen2<T>(res[w]));
+  }
+  if (p.stats_out) {
+    uint64_t s2 = 0, q2 = 0;    // the bit pattern of (0.f, 0.f)
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+      uint64_t x = vp[w];
+      if (!whole) {
+        float a, b;
+        unpack_f32x2(x, a, b);
+        x = pack_f32x2(col0 + 2 * w < p.n ? a : 0.f, col0 + 2 * w + 1 < p.n ? b : 0.f);
+      }
+      s2 = add_f32x2(s2, x); q2 = fma_f32x2(x, x, q2);
+    }
+    float s0, s1, q0, q1;
+    unpack_f32x2(s2, s0, s1); unpack_f32x2(q2, q0, q1);
+    row_sum += s0 + s1; row_sq += q0 + q1;
+  }
+  uint32_t o[8];
+#pragma unroll
+  for (int w = 0; w < 8; w++) {
+    float a, b;
+    unpack_f32x2(vp[w], a, b);
+    o[w] = pack2<T>(a, b);
+  }
+  if (in_rows) {
+    if (whole) st_global_256(crow, o);
+    else {
+      const T* tv = reinterpret_cast<const T*>(o);
+#pragma unroll
+      for (int e = 0; e < 16; e++) if (col0 + e < p.n) crow[e] = tv[e];
+    }
+  }
+}
+
 template <int BN, bool B_MN, typename T>
 __global__ void __launch_bounds__(kTcThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const TcParams p) {
@@ -951,7 +1089,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 //   full barriers     live in the even CTA; both CTAs' TMA loads credit their bytes there
 //   empty/tmem_full   one copy per CTA; the even CTA's MMA thread commits to both
 //   tmem_empty        lives in the even CTA; the epilogue warps of both CTAs arrive there
-// Everything else (warp roles, epilogue, bounded waits) is as in the single-CTA kernel.
+// Everything else (warp roles, bounded waits) is as in the single-CTA kernel; the common epilogue has sixteen warps (epilogue_unit).
 constexpr int kPairKbPerStage = 2;
 template <int BN> struct PairCfg {
   static constexpr int kABytes = BM * BK * 2;               // this CTA's 128 rows of A, one k-block
@@ -974,7 +1112,11 @@ template <int BN> struct PairCfg {
 // per-channel scales multiply the accumulator in the epilogue (exact for per-output-channel scaling), so the
 // only copy of the weights in global memory is the int8 one and no widened copy is ever written there.
 constexpr int kConvWarps = 4;
-constexpr int kTcThreadsW8 = kTcThreads + kConvWarps * 32;
+// Packed: 16-bit rows on 32 bytes, or gated results; general: everything else (staged rows, float32 results, a row argmax) with
+// eight epilogue warps; W8: int8 weights, either epilogue with eight.
+enum PairKind { kPairGeneral = 0, kPairPacked = 1, kPairW8 = 2 };
+constexpr int pair_epi_warps(int kind) { return kind == kPairPacked ? 16 : kEpiWarps; }
+constexpr int pair_threads(int kind) { return 64 + pair_epi_warps(kind) * 32 + (kind == kPairW8 ? kConvWarps * 32 : 0); }
 // Tile `rem` of a batch: bands of p.band row tiles, in a band column tile after column tile (pair_band below).
 __device__ __forceinline__ void pair_tile(const TcParams& p, int rem, int& mi, int& ni) {
   const int per = p.band * p.tiles_n, b = rem / per, r = rem - b * per, high = min(p.band, p.tiles_m - b * p.band);
@@ -1000,10 +1142,12 @@ __device__ __forceinline__ void widen_s8x4(uint32_t w, uint32_t& lo, uint32_t& h
   }
 }
 
-template <int BN, bool B_MN, typename T, bool W8 = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(W8 ? kTcThreadsW8 : kTcThreads, 1)
+template <int BN, bool B_MN, typename T, int KIND>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(KIND), 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const TcParams p) {
   using Cfg = PairCfg<BN>;
+  constexpr bool W8 = KIND == kPairW8, PACKED = KIND == kPairPacked;
+  constexpr int EW = pair_epi_warps(KIND);                  // epilogue warps
   static_assert(!W8 || (BN == 256 && !B_MN), "the int8-weight form takes a K-major [N, K] weight and 256-wide tiles");
   constexpr int STAGES = Cfg::kStages;
   constexpr int KBS = kPairKbPerStage;
@@ -1028,7 +1172,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) { mbar_init(&full_bar[s], W8 ? 1 + 2 * kConvWarps : 1); mbar_init(&empty_bar[s], 1); mbar_init(&raw_bar[s], 1); }
-    for (int a = 0; a < 2; a++) { mbar_init(&tmem_full_bar[a], 1); mbar_init(&tmem_empty_bar[a], 2 * kEpiWarps); }
+    for (int a = 0; a < 2; a++) { mbar_init(&tmem_full_bar[a], 1); mbar_init(&tmem_empty_bar[a], 2 * EW); }
     mbar_fence_init();
     prefetch_tmap(&tmap_a);
     prefetch_tmap(&tmap_b);
@@ -1208,12 +1352,27 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       const longlong2 stats_cur = stats_next;
       stats_next = ln_stats_fetch(p, tile_row(t + tile_step));
       long long c_off = (long long)(batch / p.batch_inner) * p.c_batch + (long long)(batch % p.batch_inner) * p.c_batch_inner;
+      // packed form: this warp's BN / 4 neighbouring columns; their bias and float slots go to its own shared memory as floats
+      constexpr int WC = BN / 4;
+      float* pk_bias = reinterpret_cast<float*>(smem + STAGES * Cfg::kStageBytes) + (warp - 2) * WC;
+      float* pk_scale = pk_bias + EW * WC;
+      const float* pk_fsrc = p.ln_stats ? p.ln_colsum : p.b_scales;
+      if (PACKED) {
+        const T* bias = reinterpret_cast<const T*>(p.bias);
+#pragma unroll
+        for (int i = lane; i < WC; i += 32) {
+          const int ci = n0 + pair * WC + i;
+          pk_bias[i] = (bias && ci < p.n) ? Cvt<T>::to(__ldg(bias + ci)) : 0.f;
+          if (pk_fsrc) pk_scale[i] = ci < p.n ? __ldg(pk_fsrc + ci) : 0.f;
+        }
+      }
       T* bias_s = reinterpret_cast<T*>(smem + STAGES * Cfg::kStageBytes + kStgBytes) + (warp - 2) * epi_slots(BN);
       // 16-bit C with 32-byte aligned rows: the packed epilogue takes the bias as floats; they wait in the warp's staging
       // tile, which that layout leaves unused (zeros when there is no bias)
       const bool packed_epi = p.vec_ok == 2 && !p.c_f32 && !p.argmax_keys;
       float* bias_f = reinterpret_cast<float*>(smem + STAGES * Cfg::kStageBytes + (warp - 2) * kStgBytesPerWarp);
-      if (packed_epi) {
+      if (PACKED) {
+      } else if (packed_epi) {
         const T* bias = reinterpret_cast<const T*>(p.bias);
 #pragma unroll
         for (int gi = 0; gi < BN / 64; gi++) {
@@ -1231,7 +1390,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       float* scale_s = reinterpret_cast<float*>(smem + STAGES * Cfg::kStageBytes + kStgBytes + bias_bytes(BN)) + (warp - 2) * epi_slots(BN);
       // the float slots hold the int8 per-channel scales, or the float32 bias of a float32-output product
       const float* fsrc = p.c_f32 ? reinterpret_cast<const float*>(p.bias) : (p.ln_stats ? p.ln_colsum : p.b_scales);
-      if (fsrc) {
+      if (!PACKED && fsrc) {
 #pragma unroll
         for (int gi = 0; gi < BN / 64; gi++) {
           int ci = n0 + (pair + 2 * gi) * 32 + lane;
@@ -1239,7 +1398,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
       }
       uint32_t rpre[16];
-      if (p.residual && p.vec_ok == 2 && !p.c_f32 && n0 + pair * 32 < p.n)
+      if (!PACKED && p.residual && p.vec_ok == 2 && !p.c_f32 && n0 + pair * 32 < p.n)
         load_residual_row<T>(p, reinterpret_cast<const T*>(p.residual) + c_off, row0 + lane, n0 + pair * 32, rpre);
       // folded layer_norm: this row's statistics are fetched (and turned into scale and shift) before the accumulator wait too
       float ln_mean = 0.f, ln_rstd = 1.f;
@@ -1257,7 +1416,26 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       uint8_t* stg = smem + STAGES * Cfg::kStageBytes + (warp - 2) * kStgBytesPerWarp;
       unsigned long long best_key = 0;
       float row_sum = 0.f, row_sq = 0.f;
-      if (row0 < p.m) {   // a peer CTA whose rows lie past M has nothing to store
+      if (PACKED) {
+        if (row0 < p.m) {
+          const long long gm = row0 + lane;
+          const bool in_rows = gm < p.m;
+          const long long at = c_off + gm * p.c_row + n0 + pair * WC;
+          T* crow = reinterpret_cast<T*>(p.c) + at;
+          const T* rrow = p.residual ? reinterpret_cast<const T*>(p.residual) + at : nullptr;
+          if (p.glu_n) {
+#pragma unroll 1
+            for (int g = pair; g < BN / 32 && n0 + g * 32 < p.n; g += EW / 4) glu_group<T>(p, taddr + (uint32_t)(g * 32), row0, n0 + g * 32, lane);
+          } else
+#pragma unroll 1
+          for (int i = 0; i < WC; i += 16) {
+            const int col0 = n0 + pair * WC + i;
+            if (col0 >= p.n) break;
+            epilogue_unit<T>(p, taddr + (uint32_t)(pair * WC + i), pk_bias + i, pk_fsrc ? pk_scale + i : nullptr, crow + i, rrow ? rrow + i : nullptr, in_rows, col0,
+                             ln_mean, ln_rstd, row_sum, row_sq);
+          }
+        }
+      } else if (row0 < p.m) {   // a peer CTA whose rows lie past M has nothing to store
 #pragma unroll 1
         for (int g = pair, gi = 0; g < BN / 32; g += 2, gi++) {
           if (n0 + g * 32 >= p.n) break;
@@ -1300,11 +1478,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 //   tiles         every product is cut into 256 x 256 tiles, row block by row block; the host deals the tiles of all
 //                 products, in that order, to the CTA pairs (each tile to the pair with the least work so far) and
 //                 every pair walks its own list, so the roles of a pair need no run-time scheduler
-//   dependencies  when the eight epilogue warps of a CTA have stored their parts of a tile they arrive on a shared-memory
+//   dependencies  when the epilogue warps of a CTA have stored their parts of a tile they arrive on a shared-memory
 //                 barrier; the CTA's announcer warp (one thread) waits for it, fences (proxy fence, __threadfence: the
-//                 stores it has observed through the barrier become visible GPU-wide first) and adds 8 to the counter of
+//                 stores it has observed through the barrier become visible GPU-wide first) and adds its epilogue warps to the counter of
 //                 (product, row block), so the fence's latency is not on the epilogue warps' path. The TMA thread of a
-//                 consumer tile waits (bounded) until the producer's row block has all its arrivals (16 per tile), then
+//                 consumer tile waits (bounded) until the producer's row block has all its arrivals (two CTAs a tile), then
 //                 fences the async proxy and loads. A tile only ever waits for tiles earlier in the global order, and every pair takes its
 //                 tiles in that order, so the earliest unfinished tile can always run: no cycle
 //   epilogue      row statistics and residual rows of the next tile are fetched ahead only when its row block is
@@ -1359,12 +1537,11 @@ __device__ __forceinline__ longlong2 ln_stats_fetch_cg(const TcParams& p, long l
   return __ldcg(reinterpret_cast<const longlong2*>(p.ln_stats) + gm);
 }
 
-// Epilogue warps: 8 (two per TMEM lane quarter, alternating column groups, 168 registers each). 4 (one per quarter, every
-// group, 220 registers) was measured at 146 against 112 us per GPT-2-small block: eight groups per tile in series
-// (121 us with its 255-register budget spent on accumulator loads issued a group ahead).
-constexpr int kChainEpiWarps = 8;
-constexpr int kChainGroupStep = kChainEpiWarps / 4;           // column groups between two groups of one warp
-constexpr int kChainGroups = 8 / kChainGroupStep;             // 32-column groups of a 256-wide tile per warp
+// Epilogue warps: 16, as in the CTA-pair kernel (so that row statistics add up in the same groups: results are those of separate
+// launches bit by bit). 8 with 32 columns at a time took 109 us per GPT-2-small block, 16 take 110; 4 (220 registers) took 146.
+constexpr int kChainEpiWarps = 16;
+constexpr int kChainCols = 256 * 4 / kChainEpiWarps;          // neighbouring columns of a 256-wide tile per warp
+constexpr int kChainGroups = kChainCols / 32;
 constexpr int kChainThreads = 64 + kChainEpiWarps * 32 + 32;  // TMA warp, MMA warp, epilogue warps, announcer warp
 template <typename T>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kChainThreads, 1)
@@ -1378,7 +1555,7 @@ gemm_tc_chain_kernel(const __grid_constant__ ChainMaps maps, const __grid_consta
   __shared__ uint64_t empty_bar[STAGES];
   __shared__ uint64_t tmem_full_bar[2];
   __shared__ uint64_t tmem_empty_bar[2];
-  __shared__ uint64_t stored_bar[2];        // a tile's results are stored (eight epilogue warps arrive; the announcer waits)
+  __shared__ uint64_t stored_bar[2];        // a tile's results are stored (the epilogue warps arrive; the announcer waits)
   __shared__ uint32_t tmem_base_slot;
   __shared__ int s_last;
   __shared__ TcParams s_prob[kChainMax];
@@ -1541,7 +1718,6 @@ gemm_tc_chain_kernel(const __grid_constant__ ChainMaps maps, const __grid_consta
     bool ok = true;
     bool fetched = false;            // this tile's row statistics and first residual group are already in registers
     longlong2 stats_raw = make_longlong2(0, 0);
-    uint32_t rpre[16];
     int e_next = li0 < li1 ? __ldg(cp.list + li0) : -1;
     int e_next2 = li0 + 1 < li1 ? __ldg(cp.list + li0 + 1) : -1;   // list entries are read two tiles ahead: nothing waits for them
     T col_bias[kChainGroups];                         // the next tile's bias and column sums of this lane's columns, one tile ahead
@@ -1554,7 +1730,7 @@ gemm_tc_chain_kernel(const __grid_constant__ ChainMaps maps, const __grid_consta
       const float* cs = q.ln_stats ? q.ln_colsum : nullptr;
 #pragma unroll
       for (int gi = 0; gi < kChainGroups; gi++) {
-        const int ci = n0_ + (pair + kChainGroupStep * gi) * 32 + lane;
+        const int ci = n0_ + pair * kChainCols + gi * 32 + lane;
         col_bias[gi] = (bias && ci < q.n) ? __ldg(bias + ci) : Cvt<T>::from(0.f);
         col_sum[gi] = (cs && ci < q.n) ? __ldg(cs + ci) : 0.f;
       }
@@ -1603,13 +1779,11 @@ gemm_tc_chain_kernel(const __grid_constant__ ChainMaps maps, const __grid_consta
 #pragma unroll
       for (int gi = 0; gi < kChainGroups; gi++) { bias_f[gi * 32 + lane] = Cvt<T>::to(col_bias[gi]); scale_s[gi * 32 + lane] = col_sum[gi]; }
       if (e_next >= 0) fetch_cols(e_next);
-      const bool res_ahead = p.residual && p.vec_ok == 2 && n0 + pair * 32 < p.n;
       // `fv` is a relaxed look at the counter taken one tile ago. Seeing it complete, the loads below are issued after
       // it (they depend on the branch), go to L2 (the statistics) or to lines this SM has not touched in this launch (the
       // residual rows), and the producer's stores were GPU-visible before the counter moved: they read the final values.
       if (!fetched && (need == 0 || fv >= need)) {
         stats_raw = ln_stats_fetch_cg(p, row0 + lane);
-        if (res_ahead) load_residual_row<T>(p, reinterpret_cast<const T*>(p.residual), row0 + lane, n0 + pair * 32, rpre);
         fetched = true;
       }
       __syncwarp();
@@ -1628,22 +1802,23 @@ gemm_tc_chain_kernel(const __grid_constant__ ChainMaps maps, const __grid_consta
         // accumulator this warp has just waited for follows those loads through the pipeline's barriers: the producer's
         // stores are ordered before these reads without another look at the counter.
         stats_raw = ln_stats_fetch_cg(p, row0 + lane);
-        if (res_ahead) load_residual_row<T>(p, reinterpret_cast<const T*>(p.residual), row0 + lane, n0 + pair * 32, rpre);
       }
       fetched = false;
       float ln_mean = 0.f, ln_rstd = 1.f;
       if (row0 + lane < p.m) ln_stats_finish(p, stats_raw, ln_mean, ln_rstd);
       uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * Cfg::kAccStride);
-      uint8_t* stg = nullptr;   // the staged layouts are not used here (rows are 32-byte aligned)
-      unsigned long long best_key = 0;
       float row_sum = 0.f, row_sq = 0.f;
       if (row0 < p.m) {
+        const bool in_rows = row0 + lane < p.m;
+        const long long at = (row0 + lane) * p.c_row + n0 + pair * kChainCols;
+        T* crow = reinterpret_cast<T*>(p.c) + at;
+        const T* rrow = p.residual ? reinterpret_cast<const T*>(p.residual) + at : nullptr;
 #pragma unroll 1
-        for (int gg = pair, gi = 0; gg < BN / 32; gg += kChainGroupStep, gi++) {
-          if (n0 + gg * 32 >= p.n) break;
-          int next_col0 = (gg + kChainGroupStep < BN / 32 && n0 + (gg + kChainGroupStep) * 32 < p.n) ? n0 + (gg + kChainGroupStep) * 32 : -1;
-          epilogue_group<T>(p, taddr + (uint32_t)(gg * 32), stg, nullptr, fsrc ? scale_s + gi * 32 : nullptr, rpre, row0, n0 + gg * 32, next_col0,
-                            0, lane, best_key, ln_mean, ln_rstd, row_sum, row_sq, bias_f + gi * 32);
+        for (int i = 0; i < kChainCols; i += 16) {
+          const int col0 = n0 + pair * kChainCols + i;
+          if (col0 >= p.n) break;
+          epilogue_unit<T>(p, taddr + (uint32_t)(pair * kChainCols + i), bias_f + i, fsrc ? scale_s + i : nullptr, crow + i, rrow ? rrow + i : nullptr, in_rows, col0,
+                           ln_mean, ln_rstd, row_sum, row_sq);
         }
       }
       tc_fence_before_sync();
@@ -1657,11 +1832,9 @@ gemm_tc_chain_kernel(const __grid_constant__ ChainMaps maps, const __grid_consta
         const int gn = e_next >> 24, ltn = e_next & 0xffffff;
         const TcParams& pn = s_prob[gn];
         if (cp.need[gn] == 0 || fv_next >= cp.need[gn]) {
-          const int min_ = ltn / pn.tiles_n, nin = ltn - min_ * pn.tiles_n;
+          const int min_ = ltn / pn.tiles_n;
           const long long rown = (long long)(min_ * (2 * BM) + (int)rank * BM) + quarter * 32;
           stats_raw = ln_stats_fetch_cg(pn, rown + lane);
-          if (pn.residual && pn.vec_ok == 2 && nin * BN + pair * 32 < pn.n)
-            load_residual_row<T>(pn, reinterpret_cast<const T*>(pn.residual), rown + lane, nin * BN + pair * 32, rpre);
           fetched = true;
         }
       }
@@ -1851,16 +2024,16 @@ static Status launch_tc(cudaStream_t s, const CUtensorMap& ma, const CUtensorMap
 }
 
 // Clusters of two CTAs (one CTA per SM) that can be resident at once; 0 if the query fails.
-template <int BN, bool B_MN, typename T>
+template <int BN, bool B_MN, typename T, int KIND>
 static int pair_clusters() {
   static int cached = -1;
   if (cached >= 0) return cached;
   using Cfg = PairCfg<BN>;
-  auto kern = gemm_tc_pair_kernel<BN, B_MN, T>;
+  auto kern = gemm_tc_pair_kernel<BN, B_MN, T, KIND>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess) { cudaGetLastError(); return cached = 0; }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * (sm_count() / 2)), 1, 1);
-  cfg.blockDim = dim3(kTcThreads, 1, 1);
+  cfg.blockDim = dim3(pair_threads(KIND), 1, 1);
   cfg.dynamicSmemBytes = Cfg::kSmemBytes;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
@@ -1872,26 +2045,31 @@ static int pair_clusters() {
   return cached = n;
 }
 
-template <int BN, bool B_MN, typename T>
-static Status launch_tc_pair(cudaStream_t s, const CUtensorMap& ma, const CUtensorMap& mb, const TcParams& p, long long num_tiles) {
-  int clusters = pair_clusters<BN, B_MN, T>();
+template <int BN, bool B_MN, typename T, int KIND>
+static Status launch_tc_pair_kind(cudaStream_t s, const CUtensorMap& ma, const CUtensorMap& mb, const TcParams& p, long long num_tiles) {
+  int clusters = pair_clusters<BN, B_MN, T, KIND>();
   if (clusters <= 0) return Status::compute("matmul (tcgen05, CTA pairs): no resident cluster available");
   int grid = 2 * (int)(num_tiles < clusters ? num_tiles : clusters);
-  cudaError_t le = launch_pdl(gemm_tc_pair_kernel<BN, B_MN, T>, dim3(grid), dim3(kTcThreads), PairCfg<BN>::kSmemBytes, s, ma, mb, p);
+  cudaError_t le = launch_pdl(gemm_tc_pair_kernel<BN, B_MN, T, KIND>, dim3(grid), dim3(pair_threads(KIND)), PairCfg<BN>::kSmemBytes, s, ma, mb, p);
   if (le != cudaSuccess) return cuda_status(le, "matmul (tcgen05, CTA pairs)");
   return Status::OK();
+}
+template <int BN, bool B_MN, typename T>
+static Status launch_tc_pair(cudaStream_t s, const CUtensorMap& ma, const CUtensorMap& mb, const TcParams& p, long long num_tiles) {
+  const bool packed = p.glu_n || (p.vec_ok == 2 && !p.c_f32 && !p.argmax_keys);
+  return packed ? launch_tc_pair_kind<BN, B_MN, T, kPairPacked>(s, ma, mb, p, num_tiles) : launch_tc_pair_kind<BN, B_MN, T, kPairGeneral>(s, ma, mb, p, num_tiles);
 }
 
 template <typename T>
 static Status launch_tc_pair_w8(cudaStream_t s, const CUtensorMap& ma, const CUtensorMap& mb, const TcParams& p, long long num_tiles) {
   static int clusters = -1;
-  auto kern = gemm_tc_pair_kernel<256, false, T, true>;
+  auto kern = gemm_tc_pair_kernel<256, false, T, kPairW8>;
   if (clusters < 0) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<256>::kSmemBytes) != cudaSuccess) { cudaGetLastError(); clusters = 0; }
     else {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)(2 * (sm_count() / 2)), 1, 1);
-      cfg.blockDim = dim3(kTcThreadsW8, 1, 1);
+      cfg.blockDim = dim3(pair_threads(kPairW8), 1, 1);
       cfg.dynamicSmemBytes = PairCfg<256>::kSmemBytes;
       cudaLaunchAttribute attr;
       attr.id = cudaLaunchAttributeClusterDimension;
@@ -1904,7 +2082,7 @@ static Status launch_tc_pair_w8(cudaStream_t s, const CUtensorMap& ma, const CUt
   }
   if (clusters <= 0) return Status::compute("matmul (tcgen05, int8 weights): no resident cluster available");
   int grid = 2 * (int)(num_tiles < clusters ? num_tiles : clusters);
-  cudaError_t le = launch_pdl(kern, dim3(grid), dim3(kTcThreadsW8), PairCfg<256>::kSmemBytes, s, ma, mb, p);
+  cudaError_t le = launch_pdl(kern, dim3(grid), dim3(pair_threads(kPairW8)), PairCfg<256>::kSmemBytes, s, ma, mb, p);
   if (le != cudaSuccess) return cuda_status(le, "matmul (tcgen05, int8 weights)");
   return Status::OK();
 }

@@ -165,6 +165,29 @@ def test_cta_pair_tiles_in_bands(gpu_dev, dtype, m, n, k, tile):
     assert rel_err(got, ref) <= 2.0 ** -8
 
 
+@pytest.mark.parametrize("tile", ["pair256", "pair192", "pair128"])
+@pytest.mark.parametrize("m,n", [(129, 144), (300, 272), (513, 784), (256, 1040)])
+def test_cta_pair_epilogue_units_at_the_edges(gpu_dev, tile, m, n):
+    """Rows on 32 bytes whose last columns end in any of the four warps of a lane quarter, every option of the epilogue."""
+    rng, k = np.random.default_rng(m + n), 200
+    a, w = rounded(rng.standard_normal((m, k)), "bfloat16"), rounded(rng.standard_normal((n, k)) * 0.1, "bfloat16")
+    bias, res = rounded(rng.standard_normal(n), "bfloat16"), rounded(rng.standard_normal((m, n)), "bfloat16")
+    gpu_dev.set_gemm_tile(tile)
+    try:
+        x, wt, b, r = up(gpu_dev, a, "bfloat16"), gpu_dev.transpose(up(gpu_dev, w, "bfloat16")), up(gpu_dev, bias, "bfloat16"), up(gpu_dev, res, "bfloat16")
+        plain = (x @ wt).to_numpy().astype(np.float64)
+        act = gpu_dev.gelu(gpu_dev.add_bias(x @ wt, b)).to_numpy().astype(np.float64)
+        added = (r + gpu_dev.add_bias(x @ wt, b)).to_numpy().astype(np.float64)
+    finally:
+        gpu_dev.set_gemm_tile("auto")
+    y = a.astype(np.float64) @ w.astype(np.float64).T
+    z = y + bias
+    gelu = 0.5 * z * (1 + np.tanh(np.sqrt(2 / np.pi) * (z + 0.044715 * z ** 3)))
+    for got, ref in ((plain, y), (act, gelu), (added, z + res)):
+        # one rounding to bfloat16 (2^-9 of the value) and, in the activation, the hardware tanh (2^-11)
+        assert got.shape == ref.shape and rel_err(got, ref) <= 2.0 ** -8
+
+
 def test_matmul_half_batched_and_broadcast(gpu_dev):
     rng = np.random.default_rng(5)
     a = rng.standard_normal((6, 200, 64)).astype(np.float32); b = rng.standard_normal((6, 64, 136)).astype(np.float32)
