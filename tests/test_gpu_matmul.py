@@ -522,6 +522,28 @@ def test_attention_single_kernel_matches_oracle_and_composition(gpu_dev, dtype, 
     assert gpu_dev.pipeline_status() == 0
 
 
+@pytest.mark.parametrize("causal,batch,heads,tokens", [(False, 130, 8, 300), (True, 75, 12, 400), (True, 3, 7, 13000), (False, 300, 3, 321)])
+def test_attention_in_bands_of_heads(gpu_dev, causal, batch, heads, tokens):
+    """More keys and values than the L2 keeps: heads in bands, the last one shorter (the third case: a band of 18 heads)."""
+    import torch
+    import torch.nn.functional as F
+    g = torch.Generator("cuda").manual_seed(tokens)
+    q, k, v = (torch.randn((batch, heads, tokens, 64), generator=g, device="cuda").to(torch.bfloat16) for _ in range(3))
+    q, k, v = (gpu_dev.from_torch(t) for t in (q, k, v))
+    got = (gpu_dev.attention_causal if causal else gpu_dev.attention)(q, k, v).to_numpy().astype(np.float64)
+    qt, kt, vt = (torch.from_numpy(t.to_numpy().astype(np.float32)).cuda().reshape(batch * heads, tokens, 64) for t in (q, k, v))
+    ref = np.empty((batch * heads, tokens, 64))
+    rows = torch.arange(tokens, device="cuda")
+    for i in range(batch * heads):
+        for r0 in range(0, tokens, 2048):
+            s = qt[i, r0:r0 + 2048] @ kt[i].T / 8
+            if causal:
+                s = s.masked_fill(rows[None, :] > rows[r0:r0 + 2048, None], float("-inf"))
+            ref[i, r0:r0 + 2048] = (torch.softmax(s, -1) @ vt[i]).cpu().numpy()
+    # probabilities and results rounded to bfloat16: half a step each, 2^-9 of a value
+    assert rel_err(got.reshape(ref.shape), ref) <= 2.0 ** -7
+
+
 def test_attention_on_strided_head_views(gpu_dev):
     # the GPT-2 driver's layout: Q/K/V are column slices of one [B*T, 3d] matrix viewed as [B, h, T, dh]
     rng = np.random.default_rng(13)
