@@ -49,6 +49,26 @@ def test_rms_norm(gpu_dev, rows, width, dtype):
     assert rel(got, R.rms_norm(x.astype(np.float64), w, 3e-4)) < {"float32": 1e-6, "bfloat16": 4e-3}[dtype]
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16", "float16"])
+@pytest.mark.parametrize("rows,width", [(1184, 4), (1185, 1024), (3001, 1028), (2500, 2048)])
+def test_rms_norms_of_many_rows_have_the_bits_of_few(gpu_dev, rows, width, dtype):
+    """Rows are walked by resident blocks from eight per SM on: the same sums in the same order as a block per row."""
+    rng = np.random.default_rng(rows + width)
+    x, y, w, post = rng.standard_normal((rows, width)).astype(np.float32), rng.standard_normal((rows, width)).astype(np.float32), rng.standard_normal(width).astype(np.float32), rng.standard_normal(width).astype(np.float32)
+    up = gpu_dev.from_numpy
+    norm = gpu_dev.rms_norm(up(x), up(w), eps=3e-4, dtype=dtype).to_numpy()
+    stream = up(x)
+    added = gpu_dev.rms_add(stream, up(y), up(post), up(w), eps=2e-3, dtype=dtype).to_numpy()
+    stream = stream.to_numpy()
+    for a in range(0, rows, 1000):
+        part = slice(a, min(a + 1000, rows))
+        few = up(x[part])
+        assert np.array_equal(gpu_dev.rms_norm(few, up(w), eps=3e-4, dtype=dtype).to_numpy().view(np.uint8), norm[part].view(np.uint8))
+        assert np.array_equal(gpu_dev.rms_add(few, up(y[part]), up(post), up(w), eps=2e-3, dtype=dtype).to_numpy().view(np.uint8), added[part].view(np.uint8))
+        assert np.array_equal(few.to_numpy(), stream[part])
+
+
+
 @pytest.mark.parametrize("rows,ff", [(1, 8), (7, 52), (33, 96), (5, 27)])
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_clamped_glu(gpu_dev, rows, ff, dtype):
