@@ -359,6 +359,28 @@ def test_model_layers_portions_slots(gpu_dev, name, dtype):
     assert g.pipeline_status() == 0
 
 
+@pytest.mark.parametrize("tile", ["pair256", "pair192", "pair128"])
+@pytest.mark.parametrize("width", [72, 272, 400])
+def test_float32_stream_through_cta_pair_tiles(gpu_dev, tile, width):
+    """Products that add to the float32 stream, their last columns in any of the four warps of a lane quarter, and gated ones."""
+    cfg = config(width, [("latent_attention", la(3, 16, 8, 24, 40), (72, 1.25)), ("mlstm", ml(2, 24, 40), (56, 2.0))])
+    w = weights(cfg)
+    T, trace = 290, []
+    toks = np.random.default_rng(width).integers(0, cfg["vocab"], T).tolist()
+    want = R.forward(cfg, w, toks, trace=trace)
+    eng = gpu_dev.load_gedenex(cfg, w, "bfloat16").engine(slots=1, max_len=T)
+    gpu_dev.set_gemm_tile(tile)
+    try:
+        logits, _, layers = eng.forward(toks, want=list(range(T)), layers=True)
+    finally:
+        gpu_dev.set_gemm_tile("auto")
+    for got, ref in zip(layers, trace):
+        assert close(got, ref, TOL["bfloat16"] * 3)
+    assert close(logits, want, TOL["bfloat16"] * 3)
+    eng.close()
+    assert gpu_dev.pipeline_status() == 0
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_long_decoding(gpu_dev, dtype):
     cfg = CONFIGS["looped"]
