@@ -250,14 +250,14 @@ __global__ void __launch_bounds__(kRmsThreads) rms_walk_kernel(const __grid_cons
     return i < packs ? reinterpret_cast<const float4*>(base)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   };
   float4 w1[NREG], w2[TWO ? NREG : 1], wp[POST ? NREG : 1], v[NREG], y[POST ? NREG : 1], nv[NREG], ny[POST ? NREG : 1];
+  pdl_wait();
+  pdl_trigger();
 #pragma unroll
   for (int it = 0; it < NREG; it++) {
     w1[it] = piece(p.w1, it);
     if constexpr (TWO) w2[it] = piece(p.w2, it);
     if constexpr (POST) wp[it] = piece(p.wp, it);
   }
-  pdl_wait();
-  pdl_trigger();
   auto ask = [&](long long r) {
 #pragma unroll
     for (int it = 0; it < NREG; it++) nv[it] = piece(p.x + r * p.width, it);
