@@ -7,9 +7,14 @@
 // thread per row over three serial passes; here a warp owns a row, keeps it in registers after
 // a single 16-byte-vectorised read, reduces with shuffles, and writes once.
 #include "common.cuh"
+#include "sm100.cuh"
+#include "tc_math.cuh"
+#include <type_traits>
 #include <cstdlib>
 
 namespace ag { namespace k {
+
+int* matmul_status_word();
 
 // ── layer_norm ──────────────────────────────────────────────────────────────
 // Warp-per-row; ITERS packs per lane cover cols <= 32*ITERS*Pack::N. A persistent grid (a few CTAs per SM) walks the
@@ -148,6 +153,151 @@ Status layer_norm(cudaStream_t s, const TView& in, const TView& gamma, const TVi
 }
 
 // ── softmax / softmax_causal ────────────────────────────────────────────────
+// Two 16-bit floats of one word as a pair of floats, and the larger of each of two words (a number beats NaN).
+template <typename T> __device__ __forceinline__ uint64_t widen_word(uint32_t w);
+template <> __device__ __forceinline__ uint64_t widen_word<__nv_bfloat16>(uint32_t w) { return pack_f32x2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+template <> __device__ __forceinline__ uint64_t widen_word<__half>(uint32_t w) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+  return pack_f32x2(f.x, f.y);
+}
+template <typename T> __device__ __forceinline__ uint32_t max_word(uint32_t a, uint32_t b) {
+  using T2 = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
+  const T2 m = __hmax2(*reinterpret_cast<const T2*>(&a), *reinterpret_cast<const T2*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&m);
+}
+
+// One row in a warp's registers: `valid` unmasked leading columns; put(pack index, results) for every pack of the row.
+// 16-bit rows stay as words of two, and arithmetic is on pairs: a row of 1024 took 509 instructions element by element (63 % of the
+// issue slots at 40 % of the memory's rate) and takes about half of them now. The exponential is 2^24 exp(x - max) for bfloat16, the factor
+// leaving with the sum: the hardware's exp2 gives zero for what it would not hold as a normal number, and this way that is nothing bfloat16 holds.
+template <typename T, int ITERS, bool CAUSAL, typename Put>
+__device__ __forceinline__ void softmax_row16(const Pack<T> (&cur)[ITERS], int lane, int packs, int valid, Put put) {
+  constexpr uint32_t kNegInf = std::is_same<T, __half>::value ? 0xfc00u : 0xff80u;
+  uint4 x[ITERS];
+  uint32_t top = kNegInf | kNegInf << 16;
+#pragma unroll
+  for (int it = 0; it < ITERS; it++) {
+    const int pk = lane + it * 32, left = valid - pk * 8;
+    if (pk >= packs || left <= 0) continue;
+    x[it] = reinterpret_cast<const uint4&>(cur[it]);
+    if (left < 8) {                                        // the pack the diagonal crosses
+      uint32_t* w = reinterpret_cast<uint32_t*>(&x[it]);
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        if (2 * j >= left) w[j] = kNegInf | kNegInf << 16;
+        else if (2 * j + 1 >= left) w[j] = (w[j] & 0xffffu) | kNegInf << 16;
+      }
+    }
+    top = max_word<T>(max_word<T>(top, max_word<T>(x[it].x, x[it].y)), max_word<T>(x[it].z, x[it].w));
+  }
+  float lo, hi;
+  unpack_f32x2(widen_word<T>(top), lo, hi);
+  const float m = warp_max(fmaxf(fmaxf(lo, hi), CAUSAL ? -1e9f : -INFINITY));
+  constexpr float kLog2e = 1.4426950408889634f, kUp = std::is_same<T, __half>::value ? 0.f : 24.f;
+  const uint64_t nm = pack_f32x2(-m, -m), scale = pack_f32x2(kLog2e, kLog2e), up = pack_f32x2(kUp, kUp);
+  uint64_t sums = 0;                                       // the bits of (0.f, 0.f)
+#pragma unroll
+  for (int it = 0; it < ITERS; it++) {
+    const int pk = lane + it * 32;
+    if (pk >= packs || pk * 8 >= valid) continue;
+    uint32_t* w = reinterpret_cast<uint32_t*>(&x[it]);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      float a, b;
+      unpack_f32x2(fma_f32x2(add_f32x2(widen_word<T>(w[j]), nm), scale, up), a, b);
+      a = ex2_approx(a); b = ex2_approx(b);
+      sums = add_f32x2(sums, pack_f32x2(a, b));
+      w[j] = pack2_t<T>(a, b);                             // the reference stores exp() in the storage type and divides that value
+    }
+  }
+  const float inv = __fdiv_rn(1.0f, warp_sum(sum_f32x2(sums)));      // one division per row; e * (1/sum) is within 1 ulp of e / sum
+  const uint64_t inv2 = pack_f32x2(inv, inv);
+#pragma unroll
+  for (int it = 0; it < ITERS; it++) {
+    const int pk = lane + it * 32;
+    if (pk >= packs) continue;
+    uint4 o = make_uint4(0u, 0u, 0u, 0u);
+    if (pk * 8 < valid) {
+      uint32_t* w = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        float a, b;
+        unpack_f32x2(mul_f32x2(widen_word<T>(reinterpret_cast<const uint32_t*>(&x[it])[j]), inv2), a, b);
+        w[j] = pack2_t<T>(a, b);
+      }
+    }
+    put(pk, reinterpret_cast<const Pack<T>&>(o));
+  }
+}
+template <typename T, int ITERS, bool CAUSAL, typename Put>
+__device__ __forceinline__ void softmax_row(const Pack<T> (&cur)[ITERS], int lane, int packs, int valid, Put put) {
+  if constexpr (sizeof(T) == 2) { softmax_row16<T, ITERS, CAUSAL>(cur, lane, packs, valid, put); return; }
+  constexpr int N = Pack<T>::N;
+  float v[ITERS][N];
+  float m = CAUSAL ? -1e9f : -INFINITY;
+#pragma unroll
+  for (int it = 0; it < ITERS; it++) {
+    const int c0 = (lane + it * 32) * N;
+    if (lane + it * 32 < packs && c0 < valid) {
+      if (c0 + N <= valid) {
+#pragma unroll
+        for (int e = 0; e < N; e++) { v[it][e] = Cvt<T>::to(cur[it].v[e]); m = fmaxf(m, v[it][e]); }
+      } else {
+#pragma unroll
+        for (int e = 0; e < N; e++) {
+          const float f = Cvt<T>::to(cur[it].v[e]);
+          const bool on = c0 + e < valid;
+          v[it][e] = on ? f : -INFINITY;
+          if (on) m = fmaxf(m, f);
+        }
+      }
+    }
+  }
+  m = warp_max(m);
+  float sum = 0.f;
+#pragma unroll
+  for (int it = 0; it < ITERS; it++) {
+    // packs entirely right of the diagonal (or past the row) hold only masked slots: skip their math
+    if ((lane + it * 32) * N < valid && lane + it * 32 < packs) {
+#pragma unroll
+      for (int e = 0; e < N; e++) {
+        // Masked slots hold -inf and contribute exp(-inf) = 0. __expf (hardware exp2) is within
+        // 2 ulp plus the rounding of x*log2(e): well inside the 1e-5 bar.
+        float ex = __expf(v[it][e] - m);
+        sum += ex;
+        // Half types: the reference stores exp() in the storage type and divides that value.
+        v[it][e] = Cvt<T>::to(Cvt<T>::from(ex));
+      }
+    }
+  }
+  sum = warp_sum(sum);
+  const float inv = __fdiv_rn(1.0f, sum);  // one division per row; e * (1/sum) is within 1 ulp of e / sum
+#pragma unroll
+  for (int it = 0; it < ITERS; it++) {
+    int pk = lane + it * 32;
+    int c0 = pk * N;
+    if (pk < packs) {
+      Pack<T> o;
+      if (c0 < valid) {
+        float r[N];
+#pragma unroll
+        for (int e = 0; e < N; e++) r[e] = v[it][e] * inv;     // masked slots hold exp(-inf) = 0: they store 0
+        pack_from_floats<T>(o, r);
+      } else {
+#pragma unroll
+        for (int e = 0; e < N; e++) o.v[e] = Cvt<T>::from(0.f);
+      }
+      put(pk, o);
+    }
+  }
+}
+template <bool CAUSAL>
+__device__ __forceinline__ int softmax_valid(int64_t row, int64_t total_rows, int rows_per_mat, int cols) {
+  if (!CAUSAL) return cols;
+  // 32-bit remainder where the row count allows it: the 64-bit one costs about a fifth of a 1024-column row
+  const int r = total_rows <= 0x7fffffff ? (int)((unsigned int)row % (unsigned int)rows_per_mat) : (int)(row % rows_per_mat);
+  return r + 1 < cols ? r + 1 : cols;
+}
 // Warp-per-row with the row in registers; `valid` = number of unmasked leading columns. A persistent grid walks the
 // rows and a warp keeps two rows in flight: the 16-byte loads of its next row are issued before the reductions of the
 // current one (a row's chain load -> max -> exp -> sum -> store is latency-bound on its own). Packs wholly left of the
@@ -161,12 +311,7 @@ __global__ void __launch_bounds__(128, 4) softmax_warp_kernel(const T* __restric
   const int packs = cols / N;
   pdl_wait();
   pdl_trigger();
-  auto valid_of = [&](int64_t row) -> int {
-    if (!CAUSAL) return cols;
-    // 32-bit remainder where the row count allows it: the 64-bit one costs about a fifth of a 1024-column row
-    int r = total_rows <= 0x7fffffff ? (int)((unsigned int)row % (unsigned int)rows_per_mat) : (int)(row % rows_per_mat);
-    return r + 1 < cols ? r + 1 : cols;
-  };
+  auto valid_of = [&](int64_t row) { return softmax_valid<CAUSAL>(row, total_rows, rows_per_mat, cols); };
   const int64_t stride = (int64_t)gridDim.x * wpb;
   int64_t row = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5);
   Pack<T> cur[ITERS], nxt[ITERS];
@@ -184,68 +329,95 @@ __global__ void __launch_bounds__(128, 4) softmax_warp_kernel(const T* __restric
 #pragma unroll
       for (int it = 0; it < ITERS; it++) { int pk = lane + it * 32; if (pk < packs && pk * N < next_valid) nxt[it] = ld16_stream(in + next * cols + pk * N); }
     }
-    float v[ITERS][N];
-    float m = CAUSAL ? -1e9f : -INFINITY;
-#pragma unroll
-    for (int it = 0; it < ITERS; it++) {
-      const int c0 = (lane + it * 32) * N;
-      if (lane + it * 32 < packs && c0 < valid) {
-        if (c0 + N <= valid) {
-#pragma unroll
-          for (int e = 0; e < N; e++) { v[it][e] = Cvt<T>::to(cur[it].v[e]); m = fmaxf(m, v[it][e]); }
-        } else {
-#pragma unroll
-          for (int e = 0; e < N; e++) {
-            const float f = Cvt<T>::to(cur[it].v[e]);
-            const bool on = c0 + e < valid;
-            v[it][e] = on ? f : -INFINITY;
-            if (on) m = fmaxf(m, f);
-          }
-        }
-      }
-    }
-    m = warp_max(m);
-    float sum = 0.f;
-#pragma unroll
-    for (int it = 0; it < ITERS; it++) {
-      // packs entirely right of the diagonal (or past the row) hold only masked slots: skip their math
-      if ((lane + it * 32) * N < valid && lane + it * 32 < packs) {
-#pragma unroll
-        for (int e = 0; e < N; e++) {
-          // Masked slots hold -inf and contribute exp(-inf) = 0. __expf (hardware exp2) is within
-          // 2 ulp plus the rounding of x*log2(e): well inside the 1e-5 bar.
-          float ex = __expf(v[it][e] - m);
-          sum += ex;
-          // Half types: the reference stores exp() in the storage type and divides that value.
-          v[it][e] = Cvt<T>::to(Cvt<T>::from(ex));
-        }
-      }
-    }
-    sum = warp_sum(sum);
-    const float inv = __fdiv_rn(1.0f, sum);  // one division per row; e * (1/sum) is within 1 ulp of e / sum
     T* y = out + row * cols;
-#pragma unroll
-    for (int it = 0; it < ITERS; it++) {
-      int pk = lane + it * 32;
-      int c0 = pk * N;
-      if (pk < packs) {
-        Pack<T> o;
-        if (c0 < valid) {
-          float r[N];
-#pragma unroll
-          for (int e = 0; e < N; e++) r[e] = v[it][e] * inv;     // masked slots hold exp(-inf) = 0: they store 0
-          pack_from_floats<T>(o, r);
-        } else {
-#pragma unroll
-          for (int e = 0; e < N; e++) o.v[e] = Cvt<T>::from(0.f);
-        }
-        st16_stream(y + c0, o);
-      }
-    }
+    softmax_row<T, ITERS, CAUSAL>(cur, lane, packs, valid, [&](int pk, const Pack<T>& o) { st16_stream(y + pk * N, o); });
 #pragma unroll
     for (int it = 0; it < ITERS; it++) cur[it] = nxt[it];
     valid = next_valid;
   }
+}
+
+// The same with rows that come and go by bulk copies. A warp has kSmSlots row buffers in shared memory: one lane asks for a row's
+// unmasked part two rows ahead, the row is computed in place, and the whole row leaves as one copy, zeros included. No register holds a row
+// that is on its way, so more warps fit an SM.
+// For rows of 512 to 2048 bytes (4096 of float32), 32 of them an SM. Rows in registers against bulk copies, causal, us: bfloat16 96 x
+// 1024 x 1024 65.4 / 59.6, 96 x 512 x 512 34.4 / 23.6, 96 x 256 x 256 14.5 / 10.8, 96 x 128 x 128 6.3 / 6.8, 3 x 1024 x 1024 4.9 /
+// 5.5, 8 x 2048 x 2048 20.5 / 25.5; float32 112.9 / 106.4, 36.6 / 27.7, 15.8 / 11.5, 6.8 / 6.1, 6.6 / 6.7, 61 / 82. (Element by element,
+// in registers, the first took 72: it was bound by instructions.) What bounds it now: memory, 302 MB at 5.1 TB/s.
+constexpr int kSmSlots = 4, kSmWarps = 4, kSmMinRowBytes = 512;
+template <typename T> constexpr int kSmMaxRowBytes = sizeof(T) == 4 ? 4096 : 2048;
+__device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(sm100::smem_u32(src)), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+template <typename T, int ITERS, bool CAUSAL>
+__global__ void __launch_bounds__(kSmWarps * 32) softmax_bulk_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t total_rows, int rows_per_mat, int cols, int* status) {
+  constexpr int N = Pack<T>::N;
+  extern __shared__ __align__(128) uint8_t s_rows[];
+  __shared__ uint64_t bars[kSmWarps][kSmSlots];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int packs = cols / N, row_bytes = cols * (int)sizeof(T);
+  uint8_t* const mine = s_rows + (size_t)warp * kSmSlots * row_bytes;
+  uint64_t* const bar = bars[warp];
+  if (lane == 0) {
+    for (int i = 0; i < kSmSlots; i++) sm100::mbar_init(&bar[i], 1);
+    sm100::mbar_fence_init();
+  }
+  __syncwarp();
+  pdl_wait();
+  pdl_trigger();
+  const int64_t stride = (int64_t)gridDim.x * kSmWarps, row0 = (int64_t)blockIdx.x * kSmWarps + warp;
+  auto ask = [&](int64_t row, int slot) {                    // one lane
+    const uint32_t bytes = (uint32_t)((softmax_valid<CAUSAL>(row, total_rows, rows_per_mat, cols) + N - 1) / N * 16);
+    sm100::mbar_expect_tx(&bar[slot], bytes);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(sm100::smem_u32(mine + slot * row_bytes)), "l"(in + row * cols), "r"(bytes), "r"(sm100::smem_u32(&bar[slot])) : "memory");
+  };
+  int64_t asked = row0;                                      // the next row to ask for
+  if (lane == 0) {
+    for (int i = 0; i < kSmSlots - 1 && asked < total_rows; i++, asked += stride) ask(asked, i);
+  }
+  int slot = 0, free_slot = kSmSlots - 1;
+  uint32_t phase = 0;
+  for (int64_t row = row0; row < total_rows; row += stride) {
+    if (lane == 0 && asked < total_rows) {
+      // the free slot held the row before last: its copy out must have read it
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      ask(asked, free_slot);
+      asked += stride;
+    }
+    if (!__all_sync(0xffffffffu, sm100::mbar_wait(&bar[slot], phase, status, 9))) break;
+    const int valid = softmax_valid<CAUSAL>(row, total_rows, rows_per_mat, cols);
+    uint4* const at = reinterpret_cast<uint4*>(mine + slot * row_bytes);
+    Pack<T> cur[ITERS];
+#pragma unroll
+    for (int it = 0; it < ITERS; it++) {
+      const int pk = lane + it * 32;
+      if (pk < packs && pk * N < valid) *reinterpret_cast<uint4*>(&cur[it]) = at[pk];
+    }
+    softmax_row<T, ITERS, CAUSAL>(cur, lane, packs, valid, [&](int pk, const Pack<T>& o) { at[pk] = *reinterpret_cast<const uint4*>(&o); });
+    sm100::fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) bulk_store(out + row * cols, at, (uint32_t)row_bytes);
+    free_slot = slot;
+    if (++slot == kSmSlots) { slot = 0; phase ^= 1; }
+  }
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+template <typename T, int ITERS, bool CAUSAL>
+static cudaError_t launch_softmax_bulk(cudaStream_t s, const T* x, T* y, int64_t total_rows, int64_t rows_per_mat, int64_t cols, int* status) {
+  const int smem = kSmWarps * kSmSlots * (int)(cols * (int64_t)sizeof(T));
+  auto kern = softmax_bulk_kernel<T, ITERS, CAUSAL>;
+  static bool attr = false;
+  if (!attr) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmWarps * kSmSlots * kSmMaxRowBytes<T>);
+    if (e != cudaSuccess) return e;
+    attr = true;
+  }
+  int per_sm = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSmWarps * 32, (size_t)smem);
+  if (e != cudaSuccess) return e;
+  return launch_pdl(kern, dim3((unsigned)grid_for(total_rows, kSmWarps, per_sm < 1 ? 1 : per_sm)), dim3(kSmWarps * 32), (size_t)smem, s, x, y, total_rows, (int)rows_per_mat, (int)cols, status);
 }
 
 // Block-per-row for long or unaligned rows.
@@ -288,6 +460,13 @@ static Status softmax_t(cudaStream_t s, const TView& in, const TView& out) {
     int grid = grid_for(total_rows, wpb, 4);
     int iters = (int)((packs + 31) / 32);
     cudaError_t le = cudaSuccess;
+    int* status = matmul_status_word();
+    const int64_t row_bytes = cols * (int64_t)sizeof(T);
+    if (status && row_bytes >= kSmMinRowBytes && row_bytes <= kSmMaxRowBytes<T> && total_rows >= 32 * (int64_t)sm_count()) {
+#define AG_SMB(I) le = launch_softmax_bulk<T, I, CAUSAL>(s, x, y, total_rows, rows_per_mat, cols, status)
+      if (iters <= 1) AG_SMB(1); else if (iters <= 2) AG_SMB(2); else if (iters <= 4) AG_SMB(4); else AG_SMB(8);
+#undef AG_SMB
+    } else
 #define AG_SM(I) le = launch_pdl(softmax_warp_kernel<T, I, CAUSAL>, dim3(grid), dim3(threads), 0, s, x, y, total_rows, (int)rows_per_mat, (int)cols)
     if (iters <= 1) AG_SM(1); else if (iters <= 2) AG_SM(2); else if (iters <= 4) AG_SM(4);
     else if (iters <= 8) AG_SM(8); else AG_SM(16);

@@ -202,6 +202,32 @@ def test_softmax_causal_f32(gpu_dev, shape):
     assert np.max(np.abs(got - ref)) <= 1e-5
 
 
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16", "float32"])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("shape", [(40, 128, 128), (19, 256, 256), (5, 1000, 1016), (6, 800, 1024), (3, 64, 2048), (2, 16, 4096), (3, 33, 8)])
+def test_softmax_rows_in_registers_and_by_bulk_copies(gpu_dev, dtype, causal, shape):
+    """Row lengths and counts on both sides of the rules, ragged diagonals, scores far from zero, -inf and the type's lowest value."""
+    import torch
+    t = {"bfloat16": torch.bfloat16, "float16": torch.float16, "float32": torch.float32}[dtype]
+    g = torch.Generator("cuda").manual_seed(sum(shape))
+    x = torch.randn(shape, generator=g, device="cuda") * 4
+    x[0] += 300.0
+    x[1, :, 3] = float("-inf")
+    x = x.to(t)
+    x[1, :, 5] = torch.finfo(t).min
+    got = torch.from_numpy((gpu_dev.softmax_causal if causal else gpu_dev.softmax)(gpu_dev.from_torch(x)).to_numpy().astype(np.float32)).cuda().double()
+    ref = x.double()
+    if causal:
+        ref = ref.masked_fill(torch.ones(shape[1:], dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    ref = torch.softmax(ref, -1)
+    # 16 bits: the exponential and the result are rounded to the type (half a step each: 2^-8 of the value in bfloat16), float16 also at its
+    # fixed step of 2^-24 for each; float32: exp2 within 2 ulp of an argument of up to 60 that is rounded once, 60 * 2^-24 * ln 2
+    rel, tiny = {"bfloat16": (2.0 ** -7, 1e-37), "float16": (2.0 ** -10, 2.0 ** -23), "float32": (1e-5, 1e-37)}[dtype]
+    assert torch.all((got - ref).abs() <= rel * ref + tiny)
+    if causal:
+        assert torch.all(got[ref == 0] == 0)
+
+
 def test_softmax_causal_all_masked_floor(gpu_dev):
     # the running max starts at -1e9 (kernel_templates.rs:478): values below it underflow to 0/0
     x = np.full((1, 2, 2), -2e9, np.float32); x[0, 1, 1] = 0.0
