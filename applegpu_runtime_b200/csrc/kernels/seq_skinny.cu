@@ -148,8 +148,8 @@ __global__ void __launch_bounds__(kSsThreads) seq_skinny_kernel(const SsParams p
 struct SmSeg { const void* w; const void* a; void* out; long long ld, a_ld, out_ld; int n, mode, glu, block0; float limit; };
 struct SmParams { SmSeg seg[kSeqSegs]; int n_seg, rows, kp, ranks; };       // ranks: CTAs of a cluster along K
 
-template <typename T, int NT>        // NT groups of 8 input rows
-__global__ void __launch_bounds__(kSsThreads) seq_skinny_mma_kernel(const SmParams p) {
+template <typename T, int NT, int CTAS>        // NT groups of 8 input rows, CTAS of the kernel an SM
+__global__ void __launch_bounds__(kSsThreads, CTAS) seq_skinny_mma_kernel(const SmParams p) {
   constexpr int U = 4;               // 32-column blocks in flight per warp
   __shared__ float red[kSsWarps][NT * 8][17];
   __shared__ float part[NT * 8][16];
@@ -187,6 +187,12 @@ __global__ void __launch_bounds__(kSsThreads) seq_skinny_mma_kernel(const SmPara
   fetch(rank * kSsWarps + warp);
   pdl_wait();
   pdl_trigger();
+  float old = 0.f;                                              // what this thread adds to, asked for ahead of the products
+  static_assert(NT * 8 * 16 <= kSsThreads, "a result a thread");
+  if (rank == 0 && sg.mode == (int)SeqOut::AddF32) {
+    const int m = threadIdx.x / 16, n = threadIdx.x % 16;
+    if (m < p.rows && c0 + n < sg.n) old = reinterpret_cast<const float*>(sg.out)[(long long)m * sg.out_ld + c0 + n];
+  }
   for (int kb = rank * kSsWarps + warp; kb * 32 < p.kp;) {
     uint4 b[U][NT];
 #pragma unroll
@@ -237,13 +243,13 @@ __global__ void __launch_bounds__(kSsThreads) seq_skinny_mma_kernel(const SmPara
       if (glu) reinterpret_cast<T*>(sg.out)[o] = Cvt<T>::from(glu_f(sg.glu, v, total(m, n + 8), sg.limit));
       else if (sg.mode == (int)SeqOut::Store) reinterpret_cast<T*>(sg.out)[o] = Cvt<T>::from(v);
       else if (sg.mode == (int)SeqOut::StoreF32) reinterpret_cast<float*>(sg.out)[o] = v;
-      else reinterpret_cast<float*>(sg.out)[o] += v;
+      else reinterpret_cast<float*>(sg.out)[o] = old + v;
     }
   }
   if (p.ranks > 1) sm100::cluster_sync_all();      // no CTA leaves while its sums are being read
 }
 
-template <typename T, int NT>
+template <typename T, int NT, int CTAS>
 static cudaError_t launch_sm(cudaStream_t s, const SmParams& p, int blocks) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(blocks * p.ranks)); cfg.blockDim = dim3(kSsThreads); cfg.stream = s;
@@ -251,7 +257,7 @@ static cudaError_t launch_sm(cudaStream_t s, const SmParams& p, int blocks) {
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   at[1].id = cudaLaunchAttributeClusterDimension; at[1].val.clusterDim.x = (unsigned)p.ranks; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
   cfg.attrs = at; cfg.numAttrs = p.ranks > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, seq_skinny_mma_kernel<T, NT>, p);
+  return cudaLaunchKernelEx(&cfg, seq_skinny_mma_kernel<T, NT, CTAS>, p);
 }
 
 static Status seq_skinny_mma(cudaStream_t s, const SeqSkinnyDesc& d) {
@@ -266,11 +272,22 @@ static Status seq_skinny_mma(cudaStream_t s, const SeqSkinnyDesc& d) {
     const int per = g.mode == SeqOut::Glu ? 8 : 16;
     blocks += (g.n + per - 1) / per;
   }
-  p.ranks = 1;                                     // few blocks: more CTAs along K, as long as each warp keeps a full round of it
-  while (p.ranks < 4 && blocks * p.ranks < 2 * sm_count() && p.kp / 32 >= kSsWarps * p.ranks * 4) p.ranks *= 2;
+  // Few blocks: more CTAs along K, up to what runs at once (four an SM) as long as each warp keeps a full round of four column
+  // blocks, up to two an SM with half a round.
+  p.ranks = 1;
+  for (int r = 2; r <= 4; r *= 2) {
+    const long long ctas = (long long)blocks * r, at_warp = p.kp / 32 / (kSsWarps * r);
+    if (!((at_warp >= 4 && ctas <= 4 * sm_count()) || (at_warp >= 2 && ctas <= 2 * sm_count()))) break;
+    p.ranks = r;
+  }
   cudaError_t e;
-  if (d.dtype == DType::BF16) e = d.rows <= 8 ? launch_sm<__nv_bfloat16, 1>(s, p, blocks) : launch_sm<__nv_bfloat16, 2>(s, p, blocks);
-  else e = d.rows <= 8 ? launch_sm<__half, 1>(s, p, blocks) : launch_sm<__half, 2>(s, p, blocks);
+  // More CTAs than three an SM (80 registers) take at once: four (64), which read at a higher rate; each of them is slower, so fewer
+  // stay with three. Steps of Gedenex at width 2048 with one sequence (in 1 089 CTAs, out 512): 21.2 -> 19.0 ms for 128 + 48 tokens; of Rurunex at
+  // width 1024 with eight (128 to 352) 17.5 with three, 18.0 with four.
+  const bool four = (long long)blocks * p.ranks > 3 * sm_count();
+#define AG_SM(T) (d.rows > 8 ? launch_sm<T, 2, 3>(s, p, blocks) : four ? launch_sm<T, 1, 4>(s, p, blocks) : launch_sm<T, 1, 3>(s, p, blocks))
+  e = d.dtype == DType::BF16 ? AG_SM(__nv_bfloat16) : AG_SM(__half);
+#undef AG_SM
   return cuda_status(e, "seq_skinny (tensor cores)");
 }
 

@@ -381,6 +381,22 @@ def test_float32_stream_through_cta_pair_tiles(gpu_dev, tile, width):
     assert gpu_dev.pipeline_status() == 0
 
 
+@pytest.mark.parametrize("width,ff", [(512, 96), (1024, 2816), (2048, 5632)])
+@pytest.mark.parametrize("n", [1, 8, 9])
+def test_step_products_over_clusters_along_k(gpu_dev, width, ff, n):
+    """A step's linears with one, two and four CTAs along K, three and four an SM, against the same token at the end of a portion."""
+    cfg = config(width, [("mlstm", ml(2, 24, 40), (ff, 1.25)), ("latent_attention", la(3, 16, 8, 24, 40), (ff, 2.0))])
+    toks = np.random.default_rng(width + n).integers(0, cfg["vocab"], (n, 34))
+    model = gpu_dev.load_gedenex(cfg, weights(cfg), "bfloat16")
+    eng = model.engine(slots=n, max_len=40)
+    whole = eng.forward(toks)[0]
+    eng.reset(0, n)
+    eng.forward(toks[:, :33])
+    step = eng.forward(toks[:, 33:])[0]
+    assert close(step, whole, TOL["bfloat16"] * 3)
+    eng.close()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_long_decoding(gpu_dev, dtype):
     cfg = CONFIGS["looped"]
