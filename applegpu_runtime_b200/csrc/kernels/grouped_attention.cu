@@ -17,6 +17,7 @@ struct GaParams {
   long long ld, seq_stride, y_ld, cld, v_col;
   int n_seq, T, heads, kv_heads, group, dim, vdim, pairs, window, shared, max_len, q_off, k_off, v_off;
   int hg, h_parts;                       // query heads per CTA, CTAs along a group's heads
+  int paired;                            // append: every column turns, a lane takes two neighbours of either half at a time
   float scale, cap, eps;
 };
 
@@ -29,7 +30,7 @@ static Status ga_params(const GroupedAttnDesc& d, GaParams* out) {
   p.ld = d.ld; p.seq_stride = d.seq_stride; p.y_ld = d.y_ld; p.cld = grouped_cache_ld(d.kv_heads, d.dim, d.vdim); p.v_col = grouped_v_col(d.kv_heads, d.dim);
   p.n_seq = d.n_seq; p.T = d.T; p.heads = d.heads; p.kv_heads = d.kv_heads; p.group = d.heads / d.kv_heads; p.dim = d.dim; p.vdim = d.vdim; p.pairs = d.rot_pairs;
   p.window = d.window; p.shared = d.shared ? 1 : 0; p.max_len = d.max_len; p.q_off = d.q_off; p.k_off = d.k_off; p.v_off = d.v_off;
-  p.scale = d.scale; p.cap = d.softcap; p.eps = d.eps; p.hg = 1; p.h_parts = 1;
+  p.scale = d.scale; p.cap = d.softcap; p.eps = d.eps; p.hg = 1; p.h_parts = 1; p.paired = 0;
   return Status::OK();
 }
 
@@ -48,8 +49,51 @@ __device__ __forceinline__ void ga_norm_turn(const GaParams& p, const T* src, T*
   }
   for (int i = 2 * p.pairs + lane; i < p.dim; i += 32) dst[i] = Cvt<T>::from(Cvt<T>::to(src[i]) * rs * w[i]);
 }
+// The same for 16-bit heads that turn as a whole (dim = 2 pairs <= 256, everything on the accesses' alignment): two neighbouring columns of
+// either half at a time, all of a lane's operands asked for at once and read once.
 template <typename T>
+__device__ __forceinline__ void ga_norm_turn_pairs(const GaParams& p, const T* src, T* dst, const float* w, int position, int lane) {
+  constexpr int IT = 2;                  // pairs <= 128
+  uint32_t a[IT], b[IT];
+  float2 wa[IT], wb[IT];
+  float4 cs[IT];
+#pragma unroll
+  for (int it = 0; it < IT; it++) {
+    const int i = 2 * lane + 64 * it;
+    a[it] = b[it] = 0u; wa[it] = wb[it] = make_float2(0.f, 0.f); cs[it] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i >= p.pairs) continue;
+    a[it] = *reinterpret_cast<const uint32_t*>(src + i); b[it] = *reinterpret_cast<const uint32_t*>(src + i + p.pairs);
+    wa[it] = *reinterpret_cast<const float2*>(w + i); wb[it] = *reinterpret_cast<const float2*>(w + i + p.pairs);
+    cs[it] = *reinterpret_cast<const float4*>(p.rot + (long long)position * p.pairs + i);
+  }
+  auto wide = [](uint32_t v) {
+    const T* e = reinterpret_cast<const T*>(&v);
+    return make_float2(Cvt<T>::to(e[0]), Cvt<T>::to(e[1]));
+  };
+  float sq = 0.f;
+#pragma unroll
+  for (int it = 0; it < IT; it++) {
+    const float2 u = wide(a[it]), v = wide(b[it]);
+    sq = fmaf(u.x, u.x, fmaf(u.y, u.y, fmaf(v.x, v.x, fmaf(v.y, v.y, sq))));
+  }
+  const float rs = 1.0f / sqrtf(warp_sum(sq) / (float)p.dim + p.eps);
+#pragma unroll
+  for (int it = 0; it < IT; it++) {
+    const int i = 2 * lane + 64 * it;
+    if (i >= p.pairs) continue;
+    float2 u = wide(a[it]), v = wide(b[it]);
+    u.x *= rs * wa[it].x; u.y *= rs * wa[it].y; v.x *= rs * wb[it].x; v.y *= rs * wb[it].y;
+    alignas(4) T lo[2] = {Cvt<T>::from(u.x * cs[it].x - v.x * cs[it].y), Cvt<T>::from(u.y * cs[it].z - v.y * cs[it].w)};
+    alignas(4) T hi[2] = {Cvt<T>::from(v.x * cs[it].x + u.x * cs[it].y), Cvt<T>::from(v.y * cs[it].z + u.y * cs[it].w)};
+    *reinterpret_cast<uint32_t*>(dst + i) = *reinterpret_cast<const uint32_t*>(lo);
+    *reinterpret_cast<uint32_t*>(dst + i + p.pairs) = *reinterpret_cast<const uint32_t*>(hi);
+  }
+}
+template <typename T, bool PAIRED>
 __global__ void __launch_bounds__(kGaThreads) grouped_append_kernel(const GaParams p) {
+  auto norm_turn = [&](const T* src, T* dst, const float* w, int position, int lane) {
+    if constexpr (PAIRED) ga_norm_turn_pairs<T>(p, src, dst, w, position, lane); else ga_norm_turn<T>(p, src, dst, w, position, lane);
+  };
   pdl_wait();
   pdl_trigger();
   const int r = blockIdx.x, s = r / p.T, t = r % p.T, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -59,16 +103,26 @@ __global__ void __launch_bounds__(kGaThreads) grouped_append_kernel(const GaPara
   T* crow = reinterpret_cast<T*>(p.cache) + (long long)s * p.seq_stride + (long long)position * p.cld;
   const int n = p.heads + (p.shared ? 0 : p.kv_heads);
   for (int h = warp; h < n; h += kGaThreads / 32) {
-    if (h < p.heads) { T* q = row + p.q_off + (long long)h * p.dim; ga_norm_turn<T>(p, q, q, p.q_norm, position, lane); }
-    else { const int g = h - p.heads; ga_norm_turn<T>(p, row + p.k_off + (long long)g * p.dim, crow + (long long)g * p.dim, p.k_norm, position, lane); }
+    if (h < p.heads) { T* q = row + p.q_off + (long long)h * p.dim; norm_turn(q, q, p.q_norm, position, lane); }
+    else { const int g = h - p.heads; norm_turn(row + p.k_off + (long long)g * p.dim, crow + (long long)g * p.dim, p.k_norm, position, lane); }
   }
-  if (!p.shared) for (int i = threadIdx.x; i < p.kv_heads * p.vdim; i += kGaThreads) crow[p.v_col + i] = row[p.v_off + i];
+  if (p.shared) return;
+  if constexpr (PAIRED) {                // in words: the columns of all heads lie side by side in both
+    for (int i = threadIdx.x; i < p.kv_heads * p.vdim / 2; i += kGaThreads) reinterpret_cast<uint32_t*>(crow + p.v_col)[i] = reinterpret_cast<const uint32_t*>(row + p.v_off)[i];
+  } else {
+    for (int i = threadIdx.x; i < p.kv_heads * p.vdim; i += kGaThreads) crow[p.v_col + i] = row[p.v_off + i];
+  }
 }
 Status grouped_append(cudaStream_t s, const GroupedAttnDesc& d) {
   GaParams p;
   AG_RETURN_IF_ERROR(ga_params(d, &p));
+  auto on = [](const void* q, uintptr_t n) { return (reinterpret_cast<uintptr_t>(q) & (n - 1)) == 0; };
+  p.paired = d.dtype != DType::F32 && 2 * p.pairs == p.dim && p.pairs % 2 == 0 && p.pairs <= 128 && p.ld % 2 == 0 && p.q_off % 2 == 0 && (p.shared || (p.k_off % 2 == 0 && p.v_off % 2 == 0)) &&
+             p.cld % 2 == 0 && p.v_col % 2 == 0 && p.seq_stride % 2 == 0 && p.kv_heads * p.vdim % 2 == 0 && on(p.proj, 4) && on(p.cache, 4) && on(p.q_norm, 8) && on(p.k_norm, 8) && on(p.rot, 16);
   cudaError_t e = cudaSuccess;
-  AG_DISPATCH_FLOAT(d.dtype, T, (e = launch_pdl(grouped_append_kernel<T>, dim3((unsigned)(d.n_seq * d.T)), dim3(kGaThreads), 0, s, p)));
+  const dim3 grid((unsigned)(d.n_seq * d.T)), block(kGaThreads);
+  if (p.paired) e = d.dtype == DType::BF16 ? launch_pdl(grouped_append_kernel<__nv_bfloat16, true>, grid, block, 0, s, p) : launch_pdl(grouped_append_kernel<__half, true>, grid, block, 0, s, p);
+  else AG_DISPATCH_FLOAT(d.dtype, T, (e = launch_pdl(grouped_append_kernel<T, false>, grid, block, 0, s, p)));
   return cuda_status(e, "grouped append");
 }
 
