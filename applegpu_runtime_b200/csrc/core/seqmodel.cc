@@ -332,8 +332,19 @@ struct SeqEngine {
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
   int launches = 0, step_launches = 0;
   bool last_graph = false;
+  int32_t* host_picks = nullptr;                   // page-locked: a portion's picks come back without a wait of their own
+  size_t host_picks_cap = 0;
 
-  ~SeqEngine() { drop_graphs(); }
+  ~SeqEngine() { drop_graphs(); if (host_picks) cudaFreeHost(host_picks); }
+  Status reserve_picks(size_t n) {                 // no copy into the old buffer is in flight: every portion that makes one waits for it
+    if (n <= host_picks_cap) return Status::OK();
+    if (host_picks) { cudaStreamSynchronize(DeviceCtx::get().stream); cudaFreeHost(host_picks); host_picks = nullptr; host_picks_cap = 0; }
+    const size_t cap = std::max<size_t>(n, 64);
+    void* p = nullptr;
+    if (cudaMallocHost(&p, cap * sizeof(int32_t)) != cudaSuccess) { cudaGetLastError(); return Status::compute("sequence engine: page-locked memory"); }
+    host_picks = static_cast<int32_t*>(p); host_picks_cap = cap;
+    return Status::OK();
+  }
   void drop_graphs() { for (auto& g : graphs) if (g.second) cudaGraphExecDestroy(g.second); graphs.clear(); }
 
   size_t esz() const { return dtype_size(dtype); }
@@ -775,6 +786,7 @@ Status seq_forward(uint64_t handle, int slot0, int n_seq, const int32_t* tokens,
   cudaStream_t s = ctx.stream;
   const size_t V = (size_t)e->cfg.vocab;
   const int cut = std::max(1, kMaxRows / n_seq);
+  bool handed_on = false;
   if (layers_out && T > cut) return Status::invalid("sequence engine: the portion is too long to record its layers");
   auto copy_ok = [](cudaError_t c) { return c == cudaSuccess ? Status::OK() : Status::compute(std::string("sequence engine: copy: ") + cudaGetErrorString(c)); };
   for (int t0 = 0; t0 < T; t0 += cut) {
@@ -790,12 +802,13 @@ Status seq_forward(uint64_t handle, int slot0, int n_seq, const int32_t* tokens,
     for (int i = 0; i < nw && in_order; i++) in_order = rows[i] == i;
     const bool one_token = T == 1 && !layers_out && (nw == 0 || in_order);
     AG_RETURN_IF_ERROR(e->reserve(slot0, n_seq, Ts, one_token ? n_seq : nw));
+    if (picked) AG_RETURN_IF_ERROR(e->reserve_picks((size_t)nw));
     AG_RETURN_IF_ERROR(copy_ok(cudaMemcpyAsync(e->tok.ptr(), toks.data(), toks.size() * 4, cudaMemcpyHostToDevice, s)));
     if (one_token) {
       // the step greedy generation replays; the picked token is ignored unless asked for
       AG_RETURN_IF_ERROR(copy_ok(cudaMemsetAsync(e->step.ptr(), 0, sizeof(int), s)));
       AG_RETURN_IF_ERROR(e->run_step(s, slot0, n_seq, true));
-      if (nw && picked) AG_RETURN_IF_ERROR(copy_ok(cudaMemcpyAsync(picked, e->tok.ptr(), (size_t)nw * 4, cudaMemcpyDeviceToHost, s)));
+      if (nw && picked) AG_RETURN_IF_ERROR(copy_ok(cudaMemcpyAsync(e->host_picks, e->tok.ptr(), (size_t)nw * 4, cudaMemcpyDeviceToHost, s)));
     } else {
       e->launches = 0;
       StepCtx st{s, slot0, n_seq, Ts, e->len.data() + slot0};
@@ -806,10 +819,10 @@ Status seq_forward(uint64_t handle, int slot0, int n_seq, const int32_t* tokens,
         AG_RETURN_IF_ERROR(e->enqueue_head(s, nw, in_order ? nullptr : static_cast<const int32_t*>(e->rowmap.ptr()), post));
         if (picked) {
           AG_RETURN_IF_ERROR(e->enqueue_pick(s, nw, e->picked.ptr()));
-          std::vector<int32_t> got(nw);
-          AG_RETURN_IF_ERROR(copy_ok(cudaMemcpyAsync(got.data(), e->picked.ptr(), (size_t)nw * 4, cudaMemcpyDeviceToHost, s)));
-          AG_RETURN_IF_ERROR(copy_ok(cudaStreamSynchronize(s)));
-          for (int i = 0; i < nw; i++) picked[idx[i]] = got[i];
+          AG_RETURN_IF_ERROR(copy_ok(cudaMemcpyAsync(e->host_picks, e->picked.ptr(), (size_t)nw * 4, cudaMemcpyDeviceToHost, s)));
+          // one pick per sequence, all of them here: the next step's tokens
+          if (T > 1 && t1 == T && nw == n_want && n_want == n_seq)
+            AG_RETURN_IF_ERROR(copy_ok(cudaMemcpyAsync(e->tok.ptr(), e->picked.ptr(), (size_t)nw * 4, cudaMemcpyDeviceToDevice, s)));
         }
       }
       AG_RETURN_IF_ERROR(e->count(k::seq_advance(s, static_cast<int*>(e->pos.ptr()) + slot0, n_seq, Ts, nullptr, nullptr, nullptr, 0)));
@@ -826,8 +839,12 @@ Status seq_forward(uint64_t handle, int slot0, int n_seq, const int32_t* tokens,
       }
     }
     AG_RETURN_IF_ERROR(finish(s));
+    if (picked)
+      for (int i = 0; i < nw; i++) picked[idx[i]] = e->host_picks[i];
+    handed_on = !one_token && t1 == T && nw == n_want;
   }
-  if (picked && n_want == n_seq && T > 1) AG_RETURN_IF_ERROR(copy_ok(cudaMemcpy(e->tok.ptr(), picked, (size_t)n_seq * 4, cudaMemcpyHostToDevice)));
+  // picks of several portions
+  if (picked && n_want == n_seq && T > 1 && !handed_on) AG_RETURN_IF_ERROR(copy_ok(cudaMemcpy(e->tok.ptr(), picked, (size_t)n_seq * 4, cudaMemcpyHostToDevice)));
   return Status::OK();
 }
 
