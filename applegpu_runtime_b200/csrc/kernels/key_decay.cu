@@ -15,14 +15,41 @@ namespace ag { namespace k {
 
 constexpr int kKsThreads = 512;
 
+// lanes that share a row of a low-rank matrix
+__host__ __device__ __forceinline__ int kd_lanes(int pieces) { return pieces >= 4 ? 4 : pieces >= 2 ? 2 : 1; }
+// A thread's share of such a matrix where one round of the block takes it all: its pieces, asked for long before their use, and the same
+// sums as kd_rows below.
+constexpr int kKsPieces = 4;
+template <typename T>
+__device__ __forceinline__ void kd_ask_rows(const T* w, int ld, int rank, int n, uint4 (&v)[kKsPieces]) {
+  const int pieces = (rank + Pack<T>::N - 1) / Pack<T>::N, g = kd_lanes(pieces), i = (int)threadIdx.x / g, lane = threadIdx.x % g;
+#pragma unroll
+  for (int k = 0; k < kKsPieces; k++) if (i < n && lane + k * g < pieces) v[k] = *reinterpret_cast<const uint4*>(w + (long long)i * ld + (lane + k * g) * Pack<T>::N);
+}
+template <typename T>
+__device__ __forceinline__ void kd_sum_rows(const uint4 (&v)[kKsPieces], int rank, const float* x, int n, float* out) {
+  constexpr int N = Pack<T>::N;
+  const int pieces = (rank + N - 1) / N, g = kd_lanes(pieces), i = (int)threadIdx.x / g, lane = threadIdx.x % g;
+  float a = 0.f;
+#pragma unroll
+  for (int k = 0; k < kKsPieces; k++) {
+    const int q = lane + k * g;
+    if (i < n && q < pieces) {
+      const Pack<T>& w = reinterpret_cast<const Pack<T>&>(v[k]);
+#pragma unroll
+      for (int e = 0; e < N; e++) a = fmaf(Cvt<T>::to(w.v[e]), x[q * N + e], a);
+    }
+  }
+  for (int o = g >> 1; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  if (i < n && lane == 0) out[i] = a;
+}
+
 // out[i] = sum_r w[row0 + i][r] x[r] for n rows of a [.., ld] matrix: a few lanes per row, 16-byte pieces
 template <typename T>
 __device__ __forceinline__ void kd_rows(const T* w, int ld, int rank, const float* x, int n, float* out) {
   constexpr int N = Pack<T>::N;
   const int pieces = (rank + N - 1) / N;
-  int g = 1;
-  while (g < 4 && g * 2 <= pieces) g *= 2;
-  const int lane = threadIdx.x % g;
+  const int g = kd_lanes(pieces), lane = threadIdx.x % g;
   for (int i0 = 0; i0 < n; i0 += kKsThreads / g) {
     const int i = i0 + (int)threadIdx.x / g;
     float a = 0.f;
@@ -48,8 +75,13 @@ __device__ __forceinline__ void kd_prefetch(const void* at, int bytes) {
   for (int i = threadIdx.x * 128; i < bytes; i += kKsThreads * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t*>(at) + i));
 }
 
-template <typename T, int VEC, int NR>          // NR rows of S per thread, VEC neighbouring columns of each
-__global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_step_kernel(const KdParams p, int slice, int tx_n, int sub) {      // sub: CTAs of one group of columns
+// NR rows of S per thread, VEC neighbouring columns of each. AHEAD: what a token reads is one item a thread (kd_ahead below), all of it asked
+// for before the first use. Otherwise its round trips follow one another: the taps of the convolutions 3.1 us, the low-rank products 2.8, a
+// start of the weights towards the L2 1.2 of a launch's 12.7. Rurunex of width 1024, eight sequences, a launch in a step: with the delta
+// rule 15.0 -> 10.8 us, without 10.2 -> 9.1; what is left are one round trip to memory (the state does not stay in the L2 from step to
+// step), five barriers and the cluster's sum.
+template <typename T, int VEC, int NR, bool AHEAD>
+__global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 && !AHEAD ? 2 : 1) key_decay_step_kernel(const KdParams p, int slice, int tx_n, int sub) {      // sub: CTAs of one group of columns
   extern __shared__ __align__(16) float sm[];
   __shared__ float s_sq[2], s_group[8];
   const int D = p.dim, E = p.vdim, cw = tx_n * VEC;       // cw: columns of a pass
@@ -67,11 +99,27 @@ __global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_
   float* so_all = sg + slice;            // two of them where peers read the values: one may still be at the previous token's
   float* sx = so_all + (sub > 1 ? 2 : 1) * slice;      // a1 and g1 of the token, padded with zeros to whole packs
   float* sy = sx + p.a_ld;
+  constexpr int kTaps = 4;
+  const int items = 2 * D + ne, mine = min((int)threadIdx.x, items - 1);      // AHEAD: this thread's channel
+  auto part_of_item = [&](int i) { return i < D ? 0 : i < 2 * D ? 1 : 2; };
+  auto channel_of = [&](int i, int part_of) { return part_of < 2 ? qh * D + i - part_of * D : h * E + e0 + i - 2 * D; };
+  uint4 wa[kKsPieces], wg[kKsPieces];
+  float tap[kTaps], bias_i = 0.f, norm_i = 0.f;
+  if constexpr (AHEAD) {                                   // the state and the ring start towards the L2 (whoever writes them writes there)
+    const int lines = (ne * 4 + 127) / 128;
+    const float* at = p.state(s) + (long long)h * D * E + e0;
+    for (int i = threadIdx.x; i < D * lines; i += kKsThreads) asm volatile("prefetch.global.L2 [%0];" ::"l"(at + (long long)(i / lines) * E + i % lines * 32));
+    const T* rows = p.ring_of<T>(s);
+    for (int i = threadIdx.x; i < p.ring * 3; i += kKsThreads) {
+      const int part_of = i % 3, c = part_of < 2 ? qh * D : h * E + e0, n = part_of < 2 ? D : ne;
+      for (int j = 0; j < n; j += 128 / (int)sizeof(T)) asm volatile("prefetch.global.L2 [%0];" ::"l"(rows + (long long)(i / 3) * p.channels + part_of * p.qk_heads * D + c + j));
+    }
+  }
   // weights start towards the L2 before the previous kernel is waited for
-  kd_prefetch(p.bias + h * D, D * 4);
-  if (!p.z) kd_prefetch(reinterpret_cast<const T*>(p.a2) + (long long)h * D * p.a_ld, D * p.a_ld * (int)sizeof(T));
-  if (!p.gate && p.g_rank) kd_prefetch(reinterpret_cast<const T*>(p.g2) + ((long long)h * E + e0) * p.g_ld, ne * p.g_ld * (int)sizeof(T));
-  if (p.taps) {
+  if (!AHEAD) kd_prefetch(p.bias + h * D, D * 4);
+  if (!AHEAD && !p.z) kd_prefetch(reinterpret_cast<const T*>(p.a2) + (long long)h * D * p.a_ld, D * p.a_ld * (int)sizeof(T));
+  if (!AHEAD && !p.gate && p.g_rank) kd_prefetch(reinterpret_cast<const T*>(p.g2) + ((long long)h * E + e0) * p.g_ld, ne * p.g_ld * (int)sizeof(T));
+  if (!AHEAD && p.taps) {
     const int qk = p.qk_heads * D;
     kd_prefetch(p.conv + (long long)qh * D * p.taps, D * p.taps * 4);
     kd_prefetch(p.conv + (long long)(qk + qh * D) * p.taps, D * p.taps * 4);
@@ -79,6 +127,17 @@ __global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_
   }
   pdl_wait();
   pdl_trigger();
+  const int pos = p.pos[s];
+  if constexpr (AHEAD) {
+    if (!p.z) kd_ask_rows<T>(reinterpret_cast<const T*>(p.a2) + (long long)h * D * p.a_ld, p.a_ld, p.a_rank, D, wa);
+    if (!p.gate && p.g_rank) kd_ask_rows<T>(reinterpret_cast<const T*>(p.g2) + ((long long)h * E + e0) * p.g_ld, p.g_ld, p.g_rank, ne, wg);
+    const int part_of = part_of_item(mine);
+    const float* w = p.conv + (long long)(part_of * p.qk_heads * D + channel_of(mine, part_of)) * p.taps + p.taps - 1;
+#pragma unroll
+    for (int b = 0; b < kTaps; b++) tap[b] = b < p.taps ? __ldg(w - b) : 0.f;
+    if ((int)threadIdx.x < D) bias_i = __ldg(p.bias + h * D + threadIdx.x);
+    if ((int)threadIdx.x < ne) norm_i = __ldg(p.norm + e0 + threadIdx.x);
+  }
   float* S = p.state(s) + (long long)h * D * E + e0;
   const bool resident = slice <= cw;
   float st[NR][VEC];
@@ -108,7 +167,6 @@ __global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_
     }
   };
   if (resident) load(tx * VEC);
-  const int pos = p.pos[s];
   const T* base = reinterpret_cast<const T*>(p.proj) + (long long)s * p.T * p.ld;
   T* ring = p.ring_of<T>(s);
   const float rate = p.softplus ? p.rate[h] : 0.f;
@@ -120,9 +178,36 @@ __global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_
     const int place = p.ring ? (pos + t) % p.ring : 0;            // of this token's raw inputs among the ring's rows
     const bool keep = p.ring && p.T <= kKeyDecayStepTokens;       // nothing of this launch reads the row they take
     __syncthreads();
-    for (int i = threadIdx.x; i < 2 * D + ne; i += kKsThreads) {
-      const int part_of = i < D ? 0 : i < 2 * D ? 1 : 2;
-      const int c = part_of < 2 ? qh * D + i - part_of * D : h * E + e0 + i - 2 * D;
+    if constexpr (AHEAD) {
+      const int i = threadIdx.x, part_of = part_of_item(mine), c = channel_of(mine, part_of);
+      const int col = (part_of == 0 ? p.q_off : part_of == 1 ? p.k_off : p.v_off) + c, ch = part_of * p.qk_heads * D + c;
+      const T raw = row[col];
+      float x[kTaps];
+#pragma unroll
+      for (int b = 1; b < kTaps; b++) {
+        x[b] = 0.f;
+        if (b >= p.taps) continue;
+        if (t >= b) x[b] = Cvt<T>::to(row[col - (long long)b * p.ld]);
+        else if (pos + t >= b) {
+          int q = place - b;
+          if (q < 0) q += p.ring;
+          x[b] = Cvt<T>::to(ring[(long long)q * p.channels + ch]);
+        }
+      }
+      float v = Cvt<T>::to(raw);
+      if (p.taps) {
+        v *= tap[0];
+#pragma unroll
+        for (int b = 1; b < kTaps; b++) if (b < p.taps) v = fmaf(tap[b], x[b], v);
+        v = silu_f(v);
+      }
+      if (i < items) {
+        (part_of == 0 ? sq : part_of == 1 ? sk - D : sv - 2 * D)[i] = v;
+        if (keep && (part_of == 2 || (rank == 0 && h % p.group == 0))) ring[(long long)place * p.channels + ch] = raw;
+      }
+    } else
+    for (int i = threadIdx.x; i < items; i += kKsThreads) {
+      const int part_of = part_of_item(i), c = channel_of(i, part_of);
       const int col = (part_of == 0 ? p.q_off : part_of == 1 ? p.k_off : p.v_off) + c, ch = part_of * p.qk_heads * D + c;
       const T raw = row[col];
       float v = Cvt<T>::to(raw);
@@ -147,8 +232,13 @@ __global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_
         sg[i] = p.gate ? Cvt<T>::to(reinterpret_cast<const T*>(p.gate)[r * p.gate_ld + h * E + e0 + i]) : Cvt<T>::to(row[p.g_off + h * E + e0 + i]);
     else for (int i = threadIdx.x; i < p.g_ld; i += kKsThreads) sy[i] = i < p.g_rank ? Cvt<T>::to(row[p.g_off + i]) : 0.f;
     __syncthreads();
+    if constexpr (AHEAD) {
+      if (!p.z) kd_sum_rows<T>(wa, p.a_rank, sx, D, sa);
+      if (!p.gate && p.g_rank) kd_sum_rows<T>(wg, p.g_rank, sy, ne, sg);
+    } else {
     if (!p.z) kd_rows<T>(reinterpret_cast<const T*>(p.a2) + (long long)h * D * p.a_ld, p.a_ld, p.a_rank, sx, D, sa);
     if (!p.gate && p.g_rank) kd_rows<T>(reinterpret_cast<const T*>(p.g2) + ((long long)h * E + e0) * p.g_ld, p.g_ld, p.g_rank, sy, ne, sg);
+    }
     // sums over the head, by every warp for itself
     float qq = 0.f, kk = 0.f, qk = 0.f;
     for (int i = lane; i < D; i += 32) { const float a = sq[i], b = sk[i]; qq = fmaf(a, a, qq); kk = fmaf(b, b, kk); qk = fmaf(a, b, qk); }
@@ -158,7 +248,7 @@ __global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_
     const float beta = p.delta ? sigmoid_f(beta_raw) : 1.f;
     __syncthreads();
     for (int i = threadIdx.x; i < D; i += kKsThreads) {
-      const float z = sa[i] + p.bias[h * D + i];
+      const float z = sa[i] + (AHEAD ? bias_i : p.bias[h * D + i]);
       sa[i] = p.softplus ? expf(-rate * kd_softplus(z)) : expf(-kd_softplus(-z) * p.inv_tau);
     }
     __syncthreads();
@@ -246,7 +336,7 @@ __global__ void __launch_bounds__(kKsThreads, VEC * NR <= 32 ? 2 : 1) key_decay_
     }
     const float rs = 1.0f / sqrtf(ss / (float)E + p.eps);
     T* y = reinterpret_cast<T*>(p.y) + r * p.y_ld + h * E + e0;
-    for (int i = threadIdx.x; i < ne; i += kKsThreads) y[i] = Cvt<T>::from(so[i] * rs * p.norm[e0 + i] * kd_gate(p, sg[i]));
+    for (int i = threadIdx.x; i < ne; i += kKsThreads) y[i] = Cvt<T>::from(so[i] * rs * (AHEAD ? norm_i : p.norm[e0 + i]) * kd_gate(p, sg[i]));
   }
   if (n_rank > 1) sm100::cluster_sync_all();        // no CTA leaves while another may still read its sum
 }
@@ -265,11 +355,17 @@ __global__ void __launch_bounds__(256) key_decay_tail_kernel(const KdParams p) {
   }
 }
 
-template <typename T, int VEC, int NR>
-static cudaError_t launch_ks(cudaStream_t s, const KdParams& p, int ranks, int slice, int tx_n, int sub, size_t smem) {
+// A CTA for each SM at most (its registers hold the weights), one item a thread.
+template <typename T>
+static bool kd_ahead(const KdParams& p, int ranks, int slice) {
+  auto round = [](int rank, int n) { const int pieces = (rank + Pack<T>::N - 1) / Pack<T>::N, g = kd_lanes(pieces); return n <= kKsThreads / g && pieces <= g * kKsPieces; };
+  return (long long)ranks * p.heads * p.n_seq <= sm_count() && p.taps <= 4 && 2 * p.dim + slice <= kKsThreads && (p.z || round(p.a_rank, p.dim)) && (p.gate || !p.g_rank || round(p.g_rank, slice));
+}
+template <typename T, int VEC, int NR, bool AHEAD>
+static cudaError_t launch_ks_as(cudaStream_t s, const KdParams& p, int ranks, int slice, int tx_n, int sub, size_t smem) {
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(key_decay_step_kernel<T, VEC, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(key_decay_step_kernel<T, VEC, NR, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
     if (e != cudaSuccess) return e;
     attr = true;
   }
@@ -279,7 +375,11 @@ static cudaError_t launch_ks(cudaStream_t s, const KdParams& p, int ranks, int s
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   at[1].id = cudaLaunchAttributeClusterDimension; at[1].val.clusterDim.x = (unsigned)ranks; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
   cfg.attrs = at; cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, key_decay_step_kernel<T, VEC, NR>, p, slice, tx_n, sub);
+  return cudaLaunchKernelEx(&cfg, key_decay_step_kernel<T, VEC, NR, AHEAD>, p, slice, tx_n, sub);
+}
+template <typename T, int VEC, int NR>
+static cudaError_t launch_ks(cudaStream_t s, const KdParams& p, int ranks, int slice, int tx_n, int sub, size_t smem) {
+  return kd_ahead<T>(p, ranks, slice) ? launch_ks_as<T, VEC, NR, true>(s, p, ranks, slice, tx_n, sub, smem) : launch_ks_as<T, VEC, NR, false>(s, p, ranks, slice, tx_n, sub, smem);
 }
 
 static Status key_decay_step(cudaStream_t s, DType dt, const KdParams& p) {
