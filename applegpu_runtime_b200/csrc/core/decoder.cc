@@ -60,8 +60,7 @@ class Gpt2Decoder {
   size_t small_bytes() const { return 256 + 16 * 1024 + (size_t)cfg.max_len * cfg.batch * 4; }
 
   // c = act(layer_norm?(a) @ w + bias) + residual with w [kdim, ndim] (Conv1D layout)
-  Status linear(cudaStream_t s, const void* a, int kdim, const TensorRec& wgt, const TensorRec& bias, void* c, int ndim, k::Act act, const void* residual,
-                const TensorRec* ln_g = nullptr, const TensorRec* ln_b = nullptr) {
+  k::GemmDesc linear_desc(const void* a, int kdim, const TensorRec& wgt, const TensorRec& bias, void* c, int ndim, k::Act act, const void* residual) const {
     k::GemmDesc g;
     g.dtype = dtype; g.b_dtype = dtype; g.a = a; g.b = wgt.data(); g.c = c;
     g.m = cfg.batch; g.n = ndim; g.k = kdim; g.batch = 1; g.batch_inner = 1;
@@ -69,9 +68,17 @@ class Gpt2Decoder {
     g.b_row = ndim; g.b_col = 1; g.b_batch = 0;
     g.c_row = ndim; g.c_batch = 0;
     g.ep.bias = bias.data(); g.ep.act = act; g.ep.residual = residual;
-    static const bool fuse_ln = [] { const char* v = std::getenv("APPLEGPU_DECODE_FUSE_LN"); return !(v && v[0] == '0'); }();
-    if (ln_g && fuse_ln) { g.ln_gamma = ln_g->data(); g.ln_beta = ln_b->data(); g.ln_eps = 1e-5f; }
-    if (k::decode_linear_eligible(g) && (fuse_ln || !ln_g)) {
+    return g;
+  }
+  static bool fuse_ln() {
+    static const bool on = [] { const char* v = std::getenv("APPLEGPU_DECODE_FUSE_LN"); return !(v && v[0] == '0'); }();
+    return on;
+  }
+  Status linear(cudaStream_t s, const void* a, int kdim, const TensorRec& wgt, const TensorRec& bias, void* c, int ndim, k::Act act, const void* residual,
+                const TensorRec* ln_g = nullptr, const TensorRec* ln_b = nullptr) {
+    k::GemmDesc g = linear_desc(a, kdim, wgt, bias, c, ndim, act, residual);
+    if (ln_g && fuse_ln()) { g.ln_gamma = ln_g->data(); g.ln_beta = ln_b->data(); g.ln_eps = 1e-5f; }
+    if (k::decode_linear_eligible(g) && (fuse_ln() || !ln_g)) {
       launches_per_step++;
       return k::decode_linear(s, g);
     }
@@ -124,12 +131,19 @@ class Gpt2Decoder {
     for (int l = 0; l < cfg.n_layer; l++) {
       const TensorRec* lw = &w[4 + 12 * l];
       // ln_1 and ln_2 run in the prologue of the projection that consumes them (the kernel stages its 8..16 rows whole)
-      AG_RETURN_IF_ERROR(linear(s, cur, D, lw[2], lw[3], qkv(), 3 * D, k::Act::None, nullptr, &lw[0], &lw[1]));
-      AG_RETURN_IF_ERROR(k::attention_decode(s, dtype, qkv(), kcache(l), vcache(l), att(), counters() + 1, B, cfg.n_head, cfg.max_len, scale));
+      k::GemmDesc q = linear_desc(cur, D, lw[2], lw[3], qkv(), 3 * D, k::Act::None, nullptr);
+      q.ln_gamma = lw[0].data(); q.ln_beta = lw[1].data(); q.ln_eps = 1e-5f;
+      if (fuse_ln() && k::decode_qkv_attention_eligible(q, cfg.n_head, cfg.max_len)) {
+        AG_RETURN_IF_ERROR(k::decode_qkv_attention(s, q, kcache(l), vcache(l), att(), counters() + 1, cfg.n_head, cfg.max_len, scale));
+        launches_per_step += 1;
+      } else {
+        AG_RETURN_IF_ERROR(linear(s, cur, D, lw[2], lw[3], qkv(), 3 * D, k::Act::None, nullptr, &lw[0], &lw[1]));
+        AG_RETURN_IF_ERROR(k::attention_decode(s, dtype, qkv(), kcache(l), vcache(l), att(), counters() + 1, B, cfg.n_head, cfg.max_len, scale));
+        launches_per_step += 1;
+      }
       AG_RETURN_IF_ERROR(linear(s, att(), D, lw[4], lw[5], other, D, k::Act::None, cur));           // x + c_proj(attn)
       AG_RETURN_IF_ERROR(linear(s, other, D, lw[8], lw[9], ff(), 4 * D, k::Act::GeluTanh, nullptr, &lw[6], &lw[7]));
       AG_RETURN_IF_ERROR(linear(s, ff(), 4 * D, lw[10], lw[11], cur, D, k::Act::None, other));      // x + c_proj(gelu(c_fc))
-      launches_per_step += 1;
     }
     return enqueue_head(s, cur);
   }

@@ -685,6 +685,81 @@ __global__ void __launch_bounds__(kDlThreads, LN == 4 ? 3 : 0) decode_linear_ker
   dl_finish<T, NT * 8>(p, n0, rank, ranks, &sSum[0][0][0], sFin);
 }
 
+// ── a layer's QKV projection and its attention in one launch (16-bit weights) ─
+// A cluster of eight CTAs has one head. Its first CTAs take the shares of K of the head's 192 columns, with the loads, the layer_norm and
+// the order of additions of decode_linear_kernel; instead of going to memory as q | k | v their sums go to the CTAs that attend, one
+// sequence each, whose cached rows were asked for before the dependency wait. That takes the place of a launch and of the round trip of
+// q | k | v through the L2: 8.6 us for the two, 7.5 for this; GPT-2 small, 64 + 50 tokens of eight sequences in bf16, 14.6 -> 13.55 ms, a step
+// of one sequence 221 -> 218 us. (Cached rows asked for behind the products: no gain. Two sequences a CTA for batches of up to sixteen 383 -> 393 us a
+// step; with 160 or 256 clusters' CTAs, more than SMs, at width 1280 245 -> 280 and at 2048 291 -> 322.)
+constexpr int kDqRanks = 8, kDqCols = 3 * kDlCols;
+struct DecodeAttnParams { void* kcache; void* vcache; void* out; const int* len_ptr; int heads, t_max; float scale; };
+constexpr int kDqSums = 3 * (kDlThreads / 32) * kDqRanks * kDlSumPitch, kDqFin = kDqRanks * kDqCols;      // floats
+template <typename T>
+__global__ void __launch_bounds__(kDlThreads) decode_qkv_attention_kernel(const __grid_constant__ DecodeLinearParams p, const __grid_constant__ DecodeAttnParams a, int shares) {
+  extern __shared__ __align__(16) float dq_smem[];
+  constexpr int W = kDlThreads / 32, ROWS = kDqRanks;
+  float* const sSum = dq_smem;                             // [q, k, v][warp][row][column]
+  float* const sFin = sSum + kDqSums;                      // [share][column] of this CTA's sequence
+  float* const s_scores = sFin + kDqFin;                   // [t_max]
+  __shared__ DlStats st;
+  __shared__ AttnDecodeSmem sm;
+  __shared__ float s_qkv[kDqCols];
+  const int rank = (int)sm100::cluster_ctarank(), h = blockIdx.x, d = a.heads * 64, tid = threadIdx.x, warp = tid >> 5;
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  const bool works = rank < shares, attends = rank < p.m;
+  const int k0 = rank * kDlRows;                           // rows of up to 1024 columns: a slab a share
+  uint4 wv[3][4];
+  uint2 x[1], gam = make_uint2(0u, 0u), bet = gam;
+  if (works) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) dl_load_weights<T>(p, c * d + h * 64, k0, wv[c]);
+    dl_ask_norm16<T>(p, k0, gam, bet);
+  }
+  float bias = 0.f;
+  if (tid < kDqCols && p.bias) bias = Cvt<T>::to(reinterpret_cast<const T*>(p.bias)[(tid >> 6) * d + h * 64 + (tid & 63)]);
+  const int len = attn_decode_len(*a.len_ptr, a.t_max);    // older than the launch before this one, as are the cached rows below it (attention_decode_kernel)
+  AttnDecodeRegs<T> pre;
+  const long long at_head = ((long long)rank * a.heads + h) * (long long)a.t_max * 64;
+  T* const kc = reinterpret_cast<T*>(a.kcache) + at_head;
+  T* const vc = reinterpret_cast<T*>(a.vcache) + at_head;
+  if (attends) attn_decode_fetch<T>(kc, vc, len, pre);
+  pdl_wait();      // x belongs to the step
+  pdl_trigger();
+  if (works) {
+    dl_ask_x16<T, 1>(p, k0, x);
+    dl_ln_stats<T, 4>(p, st);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      float acc[1][4][4];
+      dl_zero<1>(acc);
+      dl_products16<T, 1, true>(wv[c], x, gam, bet, st, acc);
+      dl_unit<T, 1>(acc);
+      dl_store16<1>(acc, reinterpret_cast<float (*)[kDlSumPitch]>(sSum + (c * W + warp) * ROWS * kDlSumPitch));
+    }
+  }
+  __syncthreads();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (works) {
+    for (int i = tid; i < p.m * kDqCols; i += kDlThreads) {
+      const int m = i / kDqCols, c = i - m * kDqCols;
+      float v = 0.f;
+#pragma unroll
+      for (int w = 0; w < W; w++) v += sSum[(((c >> 6) * W + w) * ROWS + m) * kDlSumPitch + (c & 63)];      // warp order = K order
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(sm100::mapa_u32(sm100::smem_u32(sFin + rank * kDqCols + c), (uint32_t)m)), "f"(v) : "memory");
+    }
+  }
+  sm100::cluster_sync_all();
+  if (!attends) return;
+  if (tid < kDqCols) {
+    float v = 0.f;
+    for (int r = 0; r < shares; r++) v += sFin[r * kDqCols + tid];
+    s_qkv[tid] = Cvt<T>::to(Cvt<T>::from(v + bias));
+  }
+  __syncthreads();
+  attn_decode_item<T>(s_qkv, kc, vc, reinterpret_cast<T*>(a.out) + (long long)rank * d + h * 64, len, a.scale, s_scores, sm, pre);
+}
+
 // float32 weights: the same on CUDA cores, x staged in shared memory; ROWS of it, eight or sixteen. The slabs of a share behind the first are
 // on their way to the L2 before the dependency wait. A step of GPT-2 small with 1 / 8 / 16 sequences, us: 463 / 579 / 793 with a CTA per
 // slab and partial sums in the L2, 518 / 590 / 780 with clusters and sixteen rows for any batch, now 372 / 444 / 808 (a box
@@ -777,6 +852,42 @@ Status decode_linear(cudaStream_t s, const GemmDesc& d) {
   else if (d.dtype == DType::BF16) e = d.m <= 8 ? launch_dl16<__nv_bfloat16, 1>(s, p, per, ranks) : launch_dl16<__nv_bfloat16, 2>(s, p, per, ranks);
   else e = d.m <= 8 ? launch_dl16<__half, 1>(s, p, per, ranks) : launch_dl16<__half, 2>(s, p, per, ranks);
   return cuda_status(e, "decode_linear");
+}
+
+// At most eight sequences (a cluster has one CTA for each) and no more clusters than run at once with one CTA an SM (238 registers): GPT-2
+// small, not large. Rows of up to 1024 columns.
+bool decode_qkv_attention_eligible(const GemmDesc& d, int heads, int t_max) {
+  return d.dtype != DType::F32 && d.ln_gamma && decode_linear_eligible(d) && heads >= 1 && d.k == heads * 64 && d.k <= 1024 && d.n == 3 * d.k && d.m <= kDqRanks &&
+         heads * kDqRanks <= sm_count() && !d.ep.residual && d.ep.act == Act::None && t_max >= 1 && t_max <= 8192;
+}
+template <typename T>
+static cudaError_t launch_dq(cudaStream_t s, const DecodeLinearParams& p, const DecodeAttnParams& a, int shares) {
+  constexpr int fixed = (kDqSums + kDqFin) * (int)sizeof(float);
+  static bool attr = false;
+  if (!attr) {
+    const cudaError_t e = cudaFuncSetAttribute(decode_qkv_attention_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, fixed + 8192 * (int)sizeof(float));
+    if (e != cudaSuccess) return e;
+    attr = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)a.heads, kDqRanks); cfg.blockDim = dim3(kDlThreads); cfg.stream = s; cfg.dynamicSmemBytes = (size_t)fixed + a.t_max * sizeof(float);
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  at[1].id = cudaLaunchAttributeClusterDimension; at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = kDqRanks; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, decode_qkv_attention_kernel<T>, p, a, shares);
+}
+Status decode_qkv_attention(cudaStream_t s, const GemmDesc& d, void* kcache, void* vcache, void* out, const int* len_ptr, int heads, int t_max, float scale) {
+  if (!decode_qkv_attention_eligible(d, heads, t_max)) return Status::invalid("decode_qkv_attention: shape or layout not supported");
+  if (!aligned16(kcache) || !aligned16(vcache)) return Status::compute("decode_qkv_attention needs 16-byte aligned caches");
+  DecodeLinearParams p;
+  p.x = d.a; p.w = d.b; p.y = nullptr; p.bias = d.ep.bias; p.residual = nullptr; p.ln_gamma = d.ln_gamma; p.ln_beta = d.ln_beta; p.ln_eps = d.ln_eps;
+  p.act = (int)Act::None; p.m = (int)d.m; p.n = (int)d.n; p.k = (int)d.k;
+  p.x_row = d.a_row; p.w_row = d.b_row; p.y_row = 0; p.partial = nullptr;
+  DecodeAttnParams a{kcache, vcache, out, len_ptr, heads, t_max, scale};
+  const int shares = dl_shares((int)d.k);
+  const cudaError_t e = d.dtype == DType::BF16 ? launch_dq<__nv_bfloat16>(s, p, a, shares) : launch_dq<__half>(s, p, a, shares);
+  return cuda_status(e, "decode_qkv_attention");
 }
 
 // ── the layers of a decode step as one persistent kernel ────────────────────

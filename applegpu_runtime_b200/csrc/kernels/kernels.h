@@ -200,6 +200,9 @@ Status attention_decode(cudaStream_t s, DType dt, const void* qkv, void* kcache,
 // and the bias / activation / residual epilogue.
 bool decode_linear_eligible(const GemmDesc& d);
 Status decode_linear(cudaStream_t s, const GemmDesc& d);
+// A layer's QKV projection with layer_norm (as decode_linear) and its attention (as attention_decode) in one launch; 16-bit weights.
+bool decode_qkv_attention_eligible(const GemmDesc& d, int heads, int t_max);
+Status decode_qkv_attention(cudaStream_t s, const GemmDesc& d, void* kcache, void* vcache, void* out, const int* len_ptr, int heads, int t_max, float scale);
 // End of a decode step: history[step] = tok, pos_ids = len + 1, step and len advance (all in device memory).
 // `keys` non-null: tok is first filled from the row-argmax keys of the LM head (and the keys cleared for the next step).
 Status decode_finish(cudaStream_t s, int32_t* tok, int32_t* history, int32_t* pos_ids, int* step_ptr, int* len_ptr, int batch, int max_steps,
