@@ -114,7 +114,7 @@ Status latent_append(cudaStream_t s, const LatentDesc& d) {
 // A generated token has one row, so the work on a head's slices of W_uk and W_uv (dim or vdim times the rank) is cut into `cuts`
 // CTAs, which start their share towards the L2 before the dependency wait. Gedenex at width 2048, one sequence, prepare / attend / merge:
 // 7.5 / 12.0 / 8.7 us a launch in a step with one CTA per head, index divisions and no load ahead of the wait, 4.7 / 8.9 / 6.8 us with them (the
-// prepare kernel with other sums than today's, whose step is 0.4 % longer).
+// prepare kernel with other sums than today's, whose step is 0.4 % longer; the merge has since gone to latent_decode_merge_ahead_kernel).
 __device__ __forceinline__ void la_prefetch(const void* at, int bytes) {
   for (int i = threadIdx.x * 128; i < bytes; i += 256 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t*>(at) + i));
 }
@@ -344,7 +344,10 @@ __global__ void __launch_bounds__(256) latent_decode_attend_mma_kernel(const LaP
     __syncthreads();
     {
       // scores: 16 heads x 8 keys per warp
-      float c4[4] = {0.f, 0.f, 0.f, 0.f};
+      // four sums side by side: a product waits for the one four before it, not for the last
+      float cc[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) { cc[i][0] = 0.f; cc[i][1] = 0.f; cc[i][2] = 0.f; cc[i][3] = 0.f; }
       const uint32_t qa = smem_addr(sqh + (lane & 15) * P + (lane >> 4) * 8), la = smem_addr(sql + (lane & 15) * P + (lane >> 4) * 8);
       const uint32_t ka = smem_addr(sk + (warp * 8 + (lane & 7)) * P + (lane >> 3) * 8);
       for (int kk = 0; kk < K; kk += 32) {
@@ -352,13 +355,16 @@ __global__ void __launch_bounds__(256) latent_decode_attend_mma_kernel(const LaP
         ldsm_x4(b, ka + kk * 2);
         ldsm_x4(a0, qa + kk * 2);
         ldsm_x4(a1, qa + kk * 2 + 32);
-        mma_16816<T>(c4, a0[0], a0[1], a0[2], a0[3], b[0], b[1]);
-        mma_16816<T>(c4, a1[0], a1[1], a1[2], a1[3], b[2], b[3]);
+        mma_16816<T>(cc[0], a0[0], a0[1], a0[2], a0[3], b[0], b[1]);
+        mma_16816<T>(cc[1], a1[0], a1[1], a1[2], a1[3], b[2], b[3]);
         ldsm_x4(a0, la + kk * 2);
         ldsm_x4(a1, la + kk * 2 + 32);
-        mma_16816<T>(c4, a0[0], a0[1], a0[2], a0[3], b[0], b[1]);
-        mma_16816<T>(c4, a1[0], a1[1], a1[2], a1[3], b[2], b[3]);
+        mma_16816<T>(cc[2], a0[0], a0[1], a0[2], a0[3], b[0], b[1]);
+        mma_16816<T>(cc[3], a1[0], a1[1], a1[2], a1[3], b[2], b[3]);
       }
+      float c4[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) c4[i] = (cc[0][i] + cc[1][i]) + (cc[2][i] + cc[3][i]);
       const int g = lane >> 2, q = lane & 3, key = warp * 8 + 2 * q;
       ss[g * (kLmKeys + 1) + key] = c4[0]; ss[g * (kLmKeys + 1) + key + 1] = c4[1];
       ss[(g + 8) * (kLmKeys + 1) + key] = c4[2]; ss[(g + 8) * (kLmKeys + 1) + key + 1] = c4[3];
@@ -391,16 +397,21 @@ __global__ void __launch_bounds__(256) latent_decode_attend_mma_kernel(const LaP
         uint32_t h0a[4], h1a[4], l0a[4], l1a[4];
         ldsm_x4(h0a, pa + kk * 2); ldsm_x4(h1a, pa + kk * 2 + 32);
         ldsm_x4(l0a, pl + kk * 2); ldsm_x4(l1a, pl + kk * 2 + 32);
+        constexpr int JB = NW < 4 ? NW : 4;            // latent tiles whose products run side by side
 #pragma unroll
-        for (int j = 0; j < NW; j++) {
-          const int c = (j * 8 + warp) * 8;
-          if (c >= p.rank) break;
-          uint32_t b[4];                               // keys kk .. kk + 31 of eight latent columns
-          ldsm_x4_t(b, smem_addr(sk + (kk + lane) * P + c));
-          mma_16816<T>(o[j], h0a[0], h0a[1], h0a[2], h0a[3], b[0], b[1]);
-          mma_16816<T>(o[j], h1a[0], h1a[1], h1a[2], h1a[3], b[2], b[3]);
-          mma_16816<T>(o[j], l0a[0], l0a[1], l0a[2], l0a[3], b[0], b[1]);
-          mma_16816<T>(o[j], l1a[0], l1a[1], l1a[2], l1a[3], b[2], b[3]);
+        for (int j0 = 0; j0 < NW; j0 += JB) {
+          if ((j0 * 8 + warp) * 8 >= p.rank) break;
+          uint32_t b[JB][4];                           // keys kk .. kk + 31 of eight latent columns (a tile behind the last one: of that)
+#pragma unroll
+          for (int j = 0; j < JB; j++) ldsm_x4_t(b[j], smem_addr(sk + (kk + lane) * P + (((j0 + j) * 8 + warp) * 8 < p.rank ? ((j0 + j) * 8 + warp) * 8 : (j0 * 8 + warp) * 8)));
+#pragma unroll
+          for (int j = 0; j < JB; j++) mma_16816<T>(o[j0 + j], h0a[0], h0a[1], h0a[2], h0a[3], b[j][0], b[j][1]);
+#pragma unroll
+          for (int j = 0; j < JB; j++) mma_16816<T>(o[j0 + j], h1a[0], h1a[1], h1a[2], h1a[3], b[j][2], b[j][3]);
+#pragma unroll
+          for (int j = 0; j < JB; j++) mma_16816<T>(o[j0 + j], l0a[0], l0a[1], l0a[2], l0a[3], b[j][0], b[j][1]);
+#pragma unroll
+          for (int j = 0; j < JB; j++) mma_16816<T>(o[j0 + j], l1a[0], l1a[1], l1a[2], l1a[3], b[j][2], b[j][3]);
         }
       }
     }
@@ -484,6 +495,76 @@ __global__ void __launch_bounds__(256) latent_decode_merge_kernel(const LaParams
   }
 }
 
+// The same where a head has at most eight splits, a warp's rows of W_uv are one pass of at most two 16-byte pieces a lane, and a thread has
+// at most two latent columns: the weights are on their way ahead of the dependency wait (they are older than the launch before this one, the
+// splits of the same call), the splits' values, maxima and sums come in one round of loads. It adds in the order of the kernel above.
+// Gedenex at width 2048, one sequence: 7.7 -> 3.7 us a launch in a step.
+constexpr int kLgSplits = 8;
+template <typename T>
+__global__ void __launch_bounds__(256) latent_decode_merge_ahead_kernel(const LaParams p, int cuts) {
+  extern __shared__ __align__(16) float so[];            // [rank]
+  constexpr int N = Pack<T>::N, R = 4, Q = 2;
+  const int h = blockIdx.x / cuts, cut = blockIdx.x % cuts, r = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int each = (p.vdim + cuts - 1) / cuts, e_lo = cut * each, e_hi = min(p.vdim, e_lo + each);       // this CTA's outputs
+  const T* uv = reinterpret_cast<const T*>(p.uv) + (long long)h * p.vdim * p.w_ld;
+  const int e0 = e_lo + warp * R, nv = p.coff / N;
+  uint4 w[Q][R];
+#pragma unroll
+  for (int k = 0; k < Q; k++)
+#pragma unroll
+    for (int i = 0; i < R; i++)
+      if (e0 < e_hi && lane + 32 * k < nv) w[k][i] = *reinterpret_cast<const uint4*>(uv + (long long)min(e0 + i, p.vdim - 1) * p.w_ld + (lane + 32 * k) * N);
+  pdl_wait();
+  pdl_trigger();
+  const float* part = p.part + ((long long)r * p.heads + h) * p.splits * (p.rank + 2);
+  float m[kLgSplits], l[kLgSplits], v[2][kLgSplits];
+#pragma unroll
+  for (int i = 0; i < kLgSplits; i++) {
+    const bool in = i < p.splits;
+    const float* at = part + (long long)i * (p.rank + 2);
+    m[i] = in ? at[0] : -INFINITY; l[i] = in ? at[1] : 0.f;
+#pragma unroll
+    for (int k = 0; k < 2; k++) v[k][i] = in && (int)threadIdx.x + 256 * k < p.rank ? at[2 + threadIdx.x + 256 * k] : 0.f;
+  }
+  float top = m[0];
+#pragma unroll
+  for (int i = 1; i < kLgSplits; i++) top = fmaxf(top, m[i]);
+  float share[kLgSplits], sum[kLgSplits];
+#pragma unroll
+  for (int i = 0; i < kLgSplits; i++) { share[i] = m[i] == -INFINITY ? 0.f : expf(m[i] - top); sum[i] = share[i] * l[i]; }
+  const float total = ((sum[0] + sum[4]) + (sum[2] + sum[6])) + ((sum[1] + sum[5]) + (sum[3] + sum[7]));      // the order of a warp's sum
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int c = threadIdx.x + 256 * k;
+    float a = 0.f;
+#pragma unroll
+    for (int i = 0; i < kLgSplits; i++) if (i < p.splits) a = fmaf(share[i] / total, v[k][i], a);
+    if (c < p.coff) so[c] = c < p.rank ? a : 0.f;
+  }
+  __syncthreads();
+  T* y = reinterpret_cast<T*>(p.y) + (long long)r * p.y_ld + (long long)h * p.vdim;
+  if (e0 >= e_hi) return;
+  float a[R];
+#pragma unroll
+  for (int i = 0; i < R; i++) a[i] = 0.f;
+#pragma unroll
+  for (int k = 0; k < Q; k++) {
+    const int c = lane + 32 * k;
+    if (c >= nv) continue;
+#pragma unroll
+    for (int q = 0; q < N; q++) {
+      const float x = so[c * N + q];
+#pragma unroll
+      for (int i = 0; i < R; i++) a[i] = fmaf(x, Cvt<T>::to(reinterpret_cast<const Pack<T>&>(w[k][i]).v[q]), a[i]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    a[i] = warp_sum(a[i]);
+    if (lane == 0 && e0 + i < e_hi) y[e0 + i] = Cvt<T>::from(a[i]);
+  }
+}
+
 static int la_splits(int rows, int heads, int max_len) {
   const int groups = rows * ((heads + kLdHeads - 1) / kLdHeads);
   int want = (2 * 148 + groups - 1) / groups, cap = (max_len + 63) / 64;
@@ -546,7 +627,8 @@ static cudaError_t latent_decode_t(cudaStream_t s, const LaParams& p) {
     else e = launch_ld<T, 32>(s, p, grid, smem);
   }
   if (e != cudaSuccess) return e;
-  return launch_pdl(latent_decode_merge_kernel<T>, dim3((unsigned)(p.heads * cuts), (unsigned)rows), dim3(256), (size_t)p.coff * sizeof(float), s, p, cuts);
+  const bool ahead = p.splits <= kLgSplits && (p.vdim + cuts - 1) / cuts <= 32 && p.coff <= 64 * Pack<T>::N && p.coff <= 512 && p.rank <= p.coff;
+  return launch_pdl(ahead ? latent_decode_merge_ahead_kernel<T> : latent_decode_merge_kernel<T>, dim3((unsigned)(p.heads * cuts), (unsigned)rows), dim3(256), (size_t)p.coff * sizeof(float), s, p, cuts);
 }
 
 Status latent_decode(cudaStream_t s, const LatentDesc& d, void* work) {
