@@ -127,6 +127,7 @@ Status grouped_append(cudaStream_t s, const GroupedAttnDesc& d) {
 }
 
 // ── decode ──────────────────────────────────────────────────────────────────
+constexpr int kGdSplits = 8;                         // CTAs of a cluster at most
 constexpr int kGdKeys = 64, kGdOut = 8;              // keys per tile; accumulators per thread: heads * vdim <= 256 * kGdOut
 static int gd_pitch(int n, size_t esz) { const int per = 16 / (int)esz, q = (n + per - 1) / per; return (q % 2 ? q : q + 1) * per; }   // an odd number of 16-byte pieces
 
@@ -195,13 +196,15 @@ __global__ void __launch_bounds__(256) grouped_decode_kernel(const GaParams p, i
     for (int hh = threadIdx.x / kGdKeys; hh < nh; hh += 256 / kGdKeys) {
       float a = -INFINITY;
       if (key < nk) {
-        a = 0.f;
+        float part[4] = {0.f, 0.f, 0.f, 0.f};          // four chains: a column waits for the one four before it
+#pragma unroll 2
         for (int q = 0; q < kpacks; q++) {
           const Pack<T> kv = *reinterpret_cast<const Pack<T>*>(sk + key * kp + q * N);
           const float* qv = sq + hh * kp + q * N;
 #pragma unroll
-          for (int e = 0; e < N; e++) a = fmaf(qv[e], Cvt<T>::to(kv.v[e]), a);
+          for (int e = 0; e < N; e++) part[e & 3] = fmaf(qv[e], Cvt<T>::to(kv.v[e]), part[e & 3]);
         }
+        a = (part[0] + part[1]) + (part[2] + part[3]);
         if (p.cap > 0.f) a = p.cap * tanhf(a / p.cap);
       }
       sp[hh * kGdKeys + key] = a;
@@ -243,14 +246,21 @@ __global__ void __launch_bounds__(256) grouped_decode_kernel(const GaParams p, i
   T* y = reinterpret_cast<T*>(p.y) + (long long)r * p.y_ld + (long long)h0 * p.vdim;
   for (int o = split * 256 + threadIdx.x; o < outs; o += splits * 256) {
     const int hh = o / p.vdim;
-    float m = -INFINITY, l = 0.f, a = 0.f;
-    for (int q = 0; q < splits; q++) m = fmaxf(m, remote(s_m + hh, q));
-    for (int q = 0; q < splits; q++) {
-      const float mq = remote(s_m + hh, q);
-      if (mq == -INFINITY) continue;
-      const float f = expf(mq - m);
-      l = fmaf(f, remote(s_l + hh, q), l);
-      a = fmaf(f, remote(so + o, q), a);
+    float m = -INFINITY, l = 0.f, a = 0.f, mq[kGdSplits], lq[kGdSplits], aq[kGdSplits];
+#pragma unroll
+    for (int q = 0; q < kGdSplits; q++) {              // all of the cluster's at once
+      mq[q] = q < splits ? remote(s_m + hh, q) : -INFINITY;
+      lq[q] = q < splits ? remote(s_l + hh, q) : 0.f;
+      aq[q] = q < splits ? remote(so + o, q) : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < kGdSplits; q++) m = fmaxf(m, mq[q]);
+#pragma unroll
+    for (int q = 0; q < kGdSplits; q++) {
+      if (mq[q] == -INFINITY) continue;
+      const float f = expf(mq[q] - m);
+      l = fmaf(f, lq[q], l);
+      a = fmaf(f, aq[q], a);
     }
     y[o] = Cvt<T>::from(a / l);
   }
@@ -284,7 +294,7 @@ Status grouped_decode(cudaStream_t s, const GroupedAttnDesc& d) {
   // splits: a cluster of up to eight; about a tile of keys each at least, and no more than fill the machine twice
   const int reach = d.window ? std::min(d.window, d.max_len) : d.max_len;
   int splits = 1;
-  while (splits < 8 && splits * 2 * 32 <= reach && splits * p.kv_heads * p.h_parts * d.n_seq * d.T < 2 * sm_count()) splits *= 2;
+  while (splits < kGdSplits && splits * 2 * 32 <= reach && splits * p.kv_heads * p.h_parts * d.n_seq * d.T < 2 * sm_count()) splits *= 2;
   cudaError_t e = cudaSuccess;
   AG_DISPATCH_FLOAT(d.dtype, T, {
     const int kp = gd_pitch(d.dim, sizeof(T)), vp = gd_pitch(d.vdim, sizeof(T));
