@@ -159,8 +159,12 @@ class Gpt2Decoder {
     g.m = B; g.n = cfg.vocab; g.k = D; g.batch = 1; g.batch_inner = 1;
     g.a_row = D; g.a_col = 1; g.a_batch = 0; g.b_row = 1; g.b_col = D; g.b_batch = 0; g.c_row = cfg.vocab; g.c_batch = 0;
     unsigned long long* finish_keys = nullptr;
-    if (dtype != DType::F32 && std::string(k::matmul_path(g)) == "tcgen05") {
-      // the keys are zero here: prefill clears them and every step's last kernel clears them again after reading them
+    // the keys are zero here: prefill clears them and every step's last kernel clears them again after reading them
+    if (k::decode_head_eligible(dtype, w[0].data(), xn(), B, D)) {
+      AG_RETURN_IF_ERROR(k::decode_head(s, dtype, w[0].data(), xn(), keys(), B, cfg.vocab, D));
+      finish_keys = keys();        // no finalize launch: the step's last kernel turns the keys into tokens
+      launches_per_step += 1;
+    } else if (dtype != DType::F32 && std::string(k::matmul_path(g)) == "tcgen05") {
       g.c = nullptr; g.ep.argmax_keys = keys();
       AG_RETURN_IF_ERROR(k::matmul(s, g));
       finish_keys = keys();        // no finalize launch: the step's last kernel turns the keys into tokens

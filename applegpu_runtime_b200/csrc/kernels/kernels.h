@@ -200,6 +200,9 @@ Status attention_decode(cudaStream_t s, DType dt, const void* qkv, void* kcache,
 // and the bias / activation / residual epilogue.
 bool decode_linear_eligible(const GemmDesc& d);
 Status decode_linear(cudaStream_t s, const GemmDesc& d);
+// The row-argmax keys (GemmEpilogue::argmax_keys) of x [m, k] against an embedding [vocab, k], 16-bit, at most 16 rows.
+bool decode_head_eligible(DType dt, const void* w, const void* x, int m, int64_t k);
+Status decode_head(cudaStream_t s, DType dt, const void* w, const void* x, unsigned long long* keys, int m, int vocab, int k);
 // A layer's QKV projection with layer_norm (as decode_linear) and its attention (as attention_decode) in one launch; 16-bit weights.
 bool decode_qkv_attention_eligible(const GemmDesc& d, int heads, int t_max);
 Status decode_qkv_attention(cudaStream_t s, const GemmDesc& d, void* kcache, void* vcache, void* out, const int* len_ptr, int heads, int t_max, float scale);

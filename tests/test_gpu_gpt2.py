@@ -122,6 +122,30 @@ def test_gpt2_int8_weights_bf16_activations_against_dequantised_oracle(gpu_dev):
     assert gpu_dev.pipeline_status() == 0
 
 
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
+@pytest.mark.parametrize("batch,heads,vocab", [(1, 1, 33), (8, 2, 97), (9, 12, 1000), (16, 3, 64), (5, 16, 130), (8, 18, 4097), (3, 20, 257)])
+def test_decoder_picks_the_largest_logit(gpu_dev, dtype, batch, heads, vocab):
+    """QKV and attention in one launch (up to eight sequences, sixteen heads) and apart, the head at vocabularies that end inside a warp's
+    sixteen rows and a block's 64: every pick has the largest logit of the float32 oracle on the same weights, to rounding."""
+    from applegpu_runtime_b200.generate import Gpt2Decoder
+    cfg = {"n_layer": 2, "n_head": heads, "n_embd": 64 * heads, "vocab_size": vocab, "n_positions": 64}
+    m = gpu_dev.init_gpt2_weights(cfg, seed=heads + vocab, dtype=dtype, std=0.08)
+    w = {k: torch.from_numpy(np.asarray(t.to_numpy()).astype(np.float32)) for k, t in m["weights"].items() if not k.startswith("__")}
+    ids = np.random.default_rng(vocab).integers(0, vocab, (batch, 7))
+    logits, kv = gpu_dev.gpt2_forward(m, ids, last_only=True)
+    first = gpu_dev.argmax(logits)
+    dec = Gpt2Decoder(m, batch, 40)
+    dec.prefill(kv, first, 7)
+    rest = np.asarray(dec.steps(6))
+    seq = np.concatenate([ids, first.to_numpy().reshape(-1, 1), rest.T], 1)
+    with torch.no_grad():
+        ref = torch_ref.gpt2_forward(w, cfg, torch.from_numpy(seq))[0].numpy()
+    # two layers of a dozen roundings to 2^-9 each, summed as if they all had one sign: under 2^-5 of a logit's scale; a pick from a wrong row is at 1
+    for i in range(7):
+        row = ref[:, 6 + i]
+        assert np.all(row.max(-1) - row[np.arange(batch), seq[:, 7 + i]] <= 2e-2 * np.abs(row).max())
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_graph_decoder_matches_the_concat_cache_engine(gpu_dev, dtype):
     """The static-shape decoder (preallocated KV cache appended in place, one captured step replayed per token) against
