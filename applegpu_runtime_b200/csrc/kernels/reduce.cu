@@ -16,6 +16,45 @@ namespace ag { namespace k {
 
 int* matmul_status_word();
 
+// ── rows in words and by bulk copies ────────────────────────────────────────
+// Two 16-bit floats of one word as a pair of floats, and the larger of each of two words (a number beats NaN).
+template <typename T> __device__ __forceinline__ uint64_t widen_word(uint32_t w);
+template <> __device__ __forceinline__ uint64_t widen_word<__nv_bfloat16>(uint32_t w) { return pack_f32x2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+template <> __device__ __forceinline__ uint64_t widen_word<__half>(uint32_t w) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+  return pack_f32x2(f.x, f.y);
+}
+template <typename T> __device__ __forceinline__ uint32_t max_word(uint32_t a, uint32_t b) {
+  using T2 = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
+  const T2 m = __hmax2(*reinterpret_cast<const T2*>(&a), *reinterpret_cast<const T2*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&m);
+}
+
+constexpr int kSmSlots = 4, kSmWarps = 4, kSmMinRowBytes = 512;       // row buffers of a warp, warps of a block
+__device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(sm100::smem_u32(src)), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  sm100::mbar_expect_tx(bar, bytes);
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(sm100::smem_u32(dst)), "l"(src), "r"(bytes), "r"(sm100::smem_u32(bar)) : "memory");
+}
+// Blocks an SM of such a kernel with `smem` bytes of row buffers each; by_registers is the kernel's own, found once.
+template <typename K>
+static cudaError_t bulk_ctas(K kern, int smem, int max_row_bytes, int* by_registers, int* per_sm) {
+  if (!*by_registers) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmWarps * kSmSlots * max_row_bytes);
+    int n = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kSmWarps * 32, 0);
+    if (e != cudaSuccess) return e;
+    *by_registers = n < 1 ? 1 : n;
+  }
+  const int by_smem = 227 * 1024 / (smem + 1024 + (int)sizeof(uint64_t) * kSmWarps * kSmSlots);
+  *per_sm = by_smem < 1 ? 1 : by_smem < *by_registers ? by_smem : *by_registers;
+  return cudaSuccess;
+}
+
 // ── layer_norm ──────────────────────────────────────────────────────────────
 // Warp-per-row; ITERS packs per lane cover cols <= 32*ITERS*Pack::N. A persistent grid (a few CTAs per SM) walks the
 // rows, and a warp keeps TWO rows in flight: the 16-byte loads of its next row are issued before the reductions of
@@ -93,6 +132,104 @@ __global__ void __launch_bounds__(256) layer_norm_warp_kernel(const T* __restric
   }
 }
 
+// The same for 16-bit rows of 512 to 2560 bytes, 32 of them an SM, that come and go by bulk copies (softmax_bulk_kernel below has the
+// pipeline), arithmetic on pairs. Rows in registers against bulk copies, bfloat16, us: 131072 x 768 77.3 / 65.6 (6.1 TB/s), 65536 x 1024
+// 68.4 / 51.7 (half of it from the L2), 16384 x 1280 19.6 / 17.3, 32768 x 256 12.6 / 11.9, 8192 x 768 7.8 / 7.8, 8192 x 2048 18.2 / 20.0.
+constexpr int kLnMaxRowBytes = 2560;
+template <typename T, int ITERS>
+__global__ void __launch_bounds__(kSmWarps * 32) layer_norm_bulk_kernel(const T* __restrict__ in, const T* __restrict__ gamma, const T* __restrict__ beta, T* __restrict__ out, int64_t rows,
+                                                                         int cols, float eps, int* status) {
+  extern __shared__ __align__(128) uint8_t s_rows[];
+  __shared__ uint64_t bars[kSmWarps][kSmSlots];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int packs = cols / 8, row_bytes = cols * 2;
+  uint8_t* const mine = s_rows + (size_t)warp * kSmSlots * row_bytes;
+  uint64_t* const bar = bars[warp];
+  if (lane == 0) {
+    for (int i = 0; i < kSmSlots; i++) sm100::mbar_init(&bar[i], 1);
+    sm100::mbar_fence_init();
+  }
+  __syncwarp();
+  pdl_wait();
+  pdl_trigger();
+  const int64_t stride = (int64_t)gridDim.x * kSmWarps, row0 = (int64_t)blockIdx.x * kSmWarps + warp;
+  int64_t asked = row0;
+  if (lane == 0) {
+    for (int i = 0; i < kSmSlots - 1 && asked < rows; i++, asked += stride) bulk_load(mine + i * row_bytes, in + asked * cols, (uint32_t)row_bytes, &bar[i]);
+  }
+  uint4 g[ITERS], b[ITERS];
+#pragma unroll
+  for (int it = 0; it < ITERS; it++) {
+    const int pk = lane + it * 32;
+    if (pk < packs) { g[it] = *(reinterpret_cast<const uint4*>(gamma) + pk); b[it] = *(reinterpret_cast<const uint4*>(beta) + pk); }
+  }
+  const float inv_cols = 1.0f / (float)cols;
+  int slot = 0, free_slot = kSmSlots - 1;
+  uint32_t phase = 0;
+  for (int64_t row = row0; row < rows; row += stride) {
+    if (lane == 0 && asked < rows) {
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the free slot's copy out has read it
+      bulk_load(mine + free_slot * row_bytes, in + asked * cols, (uint32_t)row_bytes, &bar[free_slot]);
+      asked += stride;
+    }
+    if (!__all_sync(0xffffffffu, sm100::mbar_wait(&bar[slot], phase, status, 9))) break;
+    uint4* const at = reinterpret_cast<uint4*>(mine + slot * row_bytes);
+    uint4 x[ITERS];
+    uint64_t s2 = 0;                                       // the bits of (0.f, 0.f)
+#pragma unroll
+    for (int it = 0; it < ITERS; it++) {
+      const int pk = lane + it * 32;
+      if (pk >= packs) continue;
+      x[it] = at[pk];
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(&x[it]);
+#pragma unroll
+      for (int j = 0; j < 4; j++) s2 = add_f32x2(s2, widen_word<T>(w[j]));
+    }
+    const float mean = warp_sum(sum_f32x2(s2)) * inv_cols;
+    const uint64_t nm = pack_f32x2(-mean, -mean);
+    uint64_t q2 = 0;
+#pragma unroll
+    for (int it = 0; it < ITERS; it++) {
+      if (lane + it * 32 >= packs) continue;
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(&x[it]);
+#pragma unroll
+      for (int j = 0; j < 4; j++) { const uint64_t d = add_f32x2(widen_word<T>(w[j]), nm); q2 = fma_f32x2(d, d, q2); }
+    }
+    const float inv_std = 1.0f / sqrtf(warp_sum(sum_f32x2(q2)) * inv_cols + eps);
+    const uint64_t is = pack_f32x2(inv_std, inv_std);
+#pragma unroll
+    for (int it = 0; it < ITERS; it++) {
+      const int pk = lane + it * 32;
+      if (pk >= packs) continue;
+      const uint32_t *w = reinterpret_cast<const uint32_t*>(&x[it]), *gw = reinterpret_cast<const uint32_t*>(&g[it]), *bw = reinterpret_cast<const uint32_t*>(&b[it]);
+      uint4 o;
+      uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        float lo, hi;
+        unpack_f32x2(fma_f32x2(mul_f32x2(widen_word<T>(gw[j]), add_f32x2(widen_word<T>(w[j]), nm)), is, widen_word<T>(bw[j])), lo, hi);
+        ow[j] = pack2_t<T>(lo, hi);
+      }
+      at[pk] = o;
+    }
+    sm100::fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) bulk_store(out + row * cols, at, (uint32_t)row_bytes);
+    free_slot = slot;
+    if (++slot == kSmSlots) { slot = 0; phase ^= 1; }
+  }
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+template <typename T, int ITERS>
+static cudaError_t launch_layer_norm_bulk(cudaStream_t s, const T* x, const T* g, const T* b, T* y, int64_t rows, int cols, float eps, int* status) {
+  const int smem = kSmWarps * kSmSlots * cols * (int)sizeof(T);
+  static int by_registers = 0;
+  int per_sm;
+  cudaError_t e = bulk_ctas(layer_norm_bulk_kernel<T, ITERS>, smem, kLnMaxRowBytes, &by_registers, &per_sm);
+  if (e != cudaSuccess) return e;
+  return launch_pdl(layer_norm_bulk_kernel<T, ITERS>, dim3((unsigned)grid_for(rows, kSmWarps, per_sm)), dim3(kSmWarps * 32), (size_t)smem, s, x, g, b, y, rows, cols, eps, status);
+}
+
 // Block-per-row, any cols / alignment: three passes over a row that stays in L1/L2.
 template <typename T>
 __global__ void __launch_bounds__(256) layer_norm_block_kernel(const T* __restrict__ in, const T* __restrict__ gamma, const T* __restrict__ beta,
@@ -131,6 +268,15 @@ static Status layer_norm_t(cudaStream_t s, const TView& in, const TView& gamma, 
     int grid = grid_for(rows, wpb, bps);
     int iters = (int)((packs + 31) / 32);
     cudaError_t le = cudaSuccess;
+    if constexpr (sizeof(T) == 2) {
+      int* status = matmul_status_word();
+      if (status && cols * 2 >= kSmMinRowBytes && cols * 2 <= kLnMaxRowBytes && rows >= 32 * (int64_t)sm_count() && x != y) {
+#define AG_LNB(I) le = launch_layer_norm_bulk<T, I>(s, x, g, b, y, rows, (int)cols, eps, status)
+        if (iters <= 2) AG_LNB(2); else if (iters <= 3) AG_LNB(3); else if (iters <= 4) AG_LNB(4); else AG_LNB(5);
+#undef AG_LNB
+        return cuda_status(le, "layer_norm");
+      }
+    }
 #define AG_LN(I) le = launch_pdl(layer_norm_warp_kernel<T, I>, dim3(grid), dim3(threads), 0, s, x, g, b, y, rows, (int)cols, eps)
     if (iters <= 1) AG_LN(1); else if (iters <= 2) AG_LN(2); else if (iters <= 3) AG_LN(3); else if (iters <= 4) AG_LN(4);
     else if (iters <= 6) AG_LN(6); else if (iters <= 8) AG_LN(8); else if (iters <= 12) AG_LN(12); else AG_LN(16);
@@ -153,19 +299,6 @@ Status layer_norm(cudaStream_t s, const TView& in, const TView& gamma, const TVi
 }
 
 // ── softmax / softmax_causal ────────────────────────────────────────────────
-// Two 16-bit floats of one word as a pair of floats, and the larger of each of two words (a number beats NaN).
-template <typename T> __device__ __forceinline__ uint64_t widen_word(uint32_t w);
-template <> __device__ __forceinline__ uint64_t widen_word<__nv_bfloat16>(uint32_t w) { return pack_f32x2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
-template <> __device__ __forceinline__ uint64_t widen_word<__half>(uint32_t w) {
-  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
-  return pack_f32x2(f.x, f.y);
-}
-template <typename T> __device__ __forceinline__ uint32_t max_word(uint32_t a, uint32_t b) {
-  using T2 = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
-  const T2 m = __hmax2(*reinterpret_cast<const T2*>(&a), *reinterpret_cast<const T2*>(&b));
-  return *reinterpret_cast<const uint32_t*>(&m);
-}
-
 // One row in a warp's registers: `valid` unmasked leading columns; put(pack index, results) for every pack of the row.
 // 16-bit rows stay as words of two, and arithmetic is on pairs: a row of 1024 took 509 instructions element by element (63 % of the
 // issue slots at 40 % of the memory's rate) and takes about half of them now. The exponential is 2^24 exp(x - max) for bfloat16, the factor
@@ -344,12 +477,7 @@ __global__ void __launch_bounds__(128, 4) softmax_warp_kernel(const T* __restric
 // 1024 x 1024 65.4 / 59.6, 96 x 512 x 512 34.4 / 23.6, 96 x 256 x 256 14.5 / 10.8, 96 x 128 x 128 6.3 / 6.8, 3 x 1024 x 1024 4.9 /
 // 5.5, 8 x 2048 x 2048 20.5 / 25.5; float32 112.9 / 106.4, 36.6 / 27.7, 15.8 / 11.5, 6.8 / 6.1, 6.6 / 6.7, 61 / 82. (Element by element,
 // in registers, the first took 72: it was bound by instructions.) What bounds it now: memory, 302 MB at 5.1 TB/s.
-constexpr int kSmSlots = 4, kSmWarps = 4, kSmMinRowBytes = 512;
 template <typename T> constexpr int kSmMaxRowBytes = sizeof(T) == 4 ? 4096 : 2048;
-__device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(sm100::smem_u32(src)), "r"(bytes) : "memory");
-  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
 template <typename T, int ITERS, bool CAUSAL>
 __global__ void __launch_bounds__(kSmWarps * 32) softmax_bulk_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t total_rows, int rows_per_mat, int cols, int* status) {
   constexpr int N = Pack<T>::N;
@@ -368,10 +496,7 @@ __global__ void __launch_bounds__(kSmWarps * 32) softmax_bulk_kernel(const T* __
   pdl_trigger();
   const int64_t stride = (int64_t)gridDim.x * kSmWarps, row0 = (int64_t)blockIdx.x * kSmWarps + warp;
   auto ask = [&](int64_t row, int slot) {                    // one lane
-    const uint32_t bytes = (uint32_t)((softmax_valid<CAUSAL>(row, total_rows, rows_per_mat, cols) + N - 1) / N * 16);
-    sm100::mbar_expect_tx(&bar[slot], bytes);
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(sm100::smem_u32(mine + slot * row_bytes)), "l"(in + row * cols), "r"(bytes), "r"(sm100::smem_u32(&bar[slot])) : "memory");
+    bulk_load(mine + slot * row_bytes, in + row * cols, (uint32_t)((softmax_valid<CAUSAL>(row, total_rows, rows_per_mat, cols) + N - 1) / N * 16), &bar[slot]);
   };
   int64_t asked = row0;                                      // the next row to ask for
   if (lane == 0) {
@@ -408,16 +533,11 @@ template <typename T, int ITERS, bool CAUSAL>
 static cudaError_t launch_softmax_bulk(cudaStream_t s, const T* x, T* y, int64_t total_rows, int64_t rows_per_mat, int64_t cols, int* status) {
   const int smem = kSmWarps * kSmSlots * (int)(cols * (int64_t)sizeof(T));
   auto kern = softmax_bulk_kernel<T, ITERS, CAUSAL>;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmWarps * kSmSlots * kSmMaxRowBytes<T>);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
-  int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSmWarps * 32, (size_t)smem);
+  static int by_registers = 0;
+  int per_sm;
+  cudaError_t e = bulk_ctas(kern, smem, kSmMaxRowBytes<T>, &by_registers, &per_sm);
   if (e != cudaSuccess) return e;
-  return launch_pdl(kern, dim3((unsigned)grid_for(total_rows, kSmWarps, per_sm < 1 ? 1 : per_sm)), dim3(kSmWarps * 32), (size_t)smem, s, x, y, total_rows, (int)rows_per_mat, (int)cols, status);
+  return launch_pdl(kern, dim3((unsigned)grid_for(total_rows, kSmWarps, per_sm)), dim3(kSmWarps * 32), (size_t)smem, s, x, y, total_rows, (int)rows_per_mat, (int)cols, status);
 }
 
 // Block-per-row for long or unaligned rows.

@@ -202,6 +202,21 @@ def test_softmax_causal_f32(gpu_dev, shape):
     assert np.max(np.abs(got - ref)) <= 1e-5
 
 
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
+@pytest.mark.parametrize("rows,cols", [(4735, 768), (4736, 768), (4801, 256), (5000, 1000), (4737, 1024), (6001, 1280), (4800, 1288), (4736, 248)])
+def test_layer_norm_rows_by_bulk_copies(gpu_dev, dtype, rows, cols):
+    """Both sides of the rule (32 rows an SM, 512 to 2560 bytes), every number of pieces a lane, a last piece that not every lane has."""
+    import torch
+    t = {"bfloat16": torch.bfloat16, "float16": torch.float16}[dtype]
+    g = torch.Generator("cuda").manual_seed(rows + cols)
+    x = (torch.randn((rows, cols), generator=g, device="cuda") * 3 + 5).to(t)
+    gain, shift = torch.randn(cols, generator=g, device="cuda").to(t), torch.randn(cols, generator=g, device="cuda").to(t)
+    got = torch.from_numpy(gpu_dev.layer_norm(gpu_dev.from_torch(x), gpu_dev.from_torch(gain), gpu_dev.from_torch(shift), 1e-5).to_numpy().astype(np.float32)).cuda().double()
+    ref = torch.nn.functional.layer_norm(x.double(), (cols,), gain.double(), shift.double(), 1e-5)
+    # one rounding to the type, half a step (2^-9 of the value in bfloat16, 2^-12 in float16), and float32 sums; where terms cancel, of their size
+    assert torch.all((got - ref).abs() <= (2.0 ** -8 if dtype == "bfloat16" else 2.0 ** -11) * (ref.abs() + 2.0 ** -8 * (ref - shift.double()).abs()) + 1e-5)
+
+
 @pytest.mark.parametrize("dtype", ["bfloat16", "float16", "float32"])
 @pytest.mark.parametrize("causal", [True, False])
 @pytest.mark.parametrize("shape", [(40, 128, 128), (19, 256, 256), (5, 1000, 1016), (6, 800, 1024), (3, 64, 2048), (2, 16, 4096), (3, 33, 8)])
