@@ -231,6 +231,9 @@ __device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr, uin
   d |= (uint64_t)2 << 61;
   return d;
 }
+// The descriptor `words` 16-byte words further on. Shared memory ends below the address field's 2^14 words, so the sum stays inside it:
+// one 32-bit add for the thread that issues the products, where building a descriptor anew takes it a handful of instructions.
+__device__ __forceinline__ uint64_t desc_at(uint64_t d, uint32_t words) { return (d & 0xffffffff00000000ull) | (uint32_t)((uint32_t)d + words); }
 // Instruction descriptor for kind::f16 with fp32 accumulation.
 //   [4,6) D format (1 = f32)  [7,10) A format  [10,13) B format (0 = f16, 1 = bf16)
 //   [15] A major  [16] B major (0 = K-major, 1 = MN-major)  [17,23) N>>3  [24,29) M>>4
