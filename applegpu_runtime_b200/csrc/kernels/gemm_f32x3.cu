@@ -289,15 +289,11 @@ gemm_f32x3_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
               mma(d_hi, 0, 0, on);
               on = 1u;
             }
-            const uint32_t eb = smem_u32(&empty_bar[stage]);
-            mma_commit_pair(mapa_u32(eb, 0));
-            mma_commit_pair(mapa_u32(eb, 1));
+            mma_commit_both(&empty_bar[stage]);
             if (++stage == kF3Stages) { stage = 0; phase ^= 1; }
           }
           if (!ok) break;
-          const uint32_t fb = smem_u32(&tmem_full_bar[acc]);
-          mma_commit_pair(mapa_u32(fb, 0));
-          mma_commit_pair(mapa_u32(fb, 1));
+          mma_commit_both(&tmem_full_bar[acc]);
           if (++acc == 2) { acc = 0; acc_phase ^= 1; }
         }
       }
@@ -462,11 +458,6 @@ gemm_f32x3_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         for (int kk = 0; kk < kF3Bk / 16; kk++)
           f3_mma(d, al + (uint32_t)((slot_a * kFwSlot + kk * 32) >> 4), ah, bl + (uint32_t)((slot_b * kFwSlot + kk * (B_MN ? 16 * 128 : 32)) >> 4), bh, idesc, kk ? 1u : on);
       };
-      auto done = [&](uint64_t* bar) {                 // to both CTAs, once the products so far are done
-        const uint32_t at = smem_u32(bar);
-        mma_commit_pair(mapa_u32(at, 0));
-        mma_commit_pair(mapa_u32(at, 1));
-      };
       int slot = 0; uint32_t phase = 0, hi_phase = 0, lo_phase = 0;
       auto next = [&]() { const int s = slot; if (++slot == kFwSlots) { slot = 0; phase ^= 1; } return s; };
       auto arrived = [&]() {
@@ -487,7 +478,7 @@ gemm_f32x3_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
             tc_fence_after_sync();
           }
           products(d_hi, s0, s0, kb % kFwChunk ? 1u : 0u);
-          if (kb % kFwChunk == kFwChunk - 1 || kb + 1 == p.num_kb) done(&hi_full);
+          if (kb % kFwChunk == kFwChunk - 1 || kb + 1 == p.num_kb) mma_commit_both(&hi_full);
           if (kb % kFwLowChunk == 0) {
             if (!mbar_wait(&lo_empty, lo_phase ^ 1, p.status, 6)) { ok = false; break; }
             lo_phase ^= 1;
@@ -496,14 +487,14 @@ gemm_f32x3_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           products(d_lo, s1, s1, kb % kFwLowChunk ? 1u : 0u);
           products(d_lo, s1, s0, 1u);
           products(d_lo, s0, s1, 1u);
-          done(&empty_bar[s1]);
+          mma_commit_both(&empty_bar[s1]);
           if (!arrived()) { ok = false; break; }
           const int s2 = next();
           products(d_lo, s2, s0, 1u);
           products(d_lo, s0, s2, 1u);
-          done(&empty_bar[s0]);
-          done(&empty_bar[s2]);
-          if (kb % kFwLowChunk == kFwLowChunk - 1 || kb + 1 == p.num_kb) done(&lo_full);
+          mma_commit_both(&empty_bar[s0]);
+          mma_commit_both(&empty_bar[s2]);
+          if (kb % kFwLowChunk == kFwLowChunk - 1 || kb + 1 == p.num_kb) mma_commit_both(&lo_full);
         }
       }
     }

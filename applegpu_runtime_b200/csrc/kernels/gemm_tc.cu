@@ -1328,15 +1328,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                               (r > 0 || j > 0 || kk > 0) ? 1u : 0u);
           }
           // the stage is free in both CTAs once these MMAs have read it
-          const uint32_t eb = smem_u32(&empty_bar[stage]);
-          mma_commit_pair(mapa_u32(eb, 0));
-          mma_commit_pair(mapa_u32(eb, 1));
+          mma_commit_both(&empty_bar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        const uint32_t fb = smem_u32(&tmem_full_bar[acc]);
-        mma_commit_pair(mapa_u32(fb, 0));
-        mma_commit_pair(mapa_u32(fb, 1));
+        mma_commit_both(&tmem_full_bar[acc]);
 #ifdef AG_GEMM_PROBE
         pr_main += clock64() - pc1; pr_steps += num_kb;
 #endif
@@ -1752,15 +1748,11 @@ gemm_tc_chain_kernel(const __grid_constant__ ChainMaps maps, const __grid_consta
             for (int kk = 0; kk < BK / UMMA_K; kk++)
               mma_f16_ss_pair(tmem_d, desc_at(desc_a, at + kk * (UMMA_K * 2 >> 4)), desc_at(desc_b, at + kk * (UMMA_K * 128 >> 4)), idesc, (r > 0 || j > 0 || kk > 0) ? 1u : 0u);
           }
-          const uint32_t eb = smem_u32(&empty_bar[stage]);
-          mma_commit_pair(mapa_u32(eb, 0));
-          mma_commit_pair(mapa_u32(eb, 1));
+          mma_commit_both(&empty_bar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        const uint32_t fb = smem_u32(&tmem_full_bar[acc]);
-        mma_commit_pair(mapa_u32(fb, 0));
-        mma_commit_pair(mapa_u32(fb, 1));
+        mma_commit_both(&tmem_full_bar[acc]);
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
