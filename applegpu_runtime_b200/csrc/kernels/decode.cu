@@ -854,11 +854,12 @@ Status decode_linear(cudaStream_t s, const GemmDesc& d) {
   return cuda_status(e, "decode_linear");
 }
 
-// At most eight sequences (a cluster has one CTA for each) and no more clusters than run at once with one CTA an SM (238 registers): GPT-2
-// small, not large. Rows of up to 1024 columns.
+// At most eight sequences (a cluster has one CTA for each) and no more clusters than run at once with one CTA an SM (238 registers): two
+// thirds of the SMs, as clusters of eight do not fill every group of SMs. Twelve heads are faster for it at 64 and at 700 cached rows (224 and 349 us a
+// step of eight sequences, 272 and 373 as two launches); sixteen at width 1024 took 521 us behind a prompt of 1024, 388 as two launches.
 bool decode_qkv_attention_eligible(const GemmDesc& d, int heads, int t_max) {
   return d.dtype != DType::F32 && d.ln_gamma && decode_linear_eligible(d) && heads >= 1 && d.k == heads * 64 && d.k <= 1024 && d.n == 3 * d.k && d.m <= kDqRanks &&
-         heads * kDqRanks <= sm_count() && !d.ep.residual && d.ep.act == Act::None && t_max >= 1 && t_max <= 8192;
+         heads * kDqRanks * 3 <= sm_count() * 2 && !d.ep.residual && d.ep.act == Act::None && t_max >= 1 && t_max <= 8192;
 }
 template <typename T>
 static cudaError_t launch_dq(cudaStream_t s, const DecodeLinearParams& p, const DecodeAttnParams& a, int shares) {
