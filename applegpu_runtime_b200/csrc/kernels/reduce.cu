@@ -40,6 +40,15 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(sm100::smem_u32(dst)), "l"(src), "r"(bytes), "r"(sm100::smem_u32(bar)) : "memory");
 }
+// A warp's end, one lane: rows that it asked for and will not read (a wait for one of them gave up) have landed, or had as long again each, before
+// the block's shared memory goes to another; its results have left.
+__device__ __forceinline__ void bulk_leave(uint64_t* bar, int64_t row, int64_t asked, int64_t stride, int slot, uint32_t phase, int* status) {
+  for (; row < asked; row += stride) {
+    sm100::mbar_wait_limit(&bar[slot], phase, status, 9);
+    if (++slot == kSmSlots) { slot = 0; phase ^= 1; }
+  }
+  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
 // Blocks an SM of such a kernel with `smem` bytes of row buffers each; by_registers is the kernel's own, found once.
 template <typename K>
 static cudaError_t bulk_ctas(K kern, int smem, int max_row_bytes, int* by_registers, int* per_sm) {
@@ -166,13 +175,14 @@ __global__ void __launch_bounds__(kSmWarps * 32) layer_norm_bulk_kernel(const T*
   const float inv_cols = 1.0f / (float)cols;
   int slot = 0, free_slot = kSmSlots - 1;
   uint32_t phase = 0;
-  for (int64_t row = row0; row < rows; row += stride) {
+  int64_t row = row0;
+  for (; row < rows; row += stride) {
     if (lane == 0 && asked < rows) {
       asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the free slot's copy out has read it
       bulk_load(mine + free_slot * row_bytes, in + asked * cols, (uint32_t)row_bytes, &bar[free_slot]);
       asked += stride;
     }
-    if (!__all_sync(0xffffffffu, sm100::mbar_wait(&bar[slot], phase, status, 9))) break;
+    if (!__all_sync(0xffffffffu, sm100::mbar_wait_limit(&bar[slot], phase, status, 9))) break;
     uint4* const at = reinterpret_cast<uint4*>(mine + slot * row_bytes);
     uint4 x[ITERS];
     uint64_t s2 = 0;                                       // the bits of (0.f, 0.f)
@@ -218,7 +228,7 @@ __global__ void __launch_bounds__(kSmWarps * 32) layer_norm_bulk_kernel(const T*
     free_slot = slot;
     if (++slot == kSmSlots) { slot = 0; phase ^= 1; }
   }
-  if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  if (lane == 0) bulk_leave(bar, row, asked, stride, slot, phase, status);
 }
 template <typename T, int ITERS>
 static cudaError_t launch_layer_norm_bulk(cudaStream_t s, const T* x, const T* g, const T* b, T* y, int64_t rows, int cols, float eps, int* status) {
@@ -504,14 +514,15 @@ __global__ void __launch_bounds__(kSmWarps * 32) softmax_bulk_kernel(const T* __
   }
   int slot = 0, free_slot = kSmSlots - 1;
   uint32_t phase = 0;
-  for (int64_t row = row0; row < total_rows; row += stride) {
+  int64_t row = row0;
+  for (; row < total_rows; row += stride) {
     if (lane == 0 && asked < total_rows) {
       // the free slot held the row before last: its copy out must have read it
       asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
       ask(asked, free_slot);
       asked += stride;
     }
-    if (!__all_sync(0xffffffffu, sm100::mbar_wait(&bar[slot], phase, status, 9))) break;
+    if (!__all_sync(0xffffffffu, sm100::mbar_wait_limit(&bar[slot], phase, status, 9))) break;
     const int valid = softmax_valid<CAUSAL>(row, total_rows, rows_per_mat, cols);
     uint4* const at = reinterpret_cast<uint4*>(mine + slot * row_bytes);
     Pack<T> cur[ITERS];
@@ -527,7 +538,7 @@ __global__ void __launch_bounds__(kSmWarps * 32) softmax_bulk_kernel(const T* __
     free_slot = slot;
     if (++slot == kSmSlots) { slot = 0; phase ^= 1; }
   }
-  if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  if (lane == 0) bulk_leave(bar, row, asked, stride, slot, phase, status);
 }
 template <typename T, int ITERS, bool CAUSAL>
 static cudaError_t launch_softmax_bulk(cudaStream_t s, const T* x, T* y, int64_t total_rows, int64_t rows_per_mat, int64_t cols, int* status) {

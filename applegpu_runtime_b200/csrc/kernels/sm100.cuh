@@ -60,6 +60,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
     }
   }
 }
+// The same with the limit alone, for kernels in which no other role fails: a code that another kernel left does not end the wait.
+__device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, int* status, int code) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const unsigned long long t0 = globaltimer_ns();
+  uint32_t spins = 0;
+  while (!mbar_try_wait(bar, parity))
+    if ((++spins & 0xff) == 0 && globaltimer_ns() - t0 > kWaitLimitNs) { atomicCAS(status, 0, code); return false; }
+  return true;
+}
 
 // ── TMA ─────────────────────────────────────────────────────────────────────
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* m) {

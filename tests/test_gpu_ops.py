@@ -243,6 +243,25 @@ def test_softmax_rows_in_registers_and_by_bulk_copies(gpu_dev, dtype, causal, sh
         assert torch.all(got[ref == 0] == 0)
 
 
+def test_rows_by_bulk_copies_are_whole_behind_a_failed_wait(gpu_dev):
+    """A code that another kernel's wait left in the pipeline status word does not end the waits for rows: every row is written, and the
+    code is still there to be read."""
+    import torch
+    from applegpu_runtime_b200 import _lib
+    g = torch.Generator("cuda").manual_seed(11)
+    x = torch.randn((40000, 768), generator=g, device="cuda").to(torch.bfloat16)
+    s = torch.randn((24, 1024, 1024), generator=g, device="cuda").to(torch.bfloat16)
+    gain, shift = torch.ones(768, device="cuda").to(torch.bfloat16), torch.zeros(768, device="cuda").to(torch.bfloat16)
+    x, s, gain, shift = (gpu_dev.from_torch(t) for t in (x, s, gain, shift))
+    want = [gpu_dev.layer_norm(x, gain, shift, 1e-5).to_numpy(), gpu_dev.softmax_causal(s).to_numpy()]
+    assert gpu_dev.pipeline_status() == 0
+    assert _lib.load().applegpu_test_wait_runs_out(77, 1000) == 0
+    got = [gpu_dev.layer_norm(x, gain, shift, 1e-5).eval(), gpu_dev.softmax_causal(s).eval()]
+    assert gpu_dev.pipeline_status() == 77
+    for a, b in zip(got, want):
+        assert np.array_equal(a.to_numpy().view(np.uint8), b.view(np.uint8))
+
+
 def test_softmax_causal_all_masked_floor(gpu_dev):
     # the running max starts at -1e9 (kernel_templates.rs:478): values below it underflow to 0/0
     x = np.full((1, 2, 2), -2e9, np.float32); x[0, 1, 1] = 0.0
