@@ -215,6 +215,7 @@ EXT_SYMBOLS = {
     "applegpu_ffi_mlstm": (u64, [u64, u64, u64, u64, u64, u32, u32, u32, f32, f32, i32]),
     "applegpu_ffi_latent_attention": (u64, [u64, u64, u64, u64, u64, u64, u32, u32, u32, u32, u32, u32, f32, f32, i32]),
     "applegpu_test_wait_runs_out": (i32, [i32, u32]),
+    "applegpu_test_attention_band": (i32, [i64, i64, cbool, i32]),
 }
 
 _lib = None

@@ -32,6 +32,7 @@ Status decoder_cache(uint64_t handle, int layer, bool values, TensorRec* out);
 Status decoder_set_engine(uint64_t handle, int engine);
 void decoder_destroy(uint64_t handle);
 namespace k {
+int attention_band(int64_t heads, int64_t keys, bool causal, int sms);
 void set_matmul_path(int mode);
 void set_gemm_tile(int code);
 }
@@ -1669,6 +1670,7 @@ int32_t applegpu_test_wait_runs_out(int32_t code, uint32_t limit_us) {
   if (!s.ok()) { set_ffi_error("test_wait_runs_out failed: " + s.to_string()); return -1; }
   return 0;
 }
+int32_t applegpu_test_attention_band(int64_t heads, int64_t keys, bool causal, int32_t sms) { return k::attention_band(heads, keys, causal, sms); }
 void applegpu_profile_enable(bool on) { ag::profile::enable(on); }
 void applegpu_profile_clear(void) { ag::profile::clear(); }
 void applegpu_profile_filter(const char* prefixes) { ag::profile::set_filter(prefixes ? prefixes : ""); }

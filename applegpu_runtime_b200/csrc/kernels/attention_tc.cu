@@ -71,7 +71,7 @@ __device__ unsigned long long g_attn_cta[4096][4];
 #endif
 
 // The tiles one CTA works through, the same sequence for each of its warp roles. Tiles are ranked band of heads by band of
-// heads (attention_band below), in a band heaviest first
+// heads (attention_band below; one band under a causal mask), heaviest first
 // (under a causal mask the last query tile of a head sees the most keys; every head has the same tiles), and dealt
 // to the CTAs in passes that alternate direction, so the CTA that got the heaviest tile of one pass gets the
 // lightest of the next: a fixed schedule (no counter in global memory) within ~10 % of an even split.
@@ -443,18 +443,20 @@ static Status launch_attention(cudaStream_t s, const CUtensorMap& mq, const CUte
 
 // Heads per band. Every query tile of a head reads the head's keys and values up to its own last row; ranked over all heads at
 // once, a head's tiles run one whole round of the heads apart, and keys and values that do not stay in the L2 come from
-// memory once per query tile (256 x 12 heads of 512 keys: 4 x 403 MB). So heads are taken in bands whose keys and values
-// stay. A band of as many heads as there are SMs gives each of the two CTAs of an SM whole rounds when the number of query
-// tiles is even, so that the heaviest-first order still evens out (the busiest CTA has 57 blocks of a mean of 51.9 over 640 causal
-// heads of 512 keys, banded or not). Up to 64 MB (half the L2) there is one band.
-// 256 x 12 heads of 512 tokens in a running forward: 511 -> 418 us a launch.
-static int attention_band(int64_t bh, int64_t tk) {
+// memory once per query tile (256 x 12 heads of 512 keys: 4 x 403 MB). So without a mask heads are taken in bands whose keys and
+// values stay. Up to 64 MB (half the L2) there is one band; just above there is nothing to win yet. 256 x 12 heads of 512 tokens in a running
+// forward: 511 -> 418 us a launch. One band against bands, alone, us: 3072 heads x 512 tokens (403 MB) 378 / 349, 1500 x 256 (98 MB)
+// 54.5 / 53.4, 1200 x 300 75.5 / 74.7, 648 x 512 (85 MB) 81.0 / 81.2, 600 x 450 (69 MB) 73.7 / 74.0, 40 x 8192 1035 / 1034.
+// Under a causal mask the tiles of a head differ, and the heaviest ones of every band land on the same CTAs unless a band fills whole pairs
+// of passes: 40 x 8192 515 / 713, 48 x 6000 342 / 399, 384 x 800 83.7 / 87.8; where it does, bands bring little: 2040 x 512 (267 MB)
+// 173 / 169, 640 x 512 59.3 / 59.3, 512 x 1024 137.5 / 139.2. So there is one band.
+int attention_band(int64_t heads, int64_t keys, bool causal, int sms) {
   constexpr int64_t keep = 64 << 20;
-  const int64_t per_head = tk * kD * 2 * 2;
-  if (bh * per_head <= keep) return (int)bh;
-  int64_t band = sm_count();
+  const int64_t per_head = keys * kD * 2 * 2;
+  if (causal || heads * per_head <= keep) return (int)heads;
+  int64_t band = sms;
   while (band > 16 && band * per_head > keep) band /= 2;
-  return (int)(band < bh ? band : bh);
+  return (int)(band < heads ? band : heads);
 }
 
 Status attention(cudaStream_t s, const AttnDesc& d) {
@@ -472,7 +474,7 @@ Status attention(cudaStream_t s, const AttnDesc& d) {
   p.scale_log2 = d.scale * 1.4426950408889634f;
   p.status = st;
   p.bh = (int)(d.batch * d.heads); p.q_tiles = (int)((d.tq + kQ - 1) / kQ); p.total_tiles = p.bh * p.q_tiles;
-  p.band = attention_band(p.bh, d.tk);
+  p.band = attention_band(p.bh, d.tk, d.causal, sm_count());
   // persistent CTAs: two per SM (registers and tensor-memory columns allow two), each walking its share of the tiles
   const int resident = 2 * sm_count();
   dim3 grid((unsigned)(p.total_tiles < resident ? p.total_tiles : resident), 1, 1);

@@ -209,6 +209,8 @@ APPLEGPU_API int32_t applegpu_pipeline_status(void);
  * microseconds (capped at 50 ms), on a barrier nothing arrives at, then records `code` in the pipeline
  * status word and returns. It exercises the error path of the bounded waits without a fault or a hang. */
 APPLEGPU_API int32_t applegpu_test_wait_runs_out(int32_t code, uint32_t limit_us);
+/* Test hook: how many heads' tiles the 16-bit attention kernel ranks together on a device of `sms` multiprocessors. */
+APPLEGPU_API int32_t applegpu_test_attention_band(int64_t heads, int64_t keys, bool causal, int32_t sms);
 /* CUDA-event stopwatch on the runtime stream. */
 /* Op tapes: record the graph-flavour ops one pass of a host program issues, then re-record the same
  * ops on new inputs with one call (the per-op host cost of a Python driver is paid once). Between

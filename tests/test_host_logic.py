@@ -379,3 +379,26 @@ def test_kernels_wait_for_their_predecessor_before_they_release_their_successor(
             else:
                 assert "pdl_trigger();" not in line, f"{f.name}:{i + 1}"
     assert found >= 40
+
+
+@pytest.mark.parametrize("heads,tokens", [(40, 8192), (48, 6000), (24, 16384), (21, 13000), (384, 800), (320, 1024), (300, 1000), (640, 512), (2040, 512), (1500, 256), (12, 4096)])
+def test_attention_bands_leave_the_busiest_cta_as_it_was(gpu, heads, tokens):
+    """Bands of heads must not cost balance: key blocks of the busiest of 2 x 148 CTAs, tiles dealt as in kernels/attention_tc.cu, against all
+    heads ranked at once; without a mask a band's keys and values fit the 64 MB that are kept."""
+    from applegpu_runtime_b200 import _lib
+    sms, q_tiles, blocks = 148, -(-tokens // 128), -(-tokens // 64)
+
+    def busiest(band, causal):
+        total, work = heads * q_tiles, np.zeros(2 * sms, np.int64)
+        r = np.arange(total)
+        row, at = r // (2 * sms), r % (2 * sms)
+        first = r // (band * q_tiles) * band
+        tile = q_tiles - 1 - (r - first * q_tiles) // np.minimum(band, heads - first)
+        np.add.at(work, np.where(row % 2 == 1, 2 * sms - 1 - at, at), np.minimum(blocks, 2 * (tile + 1)) if causal else blocks)
+        return work.max()
+    for causal in (True, False):
+        band = _lib.load().applegpu_test_attention_band(heads, tokens, causal, sms)
+        assert 1 <= band <= heads
+        assert busiest(band, causal) <= busiest(heads, causal)
+        if not causal and band < heads:
+            assert band * tokens * 256 <= 64 << 20 or band <= 16
