@@ -708,7 +708,7 @@ __global__ void __launch_bounds__(kDlThreads) decode_qkv_attention_kernel(const 
   const int rank = (int)sm100::cluster_ctarank(), h = blockIdx.x, d = a.heads * 64, tid = threadIdx.x, warp = tid >> 5;
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   const bool works = rank < shares, attends = rank < p.m;
-  const int k0 = rank * kDlRows;                           // rows of up to 1024 columns: a slab a share
+  const int k0 = rank * kDlRows;                           // a slab a share
   uint4 wv[3][4];
   uint2 x[1], gam = make_uint2(0u, 0u), bet = gam;
   if (works) {
@@ -854,12 +854,17 @@ Status decode_linear(cudaStream_t s, const GemmDesc& d) {
   return cuda_status(e, "decode_linear");
 }
 
-// At most eight sequences (a cluster has one CTA for each) and no more clusters than run at once with one CTA an SM (238 registers): two
-// thirds of the SMs, as clusters of eight do not fill every group of SMs. Twelve heads are faster for it at 64 and at 700 cached rows (224 and 349 us a
-// step of eight sequences, 272 and 373 as two launches); sixteen at width 1024 took 521 us behind a prompt of 1024, 388 as two launches.
+// At most eight sequences (a cluster has one CTA for each), more than four shares of K (nine heads: with fewer the two launches have clusters
+// of at most four), and no more clusters than run at once with one CTA an SM (238 registers): two thirds of the SMs, as clusters of eight do
+// not fill every group of SMs; with 148 SMs that is twelve heads. A step of six layers, us, two launches / one:
+//   heads      1          4          8          9          10         11         12         13         14         15         16
+//   1 seq.,    64 rows    70 / 74    82 / 86    97 / 100   105 / 101  107 / 102  111 / 111  113 / 111  132 / 131  135 / 138  148 / 148  149 / 167
+//   8 seq.,    64 rows    78 / 84    94 / 96    110 / 113  117 / 110  120 / 111  127 / 127  130 / 119  156 / 150  159 / 159  178 / 172  182 / 205
+//   8 seq.,   900 rows    114 / 122  129 / 133  171 / 178  189 / 183  193 / 186  199 / 197  201 / 200  225 / 220  229 / 228  246 / 243  249 / 334
+// and eight behind 7 900 rows 615 / 600 with twelve heads, 597 / 587 with nine. Thirteen to fifteen differ by -4 to +2 % and stay apart.
 bool decode_qkv_attention_eligible(const GemmDesc& d, int heads, int t_max) {
-  return d.dtype != DType::F32 && d.ln_gamma && decode_linear_eligible(d) && heads >= 1 && d.k == heads * 64 && d.k <= 1024 && d.n == 3 * d.k && d.m <= kDqRanks &&
-         heads * kDqRanks * 3 <= sm_count() * 2 && !d.ep.residual && d.ep.act == Act::None && t_max >= 1 && t_max <= 8192;
+  return d.dtype != DType::F32 && d.ln_gamma && decode_linear_eligible(d) && d.k == heads * 64 && d.k > 4 * kDlRows && d.k <= kDqRanks * kDlRows /* a slab a share */ &&
+         d.n == 3 * d.k && d.m <= kDqRanks && heads * kDqRanks * 3 <= sm_count() * 2 && !d.ep.residual && d.ep.act == Act::None && t_max >= 1 && t_max <= 8192;
 }
 template <typename T>
 static cudaError_t launch_dq(cudaStream_t s, const DecodeLinearParams& p, const DecodeAttnParams& a, int shares) {

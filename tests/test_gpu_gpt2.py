@@ -123,10 +123,12 @@ def test_gpt2_int8_weights_bf16_activations_against_dequantised_oracle(gpu_dev):
 
 
 @pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
-@pytest.mark.parametrize("batch,heads,vocab", [(1, 1, 33), (8, 2, 97), (9, 12, 1000), (16, 3, 64), (5, 16, 130), (8, 18, 4097), (3, 20, 257)])
+@pytest.mark.parametrize("batch,heads,vocab", [(1, 1, 33), (8, 2, 97), (9, 12, 1000), (16, 3, 64), (5, 16, 130), (8, 18, 4097), (3, 20, 257),
+                                                (8, 12, 500), (1, 12, 70), (3, 5, 100), (8, 9, 90), (7, 11, 129), (1, 10, 300)])
 def test_decoder_picks_the_largest_logit(gpu_dev, dtype, batch, heads, vocab):
-    """QKV and attention in one launch (up to eight sequences, twelve heads) and apart, the head at vocabularies that end inside a warp's
-    sixteen rows and a block's 64: every pick has the largest logit of the float32 oracle on the same weights, to rounding."""
+    """QKV and attention in one launch (up to eight sequences, nine to twelve heads: five and six shares of K, the last whole or half) and
+    apart, the head at vocabularies that end inside a warp's sixteen rows and a block's 64: every pick has the largest logit of the float32
+    oracle on the same weights, to rounding."""
     from applegpu_runtime_b200.generate import Gpt2Decoder
     cfg = {"n_layer": 2, "n_head": heads, "n_embd": 64 * heads, "vocab_size": vocab, "n_positions": 64}
     m = gpu_dev.init_gpt2_weights(cfg, seed=heads + vocab, dtype=dtype, std=0.08)
@@ -140,10 +142,26 @@ def test_decoder_picks_the_largest_logit(gpu_dev, dtype, batch, heads, vocab):
     seq = np.concatenate([ids, first.to_numpy().reshape(-1, 1), rest.T], 1)
     with torch.no_grad():
         ref = torch_ref.gpt2_forward(w, cfg, torch.from_numpy(seq))[0].numpy()
-    # two layers of a dozen roundings to 2^-9 each, summed as if they all had one sign: under 2^-5 of a logit's scale; a pick from a wrong row is at 1
+    # two layers of a dozen roundings to 2^-9 each, of either sign: sqrt(24) 2^-9 = 0.01 of a logit's scale for the pick and as much for the
+    # largest; a pick from a wrong row is at 1
     for i in range(7):
         row = ref[:, 6 + i]
         assert np.all(row.max(-1) - row[np.arange(batch), seq[:, 7 + i]] <= 2e-2 * np.abs(row).max())
+
+
+@pytest.mark.parametrize("batch,heads,per_layer", [(1, 1, 5), (8, 4, 5), (1, 8, 5), (8, 8, 5), (1, 9, 4), (8, 12, 4), (9, 12, 5), (1, 13, 5), (8, 16, 5)])
+def test_decoder_takes_qkv_and_attention_in_one_launch_where_it_is_faster(gpu_dev, batch, heads, per_layer):
+    from applegpu_runtime_b200.generate import Gpt2Decoder
+    launches = []
+    for layers in (1, 3):
+        cfg = {"n_layer": layers, "n_head": heads, "n_embd": 64 * heads, "vocab_size": 64, "n_positions": 32}
+        m = gpu_dev.init_gpt2_weights(cfg, seed=1, dtype="bfloat16", std=0.05)
+        logits, kv = gpu_dev.gpt2_forward(m, np.zeros((batch, 3), np.int64), last_only=True)
+        dec = Gpt2Decoder(m, batch, 16)
+        dec.prefill(kv, gpu_dev.argmax(logits), 3)
+        dec.steps(2)
+        launches.append(dec.launches_per_step)
+    assert launches[1] - launches[0] == 2 * per_layer
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
