@@ -283,14 +283,14 @@ __device__ long long g_epi_probe[8];   // [0] tmem load + wait, [1] math, [2] st
 #define AG_EPI_T(var)
 #define AG_EPI_ADD(slot, a, b)
 #endif
-template <typename T>
+template <typename T, bool DIRECT = true>      // DIRECT: p.vec_ok may be 2
 __device__ __forceinline__ void epilogue_group(const TcParams& p, uint32_t taddr, uint8_t* stg, const T* bias_s, const float* scale_s, uint32_t (&rpre)[16],
                                                long long row0, int col0, int next_col0, long long c_off, int lane, unsigned long long& best_key,
                                                float ln_mean, float ln_rstd, float& row_sum, float& row_sq, const float* bias_f = nullptr) {
   T* C = reinterpret_cast<T*>(p.c) + c_off;
   const T* R = p.residual ? reinterpret_cast<const T*>(p.residual) + c_off : nullptr;
   const int sub_row = lane >> 2, sub_chunk = lane & 3;
-  const bool direct = p.vec_ok == 2;
+  const bool direct = DIRECT && p.vec_ok == 2;
 
   // 1. residual. Direct layout: this group's row was fetched one group ahead; the next group's fetch is issued here
   //    and lands while this group is computed. Staged layouts: the tile goes to shared memory (coalesced reads).
@@ -1178,15 +1178,21 @@ template <int BN> struct PairCfg {
 // only copy of the weights in global memory is the int8 one and no widened copy is ever written there.
 constexpr int kConvWarps = 4;
 // Packed: rows on 32 bytes, or gated results; general: everything else (staged rows, a row argmax) with
-// eight epilogue warps; W8: int8 weights, either epilogue with eight.
+// eight epilogue warps; W8: int8 weights, either epilogue with eight. The general form leaves out what rows on 32 bytes alone reach: 166
+// registers, no spills in place of up to 52 bytes, us with and without: 40000 x 1000 x 520 68.3 / 59.2, with GELU 83.0 / 65.9, 8192 x 1000 x 520
+// 20.4 / 18.5, an LM head of 8192 rows with its row argmax 484 / 430.
 enum PairKind { kPairGeneral = 0, kPairPacked = 1, kPairW8 = 2 };
 constexpr int pair_epi_warps(int kind) { return kind == kPairPacked ? 16 : kEpiWarps; }
 constexpr int pair_threads(int kind) { return 64 + pair_epi_warps(kind) * 32 + (kind == kPairW8 ? kConvWarps * 32 : 0); }
 // Tile `rem` of a batch: bands of p.band row tiles, in a band column tile after column tile (pair_band below).
 __device__ __forceinline__ void pair_tile(const TcParams& p, int rem, int& mi, int& ni) {
-  const int per = p.band * p.tiles_n, b = rem / per, r = rem - b * per, high = min(p.band, p.tiles_m - b * p.band);
-  ni = r / high;
-  mi = b * p.band + r - ni * high;
+  int first = 0, high = p.tiles_m;
+  if (p.band < p.tiles_m) {
+    const int b = rem / (p.band * p.tiles_n);
+    first = b * p.band; rem -= first * p.tiles_n; high = min(p.band, p.tiles_m - first);
+  }
+  ni = rem / high;
+  mi = first + rem - ni * high;
 }
 // Four int8 values (one 32-bit word) -> two words of packed 16-bit floats, exactly. Each byte is biased to
 // unsigned (u = v + 128), dropped into the mantissa of 2^23 (0x4B000000 | u = 8388608 + u), and the float
@@ -1425,39 +1431,34 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
       }
       T* bias_s = reinterpret_cast<T*>(smem + STAGES * Cfg::kStageBytes + kStgBytes) + (warp - 2) * epi_slots(BN);
-      // 16-bit C with 32-byte aligned rows: the packed epilogue takes the bias as floats; they wait in the warp's staging
+      // int8 form, 16-bit C with 32-byte aligned rows: epilogue_group's packed path takes the bias as floats; they wait in the warp's staging
       // tile, which that layout leaves unused (zeros when there is no bias)
-      const bool packed_epi = p.vec_ok == 2 && !p.c_f32 && !p.argmax_keys;
+      const bool packed_epi = W8 && p.vec_ok == 2 && !p.c_f32 && !p.argmax_keys;
       float* bias_f = reinterpret_cast<float*>(smem + STAGES * Cfg::kStageBytes + (warp - 2) * kStgBytesPerWarp);
-      if (PACKED) {
-      } else if (packed_epi) {
-        const T* bias = reinterpret_cast<const T*>(p.bias);
-#pragma unroll
-        for (int gi = 0; gi < BN / 64; gi++) {
-          int ci = n0 + (pair + 2 * gi) * 32 + lane;
-          bias_f[gi * 32 + lane] = (bias && ci < p.n) ? Cvt<T>::to(__ldg(bias + ci)) : 0.f;
-        }
-      } else if (p.bias && !p.c_f32) {
-        const T* bias = reinterpret_cast<const T*>(p.bias);
-#pragma unroll
-        for (int gi = 0; gi < BN / 64; gi++) {
-          int ci = n0 + (pair + 2 * gi) * 32 + lane;
-          bias_s[gi * 32 + lane] = ci < p.n ? __ldg(bias + ci) : Cvt<T>::from(0.f);
-        }
-      }
       float* scale_s = reinterpret_cast<float*>(smem + STAGES * Cfg::kStageBytes + kStgBytes + bias_bytes(BN)) + (warp - 2) * epi_slots(BN);
       // the float slots hold the int8 per-channel scales, or the float32 bias of a float32-output product
       const float* fsrc = p.c_f32 ? reinterpret_cast<const float*>(p.bias) : (p.ln_stats ? p.ln_colsum : p.b_scales);
-      if (!PACKED && fsrc) {
-#pragma unroll
-        for (int gi = 0; gi < BN / 64; gi++) {
-          int ci = n0 + (pair + 2 * gi) * 32 + lane;
-          scale_s[gi * 32 + lane] = ci < p.n ? __ldg(fsrc + ci) : 0.f;
-        }
-      }
       uint32_t rpre[16];
-      if (!PACKED && p.residual && p.vec_ok == 2 && !p.c_f32 && n0 + pair * 32 < p.n)
-        load_residual_row<T>(p, reinterpret_cast<const T*>(p.residual) + c_off, row0 + lane, n0 + pair * 32, rpre);
+      if constexpr (!PACKED) {
+        if (p.bias && !p.c_f32 || packed_epi) {
+          const T* bias = reinterpret_cast<const T*>(p.bias);
+#pragma unroll
+          for (int gi = 0; gi < BN / 64; gi++) {
+            int ci = n0 + (pair + 2 * gi) * 32 + lane;
+            const T b = (bias && ci < p.n) ? __ldg(bias + ci) : Cvt<T>::from(0.f);
+            if (packed_epi) bias_f[gi * 32 + lane] = Cvt<T>::to(b); else bias_s[gi * 32 + lane] = b;
+          }
+        }
+        if (fsrc) {
+#pragma unroll
+          for (int gi = 0; gi < BN / 64; gi++) {
+            int ci = n0 + (pair + 2 * gi) * 32 + lane;
+            scale_s[gi * 32 + lane] = ci < p.n ? __ldg(fsrc + ci) : 0.f;
+          }
+        }
+        if (W8 && p.residual && p.vec_ok == 2 && !p.c_f32 && n0 + pair * 32 < p.n)
+          load_residual_row<T>(p, reinterpret_cast<const T*>(p.residual) + c_off, row0 + lane, n0 + pair * 32, rpre);
+      }
       // folded layer_norm: this row's statistics are fetched (and turned into scale and shift) before the accumulator wait too
       float ln_mean = 0.f, ln_rstd = 1.f;
       if (row0 + lane < p.m) ln_stats_finish(p, stats_cur, ln_mean, ln_rstd);
@@ -1507,11 +1508,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         for (int g = pair, gi = 0; g < BN / 32; g += 2, gi++) {
           if (n0 + g * 32 >= p.n) break;
           int next_col0 = (g + 2 < BN / 32 && n0 + (g + 2) * 32 < p.n) ? n0 + (g + 2) * 32 : -1;
-          if (p.glu_n) { glu_group<T>(p, taddr + (uint32_t)(g * 32), row0, n0 + g * 32, lane); continue; }
-          epilogue_group<T>(p, taddr + (uint32_t)(g * 32), stg, (p.bias && !p.c_f32) ? bias_s + gi * 32 : nullptr, fsrc ? scale_s + gi * 32 : nullptr, rpre, row0, n0 + g * 32, next_col0,
-                            c_off, lane, best_key, ln_mean, ln_rstd, row_sum, row_sq, packed_epi ? bias_f + gi * 32 : nullptr);
+          if (W8 && p.glu_n) { glu_group<T>(p, taddr + (uint32_t)(g * 32), row0, n0 + g * 32, lane); continue; }
+          epilogue_group<T, W8>(p, taddr + (uint32_t)(g * 32), stg, (p.bias && !p.c_f32) ? bias_s + gi * 32 : nullptr, fsrc ? scale_s + gi * 32 : nullptr, rpre, row0, n0 + g * 32, next_col0,
+                                c_off, lane, best_key, ln_mean, ln_rstd, row_sum, row_sq, packed_epi ? bias_f + gi * 32 : nullptr);
         }
-        }
+      }
       if (p.argmax_keys && best_key != 0 && row0 + lane < p.m) atomicMax(p.argmax_keys + row0 + lane, best_key);
       tc_fence_before_sync();
       __syncwarp();
