@@ -355,14 +355,17 @@ __global__ void __launch_bounds__(256) key_decay_tail_kernel(const KdParams p) {
   }
 }
 
-// A CTA for each SM at most (its registers hold the weights), one item a thread.
+// One item a thread, and all clusters at once: the kernel's registers hold the weights, so that an SM has one CTA, and clusters do not fill
+// every group of SMs (of eight CTAs fifteen fit, not eighteen). Rurunex at width 1024, us, this form never / with the SMs alone counted / now: four
+// sequences (16 clusters of eight) a step 274 / 280 / 261, 16 tokens 1371 / 1490 / 1273; nine sequences (36 clusters of four) 16 tokens 1457
+// / 1486 / 1278.
 template <typename T>
-static bool kd_ahead(const KdParams& p, int ranks, int slice) {
+static bool kd_ahead(const KdParams& p, int slice) {
   auto round = [](int rank, int n) { const int pieces = (rank + Pack<T>::N - 1) / Pack<T>::N, g = kd_lanes(pieces); return n <= kKsThreads / g && pieces <= g * kKsPieces; };
-  return (long long)ranks * p.heads * p.n_seq <= sm_count() && p.taps <= 4 && 2 * p.dim + slice <= kKsThreads && (p.z || round(p.a_rank, p.dim)) && (p.gate || !p.g_rank || round(p.g_rank, slice));
+  return p.taps <= 4 && 2 * p.dim + slice <= kKsThreads && (p.z || round(p.a_rank, p.dim)) && (p.gate || !p.g_rank || round(p.g_rank, slice));
 }
 template <typename T, int VEC, int NR, bool AHEAD>
-static cudaError_t launch_ks_as(cudaStream_t s, const KdParams& p, int ranks, int slice, int tx_n, int sub, size_t smem) {
+static cudaError_t launch_ks_as(cudaStream_t s, const KdParams& p, int ranks, int slice, int tx_n, int sub, size_t smem, bool* fits = nullptr) {
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(key_decay_step_kernel<T, VEC, NR, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
@@ -375,11 +378,30 @@ static cudaError_t launch_ks_as(cudaStream_t s, const KdParams& p, int ranks, in
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   at[1].id = cudaLaunchAttributeClusterDimension; at[1].val.clusterDim.x = (unsigned)ranks; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
   cfg.attrs = at; cfg.numAttrs = 2;
+  if (fits) {                                         // no launch: whether its clusters are all resident at once
+    static int at_once[4] = {0, 0, 0, 0};             // by cluster size 1, 2, 4, 8; less 1. The registers bound it, not the shared memory
+    int& n = at_once[ranks >= 8 ? 3 : ranks >= 4 ? 2 : ranks >= 2 ? 1 : 0];
+    if (!n) {
+      cudaLaunchConfig_t q = cfg;
+      q.attrs = at + 1; q.numAttrs = 1;
+      int got = 0;
+      const cudaError_t e = cudaOccupancyMaxActiveClusters(&got, key_decay_step_kernel<T, VEC, NR, AHEAD>, &q);
+      if (e != cudaSuccess) return e;
+      n = got + 1;
+    }
+    *fits = (long long)p.heads * p.n_seq < n;
+    return cudaSuccess;
+  }
   return cudaLaunchKernelEx(&cfg, key_decay_step_kernel<T, VEC, NR, AHEAD>, p, slice, tx_n, sub);
 }
 template <typename T, int VEC, int NR>
 static cudaError_t launch_ks(cudaStream_t s, const KdParams& p, int ranks, int slice, int tx_n, int sub, size_t smem) {
-  return kd_ahead<T>(p, ranks, slice) ? launch_ks_as<T, VEC, NR, true>(s, p, ranks, slice, tx_n, sub, smem) : launch_ks_as<T, VEC, NR, false>(s, p, ranks, slice, tx_n, sub, smem);
+  bool ahead = kd_ahead<T>(p, slice);
+  if (ahead) {
+    const cudaError_t e = launch_ks_as<T, VEC, NR, true>(s, p, ranks, slice, tx_n, sub, smem, &ahead);
+    if (e != cudaSuccess) return e;
+  }
+  return ahead ? launch_ks_as<T, VEC, NR, true>(s, p, ranks, slice, tx_n, sub, smem) : launch_ks_as<T, VEC, NR, false>(s, p, ranks, slice, tx_n, sub, smem);
 }
 
 static Status key_decay_step(cudaStream_t s, DType dt, const KdParams& p) {
