@@ -372,9 +372,9 @@ __device__ __forceinline__ void softmax_row16(const Pack<T> (&cur)[ITERS], int l
     put(pk, reinterpret_cast<const Pack<T>&>(o));
   }
 }
-template <typename T, int ITERS, bool CAUSAL, typename Put>
+template <typename T, int ITERS, bool CAUSAL, bool WORDS, typename Put>
 __device__ __forceinline__ void softmax_row(const Pack<T> (&cur)[ITERS], int lane, int packs, int valid, Put put) {
-  if constexpr (sizeof(T) == 2) { softmax_row16<T, ITERS, CAUSAL>(cur, lane, packs, valid, put); return; }
+  if constexpr (WORDS) { softmax_row16<T, ITERS, CAUSAL>(cur, lane, packs, valid, put); return; }
   constexpr int N = Pack<T>::N;
   float v[ITERS][N];
   float m = CAUSAL ? -1e9f : -INFINITY;
@@ -446,6 +446,9 @@ __device__ __forceinline__ int softmax_valid(int64_t row, int64_t total_rows, in
 // current one (a row's chain load -> max -> exp -> sum -> store is latency-bound on its own). Packs wholly left of the
 // diagonal take a mask-free path, the one pack the diagonal crosses is masked per element, packs right of it are
 // neither read nor computed: zeros are stored.
+// Rows of one pack a lane are too short for the word form, which has the longer chain: 1850 x 128 x 128 bfloat16 69.7 us element by element, 96.4 by
+// words, float16 64.6 / 97.2, causal 84.4 / 117.1; only causal bfloat16 gains, 124.3 / 117.0.
+template <typename T, int ITERS, bool CAUSAL> constexpr bool softmax_words = sizeof(T) == 2 && (ITERS > 1 || (CAUSAL && std::is_same<T, __nv_bfloat16>::value));
 template <typename T, int ITERS, bool CAUSAL>
 __global__ void __launch_bounds__(128, 4) softmax_warp_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t total_rows, int rows_per_mat, int cols) {
   constexpr int N = Pack<T>::N;
@@ -473,7 +476,7 @@ __global__ void __launch_bounds__(128, 4) softmax_warp_kernel(const T* __restric
       for (int it = 0; it < ITERS; it++) { int pk = lane + it * 32; if (pk < packs && pk * N < next_valid) nxt[it] = ld16_stream(in + next * cols + pk * N); }
     }
     T* y = out + row * cols;
-    softmax_row<T, ITERS, CAUSAL>(cur, lane, packs, valid, [&](int pk, const Pack<T>& o) { st16_stream(y + pk * N, o); });
+    softmax_row<T, ITERS, CAUSAL, softmax_words<T, ITERS, CAUSAL>>(cur, lane, packs, valid, [&](int pk, const Pack<T>& o) { st16_stream(y + pk * N, o); });
 #pragma unroll
     for (int it = 0; it < ITERS; it++) cur[it] = nxt[it];
     valid = next_valid;
@@ -481,12 +484,17 @@ __global__ void __launch_bounds__(128, 4) softmax_warp_kernel(const T* __restric
 }
 
 // The same with rows that come and go by bulk copies. A warp has kSmSlots row buffers in shared memory: one lane asks for a row's
-// unmasked part two rows ahead, the row is computed in place, and the whole row leaves as one copy, zeros included. No register holds a row
+// unmasked part three rows ahead, the row is computed in place, and the whole row leaves as one copy, zeros included. No register holds a row
 // that is on its way, so more warps fit an SM.
-// For rows of 512 to 2048 bytes (4096 of float32), 32 of them an SM. Rows in registers against bulk copies, causal, us: bfloat16 96 x
+// For rows of 512 to 2048 bytes (4096 of float32), from 32 of them an SM on (the warps of the form above ask for their third row there), of less than
+// 768 bytes from 80. Rows in registers against bulk copies, causal, us: bfloat16 96 x
 // 1024 x 1024 65.4 / 59.6, 96 x 512 x 512 34.4 / 23.6, 96 x 256 x 256 14.5 / 10.8, 96 x 128 x 128 6.3 / 6.8, 3 x 1024 x 1024 4.9 /
-// 5.5, 8 x 2048 x 2048 20.5 / 25.5; float32 112.9 / 106.4, 36.6 / 27.7, 15.8 / 11.5, 6.8 / 6.1, 6.6 / 6.7, 61 / 82. (Element by element,
+// 5.5, 8 x 2048 x 2048 20.5 / 25.5; float32 112.9 / 106.4, 36.6 / 27.7, 15.8 / 11.5, 6.8 / 6.1, 6.6 / 6.7, 61 / 82; rows of 512 bytes at 32, 64 and 97
+// an SM, float32 3.6 / 4.1, 5.0 / 5.2, 7.7 / 6.4, 256 of bfloat16 3.7 / 3.9, 5.3 / 5.7, 9.1 / 7.1. (Element by element,
 // in registers, the first took 72: it was bound by instructions.) What bounds it now: memory, 302 MB at 5.1 TB/s.
+// Without a mask: bfloat16 48 x 1024 x 1024 42.8 / 36.1, 382 x 256 x 256 43.8 / 27.6; float32 382 x 256 x 256 51.1 / 37.8, 64 x 768 x 768 57.7 / 55.2.
+// float32 rows of more than 2048 bytes and 160 MB in all stay in registers, whose loads and stores do not push one another out of the L2: 127 x
+// 768 x 768 110.0 / 110.8, 254 215 / 221, 48 x 1024 x 1024 68.4 / 73.6, 191 255 / 290; 64 x 768 x 768 (151 MB) and less as above.
 template <typename T> constexpr int kSmMaxRowBytes = sizeof(T) == 4 ? 4096 : 2048;
 template <typename T, int ITERS, bool CAUSAL>
 __global__ void __launch_bounds__(kSmWarps * 32) softmax_bulk_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t total_rows, int rows_per_mat, int cols, int* status) {
@@ -517,7 +525,7 @@ __global__ void __launch_bounds__(kSmWarps * 32) softmax_bulk_kernel(const T* __
   int64_t row = row0;
   for (; row < total_rows; row += stride) {
     if (lane == 0 && asked < total_rows) {
-      // the free slot held the row before last: its copy out must have read it
+      // the free slot held the row just done: its copy out must have read it (a warp waits here, the SM has others)
       asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
       ask(asked, free_slot);
       asked += stride;
@@ -531,7 +539,7 @@ __global__ void __launch_bounds__(kSmWarps * 32) softmax_bulk_kernel(const T* __
       const int pk = lane + it * 32;
       if (pk < packs && pk * N < valid) *reinterpret_cast<uint4*>(&cur[it]) = at[pk];
     }
-    softmax_row<T, ITERS, CAUSAL>(cur, lane, packs, valid, [&](int pk, const Pack<T>& o) { at[pk] = *reinterpret_cast<const uint4*>(&o); });
+    softmax_row<T, ITERS, CAUSAL, sizeof(T) == 2>(cur, lane, packs, valid, [&](int pk, const Pack<T>& o) { at[pk] = *reinterpret_cast<const uint4*>(&o); });
     sm100::fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) bulk_store(out + row * cols, at, (uint32_t)row_bytes);
@@ -593,7 +601,8 @@ static Status softmax_t(cudaStream_t s, const TView& in, const TView& out) {
     cudaError_t le = cudaSuccess;
     int* status = matmul_status_word();
     const int64_t row_bytes = cols * (int64_t)sizeof(T);
-    if (status && row_bytes >= kSmMinRowBytes && row_bytes <= kSmMaxRowBytes<T> && total_rows >= 32 * (int64_t)sm_count()) {
+    const bool large = !CAUSAL && row_bytes > 2048 && total_rows * row_bytes > (160ll << 20);      // float32
+    if (status && row_bytes >= kSmMinRowBytes && row_bytes <= kSmMaxRowBytes<T> && total_rows >= (row_bytes < 768 ? 80 : 32) * (int64_t)sm_count() && !large) {
 #define AG_SMB(I) le = launch_softmax_bulk<T, I, CAUSAL>(s, x, y, total_rows, rows_per_mat, cols, status)
       if (iters <= 1) AG_SMB(1); else if (iters <= 2) AG_SMB(2); else if (iters <= 4) AG_SMB(4); else AG_SMB(8);
 #undef AG_SMB

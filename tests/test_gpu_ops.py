@@ -219,7 +219,7 @@ def test_layer_norm_rows_by_bulk_copies(gpu_dev, dtype, rows, cols):
 
 @pytest.mark.parametrize("dtype", ["bfloat16", "float16", "float32"])
 @pytest.mark.parametrize("causal", [True, False])
-@pytest.mark.parametrize("shape", [(40, 128, 128), (19, 256, 256), (5, 1000, 1016), (6, 800, 1024), (3, 64, 2048), (2, 16, 4096), (3, 33, 8)])
+@pytest.mark.parametrize("shape", [(40, 128, 128), (19, 256, 256), (5, 1000, 1016), (6, 800, 1024), (3, 64, 2048), (2, 16, 4096), (3, 33, 8), (47, 256, 256), (93, 128, 128), (54, 764, 1020)])
 def test_softmax_rows_in_registers_and_by_bulk_copies(gpu_dev, dtype, causal, shape):
     """Row lengths and counts on both sides of the rules, ragged diagonals, scores far from zero, -inf and the type's lowest value."""
     import torch
