@@ -141,9 +141,16 @@ __global__ void __launch_bounds__(256) layer_norm_warp_kernel(const T* __restric
   }
 }
 
-// The same for 16-bit rows of 512 to 2560 bytes, 32 of them an SM, that come and go by bulk copies (softmax_bulk_kernel below has the
+// The same for many 16-bit rows of 512 to 2560 bytes that come and go by bulk copies (softmax_bulk_kernel below has the
 // pipeline), arithmetic on pairs. Rows in registers against bulk copies, bfloat16, us: 131072 x 768 77.3 / 65.6 (6.1 TB/s), 65536 x 1024
-// 68.4 / 51.7 (half of it from the L2), 16384 x 1280 19.6 / 17.3, 32768 x 256 12.6 / 11.9, 8192 x 768 7.8 / 7.8, 8192 x 2048 18.2 / 20.0.
+// 68.4 / 51.7 (half of it from the L2), 16384 x 1280 19.6 / 17.3, 32768 x 256 12.6 / 11.9, 8192 x 2048 18.2 / 20.0.
+// From how many rows an SM on depends on what the kernel above makes of the row (its registers hold two of them). bfloat16 / float16 at 32, 64,
+// 112 and 160 rows an SM, in registers and by copies:
+//   256 columns   5.5 5.7  5.7 5.6  7.4 7.2  9.8 9.3     / 4.5 4.5  4.8 4.6  7.3 7.2  9.6 9.4
+//   512           4.7 4.6  7.3 6.7  11.1 9.4  14.7 11.9  / 4.7 4.5  7.1 6.9  10.7 9.7  14.3 12.2
+//   768           5.9 6.7  8.1 8.5  12.4 11.9  16.5 15.1 / 4.9 5.7  8.0 8.5  12.3 12.2  16.3 16.0
+//   1024          8.4 6.8  13.1 10.7  20.2 16.3  27.2 21.5 / 6.3 6.5  9.6 10.4  14.6 15.0  19.5 19.4
+//   1280          7.8 7.1  12.6 11.8  19.6 17.1  26.5 22.1 / 9.1 7.3  15.5 12.2  18.9 17.6  25.8 22.8
 constexpr int kLnMaxRowBytes = 2560;
 template <typename T, int ITERS>
 __global__ void __launch_bounds__(kSmWarps * 32) layer_norm_bulk_kernel(const T* __restrict__ in, const T* __restrict__ gamma, const T* __restrict__ beta, T* __restrict__ out, int64_t rows,
@@ -280,7 +287,8 @@ static Status layer_norm_t(cudaStream_t s, const TView& in, const TView& gamma, 
     cudaError_t le = cudaSuccess;
     if constexpr (sizeof(T) == 2) {
       int* status = matmul_status_word();
-      if (status && cols * 2 >= kSmMinRowBytes && cols * 2 <= kLnMaxRowBytes && rows >= 32 * (int64_t)sm_count() && x != y) {
+      const int from = iters >= 5 ? 32 : iters == 4 ? (std::is_same<T, __half>::value ? 160 : 32) : iters == 2 ? 64 : 112;      // rows an SM
+      if (status && cols * 2 >= kSmMinRowBytes && cols * 2 <= kLnMaxRowBytes && rows >= from * (int64_t)sm_count() && x != y) {
 #define AG_LNB(I) le = launch_layer_norm_bulk<T, I>(s, x, g, b, y, rows, (int)cols, eps, status)
         if (iters <= 2) AG_LNB(2); else if (iters <= 3) AG_LNB(3); else if (iters <= 4) AG_LNB(4); else AG_LNB(5);
 #undef AG_LNB

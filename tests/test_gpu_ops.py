@@ -203,9 +203,10 @@ def test_softmax_causal_f32(gpu_dev, shape):
 
 
 @pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
-@pytest.mark.parametrize("rows,cols", [(4735, 768), (4736, 768), (4801, 256), (5000, 1000), (4737, 1024), (6001, 1280), (4800, 1288), (4736, 248)])
+@pytest.mark.parametrize("rows,cols", [(4735, 768), (4736, 768), (4801, 256), (5000, 1000), (4737, 1024), (6001, 1280), (4800, 1288), (4736, 248),
+                                       (16575, 768), (16576, 768), (16600, 256), (16577, 640), (9471, 512), (9473, 264), (23679, 1024), (23681, 904)])
 def test_layer_norm_rows_by_bulk_copies(gpu_dev, dtype, rows, cols):
-    """Both sides of the rule (32 rows an SM, 512 to 2560 bytes), every number of pieces a lane, a last piece that not every lane has."""
+    """Both sides of the rule (32, 64, 112 or 160 rows an SM of 512 to 2560 bytes), every number of pieces a lane, a last piece that not every lane has."""
     import torch
     t = {"bfloat16": torch.bfloat16, "float16": torch.float16}[dtype]
     g = torch.Generator("cuda").manual_seed(rows + cols)
