@@ -75,6 +75,7 @@ __device__ unsigned long long g_attn_cta[4096][4];
 // (under a causal mask the last query tile of a head sees the most keys; every head has the same tiles), and dealt
 // to the CTAs in passes that alternate direction, so the CTA that got the heaviest tile of one pass gets the
 // lightest of the next: a fixed schedule (no counter in global memory) within ~10 % of an even split.
+template <bool BANDS>
 struct TileWalk {
   int pass, cta, n_cta;
   int t;            // tiles this CTA has started so far (selects the Q buffer and barrier phases)
@@ -86,9 +87,11 @@ struct TileWalk {
     pass++; t++;
     valid = r < p.total_tiles;
     if (!valid) return;
-    const int band = r / (p.band * p.q_tiles), rem = r - band * p.band * p.q_tiles, high = min(p.band, p.bh - band * p.band);
-    qt = p.q_tiles - 1 - rem / high;
-    const int bh = band * p.band + rem % high;
+    int bh;
+    if constexpr (BANDS) {
+      const int first = r / (p.band * p.q_tiles) * p.band, rem = r - first * p.q_tiles, high = min(p.band, p.bh - first), row = rem / high;
+      qt = p.q_tiles - 1 - row; bh = first + rem - row * high;
+    } else { qt = p.q_tiles - 1 - r / p.bh; bh = r % p.bh; }
     b = bh / p.heads; h = bh % p.heads;
     q0 = qt * kQ;
     n_blocks = (p.tk + kKV - 1) / kKV;
@@ -99,7 +102,7 @@ struct TileWalk {
   }
 };
 
-template <typename T>
+template <typename T, bool BANDS>      // BANDS: heads in bands (attention_band); one band needs no division of its own, 0.5 to 2 % of short tiles
 __global__ void __launch_bounds__(kAttnThreads, 2)
 attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const AttnParams p) {
@@ -149,7 +152,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   if (warp == 0) {
     // ── TMA producer ──
     if (lane == 0) {
-      TileWalk w; w.start(p, (int)blockIdx.x, (int)gridDim.x);
+      TileWalk<BANDS> w; w.start(p, (int)blockIdx.x, (int)gridDim.x);
       int g = 0;
       bool ok = true;
       for (; w.valid && ok; w.next(p)) {
@@ -177,7 +180,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
       constexpr uint32_t idesc_s = make_idesc_f16(fmt, 0, 0, kQ, kKV);   // S = Q K^T: both K-major, N = 64
       constexpr uint32_t idesc_o = make_idesc_f16(fmt, 0, 1, kQ, kD);    // O = P V: V is N-major, N = 64
-      TileWalk ws; ws.start(p, (int)blockIdx.x, (int)gridDim.x);   // the tile whose scores are issued next
+      TileWalk<BANDS> ws; ws.start(p, (int)blockIdx.x, (int)gridDim.x);   // the tile whose scores are issued next
       int js = 0, gs = 0;
       bool ok = true;
       auto issue_s = [&]() -> bool {
@@ -199,7 +202,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       };
       ok = issue_s();
       if (ok) ok = issue_s();
-      TileWalk wp; wp.start(p, (int)blockIdx.x, (int)gridDim.x);   // the tile whose products are issued
+      TileWalk<BANDS> wp; wp.start(p, (int)blockIdx.x, (int)gridDim.x);   // the tile whose products are issued
       int gp = 0;
       for (; wp.valid && ok; wp.next(p)) {
         for (int j = 0; j < wp.n_blocks; j++, gp++) {
@@ -282,7 +285,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       return true;
     };
 
-    TileWalk w; w.start(p, (int)blockIdx.x, (int)gridDim.x);
+    TileWalk<BANDS> w; w.start(p, (int)blockIdx.x, (int)gridDim.x);
     for (; w.valid && ok; w.next(p)) {
       const int row = w.q0 + r;                   // row inside the sequence
       float m_ref = -INFINITY;   // the maximum the stored probabilities and sums are relative to
@@ -426,11 +429,11 @@ bool attention_fused_eligible(const AttnDesc& d) {
          attn_view_ok(d.v, d.v_b, d.v_h, d.v_t, d.batch, d.heads);
 }
 
-template <typename T>
-static Status launch_attention(cudaStream_t s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p,
+template <typename T, bool BANDS>
+static Status launch_attention_as(cudaStream_t s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p,
                                dim3 grid) {
   static bool attr_set = false;
-  auto kern = attention_tc_kernel<T>;
+  auto kern = attention_tc_kernel<T, BANDS>;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem);
     if (e != cudaSuccess) return cuda_status(e, "attention smem attribute");
@@ -439,6 +442,10 @@ static Status launch_attention(cudaStream_t s, const CUtensorMap& mq, const CUte
   cudaError_t le = launch_pdl(kern, dim3(grid), dim3(kAttnThreads), kAttnSmem, s, mq, mk, mv, p);
   if (le != cudaSuccess) return cuda_status(le, "attention (tcgen05)");
   return Status::OK();
+}
+template <typename T>
+static Status launch_attention(cudaStream_t s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, dim3 grid) {
+  return p.band < p.bh ? launch_attention_as<T, true>(s, mq, mk, mv, p, grid) : launch_attention_as<T, false>(s, mq, mk, mv, p, grid);
 }
 
 // Heads per band. Every query tile of a head reads the head's keys and values up to its own last row; ranked over all heads at
