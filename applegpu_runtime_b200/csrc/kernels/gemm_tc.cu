@@ -93,9 +93,7 @@ template <int BN> struct TcCfg {
 };
 
 // Epilogue staging: each epilogue warp owns a [32 rows x 32 cols] 2-byte tile in shared memory (stg_off above).
-// Results leave it through one tiled bulk store per 32 x 32 group (cp.async.bulk.tensor, issued by one lane and
-// drained by the TMA unit while the warp computes the next group) when C's rows are 16-byte aligned; otherwise,
-// and for float32 or argmax outputs, through plain global stores.
+// Results that do not go straight from a lane's registers to its row (rows off 32 bytes) are transposed through it.
 
 template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b);
 template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) {
@@ -1553,8 +1551,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 //                 consumer tile waits (bounded) until the producer's row block has all its arrivals (two CTAs a tile), then
 //                 fences the async proxy and loads. A tile only ever waits for tiles earlier in the global order, and every pair takes its
 //                 tiles in that order, so the earliest unfinished tile can always run: no cycle
-//   epilogue      row statistics and residual rows of the next tile are fetched ahead only when its row block is
-//                 already complete (its counter is read one tile earlier); otherwise after the accumulator wait
+//   epilogue      row statistics of the next tile are fetched ahead only when its row block is already complete (its counter is
+//                 read one tile earlier), otherwise after the accumulator wait; residual rows always after it, by epilogue_unit
 //   counters      zero on entry; the last CTA to leave zeroes them again
 // N-major B ([K, N] weights), 16-bit types, unbatched; the epilogue is the pair kernel's (bias, activation, residual,
 // folded layer_norm on either side).
@@ -1777,7 +1775,7 @@ gemm_tc_chain_kernel(const __grid_constant__ ChainMaps maps, const __grid_consta
     const int pair = (warp - 2) >> 2;
     int acc = 0; uint32_t acc_phase = 0;
     bool ok = true;
-    bool fetched = false;            // this tile's row statistics and first residual group are already in registers
+    bool fetched = false;            // this tile's row statistics are already in registers
     longlong2 stats_raw = make_longlong2(0, 0);
     int e_next = li0 < li1 ? __ldg(cp.list + li0) : -1;
     int e_next2 = li0 + 1 < li1 ? __ldg(cp.list + li0 + 1) : -1;   // list entries are read two tiles ahead: nothing waits for them
@@ -1840,9 +1838,9 @@ gemm_tc_chain_kernel(const __grid_constant__ ChainMaps maps, const __grid_consta
 #pragma unroll
       for (int gi = 0; gi < kChainGroups; gi++) { bias_f[gi * 32 + lane] = Cvt<T>::to(col_bias[gi]); scale_s[gi * 32 + lane] = col_sum[gi]; }
       if (e_next >= 0) fetch_cols(e_next);
-      // `fv` is a relaxed look at the counter taken one tile ago. Seeing it complete, the loads below are issued after
-      // it (they depend on the branch), go to L2 (the statistics) or to lines this SM has not touched in this launch (the
-      // residual rows), and the producer's stores were GPU-visible before the counter moved: they read the final values.
+      // `fv` is a relaxed look at the counter taken one tile ago. Seeing it complete, the load below is issued after
+      // it (it depends on the branch) and goes to L2, and the producer's stores were GPU-visible before the counter moved: it reads the
+      // final values.
       if (!fetched && (need == 0 || fv >= need)) {
         stats_raw = ln_stats_fetch_cg(p, row0 + lane);
         fetched = true;
@@ -1858,12 +1856,11 @@ gemm_tc_chain_kernel(const __grid_constant__ ChainMaps maps, const __grid_consta
       long long q2 = clock64();
       if (cp.probe && warp == 2 && lane == 0) { cp.probe[blockIdx.x * 16 + 15] += q0 - q_top; cp.probe[blockIdx.x * 16 + 5] += q1 - q0; cp.probe[blockIdx.x * 16 + 6] += q2 - q1; cp.probe[blockIdx.x * 16 + 12] += fetched ? 0 : 1; }
 #endif
-      if (!fetched) {
-        // This pair's TMA thread acquired the row block's counter before it loaded the tile's operands, and the full
-        // accumulator this warp has just waited for follows those loads through the pipeline's barriers: the producer's
-        // stores are ordered before these reads without another look at the counter.
-        stats_raw = ln_stats_fetch_cg(p, row0 + lane);
-      }
+      // This pair's TMA thread acquired the row block's counter before it loaded the tile's operands, and the full
+      // accumulator this warp has just waited for follows those loads through the pipeline's barriers: the producer's
+      // stores are ordered before what is read from here on, the statistics and epilogue_unit's residual rows (which this SM has not
+      // read in this launch before, and does not keep in its L1), without another look at the counter.
+      if (!fetched) stats_raw = ln_stats_fetch_cg(p, row0 + lane);
       fetched = false;
       float ln_mean = 0.f, ln_rstd = 1.f;
       if (row0 + lane < p.m) ln_stats_finish(p, stats_raw, ln_mean, ln_rstd);
@@ -1888,7 +1885,7 @@ gemm_tc_chain_kernel(const __grid_constant__ ChainMaps maps, const __grid_consta
       if (row0 < p.m) emit_row_stats(p, row0 + lane, n0 == 0 && pair == 0, row_sum, row_sq);
       __syncwarp();                                   // every lane's stores and atomics are issued: the announcer takes over
       if (lane == 0) mbar_arrive(&stored_bar[acc]);
-      // the next tile's statistics and first residual rows, if its row block is known to be complete
+      // the next tile's statistics, if its row block is known to be complete
       if (e_next >= 0) {
         const int gn = e_next >> 24, ltn = e_next & 0xffffff;
         const TcParams& pn = s_prob[gn];
@@ -2164,8 +2161,9 @@ static bool g_direct_store = [] { const char* v = std::getenv("APPLEGPU_GEMM_DIR
 static int g_tile_override = 0;   // APPLEGPU_GEMM_TILE / set_gemm_tile: 0 auto, else pair*1000 + bn
 static TileChoice choose_tile(const GemmDesc& d, long long nb, int force_path) {
   struct Cand { bool pair; int bn; int step; };
-  // cycles per k-step (64 deep) of one CTA's tile, measured on a B200 with the kernel's own cycle probes (pair 192:
-  // interpolated). The 256 x 192 pair tile exists for K-major B only: each CTA loads half of the B tile, and 96 columns
+  // cycles per k-step (64 deep) of one CTA's tile, measured on a B200 with the kernel's own cycle probes under eight epilogue warps (pair 192:
+  // interpolated). What a tile pays beside its products (1 800 cycles of the packed pair form at K = 768, more with an activation or a residual) is
+  // not modelled: the constant counts once, for the last tile. The 256 x 192 pair tile exists for K-major B only: each CTA loads half of the B tile, and 96 columns
   // are not a whole number of 64-column swizzle atoms of an N-major operand.
   static const Cand cands[6] = {{true, 256, 530}, {true, 192, 465}, {true, 128, 400}, {false, 256, 780}, {false, 192, 640}, {false, 128, 590}};
   const bool b_kmajor = classify_b(d) != 2;
@@ -2196,7 +2194,9 @@ static TileChoice choose_tile(const GemmDesc& d, long long nb, int force_path) {
 // band's rows stay in the L2 from one column tile to the next, and once per column tile if not; B is read once per band. Up to
 // 48 MB of A (with B and results on their way the L2 of 126 MB keeps it) there is one band, so a large B (an LM head) is read once; above
 // that bands of 16 MB. [131072, K] x [K, N], bf16, one band against bands: N x K = 2304 x 768 456 -> 379 us, 768 x 768 214 -> 191,
-// 3072 x 768 with GELU 651 -> 551, 768 x 3072 544 -> 468; [16384, 5120] x [5120, 1280] 188 -> 162.
+// 3072 x 768 with GELU 651 -> 551, 768 x 3072 544 -> 468; [16384, 5120] x [5120, 1280] 188 -> 162. At the line there is little between them, M x N x
+// K with A of 48 to 52 MB: 31000 x 768 x 768 34.3 / 33.6, 6000 x 4096 x 4096 144.7 / 143.6, 20000 x 1280 x 1280 54.5 / 52.9, 8192 x 768 x 3072 38.6 / 37.6;
+// 61 to 67 MB: 40000 x 2304 x 768 126.8 / 116.2, 8192 x 4096 x 4096 193.5 / 181.7; 8192 cubed (134 MB) 728 / 718.
 static int pair_band(const GemmDesc& d, long long tiles_m) {
   const double a_bytes = 2.0 * (double)d.m * (double)d.k;
   if (a_bytes <= 48e6) return (int)tiles_m;

@@ -586,7 +586,7 @@ static cudaError_t launch_ml_step(cudaStream_t s, const MlParams& p, int ranks, 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ranks, (unsigned)p.heads, (unsigned)p.n_seq); cfg.blockDim = dim3(kMsThreads); cfg.dynamicSmemBytes = smem; cfg.stream = s;
   const int rows = (p.dim + kMsThreads / tx_n - 1) / (kMsThreads / tx_n);       // of S, a thread's
-  const bool resident = slice <= kMsCols && slice <= tx_n * VEC && p.dim <= kMsDims && rows <= 16 && kMsCols <= kMsThreads;
+  const bool resident = slice <= kMsCols && slice <= tx_n * VEC && p.dim <= kMsDims && rows <= 16;
   cudaLaunchAttribute attr2[2];
   attr2[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr2[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   attr2[1].id = cudaLaunchAttributeClusterDimension; attr2[1].val.clusterDim.x = (unsigned)ranks; attr2[1].val.clusterDim.y = 1; attr2[1].val.clusterDim.z = 1;

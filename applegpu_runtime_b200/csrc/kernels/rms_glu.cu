@@ -239,7 +239,9 @@ __global__ void __launch_bounds__(kRmsThreads) rms_row_kernel(const __grid_const
 // keeps the norms' weights in its registers and asks for its next row before it starts on the one at hand. It is bound by memory, 14
 // bytes per element with `post`; a block per row reads the weights anew (as many bytes from the L1 as from memory) and starts with
 // nothing in flight. 8192 rows of 2048 with `post` 54.5 -> 44.9 us (5.2 TB/s), of 1024 with two outputs 13.6 -> 9.7. From eight rows
-// an SM on: four blocks fit one with rows of 2048 and `post`, so that each has a next row to ask for. It adds in the order of the kernel above.
+// an SM on: four blocks fit one with rows of 2048 and `post`, so that each has a next row to ask for. A block per row against walking, 4, 8, 16 and 32
+// rows an SM of 2048, one output 6.0 5.9, 6.0 5.9, 8.4 6.3, 15.1 10.3, with `post` 6.5 6.3, 7.8 7.3, 13.0 12.3, 23.5 22.7; of 1024 they are equal
+// up to 16. It adds in the order of the kernel above.
 template <typename T, int NREG, bool POST, bool TWO>
 __global__ void __launch_bounds__(kRmsThreads) rms_walk_kernel(const __grid_constant__ RmsParams p, int rows) {
   constexpr int W = kRmsThreads / 32;

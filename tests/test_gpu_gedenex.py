@@ -242,6 +242,21 @@ def test_latent_step_has_the_same_bits_alone_and_in_a_batch(gpu_dev, size, dtype
     assert rel(out[0][0], latent_want(c, 0, 4)) < {"float32": 3e-5, "float16": 4e-3, "bfloat16": 2e-2}[dtype]
 
 
+@pytest.mark.parametrize("max_len,T", [(500, 490), (512, 40), (513, 40), (577, 570), (2000, 40), (2000, 700)])
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+@pytest.mark.parametrize("size", [1, 4, 7])
+def test_latent_merge_of_few_and_many_splits(gpu_dev, size, dtype, max_len, T):
+    """A sequence alone has a split of the keys per 64 of its capacity: up to eight are merged in one round of loads, more one after the
+    other, most of them empty behind a short sequence."""
+    g, z = gpu_dev, LATENT_SIZES[size]
+    c = latent_case(g, T, 1, z, dtype, 50 + size, max_len)
+    cache = new_cache(g, c)
+    got = [latent_run(g, c, 0, T - 2, cache, "expanded")] + [latent_run(g, c, t, t + 1, cache, "latent") for t in (T - 2, T - 1)]
+    want = latent_want(c, 0, T)
+    for y, row in zip(got[1:], want[T - 2:]):
+        assert rel(y[0, 0], row) < {"float32": 3e-5, "float16": 4e-3, "bfloat16": 2e-2}[dtype]
+
+
 @pytest.mark.parametrize("form", ["expanded", "latent", "tensor"])
 @pytest.mark.parametrize("key,query", [(0, 299), (63, 299), (64, 128), (127, 128), (128, 128), (191, 255), (255, 256), (200, 201), (299, 299)])
 def test_latent_attention_far_key(gpu_dev, form, key, query):

@@ -300,6 +300,18 @@ def test_grouped_attention_forms_and_portions(gpu_dev, name, dtype):
     assert gpu_dev.pipeline_status() == 0
 
 
+@pytest.mark.parametrize("dim", [12, 64, 128, 132, 192, 256, 260])
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
+def test_grouped_heads_that_turn_as_a_whole(gpu_dev, dim, dtype):
+    """A lane appends one pair of neighbouring columns of either half (up to 64 pairs), two (up to 128), or column by column (above)."""
+    c = ga_case(dict(H=4, G=2, d=dim, e=40, pairs=dim // 2, window=30, cap=5.0), 40, 2, dim, 43)
+    for form in ("portion", "short"):
+        got = ga_run(gpu_dev, c, [3, 1, 20, 1, 15], dtype, form)
+        for b in range(2):
+            # the bound of the other grouped tests; float16 has eight times the steps
+            assert rel(got[b], ga_want(c, b)) < {"bfloat16": 2e-2, "float16": 2.5e-3}[dtype], form
+
+
 @pytest.mark.parametrize("window", [1, 6, 90, 0])
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_grouped_attention_shared_keys(gpu_dev, dtype, window):
