@@ -2279,8 +2279,8 @@ long long* g_chain_probe = nullptr;   // set by a probe harness
 void chain_epi_probe(long long* out) { cudaMemcpyFromSymbol(out, g_epi_probe, sizeof(long long) * 8); }
 #endif
 // Fewer rows than this and the products go out one by one: with a handful of 256-row blocks most tiles wait for the
-// tiles just before them (measured on GPT-2-small's block: chained 66 / 76 / 83 / 114 us against 54 / 72 / 86 / 145 us
-// for four launches at 1024 / 3072 / 4096 / 8192 rows).
+// tiles just before them (GPT-2-small's block, sixteen epilogue warps: chained 60 / 69 / 75 / 108 us against 49 / 64 / 80 / 124 us
+// for four launches at 1024 / 3072 / 4096 / 8192 rows; width 1280 80 / 110 / 129 / 239 against 74 / 110 / 156 / 263).
 static int64_t g_chain_min_rows = [] { const char* v = std::getenv("APPLEGPU_GEMM_CHAIN_MIN_ROWS"); return v ? (int64_t)std::atoll(v) : (int64_t)4096; }();
 void set_gemm_chain_min_rows(int64_t rows) { g_chain_min_rows = rows < 0 ? 0 : rows; }
 int64_t gemm_chain_min_rows() { return g_chain_min_rows; }
