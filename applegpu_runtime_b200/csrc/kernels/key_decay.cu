@@ -385,8 +385,7 @@ static cudaError_t launch_ks_as(cudaStream_t s, const KdParams& p, int ranks, in
       cudaLaunchConfig_t q = cfg;
       q.attrs = at + 1; q.numAttrs = 1;
       int got = 0;
-      const cudaError_t e = cudaOccupancyMaxActiveClusters(&got, key_decay_step_kernel<T, VEC, NR, AHEAD>, &q);
-      if (e != cudaSuccess) return e;
+      if (cudaOccupancyMaxActiveClusters(&got, key_decay_step_kernel<T, VEC, NR, AHEAD>, &q) != cudaSuccess) { cudaGetLastError(); got = 0; }
       n = got + 1;
     }
     *fits = (long long)p.heads * p.n_seq < n;
