@@ -1591,8 +1591,12 @@ __device__ __forceinline__ bool flag_wait(const int* f, int need, int* status, i
   while (true) {
     if (ld_acquire_gpu(f) >= need) return true;
     if ((++spins & 0x3f) == 0) {
-      if (*reinterpret_cast<volatile int*>(status) != 0) return false;
-      if (globaltimer_ns() - t0 > kWaitLimitNs) { atomicCAS(status, 0, code); return false; }
+      const bool failed = *reinterpret_cast<volatile int*>(status) != 0;
+      if (failed || globaltimer_ns() - t0 > kWaitLimitNs) {
+        if (!failed) atomicCAS(status, 0, code);
+        settle();
+        return false;
+      }
     }
   }
 }

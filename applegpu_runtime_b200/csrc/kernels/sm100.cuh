@@ -46,6 +46,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
+// Behind a wait that gave up, before its warp can leave: copies and products that the block has on their way, all of them of this GPU's memory, get
+// a millisecond (they take microseconds) to arrive in shared and tensor memory that another block has next. Every role of a
+// pipeline ends its last wait like this, so nothing is issued behind it.
+constexpr unsigned long long kSettleNs = 1000000ull;
+__device__ __forceinline__ void settle() {
+  const unsigned long long t0 = globaltimer_ns();
+  for (int i = 0; i < (1 << 20) && globaltimer_ns() - t0 < kSettleNs; i++) {}
+}
 // Returns false (and records `code`) if the phase does not complete within the limit, or if
 // another role already recorded a failure.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int code) {
@@ -55,8 +63,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((++spins & 0xff) == 0) {
-      if (*reinterpret_cast<volatile int*>(status) != 0) return false;
-      if (globaltimer_ns() - t0 > kWaitLimitNs) { atomicCAS(status, 0, code); return false; }
+      const bool failed = *reinterpret_cast<volatile int*>(status) != 0;
+      if (failed || globaltimer_ns() - t0 > kWaitLimitNs) {
+        if (!failed) atomicCAS(status, 0, code);
+        settle();
+        return false;
+      }
     }
   }
 }

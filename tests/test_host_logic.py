@@ -402,3 +402,20 @@ def test_attention_bands_leave_the_busiest_cta_as_it_was(gpu, heads, tokens):
         assert busiest(band, causal) <= busiest(heads, causal)
         if not causal and band < heads:
             assert band * tokens * 256 <= 64 << 20 or band <= 16
+
+
+def test_waits_that_give_up_settle_before_their_block_can_leave():
+    """A wait that runs out gives the block's copies in flight time to land (kernels/sm100.cuh): behind it in every polling loop that reports to
+    the status word; the rows by bulk copies wait for each copy instead (kernels/reduce.cu)."""
+    import pathlib
+    import re
+    kernels = pathlib.Path(__file__).parents[1] / "applegpu_runtime_b200" / "csrc" / "kernels"
+    text = {f.name: re.sub(r"//.*", "", f.read_text()) for f in kernels.glob("*.cu*")}
+    waits = [(name, m.group(1), m.group(2)) for name, t in text.items() for m in re.finditer(r"__device__ __forceinline__ bool (\w*wait\w*)\([^)]*int\* status, int code\) \{(.*?)\n\}", t, re.S)]
+    assert {w for _, w, _ in waits} == {"mbar_wait", "mbar_wait_limit", "flag_wait"}
+    for name, wait, body in waits:
+        if wait != "mbar_wait_limit":
+            assert re.findall(r"(\w+\(\));\s*return false;", body) == ["settle()"] and body.count("return false") == 1, (name, wait)
+    assert {name for name, t in text.items() if "mbar_wait_limit(" in t} == {"sm100.cuh", "reduce.cu"}
+    assert text["reduce.cu"].count("bulk_leave(") == 3                                    # its definition and both kernels
+    assert {name for name, t in text.items() if "mbar_try_wait(" in t} == {"sm100.cuh", "workspace.cu"}
