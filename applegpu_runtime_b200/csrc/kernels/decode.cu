@@ -897,21 +897,19 @@ Status decode_qkv_attention(cudaStream_t s, const GemmDesc& d, void* kcache, voi
 }
 
 // ── the tied LM head of a step with its greedy pick ─────────────────────────
-// x [m, k] against the embedding [vocab, k], both K-major, m <= 8: bound by reading the embedding once. A warp has 16 of its rows, which are
+// x [m, k] against the embedding [vocab, k], both K-major, m <= 16: bound by reading the embedding once. A warp has 16 of its rows, which are
 // the rows of mma.m16n8k16, over the whole of K, straight from memory (the order of K inside a block of 32 columns is free, so a lane feeds
 // two products from one 16-byte piece of either operand); what is asked for first is on its way ahead of the dependency wait. The pick is that of
 // the matrix product's argmax epilogue: values as they would be stored, the lowest column among equals, a NaN in column 0 kept. A warp
 // looks at the keys before it touches them, so that thousands of warps do not queue for one line.
-// GPT-2 small, eight sequences, bf16: 21.7 us a launch with 128 x 192 tiles on tcgen05, 15.3 with this (77 MB). Those tiles take up to 128 rows in
-// the same time; sixteen here (two groups of eight, every row of x read twice as often) took a step of one layer from 54.8 to 62.5 us, of GPT-2
-// small behind 500 tokens from 510 to 517, so more than eight rows take the tiles.
+// GPT-2 small, eight sequences, bf16: 21.7 us a launch with 128 x 192 tiles on tcgen05, 15.3 with this (77 MB).
 constexpr int kDhWarps = 4;
 __device__ __forceinline__ unsigned long long dh_key(float r, int col) {
   if (r != r) return col == 0 ? 0xffffffffffffffffull : 0ull;
   const uint32_t b = __float_as_uint(r), ord = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
   return ((unsigned long long)ord << 32) | (unsigned long long)(0xffffffffu - (uint32_t)col);
 }
-template <typename T>
+template <typename T, int NT>        // NT groups of eight rows of x
 __global__ void __launch_bounds__(kDhWarps * 32) decode_head_kernel(const T* __restrict__ w, const T* __restrict__ x, unsigned long long* keys, int m, int vocab, int k) {
   constexpr int U = 4;               // blocks of 32 columns in flight
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, n0 = (blockIdx.x * kDhWarps + (threadIdx.x >> 5)) * 16;
@@ -929,38 +927,50 @@ __global__ void __launch_bounds__(kDhWarps * 32) decode_head_kernel(const T* __r
   fetch(0);
   pdl_wait();
   pdl_trigger();
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int c0 = 0; c0 < k; c0 += U * 32) {
-    uint4 b[U];
+  float acc[NT][4];
 #pragma unroll
-    for (int u = 0; u < U; u++) b[u] = c0 + u * 32 < k && g < m ? *reinterpret_cast<const uint4*>(x + (long long)g * k + c0 + u * 32 + q * 8) : make_uint4(0u, 0u, 0u, 0u);
+  for (int t = 0; t < NT; t++) { acc[t][0] = 0.f; acc[t][1] = 0.f; acc[t][2] = 0.f; acc[t][3] = 0.f; }
+  for (int c0 = 0; c0 < k; c0 += U * 32) {
+    uint4 b[U][NT];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int t = 0; t < NT; t++)
+        b[u][t] = c0 + u * 32 < k && g + 8 * t < m ? *reinterpret_cast<const uint4*>(x + (long long)(g + 8 * t) * k + c0 + u * 32 + q * 8) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
     for (int u = 0; u < U; u++) {
       if (c0 + u * 32 >= k) break;
-      mma_16816<T>(acc, a0[u].x, a1[u].x, a0[u].y, a1[u].y, b[u].x, b[u].y);
-      mma_16816<T>(acc, a0[u].z, a1[u].z, a0[u].w, a1[u].w, b[u].z, b[u].w);
+#pragma unroll
+      for (int t = 0; t < NT; t++) {
+        mma_16816<T>(acc[t], a0[u].x, a1[u].x, a0[u].y, a1[u].y, b[u][t].x, b[u][t].y);
+        mma_16816<T>(acc[t], a0[u].z, a1[u].z, a0[u].w, a1[u].w, b[u][t].z, b[u][t].w);
+      }
     }
     if (c0 + U * 32 < k) fetch(c0 + U * 32);
   }
 #pragma unroll
-  for (int j = 0; j < 2; j++) {      // this lane: embedding rows g and g + 8 for row 2 q + j of x
-    unsigned long long key = 0ull;
-    if (n0 + g < vocab) key = dh_key(Cvt<T>::to(Cvt<T>::from(acc[j])), n0 + g);
-    if (n0 + g + 8 < vocab) { const unsigned long long o = dh_key(Cvt<T>::to(Cvt<T>::from(acc[2 + j])), n0 + g + 8); key = o > key ? o : key; }
+  for (int t = 0; t < NT; t++)
 #pragma unroll
-    for (int d = 4; d < 32; d *= 2) { const unsigned long long o = __shfl_xor_sync(0xffffffffu, key, d); key = o > key ? o : key; }
-    const int row = 2 * q + j;
-    if (g == 0 && row < m && key > *reinterpret_cast<volatile unsigned long long*>(keys + row)) atomicMax(keys + row, key);
-  }
+    for (int j = 0; j < 2; j++) {    // this lane: embedding rows g and g + 8 for row 2 q + j of x
+      unsigned long long key = 0ull;
+      if (n0 + g < vocab) key = dh_key(Cvt<T>::to(Cvt<T>::from(acc[t][j])), n0 + g);
+      if (n0 + g + 8 < vocab) { const unsigned long long o = dh_key(Cvt<T>::to(Cvt<T>::from(acc[t][2 + j])), n0 + g + 8); key = o > key ? o : key; }
+#pragma unroll
+      for (int d = 4; d < 32; d *= 2) { const unsigned long long o = __shfl_xor_sync(0xffffffffu, key, d); key = o > key ? o : key; }
+      const int row = t * 8 + 2 * q + j;
+      if (g == 0 && row < m && key > *reinterpret_cast<volatile unsigned long long*>(keys + row)) atomicMax(keys + row, key);
+    }
 }
 bool decode_head_eligible(DType dt, const void* w, const void* x, int m, int64_t k) {
-  return (dt == DType::BF16 || dt == DType::F16) && m >= 1 && m <= 8 && k >= 32 && k % 32 == 0 && k <= 65536 && aligned16(w) && aligned16(x);
+  return (dt == DType::BF16 || dt == DType::F16) && m >= 1 && m <= 16 && k >= 32 && k % 32 == 0 && k <= 65536 && aligned16(w) && aligned16(x);
 }
 Status decode_head(cudaStream_t s, DType dt, const void* w, const void* x, unsigned long long* keys, int m, int vocab, int k) {
   if (!decode_head_eligible(dt, w, x, m, k) || vocab < 1) return Status::invalid("decode_head: shape or layout not supported");
   const dim3 grid((unsigned)((vocab + 16 * kDhWarps - 1) / (16 * kDhWarps))), block(kDhWarps * 32);
-  const cudaError_t e = dt == DType::BF16 ? launch_pdl(decode_head_kernel<__nv_bfloat16>, grid, block, 0, s, (const __nv_bfloat16*)w, (const __nv_bfloat16*)x, keys, m, vocab, k)
-                                          : launch_pdl(decode_head_kernel<__half>, grid, block, 0, s, (const __half*)w, (const __half*)x, keys, m, vocab, k);
+#define AG_DH(T) (m <= 8 ? launch_pdl(decode_head_kernel<T, 1>, grid, block, 0, s, (const T*)w, (const T*)x, keys, m, vocab, k) \
+                         : launch_pdl(decode_head_kernel<T, 2>, grid, block, 0, s, (const T*)w, (const T*)x, keys, m, vocab, k))
+  const cudaError_t e = dt == DType::BF16 ? AG_DH(__nv_bfloat16) : AG_DH(__half);
+#undef AG_DH
   return cuda_status(e, "decode_head");
 }
 

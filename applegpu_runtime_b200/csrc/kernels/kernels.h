@@ -200,7 +200,7 @@ Status attention_decode(cudaStream_t s, DType dt, const void* qkv, void* kcache,
 // and the bias / activation / residual epilogue.
 bool decode_linear_eligible(const GemmDesc& d);
 Status decode_linear(cudaStream_t s, const GemmDesc& d);
-// The row-argmax keys (GemmEpilogue::argmax_keys) of x [m, k] against an embedding [vocab, k], 16-bit, at most eight rows.
+// The row-argmax keys (GemmEpilogue::argmax_keys) of x [m, k] against an embedding [vocab, k], 16-bit, at most 16 rows.
 bool decode_head_eligible(DType dt, const void* w, const void* x, int m, int64_t k);
 Status decode_head(cudaStream_t s, DType dt, const void* w, const void* x, unsigned long long* keys, int m, int vocab, int k);
 // A layer's QKV projection with layer_norm (as decode_linear) and its attention (as attention_decode) in one launch; 16-bit weights.
