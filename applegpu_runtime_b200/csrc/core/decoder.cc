@@ -148,6 +148,16 @@ class Gpt2Decoder {
     return enqueue_head(s, cur);
   }
 
+  // Whether the head takes decode_head, which reads the embedding past the L2, or the tensor-core tiles, which take up to 128 rows in one time. Up to
+  // eight rows it is the faster kernel; with sixteen it reads every row of x twice as often, and pays only where the L2 then still
+  // holds some of the layers' weights for the next step: the weights are no small part of it, and the caches of all layers leave room.
+  // A step, us, tiles / decode_head: GPT-2 small (170 MB of layers) with 16 sequences, caches of 104 MB 382 / 370, 242 MB 458 / 462, 389 MB 530 / 534;
+  // 9 sequences 58 MB 309 / 293, 136 MB 354 / 354; six layers of width 1280 (236 MB), 9 and 16 sequences, 49 MB 341 / 337, 86 MB 375 / 370, 113
+  // MB 377 / 373, 201 MB 430 / 439; one layer of width 768 (14 MB), 16 sequences 54.8 / 62.5; four of width 512 (25 MB) 102.0 / 103.2.
+  bool streamed_head() const {
+    const size_t weights = (size_t)12 * d() * d() * cfg.n_layer * esz(), caches = 2 * (size_t)cfg.n_layer * cache_layer_bytes();
+    return cfg.batch <= 8 || (weights >= ((size_t)64 << 20) && caches <= ((size_t)112 << 20));
+  }
   // ln_f, the tied LM head with the greedy pick, and the step's bookkeeping.
   Status enqueue_head(cudaStream_t s, uint8_t* cur) {
     const int B = cfg.batch, D = d();
@@ -160,7 +170,7 @@ class Gpt2Decoder {
     g.a_row = D; g.a_col = 1; g.a_batch = 0; g.b_row = 1; g.b_col = D; g.b_batch = 0; g.c_row = cfg.vocab; g.c_batch = 0;
     unsigned long long* finish_keys = nullptr;
     // the keys are zero here: prefill clears them and every step's last kernel clears them again after reading them
-    if (k::decode_head_eligible(dtype, w[0].data(), xn(), B, D)) {
+    if (streamed_head() && k::decode_head_eligible(dtype, w[0].data(), xn(), B, D)) {
       AG_RETURN_IF_ERROR(k::decode_head(s, dtype, w[0].data(), xn(), keys(), B, cfg.vocab, D));
       finish_keys = keys();        // no finalize launch: the step's last kernel turns the keys into tokens
       launches_per_step += 1;

@@ -124,10 +124,11 @@ def test_gpt2_int8_weights_bf16_activations_against_dequantised_oracle(gpu_dev):
 
 @pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
 @pytest.mark.parametrize("batch,heads,vocab", [(1, 1, 33), (8, 2, 97), (9, 12, 1000), (16, 3, 64), (5, 16, 130), (8, 18, 4097), (3, 20, 257),
-                                                (8, 12, 500), (1, 12, 70), (3, 5, 100), (8, 9, 90), (7, 11, 129), (1, 10, 300)])
+                                                (8, 12, 500), (1, 12, 70), (3, 5, 100), (8, 9, 90), (7, 11, 129), (1, 10, 300), (9, 20, 130), (16, 20, 4097)])
 def test_decoder_picks_the_largest_logit(gpu_dev, dtype, batch, heads, vocab):
     """QKV and attention in one launch (up to eight sequences, nine to twelve heads: five and six shares of K, the last whole or half) and
-    apart, the head at vocabularies that end inside a warp's sixteen rows and a block's 64: every pick has the largest logit of the float32
+    apart, the head at vocabularies that end inside a warp's sixteen rows and a block's 64 (with nine sequences and more that kernel takes the
+    models whose layers have 64 MB and more: twenty heads): every pick has the largest logit of the float32
     oracle on the same weights, to rounding."""
     from applegpu_runtime_b200.generate import Gpt2Decoder
     cfg = {"n_layer": 2, "n_head": heads, "n_embd": 64 * heads, "vocab_size": vocab, "n_positions": 64}
